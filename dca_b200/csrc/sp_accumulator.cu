@@ -2,12 +2,11 @@
 // grid per (b_i, b_j, r_i - r_j) label, and its transform to Matsubara frequencies.
 //
 // Replaces Dnfft1DGpu (dnfft_1d_gpu.hpp:38-276) whose accumulateOnDeviceKernel
-// (dnfft_1d_kernels.cu:56-138) issues one FP64 global atomicAdd per (i, j, tap), and whose
-// finalize copies f(tau) to the host for FFTW.  Here:
-//   * vertices are sorted by orbital on the host (as for the two-particle NDFT), so one CTA owns
-//     one output label and visits exactly the (i, j) pairs that land in it; the 16-tap cubic
-//     convolution (dnfft_1d.hpp:353-399, nfft_atomic_convolution.hpp:20-35) accumulates into a
-//     shared-memory copy of the label's row, which is then added to f(tau) with plain stores;
+// (dnfft_1d_kernels.cu:56-138) gives every (i, j, tap) a thread that recomputes its pair's grid
+// position, and whose finalize copies f(tau) to the host for FFTW.  Here:
+//   * a lane computes one pair's label, grid position and weight, then the warp writes the 16-tap
+//     cubic convolutions (dnfft_1d.hpp:353-399, nfft_atomic_convolution.hpp:20-35) of its 32 pairs
+//     two at a time, each as one 128-byte row of FP64 reductions;
 //   * finalize folds the halos (dnfft_1d.hpp:401-418) and evaluates the transform only at the
 //     Matsubara indices (the values transformFTauToFW, dnfft_1d.hpp:427-489, picks from its FFT),
 //     divides by the window's phi(w_n) and by n, and scales by 1/Nc
@@ -38,127 +37,207 @@ struct NfftGrid {
   double T0, Delta, one_div_Delta, t0_window, delta, one_div_delta, one_div_two_beta;
 };
 
-// One CTA per (label, spin).  Vertices of the sector are sorted by row orbital (right band/site)
-// and by column orbital (left band/site).
-__global__ void spAccumulateKernel(const NfftGrid g, const SpSector* __restrict__ sectors,
-                                   const int* __restrict__ perm_r, const int* __restrict__ perm_c,
-                                   const int* __restrict__ row_start, const int* __restrict__ col_start,
-                                   const double* __restrict__ tau, const int* __restrict__ r_of,
-                                   const double* __restrict__ coeff, double factor,
-                                   double* __restrict__ f_tau, double* __restrict__ f_tau_sqr,
-                                   double* __restrict__ f_tau_single) {
-  extern __shared__ __align__(16) double sp_smem[];
-  double* row = sp_smem;
-  double* row_sqr = sp_smem + g.n_padded;
-  const int label = blockIdx.x;
-  const int spin = blockIdx.y;
-  const SpSector sd = sectors[spin];
-  const bool sqr = f_tau_sqr != nullptr;
-  for (int t = threadIdx.x; t < g.n_padded * (sqr ? 2 : 1); t += blockDim.x)
-    sp_smem[t] = 0.0;
-  __syncthreads();
+// The two spin sectors of one measurement (by value) and their vertices: tau, row orbitals
+// b + nb r (right band / site), column orbitals (left band / site), packed by sector.
+struct SpMeasurement {
+  SpSector sector[2];
+  const double* tau;
+  const int* orb_r;
+  const int* orb_c;
+};
 
-  // label = b_i + nb (b_j + nb dr), dr = index of r_i - r_j (sp_accumulator.hpp:185-191).
-  const int b_i = label % g.nb, b_j = (label / g.nb) % g.nb, dr = label / (g.nb * g.nb);
-  const int* pr = perm_r + sd.vtx_off;
-  const int* pc = perm_c + sd.vtx_off;
-  const int* rs = row_start + spin * (g.nb * g.nc + 1);
-  const int* cs = col_start + spin * (g.nb * g.nc + 1);
-  const double* tv = tau + sd.vtx_off;
-  for (int r_j = 0; r_j < g.nc; ++r_j) {
-    const int r_i = r_of[r_j + g.nc * dr];  // x_{r_i} = x_{r_j} + x_dr
-    const int oi = b_i + g.nb * r_i, oj = b_j + g.nb * r_j;
-    const int i0 = rs[oi], ni = rs[oi + 1] - i0;
-    const int j0 = cs[oj], nj = cs[oj + 1] - j0;
-    const long pairs = long(ni) * nj * (2 * kOversampling);
-    for (long p = threadIdx.x; p < pairs; p += blockDim.x) {
-      const int tap = static_cast<int>(p % (2 * kOversampling)) + 1;
-      const long ij = p / (2 * kOversampling);
-      const int i = pr[i0 + static_cast<int>(ij % ni)];
-      const int j = pc[j0 + static_cast<int>(ij / ni)];
+// Pairs (i, j) in M's memory order, 32 to a warp step: a lane reads one M element (coalesced) and
+// computes its pair's label, grid position and interpolation argument; the warp then walks the 32
+// pairs two at a time, lane (l & 15) of a half-warp adding tap (l & 15) + 1 to the pair's 16
+// consecutive grid points with one FP64 reduction to L2 (2 x 128 contiguous bytes per warp
+// instruction; no result is read back, so nothing waits on it).
+//
+// Bound by those reductions and the coefficient reads (L1 resident, 32 KB).  Work is split over
+// pairs, not labels: a CTA per (label, spin) with the label's row in shared memory, the earlier
+// form, fills 32 of the 148 SMs on a 4x4 cluster and serialises on shared-memory FP64 atomics
+// (compare-and-swap loops).
+// One measurement, 4x4 cluster, n 50..400: 212 -> 10 us; 6x6, n 300..1000, with squares: 657 -> 64 us.
+template <bool SQR, typename Index>
+__device__ inline void spAccumulateSector(const NfftGrid& g, const SpMeasurement& m, int spin, long first, long step,
+                                          const int* __restrict__ r_sub, const double* __restrict__ coeff,
+                                          double factor, double* __restrict__ f_tau, double* __restrict__ f_tau_sqr) {
+  const SpSector sd = m.sector[spin];
+  const int lane = threadIdx.x % 32;
+  const Index n = sd.n, pairs = n * n;
+  const double* tv = m.tau + sd.vtx_off;
+  const int* orb_r = m.orb_r + sd.vtx_off;
+  const int* orb_c = m.orb_c + sd.vtx_off;
+  for (long grp = first; grp * 32 < static_cast<long>(pairs); grp += step) {
+    const Index p = static_cast<Index>(grp) * 32 + lane;
+    double f = 0, d = 0, mv = 0;
+    int row = -1, t0 = 0, tab = 0;  // row < 0: nothing to add
+    if (p < pairs) {
+      const int j = static_cast<int>(p / n), i = static_cast<int>(p % n);
       // convoluteToFTauFineCubicInterpolation (dnfft_1d.hpp:353-399), FP64.
       const double t_val = (tv[i] - tv[j]) * g.one_div_two_beta;
       const int tau_0 = static_cast<int>((t_val - g.T0) * g.one_div_Delta);
       const double t0_val_lb = g.T0 + tau_0 * g.Delta;
       const int tau_1 = static_cast<int>((t0_val_lb - t_val - g.t0_window) * g.one_div_delta);
       const double t1_val_lb = g.t0_window + tau_1 * g.delta;
-      const double d = t0_val_lb - t_val - t1_val_lb;
+      d = t0_val_lb - t_val - t1_val_lb;
       const int dti = tau_1 - kOversampling * kWindowSampling;
       const int jw = dti % kWindowSampling;
       const int iw = (dti - jw) / kWindowSampling;
-      const int t_out = tau_0 - kOversampling + tap;
-      const int ci = iw + tap;
-      if (t_out < 0 || t_out >= g.n_padded || ci < 0 || ci >= 4 * kOversampling || jw < 0)
-        continue;  // only reachable for |t_val| > 1/2, which the host rejects
-      const double* cf = coeff + 4 * (ci + 4 * kOversampling * jw);
-      const double m = sd.M[i + static_cast<long>(sd.ldm) * j];
-      const double f = factor * m;
-      const double d2 = d * d;
-      const double w = cf[0] + cf[1] * d + cf[2] * d2 + cf[3] * d2 * d;
-      atomicAdd(row + t_out, f * w);
-      if (sqr)
-        atomicAdd(row_sqr + t_out, f * m * w);
+      mv = sd.M[i + static_cast<long>(sd.ldm) * j];
+      f = factor * mv;
+      t0 = tau_0 - kOversampling;
+      tab = 4 * (iw + 4 * kOversampling * jw);
+      // Out of the table only for |t_val| > 1/2, which the host rejects.
+      if (jw >= 0 && iw >= -1 && iw + 2 * kOversampling < 4 * kOversampling) {
+        // label = b_i + nb (b_j + nb dr), dr = index of r_i - r_j (sp_accumulator.hpp:185-191).
+        const int oi = orb_r[i], oj = orb_c[j];
+        const int r_i = oi / g.nb, r_j = oj / g.nb;
+        row = oi - g.nb * r_i + g.nb * (oj - g.nb * r_j + g.nb * r_sub[r_j + g.nc * r_i]) + spin * g.n_labels;
+      }
     }
-  }
-  __syncthreads();
-  double* out = f_tau + (static_cast<long>(spin) * g.n_labels + label) * g.n_padded;
-  for (int t = threadIdx.x; t < g.n_padded; t += blockDim.x)
-    out[t] += row[t];
-  if (f_tau_single) {  // this measurement alone (replaces the previous one)
-    double* one = f_tau_single + (static_cast<long>(spin) * g.n_labels + label) * g.n_padded;
-    for (int t = threadIdx.x; t < g.n_padded; t += blockDim.x)
-      one[t] = row[t];
-  }
-  if (sqr) {
-    double* out2 = f_tau_sqr + (static_cast<long>(spin) * g.n_labels + label) * g.n_padded;
-    for (int t = threadIdx.x; t < g.n_padded; t += blockDim.x)
-      out2[t] += row_sqr[t];
+    const int tap = (lane & 15) + 1;
+#pragma unroll 4
+    for (int s = 0; s < 16; ++s) {
+      const int src = 2 * s + (lane >> 4);
+      const double fs = __shfl_sync(0xffffffffu, f, src), ds = __shfl_sync(0xffffffffu, d, src);
+      const int rs = __shfl_sync(0xffffffffu, row, src), ts = __shfl_sync(0xffffffffu, t0, src) + tap;
+      const int cs = __shfl_sync(0xffffffffu, tab, src);
+      double ms = 0;
+      if constexpr (SQR)
+        ms = __shfl_sync(0xffffffffu, mv, src);
+      if (rs < 0 || ts < 0 || ts >= g.n_padded)
+        continue;
+      const double2* cf = reinterpret_cast<const double2*>(coeff + cs + 4 * tap);
+      const double2 c01 = __ldg(cf), c23 = __ldg(cf + 1);
+      const double d2 = ds * ds;
+      const double w = c01.x + c01.y * ds + c23.x * d2 + c23.y * d2 * ds;
+      const long o = static_cast<long>(rs) * g.n_padded + ts;
+      atomicAdd(f_tau + o, fs * w);
+      if constexpr (SQR)
+        atomicAdd(f_tau_sqr + o, fs * ms * w);
+    }
   }
 }
 
-// One CTA per (label, spin): fold, then f(w) = -(1/n) sum_x f(x) e^{2 pi i x nu_w / n} / phi(w) / Nc.
-__global__ void spFinalizeKernel(const NfftGrid g, const double* __restrict__ f_tau,
-                                 const double* __restrict__ inv_phi, int n_sp,
-                                 double2* __restrict__ out) {
+template <bool SQR>
+__global__ void __launch_bounds__(256)
+spAccumulateKernel(const NfftGrid g, const SpMeasurement m, const int* __restrict__ r_sub,
+                   const double* __restrict__ coeff, double factor, double* __restrict__ f_tau,
+                   double* __restrict__ f_tau_sqr) {
+  const long warp = (static_cast<long>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
+  const long warps = static_cast<long>(gridDim.x) * blockDim.x / 32;
+  for (int spin = 0; spin < 2; ++spin) {
+    // The second sector's steps continue where the first sector's round ends, so that the warps
+    // left over there start on it.
+    const long n = m.sector[spin].n;
+    const long skip = spin ? ((static_cast<long>(m.sector[0].n) * m.sector[0].n + 31) / 32) % warps : 0;
+    const long first = (warp + warps - skip) % warps;
+    if (n <= 65535)  // 32-bit pair indices
+      spAccumulateSector<SQR, unsigned>(g, m, spin, first, warps, r_sub, coeff, factor, f_tau, f_tau_sqr);
+    else
+      spAccumulateSector<SQR, unsigned long long>(g, m, spin, first, warps, r_sub, coeff, factor, f_tau, f_tau_sqr);
+  }
+}
+
+// f(w) = -(1/n) sum_x f(x) e^{2 pi i x nu / n} / phi(w) / Nc of the folded f, nu = 2 l + 1, and its
+// conjugate at -nu.  n = 8 N (N = n_sp), so with x = a + N b
+//   sum_x f(x) e^{2 pi i x nu / n} = sum_{a < N} W^{nu a} g_c(a),   W = e^{2 pi i / n},
+//   g_c(a) = sum_{b < 8} f(a + N b) e^{2 pi i (2 c + 1) b / 8},     c = l mod 4:
+// N terms per frequency instead of 8 N.  CTA = (label, spin, kFinL frequencies); a warp sums
+// kFinU frequencies of one class c with lanes over a: nu is odd, so the lanes' table reads W^{nu a}
+// fall in distinct banks.
+//
+// Latency and shared-memory bound.  One CTA per (label, spin) over all 8 N terms with a thread per
+// frequency, the earlier form, took 1,142 us on a 4x4 cluster with N = 512; this one 20 us.
+constexpr int kFinThreads = 256, kFinU = 2;
+constexpr int kFinL = kFinThreads / 32 * kFinU;  // frequencies per CTA and pass
+constexpr int kFinPasses = 4;                    // passes per CTA
+
+__global__ void __launch_bounds__(kFinThreads)
+spFinalizeKernel(const NfftGrid g, const double* __restrict__ f_tau, const double* __restrict__ inv_phi,
+                 const double2* __restrict__ roots, int n_sp, double2* __restrict__ out) {
   extern __shared__ __align__(16) double fin_smem[];
-  double* row = fin_smem;                                       // n folded samples
-  double2* tw = reinterpret_cast<double2*>(fin_smem + g.n);     // e^{2 pi i m / n}
+  double2* tw = reinterpret_cast<double2*>(fin_smem);  // [8 N] W^m
+  double2* gc = tw + g.n;                              // [4][N]
   const int label = blockIdx.x, spin = blockIdx.y;
   const int pad = (g.n_padded - g.n) / 2;
   const double* f = f_tau + (static_cast<long>(spin) * g.n_labels + label) * g.n_padded;
-  for (int x = threadIdx.x; x < g.n; x += blockDim.x) {
-    double v = f[pad + x];
-    // foldTimeDomainBack: halo t < pad lands on t + n, halo t >= n_padded - pad on t - n.
-    const int t = pad + x;
-    if (t >= g.n && t - g.n < pad)
-      v += f[t - g.n];
-    if (t + g.n >= g.n_padded - pad && t + g.n < g.n_padded)
-      v += f[t + g.n];
-    row[x] = v;
-    double s, c;
-    sincospi(2.0 * x / g.n, &s, &c);
-    tw[x] = make_double2(c, s);
+  for (int m = threadIdx.x; m < g.n; m += blockDim.x)
+    tw[m] = roots[m];
+  for (int a = threadIdx.x; a < n_sp; a += blockDim.x) {
+    double v[8];
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      // foldTimeDomainBack: halo t < pad lands on t + n, halo t >= n_padded - pad on t - n.
+      const int t = pad + a + n_sp * b;
+      v[b] = f[t];
+      if (t >= g.n && t - g.n < pad)
+        v[b] += f[t - g.n];
+      if (t + g.n >= g.n_padded - pad && t + g.n < g.n_padded)
+        v[b] += f[t + g.n];
+    }
+    constexpr double h = 0.70710678118654752440;
+    constexpr double cs[8] = {1, h, 0, -h, -1, -h, 0, h}, sn[8] = {0, h, 1, h, 0, -h, -1, -h};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      double re = 0, im = 0;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        re = fma(v[b], cs[((2 * c + 1) * b) & 7], re);
+        im = fma(v[b], sn[((2 * c + 1) * b) & 7], im);
+      }
+      gc[c * n_sp + a] = make_double2(re, im);
+    }
   }
   __syncthreads();
   const int b1 = label % g.nb, b2 = (label / g.nb) % g.nb, r = label / (g.nb * g.nb);
   const int nb = g.nb;
-  for (int w = threadIdx.x; w < 2 * n_sp; w += blockDim.x) {
-    const int nu = w >= n_sp ? 2 * (w - n_sp) + 1 : -(2 * (n_sp - 1 - w) + 1);
-    const int step = ((nu % g.n) + g.n) % g.n;
-    double re = 0, im = 0;
-    int m = 0;
-    for (int x = 0; x < g.n; ++x) {
-      const double2 e = tw[m];
-      re = fma(row[x], e.x, re);
-      im = fma(row[x], e.y, im);
-      m += step;
-      if (m >= g.n)
-        m -= g.n;
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  for (int pass = 0; pass < kFinPasses; ++pass) {
+    // Frequencies l0 + 4 u: warps 0..3 (and 4..7, 4 kFinU further) take the four classes.
+    const int l0 = (blockIdx.z * kFinPasses + pass) * kFinL + (warp / 4) * 4 * kFinU + warp % 4;
+    if (l0 >= n_sp)
+      break;
+    double re[kFinU], im[kFinU];
+    int m[kFinU], step[kFinU];
+#pragma unroll
+    for (int u = 0; u < kFinU; ++u) {
+      const long nu = 2 * (l0 + 4 * u) + 1;
+      re[u] = im[u] = 0;
+      m[u] = static_cast<int>(nu * lane % g.n);
+      step[u] = static_cast<int>(nu * 32 % g.n);
     }
-    const double scale = -inv_phi[w] / (double(g.n) * g.nc);
-    // (b1, s, b2, s, r, w)
-    const long o = b1 + nb * (spin + 2 * (b2 + nb * (spin + 2 * (r + static_cast<long>(g.nc) * w))));
-    out[o] = make_double2(re * scale, im * scale);
+    const double2* gl = gc + (l0 & 3) * n_sp;
+    for (int a = lane; a < n_sp; a += 32) {
+      const double2 x = gl[a];
+#pragma unroll
+      for (int u = 0; u < kFinU; ++u) {
+        const double2 e = tw[m[u]];
+        re[u] = fma(x.x, e.x, re[u]);
+        re[u] = fma(-x.y, e.y, re[u]);
+        im[u] = fma(x.x, e.y, im[u]);
+        im[u] = fma(x.y, e.x, im[u]);
+        m[u] += step[u];
+        if (m[u] >= g.n)
+          m[u] -= g.n;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kFinU; ++u) {
+#pragma unroll
+      for (int s = 16; s; s /= 2) {
+        re[u] += __shfl_xor_sync(0xffffffffu, re[u], s);
+        im[u] += __shfl_xor_sync(0xffffffffu, im[u], s);
+      }
+      const int l = l0 + 4 * u;
+      if (l < n_sp && lane < 2) {
+        const int w = lane ? n_sp - 1 - l : n_sp + l;
+        const double scale = -inv_phi[w] / (double(g.n) * g.nc);
+        // (b1, s, b2, s, r, w)
+        const long o = b1 + nb * (spin + 2 * (b2 + nb * (spin + 2 * (r + static_cast<long>(g.nc) * w))));
+        out[o] = make_double2(re[u] * scale, (lane ? -im[u] : im[u]) * scale);
+      }
+    }
   }
 }
 
@@ -233,18 +312,20 @@ struct SpAccumulator::Impl {
   double beta = 0;
   bool sqr = false;
   bool stamping = false;
-  int device = 0;
+  int device = 0, n_sm = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  cudaEvent_t upload_done = nullptr;
-  std::vector<int> r_of;
-  DevBuf<double> coeff, inv_phi, f_tau, f_tau_sqr, f_tau_single, tau_d, M_d;
-  DevBuf<int> r_of_d, perm_r_d, perm_c_d, rs_d, cs_d;
-  DevBuf<SpSector> sectors_d;
-  DevBuf<double2> out_d;
-  PinBuf<double> tau_h;
-  PinBuf<int> perm_r_h, perm_c_h, rs_h, cs_h;
-  PinBuf<SpSector> sectors_h;
+  DevBuf<double> coeff, inv_phi, f_tau, f_tau_sqr, f_tau_single, M_d;
+  DevBuf<int> r_sub_d;
+  DevBuf<double2> out_d, roots;
+  // A measurement's vertices, packed (tau, row orbitals, column orbitals) so that one copy uploads
+  // them.  The pinned sets are a ring, so that the host fills the next ones while copies wait behind
+  // earlier kernels; the device set is reused in stream order.
+  static constexpr int kSets = 4;
+  PinBuf<double> vtx_h[kSets];
+  DevBuf<double> vtx_d;
+  cudaEvent_t uploaded[kSets] = {};
+  int set = 0;
   std::vector<double2> mrw, mrw_sqr;
   bool ready = false, finalized = false;
   uint64_t launches = 0;
@@ -262,17 +343,18 @@ SpAccumulator::SpAccumulator(const dcaacc_sp_config& c) : d_(new Impl) {
   d.sqr = c.accumulate_m_sqr != 0;
   d.stamping = c.stamping != 0;
   d.max_order = c.max_order;
-  // r_of[r_j + nc dr] = r_i with r_sub(r_j, r_i) = dr, i.e. x_{r_i} - x_{r_j} = x_dr.
-  d.r_of.assign(nc * nc, -1);
+  // The index of r_i - r_j for every pair of sites; each difference once per r_j.
+  const std::vector<int> r_sub(c.r_sub, c.r_sub + nc * nc);
+  std::vector<char> seen(nc * nc, 0);
   for (int rj = 0; rj < nc; ++rj)
     for (int ri = 0; ri < nc; ++ri) {
-      const int dr = c.r_sub[rj + nc * ri];
+      const int dr = r_sub[rj + nc * ri];
       if (dr < 0 || dr >= nc)
         throw Error(DCAACC_INVALID_ARG, "r_sub entry out of range");
-      d.r_of[rj + nc * dr] = ri;
+      seen[rj + nc * dr] = 1;
     }
-  for (int v : d.r_of)
-    if (v < 0)
+  for (char v : seen)
+    if (!v)
       throw Error(DCAACC_INVALID_ARG, "r_sub is not a group subtraction table");
 
   // nfft_time_domain (nfft_time_domain.hpp:112-176) with MAX_FREQUENCY = n_sp.
@@ -314,15 +396,24 @@ SpAccumulator::SpAccumulator(const dcaacc_sp_config& c) : d_(new Impl) {
   }
 
   DCAACC_CUDA_CHECK(cudaGetDevice(&d.device));
+  DCAACC_CUDA_CHECK(cudaDeviceGetAttribute(&d.n_sm, cudaDevAttrMultiProcessorCount, d.device));
   DCAACC_CUDA_CHECK(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
   d.own_stream = true;
-  DCAACC_CUDA_CHECK(cudaEventCreateWithFlags(&d.upload_done, cudaEventDisableTiming));
+  for (auto& e : d.uploaded)
+    DCAACC_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   d.coeff.alloc(cf.size());
   DCAACC_CUDA_CHECK(cudaMemcpy(d.coeff.get(), cf.data(), d.coeff.bytes(), cudaMemcpyHostToDevice));
   d.inv_phi.alloc(ip.size());
   DCAACC_CUDA_CHECK(cudaMemcpy(d.inv_phi.get(), ip.data(), d.inv_phi.bytes(), cudaMemcpyHostToDevice));
-  d.r_of_d.alloc(d.r_of.size());
-  DCAACC_CUDA_CHECK(cudaMemcpy(d.r_of_d.get(), d.r_of.data(), d.r_of_d.bytes(), cudaMemcpyHostToDevice));
+  d.r_sub_d.alloc(r_sub.size());
+  DCAACC_CUDA_CHECK(cudaMemcpy(d.r_sub_d.get(), r_sub.data(), d.r_sub_d.bytes(), cudaMemcpyHostToDevice));
+  std::vector<double2> roots(g.n);
+  for (int m = 0; m < g.n; ++m) {
+    const long double x = 2 * 3.14159265358979323846264338327950288L * m / g.n;
+    roots[m] = make_double2(double(std::cos(x)), double(std::sin(x)));
+  }
+  d.roots.alloc(roots.size());
+  DCAACC_CUDA_CHECK(cudaMemcpy(d.roots.get(), roots.data(), d.roots.bytes(), cudaMemcpyHostToDevice));
   const size_t ft = 2 * size_t(g.n_labels) * g.n_padded;
   d.f_tau.alloc(ft);
   if (d.sqr)
@@ -330,21 +421,13 @@ SpAccumulator::SpAccumulator(const dcaacc_sp_config& c) : d_(new Impl) {
   if (d.stamping)
     d.f_tau_single.alloc(ft);
   const size_t nv = 2 * size_t(d.max_order);
-  d.tau_d.alloc(nv);
   d.M_d.alloc(2 * size_t(d.max_order) * d.max_order);
-  d.perm_r_d.alloc(nv);
-  d.perm_c_d.alloc(nv);
-  d.rs_d.alloc(2 * size_t(nb * nc + 1));
-  d.cs_d.alloc(2 * size_t(nb * nc + 1));
-  d.sectors_d.alloc(2);
   d.out_d.alloc(size_t(2 * nb) * (2 * nb) * nc * 2 * d.n_sp);
-  d.tau_h.alloc(nv);
-  d.perm_r_h.alloc(nv);
-  d.perm_c_h.alloc(nv);
-  d.rs_h.alloc(2 * size_t(nb * nc + 1));
-  d.cs_h.alloc(2 * size_t(nb * nc + 1));
-  d.sectors_h.alloc(2);
-  DCAACC_CUDA_CHECK(cudaEventRecord(d.upload_done, d.stream));
+  d.vtx_d.alloc(2 * nv);  // per vertex one double and two ints
+  for (int i = 0; i < Impl::kSets; ++i) {
+    d.vtx_h[i].alloc(2 * nv);
+    DCAACC_CUDA_CHECK(cudaEventRecord(d.uploaded[i], d.stream));
+  }
   if (sizeof(double) * 2 * g.n_padded > 200 * 1024 || sizeof(double) * 3 * g.n > 200 * 1024)
     throw Error(DCAACC_INVALID_ARG, "n_sp_freq too large for the shared-memory NFFT rows");
 }
@@ -352,8 +435,9 @@ SpAccumulator::SpAccumulator(const dcaacc_sp_config& c) : d_(new Impl) {
 SpAccumulator::~SpAccumulator() {
   if (d_->stream)
     cudaStreamSynchronize(d_->stream);
-  if (d_->upload_done)
-    cudaEventDestroy(d_->upload_done);
+  for (auto& e : d_->uploaded)
+    if (e)
+      cudaEventDestroy(e);
   if (d_->own_stream && d_->stream)
     cudaStreamDestroy(d_->stream);
 }
@@ -378,9 +462,6 @@ void SpAccumulator::accumulate(const dcaacc_sector* sec, double factor) {
     throw Error(DCAACC_NOT_READY, "The accumulator is already finalized.");
   if (!sec)
     throw Error(DCAACC_INVALID_ARG, "null sectors");
-  const int n_orb = g.nb * g.nc;
-  DCAACC_CUDA_CHECK(cudaEventSynchronize(d.upload_done));
-  int vtx = 0;
   for (int s = 0; s < 2; ++s) {
     const auto& x = sec[s];
     if (x.n < 0 || x.n > d.max_order)
@@ -395,23 +476,36 @@ void SpAccumulator::accumulate(const dcaacc_sector* sec, double factor) {
       if (!(x.tau[i] >= 0.0 && x.tau[i] <= d.beta))
         throw Error(DCAACC_INVALID_ARG, "vertex time outside [0, beta]");
     }
+  }
+  const int vtx = sec[0].n + sec[1].n;
+  if (vtx == 0) {
+    if (d.stamping)  // an empty measurement: its own f(tau) is zero
+      DCAACC_CUDA_CHECK(cudaMemsetAsync(d.f_tau_single.get(), 0, d.f_tau_single.bytes(), d.stream));
+    return;
+  }
+  const int set = d.set;
+  d.set = (set + 1) % Impl::kSets;
+  DCAACC_CUDA_CHECK(cudaEventSynchronize(d.uploaded[set]));  // the set's earlier copy has been made
+  double* tau = d.vtx_h[set].get();
+  int* orb_r = reinterpret_cast<int*>(tau + vtx);
+  int* orb_c = orb_r + vtx;
+  SpMeasurement m{};
+  m.tau = d.vtx_d.get();
+  m.orb_r = reinterpret_cast<const int*>(m.tau + vtx);
+  m.orb_c = m.orb_r + vtx;
+  int off = 0;
+  long groups = 0;
+  for (int s = 0; s < 2; ++s) {
+    const auto& x = sec[s];
+    std::copy_n(x.tau, x.n, tau + off);
     // Rows: right band / site; columns: left band / site (sp_accumulator.hpp:181-187).
-    auto sort_side = [&](bool left, int* perm, int* start) {
-      std::fill(start, start + n_orb + 1, 0);
-      for (int v = 0; v < x.n; ++v)
-        start[(left ? x.left_band[v] + g.nb * x.left_site[v] : x.right_band[v] + g.nb * x.right_site[v]) + 1]++;
-      for (int o = 0; o < n_orb; ++o)
-        start[o + 1] += start[o];
-      std::vector<int> fill(start, start + n_orb);
-      for (int v = 0; v < x.n; ++v)
-        perm[fill[left ? x.left_band[v] + g.nb * x.left_site[v] : x.right_band[v] + g.nb * x.right_site[v]]++] = v;
-    };
-    sort_side(false, d.perm_r_h.get() + vtx, d.rs_h.get() + s * (n_orb + 1));
-    sort_side(true, d.perm_c_h.get() + vtx, d.cs_h.get() + s * (n_orb + 1));
-    std::copy_n(x.tau, x.n, d.tau_h.get() + vtx);
-    SpSector sd{};
+    for (int v = 0; v < x.n; ++v) {
+      orb_r[off + v] = x.right_band[v] + g.nb * x.right_site[v];
+      orb_c[off + v] = x.left_band[v] + g.nb * x.left_site[v];
+    }
+    SpSector& sd = m.sector[s];
     sd.n = x.n;
-    sd.vtx_off = vtx;
+    sd.vtx_off = off;
     sd.M = x.M;
     sd.ldm = std::max(x.ldm, 1);
     if (x.n && !x.m_on_device) {
@@ -421,33 +515,33 @@ void SpAccumulator::accumulate(const dcaacc_sector* sec, double factor) {
       sd.M = dst;
       sd.ldm = x.n;
     }
-    d.sectors_h[s] = sd;
-    vtx += x.n;
+    off += x.n;
+    groups += (long(x.n) * x.n + 31) / 32;
   }
-  if (vtx == 0) {
-    if (d.stamping)  // an empty measurement: its own f(tau) is zero
-      DCAACC_CUDA_CHECK(cudaMemsetAsync(d.f_tau_single.get(), 0, d.f_tau_single.bytes(), d.stream));
-    return;
+  DCAACC_CUDA_CHECK(cudaMemcpyAsync(d.vtx_d.get(), tau, (sizeof(double) + 2 * sizeof(int)) * vtx,
+                                    cudaMemcpyHostToDevice, d.stream));
+  DCAACC_CUDA_CHECK(cudaEventRecord(d.uploaded[set], d.stream));
+  // With stamping the measurement goes to its own f(tau) first, which is then added to the sum.
+  double* target = d.f_tau.get();
+  if (d.stamping) {
+    target = d.f_tau_single.get();
+    DCAACC_CUDA_CHECK(cudaMemsetAsync(target, 0, d.f_tau_single.bytes(), d.stream));
   }
-  auto h2d = [&](void* dst, const void* src, size_t bytes) {
-    if (bytes)
-      DCAACC_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, d.stream));
-  };
-  h2d(d.sectors_d.get(), d.sectors_h.get(), 2 * sizeof(SpSector));
-  h2d(d.tau_d.get(), d.tau_h.get(), sizeof(double) * vtx);
-  h2d(d.perm_r_d.get(), d.perm_r_h.get(), sizeof(int) * vtx);
-  h2d(d.perm_c_d.get(), d.perm_c_h.get(), sizeof(int) * vtx);
-  h2d(d.rs_d.get(), d.rs_h.get(), sizeof(int) * 2 * (n_orb + 1));
-  h2d(d.cs_d.get(), d.cs_h.get(), sizeof(int) * 2 * (n_orb + 1));
-  DCAACC_CUDA_CHECK(cudaEventRecord(d.upload_done, d.stream));
-  const size_t smem = sizeof(double) * g.n_padded * (d.sqr ? 2 : 1);
-  DCAACC_CUDA_CHECK(cudaFuncSetAttribute(spAccumulateKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  spAccumulateKernel<<<dim3(g.n_labels, 2), 256, smem, d.stream>>>(
-      g, d.sectors_d.get(), d.perm_r_d.get(), d.perm_c_d.get(), d.rs_d.get(), d.cs_d.get(),
-      d.tau_d.get(), d.r_of_d.get(), d.coeff.get(), factor, d.f_tau.get(),
-      d.sqr ? d.f_tau_sqr.get() : nullptr, d.stamping ? d.f_tau_single.get() : nullptr);
+  // Eight warps a CTA, eight CTAs to an SM at most: the reductions need many warps in flight.
+  const unsigned blocks = static_cast<unsigned>(std::max(1L, std::min((groups + 7) / 8, long(d.n_sm) * 8)));
+  if (d.sqr)
+    spAccumulateKernel<true><<<blocks, 256, 0, d.stream>>>(g, m, d.r_sub_d.get(), d.coeff.get(), factor, target,
+                                                           d.f_tau_sqr.get());
+  else
+    spAccumulateKernel<false><<<blocks, 256, 0, d.stream>>>(g, m, d.r_sub_d.get(), d.coeff.get(), factor, target,
+                                                            nullptr);
   DCAACC_LAUNCH_CHECK();
   ++d.launches;
+  if (d.stamping) {
+    addKernel<<<d.n_sm * 4, 256, 0, d.stream>>>(d.f_tau.get(), target, d.f_tau.size());
+    DCAACC_LAUNCH_CHECK();
+    ++d.launches;
+  }
 }
 
 void SpAccumulator::finalize() {
@@ -465,10 +559,12 @@ void SpAccumulator::finalize() {
 void SpAccumulator::finalizeInto(const double* f_tau, std::vector<double2>& host) {
   auto& d = *d_;
   auto& g = d.g;
-  const size_t smem = sizeof(double) * 3 * g.n;
+  const size_t smem = sizeof(double2) * (g.n + 4 * size_t(d.n_sp));
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(spFinalizeKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   DCAACC_CUDA_CHECK(cudaMemsetAsync(d.out_d.get(), 0, d.out_d.bytes(), d.stream));
-  spFinalizeKernel<<<dim3(g.n_labels, 2), 256, smem, d.stream>>>(g, f_tau, d.inv_phi.get(), d.n_sp, d.out_d.get());
+  const int splits = ceil_div(d.n_sp, kFinL * kFinPasses);
+  spFinalizeKernel<<<dim3(g.n_labels, 2, splits), kFinThreads, smem, d.stream>>>(g, f_tau, d.inv_phi.get(),
+                                                                                 d.roots.get(), d.n_sp, d.out_d.get());
   DCAACC_LAUNCH_CHECK();
   ++d.launches;
   host.resize(d.out_d.size());
@@ -555,9 +651,7 @@ void SpAccumulator::synchronize() {
 size_t SpAccumulator::deviceFingerprint() const {
   auto& d = *d_;
   return d.coeff.bytes() + d.inv_phi.bytes() + d.f_tau.bytes() + d.f_tau_sqr.bytes() + d.f_tau_single.bytes() +
-         d.tau_d.bytes() +
-         d.M_d.bytes() + d.r_of_d.bytes() + d.perm_r_d.bytes() + d.perm_c_d.bytes() + d.rs_d.bytes() +
-         d.cs_d.bytes() + d.sectors_d.bytes() + d.out_d.bytes();
+         d.M_d.bytes() + d.r_sub_d.bytes() + d.vtx_d.bytes() + d.out_d.bytes() + d.roots.bytes();
 }
 
 uint64_t SpAccumulator::kernelLaunches() const {
