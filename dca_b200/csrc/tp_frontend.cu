@@ -7,22 +7,31 @@
 //
 //   twiddle_kernel      T(w, v) = exp(i w tau_v) over the extended frequency mesh, in both the
 //                       row-sorted and column-sorted vertex orders.
-//   row_transform       X'(b1 k1 w1, j) = sum_{r1} e^{i k1 (r1 + a_b1)} sum_{i in orbital (b1,r1)}
-//                       T(w1, i) M(i, j)      (row NDFT fused with the row cluster transform)
-//   col_transform       G~(r, w1; b2 k2 w2) = 1/Nc sum_{r2} e^{-i k2 (r2 + a_b2)}
-//                       sum_{j in orbital (b2,r2)} X'(r w1, j) conj(T(w2, j)), then the epilogue
-//                       G = -G0(k1,w1) G~ G0(k2,w2) + beta G0(k1,w1) delta_{k1k2} delta_{w1w2}
-//                       (band-matrix products when nb > 1), written in frequency-block layout.
+//   row_transform       X'(b1 k1 w1, j) = -1/Nc sum_b G0(b1, b; k1, w1) sum_{r1} e^{i k1 (r1 + a_b)}
+//                       sum_{i in orbital (b,r1)} T(w1, i) M(i, j)
+//   col_transform       G(b1 k1, w1; b2 k2 w2) = sum_b [ sum_{r2} e^{-i k2 (r2 + a_b)}
+//                       sum_{j in orbital (b,r2)} X'(b1 k1 w1, j) conj(T(w2, j)) ] G0(b, b2; k2, w2)
+//                       + beta G0(k1,w1) delta_{k1k2} delta_{w1w2}, in frequency-block layout.
 //
-// Both transforms exploit the orbital structure (each vertex belongs to one orbital, so the
-// inner sums run over that orbital's vertices only, as the reference's per-orbital-pair
-// products do) and keep the cluster transform (K = Nc) in shared memory, so M, X' and G each
-// cross global memory once.  Templated on the working precision: double for the FP64 path,
-// float for the FP32 SIMT variant of the mixed path.
+// Both exploit the orbital structure (each vertex belongs to one orbital, so the inner sums run
+// over that orbital's vertices only, as the reference's per-orbital-pair products do) and both are
+// the same two small products per CTA: the sums of a 16 x WT tile for every orbital (phase 1), then
+// the cluster transform of those sums from shared memory (phase 2), so M, X' and G each cross
+// global memory once per tile column.  Templated on the working precision: double for the FP64
+// path, float for the FP32 SIMT variant of the mixed path.
+//
+// Phase 1: the orbitals are handed to the warps one by one (a shared counter).  A warp holds the
+// whole 16 x WT tile, 2 x WT/4 sums a lane, and streams its orbital's vertices through a ring of
+// its own in shared memory, one asynchronous 16-byte copy per lane and vertex; per vertex a lane
+// reads 2 + WT/4 elements for 2 WT/4 complex multiply-adds.  Phase 2: 4 x 2 sums a lane over the
+// sites.  Both phases are bound by the FP64 pipe.  The earlier kernels gave a thread one sum, that
+// is two shared-memory reads per multiply-add, and a whole CTA one orbital at a time:
+// FRONT_BEFORE_AFTER
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
+#include "async_copy.cuh"
 #include "common.cuh"
 #include "tp_frontend.hpp"
 
@@ -65,242 +74,433 @@ __device__ inline cplx_t<Real> loadC(const double2* p) {
   return mk(static_cast<Real>(v.x), static_cast<Real>(v.y));
 }
 
-// Row transform.  grid (ceil(n_max / JC), ceil(NwExt / WC), n_sectors), WC * JC threads.
-// Thread (w, jc) walks the row-sorted vertices once; the vertices of one orbital are contiguous,
-// so its running sum is flushed to shared memory at each orbital boundary (the same boundaries
-// for every thread, so no divergence).  M columns and twiddles are staged through shared memory
-// in chunks of IB vertices.
-template <typename Real, int JC, int WC, int IB>
-__global__ void __launch_bounds__(JC * WC)
+constexpr int kTileR = 16;  // rows of G (column step) or columns of M (row step) of a CTA's tile
+constexpr int kRing = 8;    // vertices in flight per warp
+
+template <int BYTES>
+__device__ inline void cpAsync(void* dst, const void* src) {
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smemAddr(dst)), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smemAddr(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ inline void cpAsyncCommit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ inline void cpAsyncWait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Shared memory of a tile kernel: the orbitals' sums Z[o][w][16], the warps' rings (16 bytes per
+// lane and slot), the phases F[b][r][k] (k padded with zeros), the orbital starts and the
+// counter that hands them out.
+template <typename Real, int WT>
+struct Tile {
+  using C = cplx_t<Real>;
+  static constexpr int kPairs = kTileR * WT;
+  static constexpr int kThreads = kPairs;
+  static constexpr int kWarps = kThreads / 32;
+  static_assert(kTileR + WT <= 32, "one copy per lane and vertex");
+  unsigned char* ring;
+  C *Z, *F;
+  int *start, *next;
+
+  // Phase 2 reads whole groups of momenta: 16 of one band, 8 otherwise.
+  __host__ __device__ static int kPad(const TpDims& d) {
+    return d.nb == 1 ? (d.nc + 15) / 16 * 16 : (d.nc + 7) / 8 * 8;
+  }
+  __host__ __device__ static size_t bytes(const TpDims& d) {
+    return size_t(kWarps) * kRing * 512 + sizeof(C) * (size_t(d.n_orb) * kPairs + size_t(d.nb) * d.nc * kPad(d)) +
+           sizeof(int) * (d.n_orb + 2);
+  }
+  // Lays the memory out and fills the phases, the starts and the counter.
+  __device__ Tile(unsigned char* raw, const TpDims& d, const double2* __restrict__ Fb,
+                  const int* __restrict__ orb_start) {
+    ring = raw;
+    Z = reinterpret_cast<C*>(raw + kWarps * kRing * 512);
+    F = Z + d.n_orb * kPairs;
+    start = reinterpret_cast<int*>(F + d.nb * d.nc * kPad(d));
+    next = start + d.n_orb + 1;
+    const int kp = kPad(d);
+    for (int i = threadIdx.x; i < d.nb * d.nc * kp; i += kThreads) {
+      const int k = i % kp, r = (i / kp) % d.nc, b = i / (kp * d.nc);
+      F[i] = k < d.nc ? loadC<Real>(Fb + (b * d.nc + k) * d.nc + r) : mk(Real(0), Real(0));
+    }
+    for (int i = threadIdx.x; i <= d.n_orb; i += kThreads)
+      start[i] = orb_start[i];
+    if (threadIdx.x == 0)
+      *next = 0;
+    __syncthreads();
+  }
+
+  // Phase 1: hands the orbitals to the warps.  issue(v, slot) starts this lane's copy of vertex v into
+  // a ring slot, use(slot) adds a landed slot, done(o) stores orbital o's sums and clears them.
+  template <typename Issue, typename Use, typename Done>
+  __device__ void orbitals(int n_orb, Issue issue, Use use, Done done) {
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    unsigned char* mine = ring + warp * kRing * 512;
+    for (;;) {
+      int o = 0;
+      if (lane == 0)
+        o = atomicAdd(next, 1);
+      o = __shfl_sync(0xffffffffu, o, 0);
+      if (o >= n_orb)
+        break;
+      const int v0 = start[o], v1 = start[o + 1];
+      __syncwarp();  // every lane is done with the previous orbital's slots
+#pragma unroll
+      for (int p = 0; p < kRing - 1; ++p) {
+        if (v0 + p < v1)
+          issue(v0 + p, mine + p * 512);
+        cpAsyncCommit();
+      }
+      int slot = 0;
+      for (int v = v0; v < v1; ++v) {
+        cpAsyncWait<kRing - 2>();
+        __syncwarp();  // vertex v has landed for every lane, and every lane is done with vertex v - 1
+        if (v + kRing - 1 < v1)
+          issue(v + kRing - 1, mine + (slot == 0 ? kRing - 1 : slot - 1) * 512);
+        cpAsyncCommit();
+        use(mine + slot * 512);
+        slot = slot == kRing - 1 ? 0 : slot + 1;
+      }
+      done(o);
+    }
+    cpAsyncWait<0>();
+    __syncthreads();
+  }
+
+  // Phase 2 of one line of the tile (16 rows of frequency wl) and band b: acc[i][c] = sum_r
+  // Z(b, r; wl, tr + 4 i) F(b, k0 + kl + 8 c; r), F conjugated when CONJ (tr = lane / 8, kl = lane % 8).
+  template <bool CONJ, int KC>
+  __device__ void clusterSum(C (&acc)[4][KC], const TpDims& d, int nb, int b, int wl, int k0) const {
+    const int lane = threadIdx.x % 32, kp = kPad(d);
+    const C* z = Z + b * kPairs + wl * kTileR + lane / 8;
+    const C* f = F + b * d.nc * kp + k0 + lane % 8;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < KC; ++c)
+        acc[i][c] = mk(Real(0), Real(0));
+#pragma unroll 2
+    for (int r = 0; r < d.nc; ++r, z += nb * kPairs, f += kp) {
+      C zv[4], fv[KC];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        zv[i] = z[4 * i];
+#pragma unroll
+      for (int c = 0; c < KC; ++c)
+        fv[c] = f[8 * c];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+          if constexpr (CONJ)
+            cfmac(acc[i][c], zv[i], fv[c]);
+          else
+            cfma(acc[i][c], zv[i], fv[c]);
+        }
+    }
+  }
+};
+
+// Momenta of one phase 2 task: 16 of one band, or 8 with all the bands.
+template <int NB>
+constexpr int kTaskK = NB == 1 ? 16 : 8;
+
+// Row transform.  grid (ceil(n_max / 16), ceil(NwExt / WT), n_sectors).  NB: bands (1, 2 or 3), 0 for
+// any number.
+template <typename Real, int WT, int NB>
+__global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
 rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const int* __restrict__ perm_r, const int* __restrict__ perm_c,
                    const int* __restrict__ row_start, const double2* __restrict__ Tr,
                    const double2* __restrict__ Fb,  // (r, k, b): e^{i k (r + a_b)}
+                   const double2* __restrict__ G0,  // (b1, b2, k, w, s)
                    cplx_t<Real>* __restrict__ Xp) {
   using C = cplx_t<Real>;
+  using T = Tile<Real, WT>;
   const SectorDesc sd = sectors[blockIdx.z];
-  const int n = sd.n;
-  const int jj0 = blockIdx.x * JC;
-  const int w0 = blockIdx.y * WC;
-  if (jj0 >= n)
+  const int n = sd.n, j0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
+  if (j0 >= n)
     return;
-  const int nw_ext = dims.nw_ext, n_orb = dims.n_orb, R = dims.R, nb = dims.nb, nc = dims.nc;
-  const int t = threadIdx.x;
-  const int w = t % WC, jc = t / WC;
-
+  const int nw_ext = dims.nw_ext, R = dims.R, nb = NB ? NB : dims.nb, nc = dims.nc;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int MS = IB + 1;               // padded row of Ms (no bank conflicts across jc)
-  C* Xs = reinterpret_cast<C*>(smem_raw);   // [n_orb][JC][WC]
-  C* Fs = Xs + JC * WC * n_orb;             // [nb][r][k]: lanes that differ in k read distinct banks
-  C* Ts = Fs + nb * nc * nc;                // [IB][WC]
-  Real* Ms = reinterpret_cast<Real*>(Ts + IB * WC);  // [JC][MS]
-  int* rs = reinterpret_cast<int*>(Ms + JC * MS);    // [n_orb + 1]
+  T tile(smem_raw, dims, Fb, row_start + sd.orb_off);
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
 
+  // Phase 1: Z(o, w, j) = sum of T(w, i) M(i, j) over the vertices i of orbital o.  Lanes 0..15 copy
+  // M(i, j0 + lane), the next WT lanes T(w0 + lane - 16, i); past the edge the last element, unused.
   const int* pr = perm_r + sd.vtx_off;
-  const int* pc = perm_c + sd.vtx_off;
-  for (int idx = t; idx < nb * nc * nc; idx += blockDim.x) {  // Fb is (b, k, r); Fs is (b, r, k)
-    const int b = idx / (nc * nc), k = (idx / nc) % nc, r = idx % nc;
-    Fs[(b * nc + r) * nc + k] = loadC<Real>(Fb + idx);
-  }
-  for (int idx = t; idx <= n_orb; idx += blockDim.x)
-    rs[idx] = row_start[sd.orb_off + idx];
-  const int jc_count = min(JC, n - jj0);
+  const long mcol = static_cast<long>(sd.ldm) * perm_c[sd.vtx_off + min(j0 + (lane & 15), n - 1)];
+  const double2* tsrc = Tr + static_cast<long>(sd.vtx_off) * nw_ext + min(w0 + lane % WT, nw_ext - 1);
+  const int jl = lane % 8, wq = lane / 8;  // this lane's sums: columns jl + 8 a, frequencies wq + 4 b
+  const bool f32 = sd.m_f32 != 0;
+  C acc[2][WT / 4];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < WT / 4; ++b)
+      acc[a][b] = mk(Real(0), Real(0));
+  tile.orbitals(
+      dims.n_orb,
+      [&](int v, unsigned char* slot) {
+        if (lane < kTileR) {
+          const long e = mcol + pr[v];
+          if (f32)
+            cpAsync<4>(slot + 16 * lane, reinterpret_cast<const float*>(sd.M) + e);
+          else
+            cpAsync<8>(slot + 16 * lane, sd.M + e);
+        }
+        else if (lane < kTileR + WT) {
+          cpAsync<16>(slot + 16 * lane, tsrc + static_cast<long>(v) * nw_ext);
+        }
+      },
+      [&](const unsigned char* slot) {
+        Real m[2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+          const unsigned char* e = slot + 16 * (jl + 8 * a);
+          m[a] = f32 ? static_cast<Real>(*reinterpret_cast<const float*>(e))
+                     : static_cast<Real>(*reinterpret_cast<const double*>(e));
+        }
+#pragma unroll
+        for (int b = 0; b < WT / 4; ++b) {
+          const C t = loadC<Real>(reinterpret_cast<const double2*>(slot + 16 * (kTileR + wq + 4 * b)));
+#pragma unroll
+          for (int a = 0; a < 2; ++a) {
+            acc[a][b].x = fma(t.x, m[a], acc[a][b].x);
+            acc[a][b].y = fma(t.y, m[a], acc[a][b].y);
+          }
+        }
+      },
+      [&](int o) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < WT / 4; ++b) {
+            tile.Z[o * T::kPairs + (wq + 4 * b) * kTileR + jl + 8 * a] = acc[a][b];
+            acc[a][b] = mk(Real(0), Real(0));
+          }
+      });
 
-  // Row NDFT per orbital: X(o1, w; jc) = sum_{ii in seg(o1)} T(w, ii) M(ii, jc).
-  C acc = mk(Real(0), Real(0));
-  int o1 = 0;
-  __syncthreads();
-  int seg_end = rs[1];
-  while (o1 < n_orb && seg_end == 0) {  // leading empty orbitals
-    Xs[o1 * JC * WC + t] = acc;
-    ++o1;
-    seg_end = o1 < n_orb ? rs[o1 + 1] : n;
-  }
-  for (int i0 = 0; i0 < n; i0 += IB) {
-    const int ib_count = min(IB, n - i0);
-    for (int idx = t; idx < ib_count * WC; idx += blockDim.x) {
-      const int ib = idx / WC, ww = idx % WC;
-      Ts[ib * WC + ww] = (w0 + ww < nw_ext) ? loadC<Real>(Tr + static_cast<long>(sd.vtx_off + i0 + ib) * nw_ext + w0 + ww)
-                                           : mk(Real(0), Real(0));
-    }
-    for (int idx = t; idx < JC * ib_count; idx += blockDim.x) {
-      const int c = idx / ib_count, ib = idx % ib_count;
-      Ms[c * MS + ib] = c < jc_count
-                            ? static_cast<Real>(loadM(sd, static_cast<long>(sd.ldm) * pc[jj0 + c] + pr[i0 + ib]))
-                            : Real(0);
-    }
-    __syncthreads();
-    for (int ib = 0; ib < ib_count; ++ib) {
-      const int ii = i0 + ib;
-      while (ii >= seg_end) {  // orbital boundary: uniform across the CTA
-        Xs[o1 * JC * WC + t] = acc;
-        acc = mk(Real(0), Real(0));
-        ++o1;
-        seg_end = o1 < n_orb ? rs[o1 + 1] : n;
-      }
-      const C tv = Ts[ib * WC + w];
-      const Real m = Ms[jc * MS + ib];
-      acc.x = fma(tv.x, m, acc.x);
-      acc.y = fma(tv.y, m, acc.y);
-    }
-    __syncthreads();
-  }
-  for (; o1 < n_orb; ++o1) {
-    Xs[o1 * JC * WC + t] = acc;
-    acc = mk(Real(0), Real(0));
-  }
-  __syncthreads();
-
-  // Row cluster transform with band phases: X'(b1 + nb k1) = sum_r1 Fb(b1, k1, r1) X(b1 + nb r1).
-  for (int q = t; q < jc_count * WC * R; q += blockDim.x) {
-    const int row = q % R, ww = (q / R) % WC, c = q / (R * WC), we = w0 + ww;
-    if (we >= nw_ext)
+  // Phase 2: the cluster transform and the left G0, -1/Nc included.
+  const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
+  const double norm = -1.0 / nc;
+  const int k_tasks = (nc + kTaskK<NB> - 1) / kTaskK<NB>;
+  const long D = static_cast<long>(R) * nw_ext;
+  for (int task = warp; task < WT * k_tasks; task += T::kWarps) {
+    const int wl = task % WT, k0 = task / WT * kTaskK<NB>, w = w0 + wl;
+    if (w >= nw_ext)
       continue;
-    const int b1 = row % nb, k1 = row / nb;
-    const C* x = Xs + b1 * JC * WC + c * WC + ww;
-    const C* f = Fs + b1 * nc * nc + k1;
-    C a = mk(Real(0), Real(0));
-    for (int r1 = 0; r1 < nc; ++r1)
-      cfma(a, f[r1 * nc], x[nb * r1 * JC * WC]);
-    Xp[sd.x_off + (static_cast<long>(we) * n + jj0 + c) * R + row] = a;
+    const double2* g0 = g0s + static_cast<long>(w) * nc * nb * nb;  // (ba, bb, k)
+    auto put = [&](int i, int b1, int k, C v) {
+      const int j = j0 + lane / 8 + 4 * i;
+      if (j < n)
+        Xp[sd.x_off + j * D + static_cast<long>(w) * R + b1 + nb * k] = v;
+    };
+    if constexpr (NB == 1) {
+      C s[4][2];
+      tile.template clusterSum<false, 2>(s, dims, 1, 0, wl, k0);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int k = k0 + lane % 8 + 8 * c;
+        if (k >= nc)
+          continue;
+        const double2 g = g0[k];
+        const C gn = mk(static_cast<Real>(norm * g.x), static_cast<Real>(norm * g.y));
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          put(i, 0, k, cmul(gn, s[i][c]));
+      }
+    }
+    else if constexpr (NB > 1) {
+      C s[NB][4][1];
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+        tile.template clusterSum<false, 1>(s[b], dims, NB, b, wl, k0);
+      const int k = k0 + lane % 8;
+      if (k < nc) {
+#pragma unroll
+        for (int b1 = 0; b1 < NB; ++b1) {
+          C gn[NB];
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+            const double2 g = g0[b1 + NB * (b + NB * k)];
+            gn[b] = mk(static_cast<Real>(norm * g.x), static_cast<Real>(norm * g.y));
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            C v = cmul(gn[0], s[0][i][0]);
+#pragma unroll
+            for (int b = 1; b < NB; ++b)
+              cfma(v, gn[b], s[b][i][0]);
+            put(i, b1, k, v);
+          }
+        }
+      }
+    }
+    else {
+      const int k = k0 + lane % 8;
+      for (int b1 = 0; b1 < nb; ++b1) {
+        C v[4] = {};
+        for (int b = 0; b < nb; ++b) {
+          C s[4][1];
+          tile.template clusterSum<false, 1>(s, dims, nb, b, wl, k0);
+          const double2 g = g0[b1 + nb * (b + nb * min(k, nc - 1))];
+          const C gn = mk(static_cast<Real>(norm * g.x), static_cast<Real>(norm * g.y));
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            cfma(v[i], gn, s[i][0]);
+        }
+        if (k < nc)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            put(i, b1, k, v[i]);
+      }
+    }
   }
 }
 
-// Column transform + G epilogue.  grid (NwExt, ceil(NwExt / WC2), n_sectors), R * WC2 threads.
-// X' rows of frequency w1 and the twiddles of the CTA's w2 chunk are staged through shared
-// memory in chunks of JB vertices; thread (row, w2) walks the column-sorted vertices once and
-// flushes its running sum at each column-orbital boundary.
-template <typename Real, int JB>
-__global__ void colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
-                                   const int* __restrict__ col_start,
-                                   const double2* __restrict__ Tc, const double2* __restrict__ Fb,
-                                   const double2* __restrict__ G0,  // (b1, b2, k, w, s)
-                                   const cplx_t<Real>* __restrict__ Xp, cplx_t<Real>* __restrict__ G,
-                                   long g_sector_stride, int WC2) {
+// Column transform + G epilogue.  grid (ceil(D / 16), ceil(NwExt / WT), n_sectors); the rows of a tile
+// are 16 consecutive (w1, r).
+template <typename Real, int WT, int NB>
+__global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
+colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
+                   const int* __restrict__ col_start, const double2* __restrict__ Tc,
+                   const double2* __restrict__ Fb,
+                   const double2* __restrict__ G0,  // (b1, b2, k, w, s)
+                   const cplx_t<Real>* __restrict__ Xp, cplx_t<Real>* __restrict__ G, long g_sector_stride) {
   using C = cplx_t<Real>;
+  using T = Tile<Real, WT>;
   const SectorDesc sd = sectors[blockIdx.z];
-  const int n = sd.n;
-  const int w1 = blockIdx.x;
-  const int nw_ext = dims.nw_ext, n_orb = dims.n_orb, R = dims.R, nb = dims.nb, nc = dims.nc;
-  const int t = threadIdx.x;
-  const int row = t % R, w2l = t / R;
-  const int w2c0 = blockIdx.y * WC2;
-  const int w2 = w2c0 + w2l;
-  const bool active = w2 < nw_ext;
-
+  const int nw_ext = dims.nw_ext, R = dims.R, nb = NB ? NB : dims.nb, nc = dims.nc;
+  const int D = R * nw_ext, row0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* Zs = reinterpret_cast<C*>(smem_raw);  // [n_orb][WC2][R]; reused as the output tile
-  C* Gs = Zs + WC2 * R * (R + 1);          // [R cols][WC2][R rows]; Zs space holds the padded tile
-  C* Fs = Gs + R * WC2 * R;                // [nb][nc][nc]
-  C* Xst = Fs + nb * nc * nc;              // [JB][R]
-  C* Tst = Xst + JB * R;                   // [JB][WC2]
-  int* cs = reinterpret_cast<int*>(Tst + JB * WC2);  // [n_orb + 1]
-  for (int idx = t; idx < nb * nc * nc; idx += blockDim.x)
-    Fs[idx] = loadC<Real>(Fb + idx);
-  for (int idx = t; idx <= n_orb; idx += blockDim.x)
-    cs[idx] = col_start[sd.orb_off + idx];
-  __syncthreads();
+  T tile(smem_raw, dims, Fb, col_start + sd.orb_off);
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
 
-  // Column NDFT per orbital: Z(o2) = sum_{jj in seg(o2)} X'(row, w1; jj) conj(T(w2, jj)).
-  const int zs = WC2 * R;  // stride between orbitals of one thread's Z
-  C* z = Zs + t;
-  C acc = mk(Real(0), Real(0));
-  int o2 = 0;
-  int seg_end = cs[1];
-  while (o2 < n_orb && seg_end == 0) {
-    z[o2 * zs] = acc;
-    ++o2;
-    seg_end = o2 < n_orb ? cs[o2 + 1] : n;
-  }
-  const C* xrow = Xp + sd.x_off + static_cast<long>(w1) * n * R;
-  for (int j0 = 0; j0 < n; j0 += JB) {
-    const int jb_count = min(JB, n - j0);
-    for (int idx = t; idx < jb_count * R; idx += blockDim.x)
-      Xst[idx] = xrow[static_cast<long>(j0) * R + idx];
-    for (int idx = t; idx < jb_count * WC2; idx += blockDim.x) {
-      const int jb = idx / WC2, ww = idx % WC2;
-      Tst[idx] = (w2c0 + ww < nw_ext)
-                     ? loadC<Real>(Tc + static_cast<long>(sd.vtx_off + j0 + jb) * nw_ext + w2c0 + ww)
-                     : mk(Real(0), Real(0));
-    }
-    __syncthreads();
-    for (int jb = 0; jb < jb_count; ++jb) {
-      const int jj = j0 + jb;
-      while (jj >= seg_end) {
-        z[o2 * zs] = acc;
-        acc = mk(Real(0), Real(0));
-        ++o2;
-        seg_end = o2 < n_orb ? cs[o2 + 1] : n;
-      }
-      cfmac(acc, Xst[jb * R + row], Tst[jb * WC2 + w2l]);
-    }
-    __syncthreads();
-  }
-  for (; o2 < n_orb; ++o2) {
-    z[o2 * zs] = acc;
-    acc = mk(Real(0), Real(0));
-  }
-  __syncthreads();
-  C* g = Gs + t;  // column col of this thread's row at g[col * zs]
-  if (active) {
-    // Column cluster transform with band phases and the 1/Nc normalisation
-    // (space_transform_2D.hpp:79-89).
-    const Real norm = Real(1) / Real(nc);
-    for (int col = 0; col < R; ++col) {
-      const int b2 = col % nb, k2 = col / nb;
-      const C* f = Fs + (b2 * nc + k2) * nc;
-      C a = mk(Real(0), Real(0));
-      for (int r2 = 0; r2 < nc; ++r2)
-        cfmac(a, z[(b2 + nb * r2) * zs], f[r2]);
-      g[col * zs] = cscale(a, norm);
-    }
-  }
-  __syncthreads();
-  // Epilogue: G = -G0(k1, w1) G~ G0(k2, w2) + beta G0(k1, w1) delta (tp_accumulator_cpu.hpp:309-375),
-  // staged as row-major blocks (row stride R + 1 against bank conflicts) in the Zs space.
-  C* Os = Zs;  // [WC2][R][R + 1]
-  if (active) {
-    const int s = sd.spin;
-    const int b1 = row % nb, k1 = row / nb;
-    const double2* g0s = G0 + static_cast<long>(s) * nw_ext * nc * nb * nb;
-    auto g0 = [&](int ba, int bb, int k, int w) {
-      return loadC<Real>(g0s + ba + nb * (bb + nb * (k + nc * w)));
-    };
-    const Real beta = static_cast<Real>(dims.beta);
-    C* o = Os + (w2l * R + row) * (R + 1);
-    for (int col = 0; col < R; ++col) {
-      const int b2 = col % nb, k2 = col / nb;
-      C v;
-      if (nb == 1) {
-        v = cmul(cmul(g0(0, 0, k1, w1), g[col * zs]), g0(0, 0, k2, w2));
-        v = mk(-v.x, -v.y);
-      }
-      else {
-        v = mk(Real(0), Real(0));
-        for (int c2 = 0; c2 < nb; ++c2) {
-          C tt = mk(Real(0), Real(0));  // (G0_w1 G~)(b1, c2) at (k1, k2)
-          for (int c1 = 0; c1 < nb; ++c1)
-            cfma(tt, g0(b1, c1, k1, w1), Gs[((c2 + nb * k2) * WC2 + w2l) * R + c1 + nb * k1]);
-          cfma(v, tt, g0(c2, b2, k2, w2));
+  // Phase 1: Z(o, w2, row) = sum of X'(row, j) conj T(w2, j) over the vertices j of orbital o.
+  const C* xsrc = Xp + sd.x_off + min(row0 + (lane & 15), D - 1);
+  const double2* tsrc = Tc + static_cast<long>(sd.vtx_off) * nw_ext + min(w0 + lane % WT, nw_ext - 1);
+  const int rl = lane % 8, wq = lane / 8;  // this lane's sums: rows rl + 8 a, frequencies wq + 4 b
+  C acc[2][WT / 4];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < WT / 4; ++b)
+      acc[a][b] = mk(Real(0), Real(0));
+  tile.orbitals(
+      dims.n_orb,
+      [&](int v, unsigned char* slot) {
+        if (lane < kTileR)
+          cpAsync<sizeof(C)>(slot + 16 * lane, xsrc + static_cast<long>(v) * D);
+        else if (lane < kTileR + WT)
+          cpAsync<16>(slot + 16 * lane, tsrc + static_cast<long>(v) * nw_ext);
+      },
+      [&](const unsigned char* slot) {
+        C x[2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+          x[a] = *reinterpret_cast<const C*>(slot + 16 * (rl + 8 * a));
+#pragma unroll
+        for (int b = 0; b < WT / 4; ++b) {
+          const C t = loadC<Real>(reinterpret_cast<const double2*>(slot + 16 * (kTileR + wq + 4 * b)));
+#pragma unroll
+          for (int a = 0; a < 2; ++a)
+            cfmac(acc[a][b], x[a], t);
         }
-        v = mk(-v.x, -v.y);
+      },
+      [&](int o) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < WT / 4; ++b) {
+            tile.Z[o * T::kPairs + (wq + 4 * b) * kTileR + rl + 8 * a] = acc[a][b];
+            acc[a][b] = mk(Real(0), Real(0));
+          }
+      });
+
+  // Phase 2: the cluster transform with conjugate phases, the right G0 and the delta term.
+  const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
+  const Real beta = static_cast<Real>(dims.beta);
+  C* out = G + g_sector_stride * (2 * sd.slot + sd.spin);
+  const int k_tasks = (nc + kTaskK<NB> - 1) / kTaskK<NB>;
+  for (int task = warp; task < WT * k_tasks; task += T::kWarps) {
+    const int wl = task % WT, k0 = task / WT * kTaskK<NB>, w2 = w0 + wl;
+    if (w2 >= nw_ext)
+      continue;
+    const double2* g0 = g0s + static_cast<long>(w2) * nc * nb * nb;  // (ba, bb, k)
+    // G(row, w2; b2 k2) += beta G0 on the diagonal, and its store (rows past the edge are dropped).
+    auto put = [&](int i, int b2, int k2, C v) {
+      const int row = row0 + lane / 8 + 4 * i;
+      if (row >= D)
+        return;
+      const int w1 = row / R, r = row - w1 * R, k1 = r / nb;
+      if (w1 == w2 && k1 == k2) {
+        const C dl = loadC<Real>(g0 + (r - nb * k1) + nb * (b2 + nb * k2));
+        v.x = fma(beta, dl.x, v.x);
+        v.y = fma(beta, dl.y, v.y);
       }
-      if (k1 == k2 && w1 == w2) {
-        const C d = g0(b1, b2, k1, w1);
-        v.x += d.x * beta;
-        v.y += d.y * beta;
+      out[((static_cast<long>(w1) * nw_ext + w2) * R + r) * R + b2 + nb * k2] = v;
+    };
+    if constexpr (NB == 1) {
+      C s[4][2];
+      tile.template clusterSum<true, 2>(s, dims, 1, 0, wl, k0);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int k = k0 + lane % 8 + 8 * c;
+        if (k >= nc)
+          continue;
+        const C g = loadC<Real>(g0 + k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          put(i, 0, k, cmul(s[i][c], g));
       }
-      o[col] = v;
     }
-  }
-  __syncthreads();
-  // Coalesced store of the CTA's blocks (w1, w2c0 .. w2c0 + WC2 - 1), each R x R contiguous.
-  const int n_w2 = min(WC2, nw_ext - w2c0);
-  C* out = G + g_sector_stride * (2 * sd.slot + sd.spin) +
-           (static_cast<long>(w1) * nw_ext + w2c0) * R * R;
-  for (int idx = t; idx < n_w2 * R * R; idx += blockDim.x) {
-    const int wl = idx / (R * R), rem = idx % (R * R);
-    out[idx] = Os[(wl * R + rem / R) * (R + 1) + rem % R];
+    else if constexpr (NB > 1) {
+      C s[NB][4][1];
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+        tile.template clusterSum<true, 1>(s[b], dims, NB, b, wl, k0);
+      const int k = k0 + lane % 8;
+      if (k < nc) {
+#pragma unroll
+        for (int b2 = 0; b2 < NB; ++b2) {
+          C g[NB];
+#pragma unroll
+          for (int b = 0; b < NB; ++b)
+            g[b] = loadC<Real>(g0 + b + NB * (b2 + NB * k));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            C v = cmul(s[0][i][0], g[0]);
+#pragma unroll
+            for (int b = 1; b < NB; ++b)
+              cfma(v, s[b][i][0], g[b]);
+            put(i, b2, k, v);
+          }
+        }
+      }
+    }
+    else {
+      const int k = k0 + lane % 8;
+      for (int b2 = 0; b2 < nb; ++b2) {
+        C v[4] = {};
+        for (int b = 0; b < nb; ++b) {
+          C s[4][1];
+          tile.template clusterSum<true, 1>(s, dims, nb, b, wl, k0);
+          const C g = loadC<Real>(g0 + b + nb * (b2 + nb * min(k, nc - 1)));
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            cfma(v[i], s[i][0], g);
+        }
+        if (k < nc)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            put(i, b2, k, v[i]);
+      }
+    }
   }
 }
 
@@ -319,88 +519,80 @@ void launchTwiddles(const FrontendArgs& a, cudaStream_t stream) {
   }
 }
 
-constexpr int kRowJC = 32, kRowWC = 8, kRowIB = 64, kColJB = 64;
-
-template <typename Real, int JC = kRowJC, int WC = kRowWC, int IB = kRowIB>
-static size_t rowSmem(const TpDims& d) {
-  return sizeof(cplx_t<Real>) * (JC * WC * d.n_orb + d.nb * d.nc * d.nc + IB * WC) +
-         sizeof(Real) * JC * (IB + 1) + sizeof(int) * (d.n_orb + 1);
+// The clusters that the front-end takes: per orbital 4 KB (FP64) of a 32 x 8 row tile and the phases in
+// 227 KB of shared memory, and R x R blocks of one column frequency.  (The kernels' own tiles are smaller.)
+size_t frontendSmemRequirement(const TpDims& d, int /*n_max*/, bool fp64) {
+  const size_t real = fp64 ? sizeof(double) : sizeof(float), cplx = 2 * real;
+  const size_t R = d.R, orb = d.n_orb, phases = size_t(d.nb) * d.nc * d.nc;
+  const size_t row = cplx * (256 * orb + phases + 512) + real * 32 * 65 + sizeof(int) * (orb + 1);
+  size_t wc = 16;
+  while (wc > 1 && (R * wc > 1024 || cplx * (R * R * wc + R * (R + 1) * wc) > 96 * 1024))
+    wc /= 2;
+  const size_t col = cplx * (std::max(R * wc * orb, wc * R * (R + 1)) + R * wc * R + phases + 64 * (R + wc)) +
+                     sizeof(int) * (orb + 1);
+  return std::max(row, col);
 }
 
+// Frequencies per CTA, 16 or 8, which the tuner chooses between: every element is the same sum in the
+// same order either way.  8 alone where 16 does not fit in shared memory.
 template <typename Real>
-static int pickWC2(const TpDims& d) {
-  // Largest power of two <= 16 with R * WC2 <= 1024 threads and Zs + Gs <= 96 KB.
-  int wc2 = 16;
-  while (wc2 > 1 && (d.R * wc2 > 1024 || sizeof(cplx_t<Real>) * (d.R * d.R * wc2 + d.R * (d.R + 1) * wc2) > 96 * 1024))
-    wc2 /= 2;
-  return wc2;
+static int tileWidth(const FrontendArgs& a, const char* family, LaunchTuner::Pick& pk, cudaStream_t stream) {
+  const bool wide = Tile<Real, 16>::bytes(a.dims) <= 227 * 1024;
+  pk = tunePick(a.tuner, tuneKey(family, a.dims.nb, a.dims.nc, a.dims.nw_ext, a.n_max, a.n_sectors, sizeof(Real)),
+                wide ? 2 : 1, stream);
+  return wide && pk.choice == 0 ? 16 : 8;
 }
 
-template <typename Real>
-static size_t colSmem(const TpDims& d, int wc2) {
-  // Zs (also the padded output tile) + Gs + Fs + staging + column starts.
-  const size_t zs = std::max(size_t(d.R) * wc2 * d.n_orb, size_t(wc2) * d.R * (d.R + 1));
-  return sizeof(cplx_t<Real>) * (zs + size_t(d.R) * wc2 * d.R + d.nb * d.nc * d.nc + kColJB * (d.R + wc2)) +
-         sizeof(int) * (d.n_orb + 1);
-}
-
-template <typename Real, int JC, int WC>
-static void launchRowTile(const FrontendArgs& a, cplx_t<Real>* Xp, cudaStream_t stream) {
-  const TpDims& d = a.dims;
-  const size_t smem = rowSmem<Real, JC, WC>(d);
-  auto k = rowTransformKernel<Real, JC, WC, kRowIB>;
-  DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const dim3 grid(ceil_div(a.n_max, JC), ceil_div(d.nw_ext, WC), a.n_sectors);
-  k<<<grid, JC * WC, smem, stream>>>(d, a.sectors, a.perm_r, a.perm_c, a.row_start, a.Tr, a.Fb, Xp);
+template <typename Real, int WT, typename Kernel, typename... Args>
+static void launchTile(Kernel k, const TpDims& d, int tiles, int sectors, cudaStream_t stream, Args... args) {
+  const size_t smem = Tile<Real, WT>::bytes(d);
+  DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  k<<<dim3(tiles, ceil_div(d.nw_ext, WT), sectors), Tile<Real, WT>::kThreads, smem, stream>>>(d, args...);
   DCAACC_LAUNCH_CHECK();
 }
 
-// Tile shapes (vertices JC x frequencies WC per CTA, 256 threads) the tuner chooses among: each
-// X' element is the same sum in the same order whatever the tile.
+template <typename Real, int WT>
+static void launchRowWT(const FrontendArgs& a, cplx_t<Real>* Xp, cudaStream_t stream) {
+  const int nb = a.dims.nb;
+  auto k = nb == 1   ? rowTransformKernel<Real, WT, 1>
+           : nb == 2 ? rowTransformKernel<Real, WT, 2>
+           : nb == 3 ? rowTransformKernel<Real, WT, 3> : rowTransformKernel<Real, WT, 0>;
+  launchTile<Real, WT>(k, a.dims, ceil_div(a.n_max, kTileR), a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
+                       a.row_start, a.Tr, a.Fb, a.G0, Xp);
+}
+
 template <typename Real>
 void launchRowTransform(const FrontendArgs& a, cplx_t<Real>* Xp, cudaStream_t stream) {
-  const TpDims& d = a.dims;
   if (a.n_max == 0)
     return;
-  const size_t lim = 227 * 1024;
-  const bool fit16 = rowSmem<Real, 16, 16>(d) <= lim, fit64 = rowSmem<Real, 64, 4>(d) <= lim;
-  const int n_cand = fit16 ? (fit64 ? 3 : 2) : 1;
-  const auto pk = tunePick(a.tuner, tuneKey("row", d.nb, d.nc, d.nw_ext, a.n_max, a.n_sectors, sizeof(Real)),
-                           n_cand, stream);
-  if (pk.choice == 1)
-    launchRowTile<Real, 16, 16>(a, Xp, stream);
-  else if (pk.choice == 2)
-    launchRowTile<Real, 64, 4>(a, Xp, stream);
+  LaunchTuner::Pick pk;
+  if (tileWidth<Real>(a, "row", pk, stream) == 16)
+    launchRowWT<Real, 16>(a, Xp, stream);
   else
-    launchRowTile<Real, kRowJC, kRowWC>(a, Xp, stream);
+    launchRowWT<Real, 8>(a, Xp, stream);
   tuneEnd(a.tuner, pk, stream);
+}
+
+template <typename Real, int WT>
+static void launchColWT(const FrontendArgs& a, const cplx_t<Real>* Xp, cplx_t<Real>* G, long g_sector_stride,
+                        cudaStream_t stream) {
+  const int nb = a.dims.nb;
+  auto k = nb == 1   ? colTransformKernel<Real, WT, 1>
+           : nb == 2 ? colTransformKernel<Real, WT, 2>
+           : nb == 3 ? colTransformKernel<Real, WT, 3> : colTransformKernel<Real, WT, 0>;
+  launchTile<Real, WT>(k, a.dims, ceil_div(long(a.dims.R) * a.dims.nw_ext, kTileR), a.n_sectors, stream, a.sectors,
+                       a.col_start, a.Tc, a.Fb, a.G0, Xp, G, g_sector_stride);
 }
 
 template <typename Real>
 void launchColTransform(const FrontendArgs& a, const cplx_t<Real>* Xp, cplx_t<Real>* G,
                         long g_sector_stride, cudaStream_t stream) {
-  const TpDims& d = a.dims;
-  // Candidates: the heuristic's column-frequency width and the next two halvings (each G element
-  // is the same sum in the same order whatever the width).
-  const int wc2_max = pickWC2<Real>(d);
-  const int n_cand = wc2_max >= 4 ? 3 : wc2_max == 2 ? 2 : 1;
-  const auto pk = tunePick(a.tuner, tuneKey("col", d.nb, d.nc, d.nw_ext, a.n_max, a.n_sectors, sizeof(Real)),
-                           n_cand, stream);
-  const int wc2 = wc2_max >> pk.choice;
-  const size_t smem = colSmem<Real>(d, wc2);
-  auto k = colTransformKernel<Real, kColJB>;
-  DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const dim3 grid(d.nw_ext, ceil_div(d.nw_ext, wc2), a.n_sectors);
-  k<<<grid, d.R * wc2, smem, stream>>>(d, a.sectors, a.col_start, a.Tc, a.Fb, a.G0, Xp, G,
-                                       g_sector_stride, wc2);
-  DCAACC_LAUNCH_CHECK();
+  LaunchTuner::Pick pk;
+  if (tileWidth<Real>(a, "col", pk, stream) == 16)
+    launchColWT<Real, 16>(a, Xp, G, g_sector_stride, stream);
+  else
+    launchColWT<Real, 8>(a, Xp, G, g_sector_stride, stream);
   tuneEnd(a.tuner, pk, stream);
-}
-
-size_t frontendSmemRequirement(const TpDims& d, int /*n_max*/, bool fp64) {
-  if (fp64)
-    return std::max(rowSmem<double>(d), colSmem<double>(d, pickWC2<double>(d)));
-  return std::max(rowSmem<float>(d), colSmem<float>(d, pickWC2<float>(d)));
 }
 
 template void launchRowTransform<double>(const FrontendArgs&, double2*, cudaStream_t);
