@@ -272,50 +272,61 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     d.signs.alloc(max_batch_);
     d.M.alloc(n_sec * size_t(max_order_) * max_order_);
   }
-  Tr_d_.alloc(n_vtx * nw_ext);
-  if (non_density_)
-    Tc_d_.alloc(n_vtx * nw_ext);
   // Launch-shape tuning (launch_tuner.hpp), unless DCAACC_TUNE=0 keeps the built-in shapes.
   const char* tune_env = std::getenv("DCAACC_TUNE");
   tuner_.setEnabled(!(tune_env && std::strcmp(tune_env, "0") == 0));
   const size_t x_elems = n_sec * size_t(R) * max_order_ * nw_ext;
   const size_t g_elems = n_sec * size_t(g_sector_stride_);
   if (mixed_) {
-    // The mixed path runs its front-end and the disconnected terms of the one-band PH channels on
-    // the tensor cores, unless DCAACC_TP_SIMT_ONLY=1 selects the all-SIMT kernels (kept to compare
-    // both paths).
     const char* graphs_env = std::getenv("DCAACC_TP_GRAPHS");
     graphs_on_ = !(graphs_env && std::strcmp(graphs_env, "0") == 0);
+    // DCAACC_TP_SIMT_ONLY=1 selects the all-SIMT G4 kernels and the whole of G (kept to compare both paths).
     const char* simt_env = std::getenv("DCAACC_TP_SIMT_ONLY");
-    const bool simt_only = simt_env && std::strcmp(simt_env, "1") == 0;
+    simt_only_ = simt_env && std::strcmp(simt_env, "1") == 0;
     G32_.alloc(g_elems);
-    if (simt_only) {
-      X32_.alloc(x_elems);
+    // Front-end: factored by orbital in FP32 (tp_frontend32.cu) for one band on a 4x4 or 6x6 cluster, where the
+    // factoring saves 16 or 36 times the flops and the cluster transform is an FFT (a batch of 64, Nw = 64: 0.47
+    // against 0.66 ms; 6x6, Nw = 32, batch of 128: 4.0 against 8.7 ms); dense tensor-core products
+    // (tp_frontend_tc.cu) elsewhere (8 sites, one band, Nw = 24 + 2, batch of 32: 0.085 against 0.093 ms;
+    // three bands on 8 sites take 0.50 against 0.37 ms, but beside the FP32-bound pairing update of
+    // another batch the tensor cores' are the cheaper ones).  DCAACC_TP_FACTORED_COL selects the
+    // tensor-core front-end with one of its column steps: 0 the dense GEMM; 1 one band, 4x4 or
+    // 6x6 cluster: factored by orbital on mma.sync or the CUDA cores (DCAACC_TP_COL_FFT=0: with the
+    // matrix transform instead of the FFT); 2 one band, 4x4: factored with the sums in tensor memory.
+    const char* fact_env = std::getenv("DCAACC_TP_FACTORED_COL");
+    const char* fft_env = std::getenv("DCAACC_TP_COL_FFT");
+    if (fft_env && std::strcmp(fft_env, "0") == 0)
+      fft.on = 0;
+    const bool fact_off = fact_env && std::strcmp(fact_env, "0") == 0;
+    const bool fact_on = fact_env && std::strcmp(fact_env, "1") == 0;
+    const bool fact_tc = fact_env && std::strcmp(fact_env, "2") == 0;
+    front32_ = simt_only_ || (!fact_off && !fact_on && !fact_tc && fft.on && front32Applies(dims_, max_order_));
+    tc_front_ = !front32_;
+    if (front32_) {
+      const size_t Kr = (size_t(max_order_) + 63) / 64 * 64;
+      T2_d_.alloc((n_vtx + kFront32Pad) * nw_ext);
+      T4_d_.alloc((n_vtx + kFront32Pad) * nw_ext);
+      Ms_d_.alloc(n_sec * Kr * Kr);
+      X32_.alloc(x_elems + size_t(kFront32Pad) * R * nw_ext);
+      f32_.T2 = T2_d_.get();
+      f32_.T4 = T4_d_.get();
+      f32_.Ms = Ms_d_.get();
+      f32_.X = X32_.get();
+      f32_.Kr = int(Kr);
+      f32_.fft = fft;
     }
     else {
-      tc_front_ = true;
+      Tr_d_.alloc(n_vtx * nw_ext);
+      if (non_density_)
+        Tc_d_.alloc(n_vtx * nw_ext);
       const FrontTcShape fs = frontTcShape(dims_, int(n_sec), max_order_);
       ftc_mem_.alloc(frontTcBytes(fs));
       // Padding rows stay zero; ordered before the scale kernel frontTcInit launches on stream_.
       DCAACC_CUDA_CHECK(cudaMemsetAsync(ftc_mem_.get(), 0, ftc_mem_.bytes(), stream_));
       frontTcInit(ftc_, fs, ftc_mem_.get(), dims_, G0_.get(), stream_);
-      // One band on a 4 x 4 cluster: the column step runs factored by orbital (12x fewer flops than
-      // the dense GEMM) on tcgen05 with the per-site sums in tensor memory (tp_colfactor_tc.cu),
-      // which also spares the dense step's Q operand.  DCAACC_TP_FACTORED_COL=0 keeps the dense
-      // GEMM; =1 selects the other factored forms (mma.sync with the 4 x 4 FFT, or the CUDA cores
-      // with the 16 x 16 matrix transform, which DCAACC_TP_COL_FFT=0 forces), both slower.  One
-      // band on a 6 x 6 cluster: DCAACC_TP_FACTORED_COL=1 selects the factored form on the CUDA
-      // cores with the 6 x 6 FFT (24x fewer flops than the dense GEMM, yet slower on B200: 57 ms
-      // against 39 ms per batch of 128 at Nw = 128).
-      const char* fact_env = std::getenv("DCAACC_TP_FACTORED_COL");
-      const char* fft_env = std::getenv("DCAACC_TP_COL_FFT");
       ftc_.fft = fft;
-      if (fft_env && std::strcmp(fft_env, "0") == 0)
-        ftc_.fft.on = 0;
-      const bool fact_off = fact_env && std::strcmp(fact_env, "0") == 0;
-      const bool fact_on = fact_env && std::strcmp(fact_env, "1") == 0;
       const int row0 = dims_.half_g ? fs.D / 2 : 0;
-      ftc_.col_tc = !fact_off && !fact_on && colFactorApplies(dims_) && ftc_.fft.on &&
+      ftc_.col_tc = fact_tc && colFactorApplies(dims_) && ftc_.fft.on &&
                     colFactorTcApplies(dims_, fs.D, row0, max_order_);
       const bool wide = colFactorWideApplies(dims_) && ftc_.fft.on && ftc_.fft.L == 6 && fact_on;
       ftc_.factored_col = (colFactorApplies(dims_) && (fact_on || ftc_.col_tc)) || wide;
@@ -328,6 +339,9 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
         if (non_density_)
           d.orb_c.alloc(n_vtx);
       }
+    }
+    if (!simt_only_) {
+      // The disconnected terms of the one-band PH channels run on the tensor cores.
       gmax_d_.alloc(2 * size_t(max_batch_));
       if (discGemmApplies(dims_, max_batch_)) {
         disc_.alloc(discScratchBytes(dims_, max_batch_));
@@ -398,6 +412,9 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     }
   }
   else {
+    Tr_d_.alloc(n_vtx * nw_ext);
+    if (non_density_)
+      Tc_d_.alloc(n_vtx * nw_ext);
     X64_.alloc(x_elems);
     G64_.alloc(g_elems);
   }
@@ -416,7 +433,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   for (auto& d : dstage_)
     DCAACC_CUDA_CHECK(cudaEventRecord(d.consumed, stream_));
 
-  if (!tc_front_ && frontendSmemRequirement(dims_, max_order_, !mixed_) > 227 * 1024)
+  if ((!mixed_ || simt_only_) && frontendSmemRequirement(dims_, max_order_, !mixed_) > 227 * 1024)
     invalid("max_order too large for the front-end's shared-memory tiles");
   G4_host_.assign(c.n_channels, {});
 }
@@ -741,10 +758,10 @@ void TpAccumulator::process() {
   fa.Fb = Fb_.get();
   fa.G0 = G0_.get();
   fa.tuner = &tuner_;
-  // Tensor-core path: the launch shapes take the order bound in steps of 128 (the GEMM tile);
-  // every kernel reads each sector's own order, so the results do not depend on it, and batches
-  // of similar orders share one captured graph.
-  if (tc_front_ && n_max_batch_ > 0)
+  // Mixed path: the launch shapes take the order bound in steps of 128; every kernel reads each
+  // sector's own order, so the results do not depend on it, and batches of similar orders share one
+  // captured graph.
+  if (mixed_ && n_max_batch_ > 0)
     fa.n_max = (n_max_batch_ + 127) / 128 * 128;
   G4Args ga{};
   ga.dims = dims_;
@@ -765,14 +782,14 @@ void TpAccumulator::process() {
     ga.q_all = distinct == dims_.nc && int(q_list_.size()) == dims_.nc;
   }
   ga.disc = have_disc_ ? &disc_ws_ : nullptr;
-  ga.gmax = tc_front_ ? gmax_d_.get() : nullptr;
+  ga.gmax = gmax_d_.get();  // null in FP64 and all-SIMT runs
   ga.tile_order = dims_.half_g4 ? tile_order_d_.get() : nullptr;
   ga.n_sm = n_sm_;
   ga.tuner = &tuner_;
   ga.wait_limit = wait_limit_;
   ga.fault_stop_step = fault_stop_step_;
 
-  const bool graphable = graphs_on_ && tc_front_ && !timing_ && n_max_batch_ > 0 && stream_ != nullptr &&
+  const bool graphable = graphs_on_ && mixed_ && !simt_only_ && !timing_ && n_max_batch_ > 0 && stream_ != nullptr &&
                          stream_ != cudaStreamLegacy && stream_ != cudaStreamPerThread;
   if (graphable)
     launches_ += launchBatchGraph(set, fa, ga, ds);
@@ -804,7 +821,10 @@ int TpAccumulator::launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStag
       launched += 1;
     }
     int n_prep;
-    if (tc_front_) {
+    if (front32_) {
+      n_prep = launchFront32Prep(fa, f32_, stream_);
+    }
+    else if (tc_front_) {
       n_prep = launchFrontendTcPrep(fa, ftc_, ds.orb_r.get(), non_density_ ? ds.orb_c.get() : ds.orb_r.get(),
                                     stream_);
     }
@@ -818,19 +838,19 @@ int TpAccumulator::launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStag
   timeBegin(DCAACC_STAGE_ROW, &b);
   if (tc_front_)
     launchFrontendTcRow(fa, ftc_, err_d_.get(), stream_);
-  else if (mixed_)
-    launchRowTransform<float>(fa, X32_.get(), stream_);
+  else if (front32_)
+    launchFront32Row(fa, f32_, stream_);
   else
-    launchRowTransform<double>(fa, X64_.get(), stream_);
+    launchRowTransform(fa, X64_.get(), stream_);
   timeEnd(DCAACC_STAGE_ROW, b, 1);
   timeBegin(DCAACC_STAGE_COL, &b);
   int col_launches = 1;
   if (tc_front_)
     col_launches = launchFrontendTcCol(fa, ftc_, G32_.get(), g_sector_stride_, gmax_d_.get(), err_d_.get(), stream_);
-  else if (mixed_)
-    launchColTransform<float>(fa, X32_.get(), G32_.get(), g_sector_stride_, stream_);
+  else if (front32_)
+    launchFront32Col(fa, f32_, G32_.get(), g_sector_stride_, gmax_d_.get(), stream_);
   else
-    launchColTransform<double>(fa, X64_.get(), G64_.get(), g_sector_stride_, stream_);
+    launchColTransform(fa, X64_.get(), G64_.get(), g_sector_stride_, stream_);
   timeEnd(DCAACC_STAGE_COL, b, col_launches);
   timeBegin(DCAACC_STAGE_G4, &b);
   const int g4_launches = mixed_ ? launchUpdateG4<float2>(ga, G32_.get(), g_sector_stride_, stream_)
@@ -1167,7 +1187,7 @@ void TpAccumulator::synchronize() {
 size_t TpAccumulator::deviceFingerprint() const {
   size_t b = G0_.bytes() + Fb_.bytes() + k_add_d_.bytes() + k_sub_d_.bytes() + q_d_.bytes() +
              wex_d_.bytes() + G4_ptrs_.bytes() + Tr_d_.bytes() + Tc_d_.bytes() + X64_.bytes() +
-             G64_.bytes() + X32_.bytes() + G32_.bytes() + err_d_.bytes();
+             G64_.bytes() + X32_.bytes() + G32_.bytes() + err_d_.bytes() + T2_d_.bytes() + T4_d_.bytes() + Ms_d_.bytes();
   for (const auto& g : g4())  // a shared G4 is counted by every handle that shares it
     b += g.bytes();
   for (const auto& d : dstage_)

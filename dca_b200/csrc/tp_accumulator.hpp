@@ -226,9 +226,13 @@ private:
   DevBuf<unsigned char> disc_;  // mixed mode, one band: tensor-core disconnected-term workspace
   DiscWorkspace disc_ws_{};
   bool have_disc_ = false;
-  // Mixed mode: tensor-core front-end (operand planes + TMA descriptors) and the orbital of each
-  // vertex in row / column order.
-  bool tc_front_ = false;
+  // Mixed mode: the FP32 front-end's twiddles and sorted M, or the tensor-core front-end's operand
+  // planes and TMA descriptors (with the orbital of each vertex in row / column order).
+  bool front32_ = false, tc_front_ = false, simt_only_ = false;
+  DevBuf<float2> T2_d_;
+  DevBuf<float4> T4_d_;
+  DevBuf<float> Ms_d_;
+  Front32Workspace f32_{};
   DevBuf<unsigned char> ftc_mem_;
   DevBuf<unsigned char> col_tp_;  // factored column step, FFT form: FP16 planes of the column twiddles
   FrontTcWorkspace ftc_{};

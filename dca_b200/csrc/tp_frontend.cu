@@ -17,8 +17,7 @@
 // over that orbital's vertices only, as the reference's per-orbital-pair products do) and both are
 // the same two small products per CTA: the sums of a 16 x WT tile for every orbital (phase 1), then
 // the cluster transform of those sums from shared memory (phase 2), so M, X' and G each cross
-// global memory once per tile column.  Templated on the working precision: double for the FP64
-// path, float for the FP32 SIMT variant of the mixed path.
+// global memory once per tile column.
 //
 // Phase 1: the orbitals are handed to the warps one by one (a shared counter).  A warp holds the
 // whole 16 x WT tile, 2 x WT/4 sums a lane, and streams its orbital's vertices through a ring of
@@ -68,12 +67,6 @@ __global__ void twiddleKernel(const SectorDesc* __restrict__ sectors,
   }
 }
 
-template <typename Real>
-__device__ inline cplx_t<Real> loadC(const double2* p) {
-  const double2 v = *p;
-  return mk(static_cast<Real>(v.x), static_cast<Real>(v.y));
-}
-
 constexpr int kTileR = 16;  // rows of G (column step) or columns of M (row step) of a CTA's tile
 constexpr int kRing = 8;    // vertices in flight per warp
 
@@ -95,15 +88,14 @@ __device__ inline void cpAsyncWait() {
 // Shared memory of a tile kernel: the orbitals' sums Z[o][w][16], the warps' rings (16 bytes per
 // lane and slot), the phases F[b][r][k] (k padded with zeros), the orbital starts and the
 // counter that hands them out.
-template <typename Real, int WT>
+template <int WT>
 struct Tile {
-  using C = cplx_t<Real>;
   static constexpr int kPairs = kTileR * WT;
   static constexpr int kThreads = kPairs;
   static constexpr int kWarps = kThreads / 32;
   static_assert(kTileR + WT <= 32, "one copy per lane and vertex");
   unsigned char* ring;
-  C *Z, *F;
+  double2 *Z, *F;
   int *start, *next;
 
   // Phase 2 reads whole groups of momenta: 16 of one band, 8 otherwise.
@@ -111,21 +103,21 @@ struct Tile {
     return d.nb == 1 ? (d.nc + 15) / 16 * 16 : (d.nc + 7) / 8 * 8;
   }
   __host__ __device__ static size_t bytes(const TpDims& d) {
-    return size_t(kWarps) * kRing * 512 + sizeof(C) * (size_t(d.n_orb) * kPairs + size_t(d.nb) * d.nc * kPad(d)) +
+    return size_t(kWarps) * kRing * 512 + sizeof(double2) * (size_t(d.n_orb) * kPairs + size_t(d.nb) * d.nc * kPad(d)) +
            sizeof(int) * (d.n_orb + 2);
   }
   // Lays the memory out and fills the phases, the starts and the counter.
   __device__ Tile(unsigned char* raw, const TpDims& d, const double2* __restrict__ Fb,
                   const int* __restrict__ orb_start) {
     ring = raw;
-    Z = reinterpret_cast<C*>(raw + kWarps * kRing * 512);
+    Z = reinterpret_cast<double2*>(raw + kWarps * kRing * 512);
     F = Z + d.n_orb * kPairs;
     start = reinterpret_cast<int*>(F + d.nb * d.nc * kPad(d));
     next = start + d.n_orb + 1;
     const int kp = kPad(d);
     for (int i = threadIdx.x; i < d.nb * d.nc * kp; i += kThreads) {
       const int k = i % kp, r = (i / kp) % d.nc, b = i / (kp * d.nc);
-      F[i] = k < d.nc ? loadC<Real>(Fb + (b * d.nc + k) * d.nc + r) : mk(Real(0), Real(0));
+      F[i] = k < d.nc ? Fb[(b * d.nc + k) * d.nc + r] : mk(double(0), double(0));
     }
     for (int i = threadIdx.x; i <= d.n_orb; i += kThreads)
       start[i] = orb_start[i];
@@ -174,18 +166,18 @@ struct Tile {
   // Phase 2 of one line of the tile (16 rows of frequency wl) and band b: acc[i][c] = sum_r
   // Z(b, r; wl, tr + 4 i) F(b, k0 + kl + 8 c; r), F conjugated when CONJ (tr = lane / 8, kl = lane % 8).
   template <bool CONJ, int KC>
-  __device__ void clusterSum(C (&acc)[4][KC], const TpDims& d, int nb, int b, int wl, int k0) const {
+  __device__ void clusterSum(double2 (&acc)[4][KC], const TpDims& d, int nb, int b, int wl, int k0) const {
     const int lane = threadIdx.x % 32, kp = kPad(d);
-    const C* z = Z + b * kPairs + wl * kTileR + lane / 8;
-    const C* f = F + b * d.nc * kp + k0 + lane % 8;
+    const double2* z = Z + b * kPairs + wl * kTileR + lane / 8;
+    const double2* f = F + b * d.nc * kp + k0 + lane % 8;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int c = 0; c < KC; ++c)
-        acc[i][c] = mk(Real(0), Real(0));
+        acc[i][c] = mk(double(0), double(0));
 #pragma unroll 2
     for (int r = 0; r < d.nc; ++r, z += nb * kPairs, f += kp) {
-      C zv[4], fv[KC];
+      double2 zv[4], fv[KC];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         zv[i] = z[4 * i];
@@ -211,16 +203,15 @@ constexpr int kTaskK = NB == 1 ? 16 : 8;
 
 // Row transform.  grid (ceil(n_max / 16), ceil(NwExt / WT), n_sectors).  NB: bands (1, 2 or 3), 0 for
 // any number.
-template <typename Real, int WT, int NB>
+template <int WT, int NB>
 __global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
 rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const int* __restrict__ perm_r, const int* __restrict__ perm_c,
                    const int* __restrict__ row_start, const double2* __restrict__ Tr,
                    const double2* __restrict__ Fb,  // (r, k, b): e^{i k (r + a_b)}
                    const double2* __restrict__ G0,  // (b1, b2, k, w, s)
-                   cplx_t<Real>* __restrict__ Xp) {
-  using C = cplx_t<Real>;
-  using T = Tile<Real, WT>;
+                   double2* __restrict__ Xp) {
+  using T = Tile<WT>;
   const SectorDesc sd = sectors[blockIdx.z];
   const int n = sd.n, j0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
   if (j0 >= n)
@@ -237,12 +228,12 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   const double2* tsrc = Tr + static_cast<long>(sd.vtx_off) * nw_ext + min(w0 + lane % WT, nw_ext - 1);
   const int jl = lane % 8, wq = lane / 8;  // this lane's sums: columns jl + 8 a, frequencies wq + 4 b
   const bool f32 = sd.m_f32 != 0;
-  C acc[2][WT / 4];
+  double2 acc[2][WT / 4];
 #pragma unroll
   for (int a = 0; a < 2; ++a)
 #pragma unroll
     for (int b = 0; b < WT / 4; ++b)
-      acc[a][b] = mk(Real(0), Real(0));
+      acc[a][b] = mk(double(0), double(0));
   tile.orbitals(
       dims.n_orb,
       [&](int v, unsigned char* slot) {
@@ -258,16 +249,16 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
         }
       },
       [&](const unsigned char* slot) {
-        Real m[2];
+        double m[2];
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
           const unsigned char* e = slot + 16 * (jl + 8 * a);
-          m[a] = f32 ? static_cast<Real>(*reinterpret_cast<const float*>(e))
-                     : static_cast<Real>(*reinterpret_cast<const double*>(e));
+          m[a] = f32 ? static_cast<double>(*reinterpret_cast<const float*>(e))
+                     : *reinterpret_cast<const double*>(e);
         }
 #pragma unroll
         for (int b = 0; b < WT / 4; ++b) {
-          const C t = loadC<Real>(reinterpret_cast<const double2*>(slot + 16 * (kTileR + wq + 4 * b)));
+          const double2 t = *reinterpret_cast<const double2*>(slot + 16 * (kTileR + wq + 4 * b));
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
             acc[a][b].x = fma(t.x, m[a], acc[a][b].x);
@@ -281,7 +272,7 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
 #pragma unroll
           for (int b = 0; b < WT / 4; ++b) {
             tile.Z[o * T::kPairs + (wq + 4 * b) * kTileR + jl + 8 * a] = acc[a][b];
-            acc[a][b] = mk(Real(0), Real(0));
+            acc[a][b] = mk(double(0), double(0));
           }
       });
 
@@ -295,13 +286,13 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
     if (w >= nw_ext)
       continue;
     const double2* g0 = g0s + static_cast<long>(w) * nc * nb * nb;  // (ba, bb, k)
-    auto put = [&](int i, int b1, int k, C v) {
+    auto put = [&](int i, int b1, int k, double2 v) {
       const int j = j0 + lane / 8 + 4 * i;
       if (j < n)
         Xp[sd.x_off + j * D + static_cast<long>(w) * R + b1 + nb * k] = v;
     };
     if constexpr (NB == 1) {
-      C s[4][2];
+      double2 s[4][2];
       tile.template clusterSum<false, 2>(s, dims, 1, 0, wl, k0);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -309,14 +300,14 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
         if (k >= nc)
           continue;
         const double2 g = g0[k];
-        const C gn = mk(static_cast<Real>(norm * g.x), static_cast<Real>(norm * g.y));
+        const double2 gn = mk(norm * g.x, norm * g.y);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           put(i, 0, k, cmul(gn, s[i][c]));
       }
     }
     else if constexpr (NB > 1) {
-      C s[NB][4][1];
+      double2 s[NB][4][1];
 #pragma unroll
       for (int b = 0; b < NB; ++b)
         tile.template clusterSum<false, 1>(s[b], dims, NB, b, wl, k0);
@@ -324,15 +315,15 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
       if (k < nc) {
 #pragma unroll
         for (int b1 = 0; b1 < NB; ++b1) {
-          C gn[NB];
+          double2 gn[NB];
 #pragma unroll
           for (int b = 0; b < NB; ++b) {
             const double2 g = g0[b1 + NB * (b + NB * k)];
-            gn[b] = mk(static_cast<Real>(norm * g.x), static_cast<Real>(norm * g.y));
+            gn[b] = mk(norm * g.x, norm * g.y);
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            C v = cmul(gn[0], s[0][i][0]);
+            double2 v = cmul(gn[0], s[0][i][0]);
 #pragma unroll
             for (int b = 1; b < NB; ++b)
               cfma(v, gn[b], s[b][i][0]);
@@ -344,12 +335,12 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
     else {
       const int k = k0 + lane % 8;
       for (int b1 = 0; b1 < nb; ++b1) {
-        C v[4] = {};
+        double2 v[4] = {};
         for (int b = 0; b < nb; ++b) {
-          C s[4][1];
+          double2 s[4][1];
           tile.template clusterSum<false, 1>(s, dims, nb, b, wl, k0);
           const double2 g = g0[b1 + nb * (b + nb * min(k, nc - 1))];
-          const C gn = mk(static_cast<Real>(norm * g.x), static_cast<Real>(norm * g.y));
+          const double2 gn = mk(norm * g.x, norm * g.y);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             cfma(v[i], gn, s[i][0]);
@@ -365,15 +356,14 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
 
 // Column transform + G epilogue.  grid (ceil(D / 16), ceil(NwExt / WT), n_sectors); the rows of a tile
 // are 16 consecutive (w1, r).
-template <typename Real, int WT, int NB>
+template <int WT, int NB>
 __global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
 colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const int* __restrict__ col_start, const double2* __restrict__ Tc,
                    const double2* __restrict__ Fb,
                    const double2* __restrict__ G0,  // (b1, b2, k, w, s)
-                   const cplx_t<Real>* __restrict__ Xp, cplx_t<Real>* __restrict__ G, long g_sector_stride) {
-  using C = cplx_t<Real>;
-  using T = Tile<Real, WT>;
+                   const double2* __restrict__ Xp, double2* __restrict__ G, long g_sector_stride) {
+  using T = Tile<WT>;
   const SectorDesc sd = sectors[blockIdx.z];
   const int nw_ext = dims.nw_ext, R = dims.R, nb = NB ? NB : dims.nb, nc = dims.nc;
   const int D = R * nw_ext, row0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
@@ -382,31 +372,31 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
 
   // Phase 1: Z(o, w2, row) = sum of X'(row, j) conj T(w2, j) over the vertices j of orbital o.
-  const C* xsrc = Xp + sd.x_off + min(row0 + (lane & 15), D - 1);
+  const double2* xsrc = Xp + sd.x_off + min(row0 + (lane & 15), D - 1);
   const double2* tsrc = Tc + static_cast<long>(sd.vtx_off) * nw_ext + min(w0 + lane % WT, nw_ext - 1);
   const int rl = lane % 8, wq = lane / 8;  // this lane's sums: rows rl + 8 a, frequencies wq + 4 b
-  C acc[2][WT / 4];
+  double2 acc[2][WT / 4];
 #pragma unroll
   for (int a = 0; a < 2; ++a)
 #pragma unroll
     for (int b = 0; b < WT / 4; ++b)
-      acc[a][b] = mk(Real(0), Real(0));
+      acc[a][b] = mk(double(0), double(0));
   tile.orbitals(
       dims.n_orb,
       [&](int v, unsigned char* slot) {
         if (lane < kTileR)
-          cpAsync<sizeof(C)>(slot + 16 * lane, xsrc + static_cast<long>(v) * D);
+          cpAsync<sizeof(double2)>(slot + 16 * lane, xsrc + static_cast<long>(v) * D);
         else if (lane < kTileR + WT)
           cpAsync<16>(slot + 16 * lane, tsrc + static_cast<long>(v) * nw_ext);
       },
       [&](const unsigned char* slot) {
-        C x[2];
+        double2 x[2];
 #pragma unroll
         for (int a = 0; a < 2; ++a)
-          x[a] = *reinterpret_cast<const C*>(slot + 16 * (rl + 8 * a));
+          x[a] = *reinterpret_cast<const double2*>(slot + 16 * (rl + 8 * a));
 #pragma unroll
         for (int b = 0; b < WT / 4; ++b) {
-          const C t = loadC<Real>(reinterpret_cast<const double2*>(slot + 16 * (kTileR + wq + 4 * b)));
+          const double2 t = *reinterpret_cast<const double2*>(slot + 16 * (kTileR + wq + 4 * b));
 #pragma unroll
           for (int a = 0; a < 2; ++a)
             cfmac(acc[a][b], x[a], t);
@@ -418,14 +408,14 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
 #pragma unroll
           for (int b = 0; b < WT / 4; ++b) {
             tile.Z[o * T::kPairs + (wq + 4 * b) * kTileR + rl + 8 * a] = acc[a][b];
-            acc[a][b] = mk(Real(0), Real(0));
+            acc[a][b] = mk(double(0), double(0));
           }
       });
 
   // Phase 2: the cluster transform with conjugate phases, the right G0 and the delta term.
   const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
-  const Real beta = static_cast<Real>(dims.beta);
-  C* out = G + g_sector_stride * (2 * sd.slot + sd.spin);
+  const double beta = dims.beta;
+  double2* out = G + g_sector_stride * (2 * sd.slot + sd.spin);
   const int k_tasks = (nc + kTaskK<NB> - 1) / kTaskK<NB>;
   for (int task = warp; task < WT * k_tasks; task += T::kWarps) {
     const int wl = task % WT, k0 = task / WT * kTaskK<NB>, w2 = w0 + wl;
@@ -433,34 +423,34 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
       continue;
     const double2* g0 = g0s + static_cast<long>(w2) * nc * nb * nb;  // (ba, bb, k)
     // G(row, w2; b2 k2) += beta G0 on the diagonal, and its store (rows past the edge are dropped).
-    auto put = [&](int i, int b2, int k2, C v) {
+    auto put = [&](int i, int b2, int k2, double2 v) {
       const int row = row0 + lane / 8 + 4 * i;
       if (row >= D)
         return;
       const int w1 = row / R, r = row - w1 * R, k1 = r / nb;
       if (w1 == w2 && k1 == k2) {
-        const C dl = loadC<Real>(g0 + (r - nb * k1) + nb * (b2 + nb * k2));
+        const double2 dl = g0[(r - nb * k1) + nb * (b2 + nb * k2)];
         v.x = fma(beta, dl.x, v.x);
         v.y = fma(beta, dl.y, v.y);
       }
       out[((static_cast<long>(w1) * nw_ext + w2) * R + r) * R + b2 + nb * k2] = v;
     };
     if constexpr (NB == 1) {
-      C s[4][2];
+      double2 s[4][2];
       tile.template clusterSum<true, 2>(s, dims, 1, 0, wl, k0);
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int k = k0 + lane % 8 + 8 * c;
         if (k >= nc)
           continue;
-        const C g = loadC<Real>(g0 + k);
+        const double2 g = g0[k];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
           put(i, 0, k, cmul(s[i][c], g));
       }
     }
     else if constexpr (NB > 1) {
-      C s[NB][4][1];
+      double2 s[NB][4][1];
 #pragma unroll
       for (int b = 0; b < NB; ++b)
         tile.template clusterSum<true, 1>(s[b], dims, NB, b, wl, k0);
@@ -468,13 +458,13 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
       if (k < nc) {
 #pragma unroll
         for (int b2 = 0; b2 < NB; ++b2) {
-          C g[NB];
+          double2 g[NB];
 #pragma unroll
           for (int b = 0; b < NB; ++b)
-            g[b] = loadC<Real>(g0 + b + NB * (b2 + NB * k));
+            g[b] = g0[b + NB * (b2 + NB * k)];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            C v = cmul(s[0][i][0], g[0]);
+            double2 v = cmul(s[0][i][0], g[0]);
 #pragma unroll
             for (int b = 1; b < NB; ++b)
               cfma(v, s[b][i][0], g[b]);
@@ -486,11 +476,11 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
     else {
       const int k = k0 + lane % 8;
       for (int b2 = 0; b2 < nb; ++b2) {
-        C v[4] = {};
+        double2 v[4] = {};
         for (int b = 0; b < nb; ++b) {
-          C s[4][1];
+          double2 s[4][1];
           tile.template clusterSum<true, 1>(s, dims, nb, b, wl, k0);
-          const C g = loadC<Real>(g0 + b + nb * (b2 + nb * min(k, nc - 1)));
+          const double2 g = g0[b + nb * (b2 + nb * min(k, nc - 1))];
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             cfma(v[i], s[i][0], g);
@@ -535,69 +525,63 @@ size_t frontendSmemRequirement(const TpDims& d, int /*n_max*/, bool fp64) {
 
 // Frequencies per CTA, 16 or 8, which the tuner chooses between: every element is the same sum in the
 // same order either way.  8 alone where 16 does not fit in shared memory.
-template <typename Real>
 static int tileWidth(const FrontendArgs& a, const char* family, LaunchTuner::Pick& pk, cudaStream_t stream) {
-  const bool wide = Tile<Real, 16>::bytes(a.dims) <= 227 * 1024;
-  pk = tunePick(a.tuner, tuneKey(family, a.dims.nb, a.dims.nc, a.dims.nw_ext, a.n_max, a.n_sectors, sizeof(Real)),
+  const bool wide = Tile<16>::bytes(a.dims) <= 227 * 1024;
+  pk = tunePick(a.tuner, tuneKey(family, a.dims.nb, a.dims.nc, a.dims.nw_ext, a.n_max, a.n_sectors, 8),
                 wide ? 2 : 1, stream);
   return wide && pk.choice == 0 ? 16 : 8;
 }
 
-template <typename Real, int WT, typename Kernel, typename... Args>
+template <int WT, typename Kernel, typename... Args>
 static void launchTile(Kernel k, const TpDims& d, int tiles, int sectors, cudaStream_t stream, Args... args) {
-  const size_t smem = Tile<Real, WT>::bytes(d);
+  const size_t smem = Tile<WT>::bytes(d);
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  k<<<dim3(tiles, ceil_div(d.nw_ext, WT), sectors), Tile<Real, WT>::kThreads, smem, stream>>>(d, args...);
+  DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         int(cudaSharedmemCarveoutMaxShared)));
+  k<<<dim3(tiles, ceil_div(d.nw_ext, WT), sectors), Tile<WT>::kThreads, smem, stream>>>(d, args...);
   DCAACC_LAUNCH_CHECK();
 }
 
-template <typename Real, int WT>
-static void launchRowWT(const FrontendArgs& a, cplx_t<Real>* Xp, cudaStream_t stream) {
+template <int WT>
+static void launchRowWT(const FrontendArgs& a, double2* Xp, cudaStream_t stream) {
   const int nb = a.dims.nb;
-  auto k = nb == 1   ? rowTransformKernel<Real, WT, 1>
-           : nb == 2 ? rowTransformKernel<Real, WT, 2>
-           : nb == 3 ? rowTransformKernel<Real, WT, 3> : rowTransformKernel<Real, WT, 0>;
-  launchTile<Real, WT>(k, a.dims, ceil_div(a.n_max, kTileR), a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
+  auto k = nb == 1   ? rowTransformKernel<WT, 1>
+           : nb == 2 ? rowTransformKernel<WT, 2>
+           : nb == 3 ? rowTransformKernel<WT, 3> : rowTransformKernel<WT, 0>;
+  launchTile<WT>(k, a.dims, ceil_div(a.n_max, kTileR), a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
                        a.row_start, a.Tr, a.Fb, a.G0, Xp);
 }
 
-template <typename Real>
-void launchRowTransform(const FrontendArgs& a, cplx_t<Real>* Xp, cudaStream_t stream) {
+void launchRowTransform(const FrontendArgs& a, double2* Xp, cudaStream_t stream) {
   if (a.n_max == 0)
     return;
   LaunchTuner::Pick pk;
-  if (tileWidth<Real>(a, "row", pk, stream) == 16)
-    launchRowWT<Real, 16>(a, Xp, stream);
+  if (tileWidth(a, "row", pk, stream) == 16)
+    launchRowWT<16>(a, Xp, stream);
   else
-    launchRowWT<Real, 8>(a, Xp, stream);
+    launchRowWT<8>(a, Xp, stream);
   tuneEnd(a.tuner, pk, stream);
 }
 
-template <typename Real, int WT>
-static void launchColWT(const FrontendArgs& a, const cplx_t<Real>* Xp, cplx_t<Real>* G, long g_sector_stride,
+template <int WT>
+static void launchColWT(const FrontendArgs& a, const double2* Xp, double2* G, long g_sector_stride,
                         cudaStream_t stream) {
   const int nb = a.dims.nb;
-  auto k = nb == 1   ? colTransformKernel<Real, WT, 1>
-           : nb == 2 ? colTransformKernel<Real, WT, 2>
-           : nb == 3 ? colTransformKernel<Real, WT, 3> : colTransformKernel<Real, WT, 0>;
-  launchTile<Real, WT>(k, a.dims, ceil_div(long(a.dims.R) * a.dims.nw_ext, kTileR), a.n_sectors, stream, a.sectors,
+  auto k = nb == 1   ? colTransformKernel<WT, 1>
+           : nb == 2 ? colTransformKernel<WT, 2>
+           : nb == 3 ? colTransformKernel<WT, 3> : colTransformKernel<WT, 0>;
+  launchTile<WT>(k, a.dims, ceil_div(long(a.dims.R) * a.dims.nw_ext, kTileR), a.n_sectors, stream, a.sectors,
                        a.col_start, a.Tc, a.Fb, a.G0, Xp, G, g_sector_stride);
 }
 
-template <typename Real>
-void launchColTransform(const FrontendArgs& a, const cplx_t<Real>* Xp, cplx_t<Real>* G,
+void launchColTransform(const FrontendArgs& a, const double2* Xp, double2* G,
                         long g_sector_stride, cudaStream_t stream) {
   LaunchTuner::Pick pk;
-  if (tileWidth<Real>(a, "col", pk, stream) == 16)
-    launchColWT<Real, 16>(a, Xp, G, g_sector_stride, stream);
+  if (tileWidth(a, "col", pk, stream) == 16)
+    launchColWT<16>(a, Xp, G, g_sector_stride, stream);
   else
-    launchColWT<Real, 8>(a, Xp, G, g_sector_stride, stream);
+    launchColWT<8>(a, Xp, G, g_sector_stride, stream);
   tuneEnd(a.tuner, pk, stream);
 }
-
-template void launchRowTransform<double>(const FrontendArgs&, double2*, cudaStream_t);
-template void launchRowTransform<float>(const FrontendArgs&, float2*, cudaStream_t);
-template void launchColTransform<double>(const FrontendArgs&, const double2*, double2*, long, cudaStream_t);
-template void launchColTransform<float>(const FrontendArgs&, const float2*, float2*, long, cudaStream_t);
 
 }  // namespace dcaacc

@@ -29,15 +29,13 @@ struct FrontendArgs {
 
 void launchTwiddles(const FrontendArgs& a, cudaStream_t stream);
 
-// Row transform: M -> X' for every sector.
-template <typename Real>
-void launchRowTransform(const FrontendArgs& a, cplx_t<Real>* Xp, cudaStream_t stream);
+// FP64 row transform: M -> X' for every sector.
+void launchRowTransform(const FrontendArgs& a, double2* Xp, cudaStream_t stream);
 
-// Column transform + G epilogue: X' -> G, one D x D block-layout matrix per (slot, spin) at
+// FP64 column transform + G epilogue: X' -> G, one D x D block-layout matrix per (slot, spin) at
 // offset g_sector_stride * (2 * slot + spin).
-template <typename Real>
-void launchColTransform(const FrontendArgs& a, const cplx_t<Real>* Xp, cplx_t<Real>* G,
-                        long g_sector_stride, cudaStream_t stream);
+void launchColTransform(const FrontendArgs& a, const double2* Xp, double2* G, long g_sector_stride,
+                        cudaStream_t stream);
 
 size_t frontendSmemRequirement(const TpDims& d, int n_max, bool fp64);
 
@@ -60,6 +58,25 @@ struct ColFft {
   int L;
   unsigned char rmap[36], kmap[36];
 };
+
+// ---- FP32 front-end of the mixed path, factored by orbital (tp_frontend32.cu) ----
+struct Front32Workspace {
+  // Each of T2, T4 and X is followed by kFront32Pad vertices' worth of memory that copies may run into.
+  float2* T2 = nullptr;  // [vertex][w] row twiddles (c, s)
+  float4* T4 = nullptr;  // [vertex][w] column twiddles (c, c, s, s)
+  float* Ms = nullptr;   // [sector][Kr][Kr] M in sorted order
+  float2* X = nullptr;   // X', (row, j) per sector at SectorDesc::x_off
+  int Kr = 0;            // max_order rounded up to 64
+  ColFft fft{};
+};
+constexpr int kFront32Pad = 4;
+// Its shared-memory tiles hold the cluster's orbitals (nb Nc up to about 100).
+bool front32Applies(const TpDims& d, int max_order);
+// Twiddles and sorted M (returns the launches); X' (one launch); G and, with gmax, each sector's largest |G| (one).
+int launchFront32Prep(const FrontendArgs& a, const Front32Workspace& w, cudaStream_t stream);
+void launchFront32Row(const FrontendArgs& a, const Front32Workspace& w, cudaStream_t stream);
+void launchFront32Col(const FrontendArgs& a, const Front32Workspace& w, float2* G, long g_sector_stride, int* gmax,
+                      cudaStream_t stream);
 
 struct FrontTcWorkspace {
   FrontTcShape shape;

@@ -12,7 +12,8 @@ constexpr int kMaxChannels = 4;
 // Static sizes.  Index conventions (all "first index fastest"):
 //   G0   (b1, b2, k, w_ext, s)                      nb^2 Nc NwExt 2
 //   X'   per sector: (row, w1_ext, jj) with row = b1 + nb k1 and jj the column of M in
-//        column-sorted order (FP64 and SIMT front-end)
+//        column-sorted order (FP64 and FP32 front-ends; rows of the
+//        upper frequency half only with half_g)
 //   G    per sector, frequency-block layout: (c, r, w_c, w_r) with r = b_r + nb k_r and
 //        c = b_c + nb k_c, i.e. one R x R block (row-major inside the block) per pair of
 //        extended frequencies (w_r, w_c).  G(r, w_r; c, w_c) is the reference's

@@ -257,9 +257,9 @@ void computeGNoAlloc(const dcaacc_tp_config& c, const double* G0_dev, const dcaa
   double2* Xp = reinterpret_cast<double2*>(base + o_x);
   if (fa.n_max > 0) {
     launchTwiddles(fa, stream);
-    launchRowTransform<double>(fa, Xp, stream);
+    launchRowTransform(fa, Xp, stream);
   }
-  launchColTransform<double>(fa, Xp, reinterpret_cast<double2*>(G_out), long(nw_ext) * nw_ext * R * R,
+  launchColTransform(fa, Xp, reinterpret_cast<double2*>(G_out), long(nw_ext) * nw_ext * R * R,
                              stream);
 }
 
