@@ -247,7 +247,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   }
   err_d_.alloc(1);
   DCAACC_CUDA_CHECK(cudaMemset(err_d_.get(), 0, sizeof(int)));
-  G4_ptrs_.alloc(c.n_channels);
+  G4_ptrs_.alloc(2 * c.n_channels);
   uploadG4Ptrs();
 
   // ---- batch workspace ----
@@ -343,25 +343,22 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     if (!simt_only_) {
       // The disconnected terms of the one-band PH channels run on the tensor cores.
       gmax_d_.alloc(2 * size_t(max_batch_));
-      if (discGemmApplies(dims_, max_batch_)) {
-        disc_.alloc(discScratchBytes(dims_, max_batch_));
-        discInit(disc_ws_, dims_, max_batch_, disc_.get(), disc_.bytes());
+      const TpDims ph = phChannels(dims_);
+      if (discGemmApplies(ph, max_batch_)) {
+        disc_.alloc(discScratchBytes(ph, max_batch_));
+        discInit(disc_ws_, ph, max_batch_, disc_.get(), disc_.bytes());
         have_disc_ = true;
       }
-      // Half G (mirror symmetry) when the direct-term kernel reads mirrored G blocks: one band,
-      // all momentum transfers, Nc = 16 (tensor-core direct term) or Nc = 36 (split FP32 direct
-      // term), and half of D a whole number of 128-row tiles.  DCAACC_TP_FULL_G=1 computes the
-      // whole of G instead (for comparisons).
-      std::vector<int> seen(nc, 0);
-      int distinct = 0;
-      for (int q : q_list_)
-        distinct += seen[q]++ == 0;
-      const bool q_all = distinct == nc && int(q_list_.size()) == nc;
+      // Half G (mirror symmetry) when the direct-term kernels read mirrored G blocks: one band, Nc = 16
+      // (tensor cores, or the transfer-subset kernel) or Nc = 36 (split FP32, or the subset kernel), and half
+      // of D a whole number of 128-row tiles (tensor-core front-end) or half the frequencies an even number
+      // (FP32 front-end, which copies them in pairs).  DCAACC_TP_FULL_G=1 computes the whole of G instead
+      // (for comparisons).
       const char* full_env = std::getenv("DCAACC_TP_FULL_G");
       const bool full_g = full_env && std::strcmp(full_env, "1") == 0;
-      if (have_disc_ && mirror_ok && !full_g && nb == 1 && (nc == kMaxMirrorNc || nc == 36) && q_all &&
-          c.n_channels <= 2 &&
-          nw_ext % 2 == 0 && (long(R) * nw_ext / 2) % 128 == 0) {
+      if (have_disc_ && mirror_ok && !full_g && nb == 1 && (nc == kMaxMirrorNc || nc == 36) &&
+          ph.n_channels == c.n_channels &&
+          nw_ext % 2 == 0 && (front32_ ? nw_ext % 4 == 0 : (long(R) * nw_ext / 2) % 128 == 0)) {
         dims_.half_g = 1;
         for (int k = 0; k < nc; ++k)
           dims_.kneg[k] = static_cast<unsigned char>(kneg[k]);
@@ -376,7 +373,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
             if (wex_list_[j] == -wex_list_[i])
               wm[i] = int(j);
         const bool closed = std::count(qm.begin(), qm.end(), -1) == 0 && std::count(wm.begin(), wm.end(), -1) == 0;
-        if (closed && nw % 2 == 0 && (nc * nw / 2) % 128 == 0) {
+        if (closed && nw % 2 == 0) {
           dims_.half_g4 = 1;
           upload_ints(q_mirror_d_, qm);
           upload_ints(wq_mirror_d_, wm);
@@ -486,9 +483,18 @@ void TpAccumulator::setFaultInjection(int stop_step, uint32_t wait_polls) {
 }
 
 void TpAccumulator::uploadG4Ptrs() {
+  // In channel order, then sorted for G4Args::G4_sorted.
   std::vector<double2*> ptrs;
   for (auto& g : g4())
     ptrs.push_back(g.get());
+  const int ph[2] = {DCAACC_PH_MAGNETIC, DCAACC_PH_CHARGE};
+  for (int c = 0; c < dims_.n_channels; ++c)
+    if (dims_.channels[c] == ph[0] || dims_.channels[c] == ph[1])
+      ptrs.push_back(g4()[c].get());
+  for (int ch : {DCAACC_PH_TRANSVERSE, DCAACC_PP_UP_DOWN})
+    for (int c = 0; c < dims_.n_channels; ++c)
+      if (dims_.channels[c] == ch)
+        ptrs.push_back(g4()[c].get());
   DCAACC_CUDA_CHECK(cudaMemcpy(G4_ptrs_.get(), ptrs.data(), G4_ptrs_.bytes(), cudaMemcpyHostToDevice));
 }
 
@@ -772,6 +778,8 @@ void TpAccumulator::process() {
   ga.q_list = q_d_.get();
   ga.wex_list = wex_d_.get();
   ga.G4 = G4_ptrs_.get();
+  ga.G4_sorted = G4_ptrs_.get() + dims_.n_channels;
+  ga.simt_only = simt_only_;
   ga.atomic = atomic_;
   ga.err = err_d_.get();
   {

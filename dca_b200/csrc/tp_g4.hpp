@@ -21,8 +21,10 @@ struct G4Args {
   const int* q_list;    // [nq] momentum-transfer indices (device)
   const int* wex_list;  // [nwq] frequency transfers (device)
   double2* const* G4;   // [n_channels] device pointers to each channel's running sum (device array)
+  double2* const* G4_sorted = nullptr;  // the same, PH-magnetic / PH-charge first (in order), then transverse, then pairing
   bool atomic;          // several accumulators share G4
   int* err;             // device error word (async_copy.cuh kErr* bits)
+  bool simt_only = false;         // no tensor-core terms (mixed path, comparisons)
   bool q_all = false;             // q_list is a permutation of all Nc cluster momenta
   const struct DiscWorkspace* disc = nullptr;  // tensor-core disconnected-term workspace (or null)
   const int* gmax = nullptr;  // [2 slot + spin] largest |G| of each sector as float bits (or null)
@@ -52,12 +54,13 @@ struct DiscWorkspace {
 // dst += src; src = 0 (sumTo of two accumulators on the same device).
 void launchAddAndClear(double2* dst, double2* src, size_t n, cudaStream_t stream);
 
-// Batched FP32 single-band PH update (tp_g4_batched.cu): one band, Nc in {4, 8, 16}, channels
-// PH-magnetic / PH-charge only.
+// Batched FP32 single-band update (tp_g4_batched.cu): one band, Nc in {4, 8, 16, 36}, no channel twice.
 bool singlebandBatchedApplies(const TpDims& d);
+// d with its PH-magnetic / PH-charge channels alone.
+TpDims phChannels(const TpDims& d);
 // Returns the number of kernels launched, 0 when the configuration is not covered (then
-// launchUpdateG4 uses the general kernels).  With a.disc_scratch large enough, the disconnected
-// terms run on the tensor cores (launchDiscGemm) and the update kernel only adds the direct term.
+// launchUpdateG4 uses the general kernels).  The disconnected terms run on the tensor cores
+// (launchDiscGemm) and the update kernels add the second-order terms, one kernel per kind.
 int launchUpdateG4SinglebandBatched(const G4Args& a, const float2* G, long g_sector_stride,
                                     cudaStream_t stream);
 
@@ -65,7 +68,7 @@ int launchUpdateG4SinglebandBatched(const G4Args& a, const float2* G, long g_sec
 // alone, full G and G4.  Returns false (nothing launched) when the configuration is not covered.
 bool launchUpdateG4PPMultiband(const G4Args& a, const float2* G, long g_sector_stride, cudaStream_t stream);
 
-// Tensor-core disconnected terms (tp_g4_disc.cu): one band, PH channels, batches of at most 256.
+// Tensor-core disconnected terms (tp_g4_disc.cu): one band, d a phChannels list, batches of at most 256.
 // discInit carves `mem` (discScratchBytes) and builds the descriptors; launchDiscGemm returns the
 // device result (per problem an M x M FP32 matrix), or null without a workspace.
 bool discGemmApplies(const TpDims& d, int max_batch);

@@ -17,6 +17,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "../../include/dcaacc.h"
 #include "async_copy.cuh"
 #include "common.cuh"
 #include "tp_g4.hpp"
@@ -233,144 +234,266 @@ updateG4SinglebandBatched(const TpDims dims, const float2* __restrict__ G, long 
   }
 }
 
-// Direct term only: sum_m sum_s -s_m/2 G_s(k1 w1; k2 w2) G_s(k2+q w2+x; k1+q w1+x), which is the same
-// for PH-magnetic and PH-charge with one band.  The disconnected terms come from the tensor-core
-// GEMM (tp_g4_disc.cu) in `disc`: per problem (iwq, iq, channel) an M x M matrix (M = Nc Nw) with
-// m = k1 + Nc w1 fastest.  Only the A and B blocks are staged.  The flush goes through shared
-// memory so that consecutive lanes touch consecutive k1 of G4 and of `disc`.
-template <int NC>
-__global__ void __launch_bounds__(256, 2)
-updateG4SinglebandDirect(const TpDims dims, const float2* __restrict__ G, long g_sector_stride,
-                         const int* __restrict__ signs, int n_slots, const int* __restrict__ k_add,
-                         const int* __restrict__ q_list, const int* __restrict__ wex_list,
-                         const float2* __restrict__ disc, double2* const* __restrict__ G4, bool atomic,
-                         int q_chunk, int* __restrict__ err) {
-  constexpr int R = NC;
-  constexpr int BLK = R * R;
-  const int nw = dims.nw, nw_ext = dims.nw_ext, nq = dims.nq;
-  const int tiles = nw * nw;
-  const int n_qchunks = (nq + q_chunk - 1) / q_chunk;
-  int w1, w2;
-  tileOfIndex(blockIdx.x % tiles, nw, w1, w2);
-  const int rest = blockIdx.x / tiles;
-  const int iwq = rest / n_qchunks, q0 = (rest % n_qchunks) * q_chunk;
-  const int wex = wex_list[iwq];
-  const int ext = dims.ext;
-  const int t = threadIdx.x;
-  const int qp = q_chunk + 1;  // padded row of the flush table
-  const int ql = t % q_chunk, k1 = t / q_chunk;
-  const int iq = q0 + ql;
-  const bool active = iq < nq && k1 < NC;
-  const int q = active ? q_list[iq] : 0;
+// Second-order terms of the batched update, per entry (k1 w1, k2 w2, q, x) with one band:
+//   kDirectPH     -s/2 sum_s G_s(k1 w1; k2 w2) G_s(k2+q w2+x; k1+q w1+x)   (PH-magnetic and PH-charge;
+//                 their disconnected terms come from the tensor-core GEMM, tp_g4_disc.cu, in `disc`: per
+//                 problem (iwq, iq, channel) an M x M matrix, M = Nc Nw, with m = k1 + Nc w1 fastest)
+//   kTransverse   -s/2 sum_s G_s(k1 w1; k2 w2) G_-s(k2+q w2+x; k1+q w1+x)
+//   kPairing       s/2 sum_s G_s(k1 w1; k2 w2) G_-s(q-k1 m1; q-k2 m2),  m = x + Nw - 1 - w
+// (tp_accumulator_cpu.hpp:454-546, 628-661).  Every form is a sum of A(k1; k2) B(..) over the batch, A and B
+// one G block each; with d = k1 - k2 fixed, A depends on k1 alone and B on l1 alone,
+//   l1 = k1 + q, B(l1 - d; l1)   (particle-hole)        l1 = q - k1, B(l1; l1 + d)   (pairing).
+enum SecondOrder { kDirectPH = 0, kTransverse = 1, kPairing = 2 };
 
-  const int w1e = w1 + ext, w2e = w2 + ext, w1x = w1e + wex, w2x = w2e + wex;
-  const long b_A = (static_cast<long>(w1e) * nw_ext + w2e) * BLK;
-  const long b_B = (static_cast<long>(w2x) * nw_ext + w1x) * BLK;
+// Block (row, column frequency) that B is read from, for the tile (w1, w2) and transfer wex.
+template <int MODE>
+__device__ inline void secondBlock(const TpDims& d, int w1, int w2, int wex, int& wr, int& wc) {
+  if (MODE == kPairing) {
+    wr = wex + d.nw - 1 - w1 + d.ext;
+    wc = wex + d.nw - 1 - w2 + d.ext;
+  }
+  else {
+    wr = w2 + d.ext + wex;
+    wc = w1 + d.ext + wex;
+  }
+}
+
+// A subset of the momentum transfers.  CTA = one (w1, w2, wq) tile and up to TQ QT transfers; thread =
+// (k1, d = k1 - k2, transfer), KI values of d and QT transfers each, so that the lanes of a half-warp read
+// consecutive columns of A and of B: whole blocks can be bulk-copied and the gathers stay free of bank
+// conflicts.  Per measurement a thread reads KI alphas and KI QT betas a spin.  Measurements are staged DEPTH
+// deep; per-stage "empty" barriers let the warps drift apart.  Half G (dims.half_g): a block of the lower
+// frequency half is read as the conjugate of its mirror with k -> -k; half G4 (tile_order non-null): only
+// the tiles listed there run.  With one entry a thread its G4 and disconnected-term loads are issued before
+// the batch loop.
+//
+// Bound by the read of G, once (with its L2 reread as B).  The earlier kernel gave a thread all k2 of one
+// (k1, transfer), sixteen threads to a CTA with one transfer on a 4x4 cluster (Nw = 64, batch of 64): 0.477 ms
+// with the whole of G; this one 0.147 ms, with the half that it can read (0.54 GB, 0.083 ms at the copy rate).
+template <int NC>
+struct FewShape;  // threads, transfers side by side, d values per thread, staged measurements
+template <>
+struct FewShape<4> {
+  static constexpr int NT = 256, TQ = 16, KI = 1, DEPTH = 16;
+};
+template <>
+struct FewShape<8> {
+  static constexpr int NT = 256, TQ = 4, KI = 1, DEPTH = 12;
+};
+template <>
+struct FewShape<16> {
+  static constexpr int NT = 256, TQ = 1, KI = 1, DEPTH = 6;
+};
+template <>
+struct FewShape<36> {
+  static constexpr int NT = 432, TQ = 1, KI = 3, DEPTH = 4;
+};
+
+template <int NC, int QT, int MODE>
+__global__ void __launch_bounds__(FewShape<NC>::NT)
+updateG4SinglebandFew(const TpDims dims, const float2* __restrict__ G, long g_sector_stride,
+                      const int* __restrict__ signs, int n_slots, const int* __restrict__ k_sub,
+                      const int* __restrict__ q_list, const int* __restrict__ wex_list,
+                      const unsigned* __restrict__ tile_order, const float2* __restrict__ disc,
+                      double2* const* __restrict__ G4, bool atomic, int* __restrict__ err) {
+  using S = FewShape<NC>;
+  constexpr int NT = S::NT, TQ = S::TQ, KI = S::KI, DEPTH = S::DEPTH;
+  constexpr int BLK = NC * NC, PAIRS = BLK / KI;
+  static_assert(NT == PAIRS * TQ && NC % KI == 0, "thread layout");
+  constexpr bool kPrefetch = KI * QT == 1;
+  const int nw = dims.nw, nw_ext = dims.nw_ext, nq = dims.nq, n_ch = dims.n_channels;
+  const int n_chunks = (nq + TQ * QT - 1) / (TQ * QT);
+  const int q0 = static_cast<int>(blockIdx.x % n_chunks) * TQ * QT;
+  const int tile = blockIdx.x / n_chunks;
+  const int per_wq = tile_order ? nw * nw / 2 : nw * nw;
+  int w1, w2;
+  if (tile_order) {
+    const unsigned v = tile_order[tile % per_wq];
+    w1 = static_cast<int>(v & 0xffffu);
+    w2 = static_cast<int>(v >> 16);
+  }
+  else {
+    tileOfIndex(tile % per_wq, nw, w1, w2);
+  }
+  const int iwq = tile / per_wq, wex = wex_list[iwq];
+  const int t = threadIdx.x, lane = t % 32;
+  const int k1 = t % NC, d0 = (t % PAIRS) / NC, tq = t / PAIRS;
+
+  const int wa1 = w1 + dims.ext, wa2 = w2 + dims.ext;
+  int wb1, wb2;
+  secondBlock<MODE>(dims, w1, w2, wex, wb1, wb2);
+  const bool mir_a = dims.half_g && 2 * wa1 < nw_ext, mir_b = dims.half_g && 2 * wb1 < nw_ext;
+  auto block = [&](int wr, int wc, bool mir) {
+    return (mir ? static_cast<long>(nw_ext - 1 - wr) * nw_ext + nw_ext - 1 - wc
+                : static_cast<long>(wr) * nw_ext + wc) * BLK;
+  };
+  const long b_A = block(wa1, wa2, mir_a), b_B = block(wb1, wb2, mir_b);
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);     // [2]
-  float2* stage = reinterpret_cast<float2*>(smem_raw + 16);  // [2][A0 B0 A1 B1][BLK]
-
-  int b_off[NC];
-  const int k1q = k_add[k1 % NC + NC * q];
-#pragma unroll
-  for (int j = 0; j < NC; ++j)
-    b_off[j] = k_add[j + NC * q] * R + k1q;
-  const int a_off = (k1 % NC) * R;
-
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);  // [DEPTH] copies landed
+  uint64_t* empty = full + DEPTH;                          // [DEPTH] all warps done reading
+  int* ksub = reinterpret_cast<int*>(empty + DEPTH);       // [NC * NC], a + NC b: b - a
+  constexpr int kHead = (16 * DEPTH + 4 * BLK + 15) / 16 * 16;
+  float2* stage = reinterpret_cast<float2*>(smem_raw + kHead);  // [DEPTH][A0 B0 A1 B1][BLK]
+  float2* T = stage;                                            // flush table, after the batch loop
   constexpr uint32_t blk_bytes = BLK * sizeof(float2);
-  auto issue = [&](int slot, int st) {
+  auto issue = [&](int slot) {
+    const int st = slot % DEPTH;
     float2* dst = stage + st * 4 * BLK;
-    mbarArriveExpectTx(&bar[st], 4 * blk_bytes);
+    mbarArriveExpectTx(&full[st], 4 * blk_bytes);
     const float2* src0 = G + g_sector_stride * (2 * slot);
     const float2* src1 = src0 + g_sector_stride;
-    bulkCopyG2S(dst + 0 * BLK, src0 + b_A, blk_bytes, &bar[st]);
-    bulkCopyG2S(dst + 1 * BLK, src0 + b_B, blk_bytes, &bar[st]);
-    bulkCopyG2S(dst + 2 * BLK, src1 + b_A, blk_bytes, &bar[st]);
-    bulkCopyG2S(dst + 3 * BLK, src1 + b_B, blk_bytes, &bar[st]);
+    bulkCopyG2S(dst + 0 * BLK, src0 + b_A, blk_bytes, &full[st]);
+    bulkCopyG2S(dst + 1 * BLK, src0 + b_B, blk_bytes, &full[st]);
+    bulkCopyG2S(dst + 2 * BLK, src1 + b_A, blk_bytes, &full[st]);
+    bulkCopyG2S(dst + 3 * BLK, src1 + b_B, blk_bytes, &full[st]);
   };
+  for (int e = t; e < BLK; e += NT)
+    ksub[e] = k_sub[e];
   if (t == 0) {
-    mbarInit(&bar[0], 1);
-    mbarInit(&bar[1], 1);
+    for (int s = 0; s < DEPTH; ++s) {
+      mbarInit(&full[s], 1);
+      mbarInit(&empty[s], (NT + 31) / 32);
+    }
     fenceBarrierInit();
   }
   __syncthreads();
-  if (t == 0) {
-    issue(0, 0);
-    if (n_slots > 1)
-      issue(1, 1);
-  }
+  if (t == 0)
+    for (int m = 0; m < DEPTH && m < n_slots; ++m)
+      issue(m);
 
-  float2 acc[NC];
+  // -k = k_z - k with z = k_0 - k_0 the zero momentum.
+  const int z0 = ksub[0];
+  auto neg = [&](int k) { return ksub[k + NC * z0]; };
+  auto elem = [&](int r, int c, bool mir) { return mir ? neg(r) * NC + neg(c) : r * NC + c; };
+  int oa[KI], ob[KI][QT];
 #pragma unroll
-  for (int j = 0; j < NC; ++j)
-    acc[j] = make_float2(0.f, 0.f);
-
-  for (int m = 0; m < n_slots; ++m) {
-    const int st = m & 1;
-    const bool ok = mbarWait(&bar[st], (m >> 1) & 1, err);
-    if (!__syncthreads_and(ok))
-      return;  // uniform bail-out; the host reports the error word
-    float2* S = stage + st * 4 * BLK;
-    const float nhs = -0.5f * static_cast<float>(signs[m]);
-    for (int e = t; e < BLK; e += blockDim.x) {  // A_0, A_1 *= -s/2
-      float2 a = S[e];
-      S[e] = make_float2(nhs * a.x, nhs * a.y);
-      a = S[2 * BLK + e];
-      S[2 * BLK + e] = make_float2(nhs * a.x, nhs * a.y);
-    }
-    __syncthreads();
-    if (active) {
-      const float2* A0 = S + a_off;
-      const float2* B0 = S + 1 * BLK;
-      const float2* A1 = S + 2 * BLK + a_off;
-      const float2* B1 = S + 3 * BLK;
+  for (int i = 0; i < KI; ++i) {
+    const int d = d0 + i * (NC / KI);
+    oa[i] = elem(k1, ksub[d + NC * k1], mir_a);
 #pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        cfma(acc[j], A0[j], B0[b_off[j]]);
-        cfma(acc[j], A1[j], B1[b_off[j]]);
-      }
-    }
-    fenceProxyAsync();  // this thread's generic writes to the stage precede the next bulk copy
-    __syncthreads();    // stage st is free again
-    if (t == 0 && m + 2 < n_slots)
-      issue(m + 2, st);
-  }
-
-  // Flush: table T[j][k1][ql] (rows padded to qp), then lanes take consecutive k1.
-  float2* T = stage;
-  if (active) {
-#pragma unroll
-    for (int j = 0; j < NC; ++j)
-      T[(j * NC + k1) * qp + ql] = acc[j];
-  }
-  __syncthreads();
-  const long M = static_cast<long>(NC) * nw;
-  const long s_w1 = NC, s_k2 = s_w1 * nw, s_w2 = s_k2 * NC, s_q = s_w2 * nw, s_wq = s_q * nq;
-  const int n_ch = dims.n_channels;
-  for (int idx = t; idx < NC * NC * q_chunk; idx += blockDim.x) {
-    const int fk1 = idx % NC, j = (idx / NC) % NC, fql = idx / (NC * NC);
-    const int fiq = q0 + fql;
-    if (fiq >= nq)
-      continue;
-    const float2 v = T[(j * NC + fk1) * qp + fql];
-    const long g4i = fk1 + w1 * s_w1 + j * s_k2 + w2 * s_w2 + fiq * s_q + iwq * s_wq;
-    const long di = (j + static_cast<long>(NC) * w2) * M + fk1 + static_cast<long>(NC) * w1;
-    for (int c = 0; c < n_ch; ++c) {
-      const float2 dv = disc[(static_cast<long>(iwq * nq + fiq) * n_ch + c) * M * M + di];
-      double2* p = G4[c] + g4i;
-      const double re = static_cast<double>(v.x + dv.x), im = static_cast<double>(v.y + dv.y);
-      if (atomic) {
-        atomicAdd(&p->x, re);
-        atomicAdd(&p->y, im);
+    for (int j = 0; j < QT; ++j) {
+      const int q = q_list[min(q0 + tq + TQ * j, nq - 1)];
+      if (MODE == kPairing) {
+        const int l1 = ksub[k1 + NC * q];
+        ob[i][j] = elem(l1, ksub[neg(d) + NC * l1], mir_b);
       }
       else {
-        double2 o = *p;
-        o.x += re;
-        o.y += im;
-        *p = o;
+        const int l1 = ksub[neg(k1) + NC * q];
+        ob[i][j] = elem(ksub[d + NC * l1], l1, mir_b);
       }
     }
+  }
+  const long M = static_cast<long>(NC) * nw;
+  const long s_w1 = NC, s_k2 = s_w1 * nw, s_w2 = s_k2 * NC, s_q = s_w2 * nw, s_wq = s_q * nq;
+  // Entry idx of the flush: k1 fastest, then k2, then the transfer.
+  const int total = BLK * min(TQ * QT, nq - q0);
+  auto g4At = [&](int idx) {
+    const int fk1 = idx % NC, fk2 = (idx / NC) % NC, iq = q0 + idx / BLK;
+    return fk1 + w1 * s_w1 + fk2 * s_k2 + w2 * s_w2 + iq * s_q + iwq * s_wq;
+  };
+  auto discAt = [&](int idx, int c) {
+    const int fk1 = idx % NC, fk2 = (idx / NC) % NC, iq = q0 + idx / BLK;
+    return ((static_cast<long>(iwq * nq + iq) * n_ch + c) * M + fk2 + static_cast<long>(NC) * w2) * M + fk1 +
+           static_cast<long>(NC) * w1;
+  };
+  double2 o[2];
+  float2 dv[2];
+  if (kPrefetch && t < total) {
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      if (c < n_ch) {
+        o[c] = atomic ? make_double2(0., 0.) : G4[c][g4At(t)];
+        dv[c] = MODE == kDirectPH ? __ldg(disc + discAt(t, c)) : make_float2(0.f, 0.f);
+      }
+  }
+
+  float2 acc[KI][QT];
+#pragma unroll
+  for (int i = 0; i < KI; ++i)
+#pragma unroll
+    for (int j = 0; j < QT; ++j)
+      acc[i][j] = make_float2(0.f, 0.f);
+  const float ia = mir_a ? -1.f : 1.f, ib = mir_b ? -1.f : 1.f;
+  const unsigned warp_mask = t / 32 == NT / 32 ? (1u << (NT % 32)) - 1 : ~0u;  // the last warp may be partial
+  bool ok = true;
+  for (int m = 0; m < n_slots; ++m) {
+    const int st = m % DEPTH;
+    const float half = (MODE == kPairing ? 0.5f : -0.5f) * static_cast<float>(__ldg(signs + m));
+    ok = __all_sync(warp_mask, mbarWait(&full[st], (m / DEPTH) & 1, err));
+    if (!ok)
+      break;
+    const float2* Sm = stage + st * 4 * BLK;
+#pragma unroll
+    for (int spin = 0; spin < 2; ++spin) {
+      const float2* A = Sm + 2 * spin * BLK;
+      const float2* B = Sm + (2 * (MODE == kDirectPH ? spin : 1 - spin) + 1) * BLK;
+#pragma unroll
+      for (int i = 0; i < KI; ++i) {
+        float2 av = A[oa[i]];
+        av = make_float2(half * av.x, half * ia * av.y);
+#pragma unroll
+        for (int j = 0; j < QT; ++j) {
+          float2 bv = B[ob[i][j]];
+          bv.y *= ib;
+          cfma(acc[i][j], av, bv);
+        }
+      }
+    }
+    __syncwarp(warp_mask);
+    if (lane == 0)
+      mbarArrive(&empty[st]);  // release: this warp's reads of the stage are done
+    if (t == 0 && m + DEPTH < n_slots) {
+      if (!mbarWait(&empty[st], (m / DEPTH) & 1, err)) {
+        ok = false;  // the other warps see the missing copy as a timeout of their own
+        break;
+      }
+      issue(m + DEPTH);
+    }
+  }
+  if (__syncthreads_or(!ok))
+    return;  // uniform bail-out; the host reports the error word
+
+  // T[transfer][k2][k1], then consecutive lanes take consecutive k1 of G4 and of `disc`.
+#pragma unroll
+  for (int i = 0; i < KI; ++i)
+#pragma unroll
+    for (int j = 0; j < QT; ++j)
+      T[((tq + TQ * j) * NC + ksub[d0 + i * (NC / KI) + NC * k1]) * NC + k1] = acc[i][j];
+  __syncthreads();
+  auto add = [&](int idx, int c, double2 old, float2 dc) {
+    const float2 v = T[idx];
+    double2* p = G4[c] + g4At(idx);
+    const double re = static_cast<double>(v.x + dc.x), im = static_cast<double>(v.y + dc.y);
+    if (atomic) {
+      atomicAdd(&p->x, re);
+      atomicAdd(&p->y, im);
+    }
+    else {
+      *p = make_double2(old.x + re, old.y + im);
+    }
+  };
+  if constexpr (kPrefetch) {
+    if (t < total)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (c < n_ch)
+          add(t, c, o[c], dv[c]);
+  }
+  else {
+    for (int base = t; base < total; base += 2 * NT)
+      for (int c = 0; c < n_ch; ++c) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int idx = min(base + u * NT, total - 1);
+          o[u] = atomic ? make_double2(0., 0.) : G4[c][g4At(idx)];
+          dv[u] = MODE == kDirectPH ? __ldg(disc + discAt(idx, c)) : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (base + u * NT < total)
+            add(base + u * NT, c, o[u], dv[u]);
+      }
   }
 }
 
@@ -378,13 +501,13 @@ updateG4SinglebandDirect(const TpDims dims, const float2* __restrict__ G, long g
 // Grouping the entries by d = k1 - k2 turns the term into outer products: with l1 = k1 + q,
 //   D(k1, k2 = k1 - d, q = l1 - k1) = sum_m sum_s alpha_sd(k1) beta_sd(l1),
 //   alpha_sd(k1) = -s_m/2 G_s(k1 w1; k1-d w2),   beta_sd(l1) = G_s(l1-d w2+x; l1 w1+x),
-// (the cluster momenta form a group, so k2 + q = l1 - d).  Thread (d, k1 block, l1 block) keeps a
+// (the cluster momenta form a group, so k2 + q = l1 - d), and likewise for the other second-order forms.  Thread (d, k1 block, l1 block) keeps a
 // TA x TB tile of complex sums in registers and, per measurement and spin, gathers its TA alphas
 // and TB betas straight from the staged G blocks (fixed shared-memory offsets, computed once) for
 // TA TB complex FMAs.  Measurements are staged eight deep (bulk copies); per-stage "empty"
 // barriers let the warps drift apart instead of meeting at a block barrier per measurement.  The flush goes through a shared table so that lanes touch consecutive k1
 // of G4 and of `disc`.
-template <int NC, int TA, int TB>
+template <int NC, int TA, int TB, int MODE>
 __global__ void __launch_bounds__(NC * (NC / TA) * (NC / TB))
 updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_sector_stride,
                         const int* __restrict__ signs, int n_slots, const int* __restrict__ k_sub,
@@ -401,14 +524,14 @@ updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_
   tileOfIndex(blockIdx.x % (nw * nw), nw, w1, w2);
   const int iwq = blockIdx.x / (nw * nw);
   const int wex = wex_list[iwq];
-  const int ext = dims.ext;
   const int t = threadIdx.x;
   const int d = t / (NKB * NLB), sub = t % (NKB * NLB);
   const int k1_0 = (sub / NLB) * TA, l1_0 = (sub % NLB) * TB;
 
-  const int w1e = w1 + ext, w2e = w2 + ext, w1x = w1e + wex, w2x = w2e + wex;
-  const long b_A = (static_cast<long>(w1e) * nw_ext + w2e) * BLK;
-  const long b_B = (static_cast<long>(w2x) * nw_ext + w1x) * BLK;
+  int wb1, wb2;
+  secondBlock<MODE>(dims, w1, w2, wex, wb1, wb2);
+  const long b_A = (static_cast<long>(w1 + dims.ext) * nw_ext + w2 + dims.ext) * BLK;
+  const long b_B = (static_cast<long>(wb1) * nw_ext + wb2) * BLK;
 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);      // [DEPTH] copies landed
@@ -451,16 +574,19 @@ updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_
       issue(m);
 
   // Fixed gather offsets inside a staged block: alpha from A (row k1, column k1 - d), beta from B
-  // (row l1 - d, column l1).
+  // (row l1 - d, column l1; pairing: row l1, column l1 + d).  -k = k_z - k with z = k_0 - k_0.
+  const int z0 = ksub[0];
+  auto neg = [&](int k) { return ksub[k + NC * z0]; };
   int oa[TA], ob[TB];
 #pragma unroll
   for (int a = 0; a < TA; ++a)
     oa[a] = (k1_0 + a) * NC + ksub[d + NC * (k1_0 + a)];
 #pragma unroll
   for (int b = 0; b < TB; ++b)
-    ob[b] = ksub[d + NC * (l1_0 + b)] * NC + l1_0 + b;
+    ob[b] = MODE == kPairing ? (l1_0 + b) * NC + ksub[neg(d) + NC * (l1_0 + b)]
+                             : ksub[d + NC * (l1_0 + b)] * NC + l1_0 + b;
 
-  // Sums of -s_m alpha beta (the factor 1/2 is applied at the flush); the sign selects the loop
+  // Sums of -s_m alpha beta (pairing: +; the factor 1/2 is applied at the flush); the sign selects the loop
   // body (uniform across the CTA), so no multiply is spent on it.
   float2 acc[TA][TB];
 #pragma unroll
@@ -481,11 +607,11 @@ updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_
     if (!ok)
       break;
     const float2* S = stage + st * 4 * BLK;
-    const bool add = sg < 0;
+    const bool add = MODE == kPairing ? sg > 0 : sg < 0;
 #pragma unroll
     for (int spin = 0; spin < 2; ++spin) {
       const float2* A = S + (2 * spin) * BLK;
-      const float2* B = S + (2 * spin + 1) * BLK;
+      const float2* B = S + (2 * (MODE == kDirectPH ? spin : 1 - spin) + 1) * BLK;
       float2 av[TA], bv[TB];
 #pragma unroll
       for (int a = 0; a < TA; ++a)
@@ -535,7 +661,7 @@ updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_
     for (int b = 0; b < TB; ++b) {
       const int k1 = k1_0 + a, l1 = l1_0 + b;
       const int k2 = ksub[d + NC * k1];
-      const int qi = qinv[ksub[k1 + NC * l1]];
+      const int qi = qinv[ksub[(MODE == kPairing ? neg(k1) : k1) + NC * l1]];
       T[(k2 * NC + k1) * QP + qi] = make_float2(0.5f * acc[a][b].x, 0.5f * acc[a][b].y);
     }
   __syncthreads();
@@ -563,7 +689,7 @@ updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_
       double2 o[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        dv[u] = __ldg(disc + di[u] + static_cast<long>(c) * M * M);
+        dv[u] = MODE == kDirectPH ? __ldg(disc + di[u] + static_cast<long>(c) * M * M) : make_float2(0.f, 0.f);
         o[u] = atomic ? make_double2(0., 0.) : G4[c][g4i[u]];
       }
 #pragma unroll
@@ -915,18 +1041,47 @@ size_t outerSmem() {
   return 16 * 8 + 4 * (BLK + NC + 4) + std::max(loop, table);
 }
 
-template <int NC>
+template <int NC, int MODE>
 void launchOuter(const G4Args& a, const float2* G, long stride, const float2* disc, cudaStream_t stream) {
   const TpDims& d = a.dims;
   constexpr int TA = OuterTile<NC>::TA, TB = OuterTile<NC>::TB;
   const size_t smem = outerSmem<NC>();
-  auto k = updateG4SinglebandOuter<NC, TA, TB>;
+  auto k = updateG4SinglebandOuter<NC, TA, TB, MODE>;
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const long blocks = long(d.nw) * d.nw * d.nwq;
   constexpr int threads = NC * (NC / TA) * (NC / TB);
   k<<<static_cast<unsigned>(blocks), threads, smem, stream>>>(d, G, stride, a.signs, a.n_slots, a.k_sub, a.q_list,
                                                               a.wex_list, disc, a.G4, a.atomic, a.err);
   DCAACC_LAUNCH_CHECK();
+}
+
+template <int NC, int QT, int MODE>
+void launchFewQT(const G4Args& a, const float2* G, long stride, const float2* disc, cudaStream_t stream) {
+  using S = FewShape<NC>;
+  const TpDims& d = a.dims;
+  constexpr size_t head = (16 * S::DEPTH + 4 * NC * NC + 15) / 16 * 16;
+  constexpr size_t smem = head + sizeof(float2) * NC * NC * size_t(std::max(4 * S::DEPTH, S::TQ * QT));
+  static_assert(smem <= 227 * 1024, "shared memory per CTA");
+  auto k = updateG4SinglebandFew<NC, QT, MODE>;
+  DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const long tiles = long(d.nw) * d.nw * d.nwq / (a.tile_order ? 2 : 1);  // half G4: w1 >= Nw / 2 only
+  const long blocks = tiles * ((d.nq + S::TQ * QT - 1) / (S::TQ * QT));
+  k<<<static_cast<unsigned>(blocks), S::NT, smem, stream>>>(d, G, stride, a.signs, a.n_slots, a.k_sub, a.q_list,
+                                                            a.wex_list, a.tile_order, disc, a.G4, a.atomic, a.err);
+  DCAACC_LAUNCH_CHECK();
+}
+
+// One, two or four transfers a thread: the fewest that cover the list, since each further chunk of
+// transfers stages the blocks again.
+template <int NC, int MODE>
+void launchFew(const G4Args& a, const float2* G, long stride, const float2* disc, cudaStream_t stream) {
+  const int per = (a.dims.nq + FewShape<NC>::TQ - 1) / FewShape<NC>::TQ;
+  if (per <= 1)
+    launchFewQT<NC, 1, MODE>(a, G, stride, disc, stream);
+  else if (per == 2)
+    launchFewQT<NC, 2, MODE>(a, G, stride, disc, stream);
+  else
+    launchFewQT<NC, 4, MODE>(a, G, stride, disc, stream);
 }
 
 template <int NC, bool MAG, bool CHARGE>
@@ -946,81 +1101,111 @@ void launchBatched(const G4Args& a, const float2* G, long stride, cudaStream_t s
   DCAACC_LAUNCH_CHECK();
 }
 
-template <int NC>
-void launchDirect(const G4Args& a, const float2* G, long stride, const float2* disc, cudaStream_t stream) {
-  const TpDims& d = a.dims;
-  const int q_chunk = std::max(1, std::min(d.nq, 256 / NC));
-  const int threads = NC * q_chunk;
-  const int qp = q_chunk + 1;
-  const size_t smem = 16 + sizeof(float2) * std::max<size_t>(2 * 4 * NC * NC, size_t(NC) * NC * qp);
-  auto k = updateG4SinglebandDirect<NC>;
-  DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int n_qchunks = (d.nq + q_chunk - 1) / q_chunk;
-  const long blocks = long(d.nw) * d.nw * d.nwq * n_qchunks;
-  k<<<static_cast<unsigned>(blocks), threads, smem, stream>>>(d, G, stride, a.signs, a.n_slots, a.k_add,
-                                                              a.q_list, a.wex_list, disc, a.G4, a.atomic,
-                                                              q_chunk, a.err);
-  DCAACC_LAUNCH_CHECK();
+// The second-order term of MODE: outer products with all transfers (Nc <= 16), else the subset kernel.
+template <int NC, int MODE>
+void launchSecondOrder(const G4Args& a, const float2* G, long stride, const float2* disc, cudaStream_t s) {
+  if constexpr (NC <= 16) {
+    if (a.q_all) {
+      launchOuter<NC, MODE>(a, G, stride, disc, s);
+      return;
+    }
+  }
+  launchFew<NC, MODE>(a, G, stride, disc, s);
 }
 
 template <int NC>
-int launchForNc(const G4Args& a, const float2* G, long stride, bool mag, bool charge, cudaStream_t s) {
-  if (const float2* disc = launchDiscGemm(a, G, stride, s)) {
-    if (NC == 16 && directTcApplies(a))
-      launchDirectTc(a, G, stride, disc, a.n_sm, s);
-    else if (a.q_all)
-      launchOuter<NC>(a, G, stride, disc, s);
+int launchForNc(const G4Args& a, const float2* G, long stride, cudaStream_t s) {
+  // Each group of channels with its own term and its own run of the sorted G4 pointers.
+  int launched = 0;
+  G4Args p = a;
+  p.dims = phChannels(a.dims);
+  p.G4 = a.G4_sorted;
+  if (p.dims.n_channels > 0) {
+    const float2* disc = launchDiscGemm(p, G, stride, s);
+    if (!disc)
+      return 0;
+    if (NC == 16 && directTcApplies(p))
+      launchDirectTc(p, G, stride, disc, p.n_sm, s);
+    else if (NC == 36 && p.q_all)
+      launchOuterSplit(p, G, stride, disc, s);
     else
-      launchDirect<NC>(a, G, stride, disc, s);
-    return 3;
+      launchSecondOrder<NC, kDirectPH>(p, G, stride, disc, s);
+    launched += 3;
+    p.G4 += p.dims.n_channels;
   }
-  if (mag && charge)
-    launchBatched<NC, true, true>(a, G, stride, s);
-  else if (mag)
-    launchBatched<NC, true, false>(a, G, stride, s);
-  else
-    launchBatched<NC, false, true>(a, G, stride, s);
-  return 1;
+  for (int ch : {DCAACC_PH_TRANSVERSE, DCAACC_PP_UP_DOWN})
+    for (int c = 0; c < a.dims.n_channels; ++c)
+      if (a.dims.channels[c] == ch) {
+        p.dims = a.dims;
+        p.dims.n_channels = 1;
+        p.dims.channels[0] = ch;
+        if (ch == DCAACC_PH_TRANSVERSE)
+          launchSecondOrder<NC, kTransverse>(p, G, stride, nullptr, s);
+        else
+          launchSecondOrder<NC, kPairing>(p, G, stride, nullptr, s);
+        ++launched;
+        ++p.G4;
+      }
+  return launched;
 }
 
 }  // namespace
+
+TpDims phChannels(const TpDims& d) {
+  TpDims p = d;
+  p.n_channels = 0;
+  for (int c = 0; c < d.n_channels; ++c)
+    if (d.channels[c] == DCAACC_PH_MAGNETIC || d.channels[c] == DCAACC_PH_CHARGE)
+      p.channels[p.n_channels++] = d.channels[c];
+  return p;
+}
 
 int launchUpdateG4SinglebandBatched(const G4Args& a, const float2* G, long g_sector_stride,
                                     cudaStream_t stream) {
   const TpDims& d = a.dims;
   if (!singlebandBatchedApplies(d))
     return 0;
+  if (!a.simt_only && a.n_slots <= kSplitMaxSlots) {
+    const int n = d.nc == 4    ? launchForNc<4>(a, G, g_sector_stride, stream)
+                  : d.nc == 8  ? launchForNc<8>(a, G, g_sector_stride, stream)
+                  : d.nc == 16 ? launchForNc<16>(a, G, g_sector_stride, stream)
+                               : launchForNc<kSplitNc>(a, G, g_sector_stride, stream);
+    if (n)
+      return n;
+  }
+  // Without the disconnected terms' workspace (all-SIMT runs, batches beyond its limit): all channels
+  // particle-hole and Nc <= 16, one kernel with those terms in place.
+  if (phChannels(d).n_channels != d.n_channels || d.nc == kSplitNc)
+    return 0;
   bool mag = false, charge = false;
   for (int c = 0; c < d.n_channels; ++c)
-    (d.channels[c] == 2 ? mag : charge) = true;
-  switch (d.nc) {
-    case 4:
-      return launchForNc<4>(a, G, g_sector_stride, mag, charge, stream);
-    case 8:
-      return launchForNc<8>(a, G, g_sector_stride, mag, charge, stream);
-    case kSplitNc:
-      // Disconnected terms on the tensor cores and the split direct term (both read mirrored
-      // blocks for half G and run the w1 >= Nw / 2 tiles for half G4); without the workspace or
-      // with a subset of the transfers, the general one-band kernel (return 0; half G is never
-      // enabled then).
-      if (!a.q_all || a.n_slots > kSplitMaxSlots)
-        return 0;
-      if (const float2* disc = launchDiscGemm(a, G, g_sector_stride, stream)) {
-        launchOuterSplit(a, G, g_sector_stride, disc, stream);
-        return 3;
-      }
-      return 0;
-    default:
-      return launchForNc<16>(a, G, g_sector_stride, mag, charge, stream);
-  }
+    (d.channels[c] == DCAACC_PH_MAGNETIC ? mag : charge) = true;
+  auto go = [&](auto nc) {
+    constexpr int NC = decltype(nc)::value;
+    if (mag && charge)
+      launchBatched<NC, true, true>(a, G, g_sector_stride, stream);
+    else if (mag)
+      launchBatched<NC, true, false>(a, G, g_sector_stride, stream);
+    else
+      launchBatched<NC, false, true>(a, G, g_sector_stride, stream);
+  };
+  if (d.nc == 4)
+    go(std::integral_constant<int, 4>{});
+  else if (d.nc == 8)
+    go(std::integral_constant<int, 8>{});
+  else
+    go(std::integral_constant<int, 16>{});
+  return 1;
 }
 
+// Each channel at most once: the groups' pointers are sorted by channel.
 bool singlebandBatchedApplies(const TpDims& d) {
   if (d.nb != 1 || (d.nc != 4 && d.nc != 8 && d.nc != 16 && d.nc != kSplitNc))
     return false;
   for (int c = 0; c < d.n_channels; ++c)
-    if (d.channels[c] != 2 && d.channels[c] != 3)
-      return false;
+    for (int e = 0; e < c; ++e)
+      if (d.channels[c] == d.channels[e])
+        return false;
   return d.n_channels > 0;
 }
 

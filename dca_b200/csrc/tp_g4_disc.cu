@@ -58,7 +58,7 @@ size_t align256(size_t b) {
 __global__ void __launch_bounds__(256)
 discPlanesKernel(const TpDims dims, const float2* __restrict__ G, long g_sector_stride,
                  const int* __restrict__ signs, int n_slots, int Kb, int Mp, const int* __restrict__ k_add,
-                 const int* __restrict__ q_list, const int* __restrict__ wex_list, __half* __restrict__ Up,
+                 const int* __restrict__ q_list, const int* __restrict__ wex_list, int u_row0, __half* __restrict__ Up,
                  __half* __restrict__ Vp, int* __restrict__ eU, int* __restrict__ eV) {
   const int nc = dims.nc, ext = dims.ext;
   const int M = nc * dims.nw;
@@ -81,8 +81,8 @@ discPlanesKernel(const TpDims dims, const float2* __restrict__ G, long g_sector_
     long bc = 0, be = 0;
     bool cc = false, ce = false;  // read from the conjugated mirror (half G)
     const bool in_row = row < M;
-    // Half G4: the GEMM reads U only for the rows (k1, w1) with w1 >= Nw / 2.
-    const bool need_u = in_row && !(dims.half_g4 && 2 * (row / nc) < dims.nw);
+    // Half G4: the GEMM reads U only from the row tile of (k1 = 0, w1 = Nw / 2) on.
+    const bool need_u = in_row && row >= u_row0;
     if (in_row) {
       const int k = row % nc, w = row / nc;
       const int kq = k_add[k + nc * q];
@@ -139,7 +139,7 @@ discPlanesKernel(const TpDims dims, const float2* __restrict__ G, long g_sector_
     const long o = static_cast<long>(row) * kp + slot0;
 #pragma unroll
     for (int pl = 0; pl < kPl; ++pl) {
-      if (need_u || !dims.half_g4) {
+      if (row >= u_row0) {
         store8(U + pl * plane + o, ur[pl]);
         store8(U + pl * plane + o + Kb, ui[pl]);
       }
@@ -156,7 +156,7 @@ discPlanesKernel(const TpDims dims, const float2* __restrict__ G, long g_sector_
 }  // namespace
 
 bool discGemmApplies(const TpDims& d, int max_batch) {
-  return singlebandBatchedApplies(d) && max_batch <= 256;
+  return d.n_channels > 0 && singlebandBatchedApplies(d) && max_batch <= 256;
 }
 
 size_t discScratchBytes(const TpDims& d, int max_batch) {
@@ -194,12 +194,13 @@ const float2* launchDiscGemm(const G4Args& a, const float2* G, long g_sector_str
     return nullptr;
   const TpDims& d = a.dims;
   const DiscShape s = discShape(d, w->max_batch);
+  const int mt0 = d.half_g4 ? s.M / 2 / kBM : 0;  // half G4: the row tiles that hold w1 >= Nw / 2
   {
     const long work = long(s.Kb / 8) * s.Mp;
     const dim3 grid(static_cast<unsigned>(std::max(1L, std::min(1024L, (work + 255) / 256))), d.nq * d.nwq,
                     d.n_channels);
     discPlanesKernel<<<grid, 256, 0, stream>>>(d, G, g_sector_stride, a.signs, a.n_slots, s.Kb, s.Mp, a.k_add,
-                                               a.q_list, a.wex_list, static_cast<__half*>(w->U),
+                                               a.q_list, a.wex_list, mt0 * kBM, static_cast<__half*>(w->U),
                                                static_cast<__half*>(w->V), w->eU, w->eV);
     DCAACC_LAUNCH_CHECK();
   }
@@ -209,7 +210,7 @@ const float2* launchDiscGemm(const G4Args& a, const float2* G, long g_sector_str
   p.D = s.M;
   p.Dp = s.Mp;
   p.Kr = s.Kb;
-  p.mt0 = d.half_g4 ? s.M / 2 / kBM : 0;  // half G4: the rows (k1, w1) with w1 >= Nw / 2 only
+  p.mt0 = mt0;
   p.mt = s.Mp / kBM - p.mt0;
   p.nt = s.Mp / kBN;
   p.err = a.err;

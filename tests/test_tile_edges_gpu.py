@@ -1,0 +1,124 @@
+"""Sizes at which the tiled kernels can go wrong: clusters, bands, frequencies and expansion orders that
+do not fill a tile, orbitals without vertices, transfer lists that are cut, unsorted or repeated.  Against
+the oracle, at the tolerances of the other GPU tests (the same arithmetic at other sizes)."""
+
+import numpy as np
+import pytest
+
+from helpers import rel_err
+from dca_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+FP64_TOL, MIXED_TOL, SP_TOL = 1e-12, 1e-6, 1e-9
+
+CLUSTERS = {"2x1": W.make_cluster((2, 0), (0, 1)), "3x2": W.make_cluster((3, 0), (0, 2)),
+            "2x2": W.square_cluster(2), "betts8": W.betts8_cluster(), "4x4": W.square_cluster(4),
+            "5x5": W.square_cluster(5), "6x6": W.square_cluster(6)}
+
+
+def _g0(rng, nb, cl, n_sp):
+    """A G0 with the layout of workloads.make_g0 and random band blocks (nb = 1: time-reversal symmetric,
+    as the models' is, so that the mirrored path runs)."""
+    if nb == 1:
+        return W.make_g0(W.Model("single", tp=-0.1), cl, 7.0, 0.3, n_sp)
+    nc = cl.nc
+    g = np.zeros((2 * n_sp, nc, 2, nb, 2, nb), complex)
+    for s in range(2):
+        g[:, :, s, :, s, :] = rng.normal(size=(2 * n_sp, nc, nb, nb)) + 1j * rng.normal(size=(2 * n_sp, nc, nb, nb))
+    return g
+
+
+def _measurements(rng, nb, nc, orders):
+    # One sign in five negative: with as many of both the beta^2 G0 G0 terms, the same in every measurement,
+    # cancel, and their FP32 rounding (6e-8 of the uncancelled sum) is all that a relative error sees.
+    return [W.Measurement(-1 if i % 5 == 4 else 1, tuple(W.make_sector(rng, n, nb, nc, 7.0) for n in pair))
+            for i, pair in enumerate(orders)]
+
+
+def _params(nb, cl, nw_half, n_sp, channels, k_ex, w_ex, orders, **kw):
+    from dca_b200.accumulators import TpParameters
+    a_vecs = np.zeros((1, 2)) if nb == 1 else np.linspace(0, 0.5, 2 * nb).reshape(nb, 2)
+    return TpParameters(nb, cl.nc, nw_half, n_sp, 7.0, channels, k_ex, w_ex, cl.r_vecs, cl.k_vecs, a_vecs, cl.k_add,
+                        cl.k_sub, cl.r_sub, max_order=max(1, max(max(p) for p in orders)), **kw)
+
+
+def _compare(oracle_lib, g0, measurements, params, tol):
+    from dca_b200.accumulators import TpAccumulator
+    ora = oracle_lib.OracleTp(g0, params)
+    acc = TpAccumulator(g0, params)
+    acc.resetAccumulation(0)
+    for m in measurements:
+        for a in (ora, acc):
+            a.accumulate([s.M for s in m.sectors], list(m.sectors), m.sign)
+    acc.finalize()
+    for got, want in zip(acc.get_G4(), ora.get_G4()):
+        assert np.all(np.isfinite(got))
+        assert rel_err(got, want) <= tol
+    return acc
+
+
+@pytest.mark.parametrize("precision,tol", [(0, FP64_TOL), (1, MIXED_TOL)])
+@pytest.mark.parametrize("cluster,nb,nw_half,w_ex,orders", [
+    ("2x1", 1, 1, [0], [(1, 0), (3, 2)]),             # D = 4: less than one tile of rows
+    ("3x2", 1, 5, [0, 1], [(33, 31), (1, 64)]),       # 6 sites: no FFT, momenta not a multiple of 8
+    ("2x2", 2, 3, [1], [(17, 40), (0, 5)]),           # two bands
+    ("2x1", 4, 2, [0], [(9, 30), (32, 1)]),           # more bands than the compiled cases
+    ("betts8", 3, 3, [0, 2], [(47, 18), (5, 100)]),   # three bands, rows not a multiple of the tile
+    ("4x4", 1, 5, [0], [(1, 33), (130, 7)]),          # 4 x 4 FFT, 10 frequencies, most orbitals empty
+    ("5x5", 1, 2, [0], [(40, 70), (2, 25)]),          # 25 sites: matrix transform
+    ("6x6", 1, 3, [0], [(40, 0), (97, 5)]),           # 6 x 6 FFT, 6 frequencies
+])
+def test_front_end_tiles(oracle_lib, precision, tol, cluster, nb, nw_half, w_ex, orders):
+    rng = np.random.default_rng(5)
+    cl = CLUSTERS[cluster]
+    n_sp = nw_half + max(w_ex) + 3
+    params = _params(nb, cl, nw_half, n_sp, [W.PH_MAGNETIC], [cl.nc - 1], w_ex, orders, precision=precision,
+                     max_batch=2 if precision else 1)
+    _compare(oracle_lib, _g0(rng, nb, cl, n_sp), _measurements(rng, nb, cl.nc, orders), params, tol)
+
+
+@pytest.mark.parametrize("cluster,k_ex,n_meas,max_batch", [
+    ("2x2", [3], 20, 20), ("2x2", [2, 0, 2], 3, 2), ("betts8", [1, 5, 2, 7, 0], 15, 15), ("4x4", [15], 8, 7),
+    ("4x4", [3, 9, 1, 14, 8], 3, 3), ("6x6", [20], 5, 5), ("6x6", [35, 1], 2, 1)])
+@pytest.mark.parametrize("channels", [[2, 3], [4, 2, 1]])
+def test_transfer_subsets(oracle_lib, cluster, k_ex, n_meas, max_batch, channels):
+    """Mixed path, cut transfer lists (the list's length against the threads' transfers, batches beyond the
+    staged measurements), the second-order terms of every channel; PH channels alone run with half of G."""
+    rng = np.random.default_rng(6)
+    cl = CLUSTERS[cluster]
+    orders = [(int(a), int(b)) for a, b in rng.integers(0, 30, (n_meas, 2))]
+    nw_half = {"4x4": 8, "6x6": 4}.get(cluster, 2)
+    params = _params(1, cl, nw_half, nw_half + 4, channels, k_ex, [0, 1] if cluster == "2x2" else [0], orders,
+                     precision=1, max_batch=max_batch)
+    _compare(oracle_lib, _g0(rng, 1, cl, nw_half + 4), _measurements(rng, 1, cl.nc, orders), params, MIXED_TOL)
+
+
+@pytest.mark.parametrize("cluster", ["2x2", "betts8", "4x4"])
+def test_all_transfers_all_channels(oracle_lib, cluster):
+    """Mixed path, every transfer, four channels in another order than their terms run."""
+    rng = np.random.default_rng(7)
+    cl = CLUSTERS[cluster]
+    orders = [(12, 7), (0, 0), (3, 25), (31, 2)]
+    k_ex = list(rng.permutation(cl.nc))
+    params = _params(1, cl, 2, 8, [3, 4, 1, 2], k_ex, [0, 1], orders, precision=1, max_batch=3)
+    _compare(oracle_lib, _g0(rng, 1, cl, 8), _measurements(rng, 1, cl.nc, orders), params, MIXED_TOL)
+
+
+@pytest.mark.parametrize("cluster,nb,n_sp,orders", [
+    ("2x2", 1, 5, [(0, 1), (2, 0)]), ("betts8", 3, 37, [(31, 32), (33, 65)]), ("3x2", 2, 64, [(7, 129)])])
+def test_single_particle_pairs(oracle_lib, cluster, nb, n_sp, orders):
+    """Pair counts around the warps' 32, frequency counts that do not fill the finalize passes."""
+    from dca_b200.accumulators import SpAccumulator, SpParameters
+    rng = np.random.default_rng(8)
+    cl = CLUSTERS[cluster]
+    params = SpParameters(nb, cl.nc, n_sp, 7.0, cl.r_sub, max_order=max(max(p) for p in orders))
+    acc, ora = SpAccumulator(params, True), oracle_lib.OracleSp(params, True)
+    acc.resetAccumulation()
+    for m in _measurements(rng, nb, cl.nc, orders):
+        for a in (acc, ora):
+            a.accumulate([s.M for s in m.sectors], list(m.sectors), m.sign)
+    acc.finalize()
+    ora.finalize()
+    assert rel_err(acc.get_sign_times_M_r_w(), ora.get()) <= SP_TOL
+    assert rel_err(acc.get_sign_times_M_r_w_sqr(), ora.get(True)) <= SP_TOL
