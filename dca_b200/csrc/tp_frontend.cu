@@ -23,12 +23,14 @@
 // whole 16 x WT tile, 2 x WT/4 sums a lane, and streams its orbital's vertices through a ring of
 // its own in shared memory, one asynchronous 16-byte copy per lane and vertex; per vertex a lane
 // reads 2 + WT/4 elements for 2 WT/4 complex multiply-adds.  Phase 2: 4 x 2 sums a lane over the
-// sites.  Both phases are bound by the FP64 pipe.  The earlier kernels gave a thread one sum, that
+// sites, or on a 4 x 4 cluster an FFT (a fifth of the matrix's FP64 operations, which were more than
+// phase 1's), one (row, frequency) pair a thread.  Both phases are bound by the FP64 pipe.  The earlier kernels gave a thread one sum, that
 // is two shared-memory reads per multiply-add, and a whole CTA one orbital at a time:
 // FRONT_BEFORE_AFTER
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "async_copy.cuh"
 #include "common.cuh"
@@ -85,12 +87,24 @@ __device__ inline void cpAsyncWait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// X[m] = sum_x e^{SIGN i pi m x / 2} z[x], in place.
+template <int SIGN>
+__device__ inline void dft4(double2& z0, double2& z1, double2& z2, double2& z3) {
+  const double2 t0 = cadd(z0, z2), t1 = csub(z0, z2), t2 = cadd(z1, z3), d = csub(z1, z3);
+  const double2 t3 = SIGN < 0 ? mk(d.y, -d.x) : mk(-d.y, d.x);
+  z0 = cadd(t0, t2);
+  z2 = csub(t0, t2);
+  z1 = cadd(t1, t3);
+  z3 = csub(t1, t3);
+}
+
 // Shared memory of a tile kernel: the orbitals' sums Z[o][w][16], the warps' rings (16 bytes per
 // lane and slot), the phases F[b][r][k] (k padded with zeros), the orbital starts and the
 // counter that hands them out.
-template <int WT>
+template <int WT, int L>
 struct Tile {
   static constexpr int kPairs = kTileR * WT;
+  static constexpr int kSums = kPairs + (L ? 1 : 0);  // stride of an orbital's sums (FFT: lanes along k, distinct banks)
   static constexpr int kThreads = kPairs;
   static constexpr int kWarps = kThreads / 32;
   static_assert(kTileR + WT <= 32, "one copy per lane and vertex");
@@ -102,22 +116,32 @@ struct Tile {
   __host__ __device__ static int kPad(const TpDims& d) {
     return d.nb == 1 ? (d.nc + 15) / 16 * 16 : (d.nc + 7) / 8 * 8;
   }
+  __host__ __device__ static int factors(const TpDims& d) {
+    return L ? WT * L * L : d.nb * d.nc * kPad(d);
+  }
   __host__ __device__ static size_t bytes(const TpDims& d) {
-    return size_t(kWarps) * kRing * 512 + sizeof(double2) * (size_t(d.n_orb) * kPairs + size_t(d.nb) * d.nc * kPad(d)) +
+    return size_t(kWarps) * kRing * 512 + sizeof(double2) * (size_t(d.n_orb) * kSums + factors(d)) +
            sizeof(int) * (d.n_orb + 2);
   }
-  // Lays the memory out and fills the phases, the starts and the counter.
+  // Lays the memory out and fills the phases (FFT: factor(w, k), in slot order), the starts and the counter.
+  template <typename Factor>
   __device__ Tile(unsigned char* raw, const TpDims& d, const double2* __restrict__ Fb,
-                  const int* __restrict__ orb_start) {
+                  const int* __restrict__ orb_start, const ColFft& fft, Factor factor) {
     ring = raw;
     Z = reinterpret_cast<double2*>(raw + kWarps * kRing * 512);
-    F = Z + d.n_orb * kPairs;
-    start = reinterpret_cast<int*>(F + d.nb * d.nc * kPad(d));
+    F = Z + d.n_orb * kSums;
+    start = reinterpret_cast<int*>(F + factors(d));
     next = start + d.n_orb + 1;
-    const int kp = kPad(d);
-    for (int i = threadIdx.x; i < d.nb * d.nc * kp; i += kThreads) {
-      const int k = i % kp, r = (i / kp) % d.nc, b = i / (kp * d.nc);
-      F[i] = k < d.nc ? Fb[(b * d.nc + k) * d.nc + r] : mk(double(0), double(0));
+    if constexpr (L > 0) {
+      for (int i = threadIdx.x; i < WT * L * L; i += kThreads)
+        F[i] = factor(i / (L * L), static_cast<int>(fft.kmap[i % (L * L)]));
+    }
+    else {
+      const int kp = kPad(d);
+      for (int i = threadIdx.x; i < d.nb * d.nc * kp; i += kThreads) {
+        const int k = i % kp, r = (i / kp) % d.nc, b = i / (kp * d.nc);
+        F[i] = k < d.nc ? Fb[(b * d.nc + k) * d.nc + r] : mk(0., 0.);
+      }
     }
     for (int i = threadIdx.x; i <= d.n_orb; i += kThreads)
       start[i] = orb_start[i];
@@ -168,7 +192,7 @@ struct Tile {
   template <bool CONJ, int KC>
   __device__ void clusterSum(double2 (&acc)[4][KC], const TpDims& d, int nb, int b, int wl, int k0) const {
     const int lane = threadIdx.x % 32, kp = kPad(d);
-    const double2* z = Z + b * kPairs + wl * kTileR + lane / 8;
+    const double2* z = Z + b * kSums + wl * kTileR + lane / 8;
     const double2* f = F + b * d.nc * kp + k0 + lane % 8;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -176,7 +200,7 @@ struct Tile {
       for (int c = 0; c < KC; ++c)
         acc[i][c] = mk(double(0), double(0));
 #pragma unroll 2
-    for (int r = 0; r < d.nc; ++r, z += nb * kPairs, f += kp) {
+    for (int r = 0; r < d.nc; ++r, z += nb * kSums, f += kp) {
       double2 zv[4], fv[KC];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
@@ -195,6 +219,29 @@ struct Tile {
         }
     }
   }
+
+  // FFT form of phase 2 (L = 4), for the 32 pairs of this warp from line wl on (two lines): the sums of site
+  // (a, b) become factor times the transform e^{SIGN i k r}, element k in place of orbital k.
+  template <int SIGN>
+  __device__ void fftLines(const ColFft& fft, int wl) const {
+    const int lane = threadIdx.x % 32;
+    double2* p = Z + wl * kTileR + lane;
+    double2 z[16];
+#pragma unroll
+    for (int g = 0; g < 16; ++g)
+      z[g] = p[fft.rmap[g] * kSums];
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      dft4<SIGN>(z[4 * b], z[4 * b + 1], z[4 * b + 2], z[4 * b + 3]);
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+      dft4<SIGN>(z[m], z[m + 4], z[m + 8], z[m + 12]);
+    const double2* f = F + (wl + lane / kTileR) * 16;
+#pragma unroll
+    for (int g = 0; g < 16; ++g)
+      p[fft.kmap[g] * kSums] = cmul(f[g], z[g]);
+    __syncwarp();
+  }
 };
 
 // Momenta of one phase 2 task: 16 of one band, or 8 with all the bands.
@@ -203,22 +250,27 @@ constexpr int kTaskK = NB == 1 ? 16 : 8;
 
 // Row transform.  grid (ceil(n_max / 16), ceil(NwExt / WT), n_sectors).  NB: bands (1, 2 or 3), 0 for
 // any number.
-template <int WT, int NB>
+template <int WT, int L, int NB>
 __global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
 rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const int* __restrict__ perm_r, const int* __restrict__ perm_c,
                    const int* __restrict__ row_start, const double2* __restrict__ Tr,
                    const double2* __restrict__ Fb,  // (r, k, b): e^{i k (r + a_b)}
                    const double2* __restrict__ G0,  // (b1, b2, k, w, s)
-                   double2* __restrict__ Xp) {
-  using T = Tile<WT>;
+                   const __grid_constant__ ColFft fft, double2* __restrict__ Xp) {
+  using T = Tile<WT, L>;
   const SectorDesc sd = sectors[blockIdx.z];
   const int n = sd.n, j0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
   if (j0 >= n)
     return;
   const int nw_ext = dims.nw_ext, R = dims.R, nb = NB ? NB : dims.nb, nc = dims.nc;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T tile(smem_raw, dims, Fb, row_start + sd.orb_off);
+  const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
+  const double norm = -1.0 / nc;
+  T tile(smem_raw, dims, Fb, row_start + sd.orb_off, fft, [&](int w, int k) {
+    const double2 g = cmul(g0s[k + nc * min(w0 + w, nw_ext - 1)], Fb[k * nc + fft.r0]);
+    return mk(norm * g.x, norm * g.y);
+  });
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
 
   // Phase 1: Z(o, w, j) = sum of T(w, i) M(i, j) over the vertices i of orbital o.  Lanes 0..15 copy
@@ -271,16 +323,27 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
         for (int a = 0; a < 2; ++a)
 #pragma unroll
           for (int b = 0; b < WT / 4; ++b) {
-            tile.Z[o * T::kPairs + (wq + 4 * b) * kTileR + jl + 8 * a] = acc[a][b];
+            tile.Z[o * T::kSums + (wq + 4 * b) * kTileR + jl + 8 * a] = acc[a][b];
             acc[a][b] = mk(double(0), double(0));
           }
       });
 
   // Phase 2: the cluster transform and the left G0, -1/Nc included.
-  const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
-  const double norm = -1.0 / nc;
-  const int k_tasks = (nc + kTaskK<NB> - 1) / kTaskK<NB>;
   const long D = static_cast<long>(R) * nw_ext;
+  if constexpr (L > 0) {
+    for (int wl = 2 * warp; wl < WT; wl += 2 * T::kWarps) {
+      tile.template fftLines<1>(fft, wl);
+      const int k = lane % 16;
+#pragma unroll 4
+      for (int i = 0; i < kTileR; ++i) {  // two elements of the line pair a step: j = j0 + (e % 16)
+        const int e = 2 * i + lane / 16, w = w0 + wl + e / kTileR, j = j0 + e % kTileR;
+        if (w < nw_ext && j < n)
+          Xp[sd.x_off + j * D + static_cast<long>(w) * R + k] = tile.Z[k * T::kSums + wl * kTileR + e];
+      }
+    }
+    return;
+  }
+  const int k_tasks = (nc + kTaskK<NB> - 1) / kTaskK<NB>;
   for (int task = warp; task < WT * k_tasks; task += T::kWarps) {
     const int wl = task % WT, k0 = task / WT * kTaskK<NB>, w = w0 + wl;
     if (w >= nw_ext)
@@ -356,19 +419,22 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
 
 // Column transform + G epilogue.  grid (ceil(D / 16), ceil(NwExt / WT), n_sectors); the rows of a tile
 // are 16 consecutive (w1, r).
-template <int WT, int NB>
+template <int WT, int L, int NB>
 __global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
 colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const int* __restrict__ col_start, const double2* __restrict__ Tc,
                    const double2* __restrict__ Fb,
                    const double2* __restrict__ G0,  // (b1, b2, k, w, s)
-                   const double2* __restrict__ Xp, double2* __restrict__ G, long g_sector_stride) {
-  using T = Tile<WT>;
+                   const __grid_constant__ ColFft fft, const double2* __restrict__ Xp, double2* __restrict__ G,
+                   long g_sector_stride) {
+  using T = Tile<WT, L>;
   const SectorDesc sd = sectors[blockIdx.z];
   const int nw_ext = dims.nw_ext, R = dims.R, nb = NB ? NB : dims.nb, nc = dims.nc;
   const int D = R * nw_ext, row0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T tile(smem_raw, dims, Fb, col_start + sd.orb_off);
+  const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
+  T tile(smem_raw, dims, Fb, col_start + sd.orb_off, fft,
+         [&](int w, int k) { return cmulc(g0s[k + nc * min(w0 + w, nw_ext - 1)], Fb[k * nc + fft.r0]); });
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
 
   // Phase 1: Z(o, w2, row) = sum of X'(row, j) conj T(w2, j) over the vertices j of orbital o.
@@ -407,15 +473,35 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
         for (int a = 0; a < 2; ++a)
 #pragma unroll
           for (int b = 0; b < WT / 4; ++b) {
-            tile.Z[o * T::kPairs + (wq + 4 * b) * kTileR + rl + 8 * a] = acc[a][b];
+            tile.Z[o * T::kSums + (wq + 4 * b) * kTileR + rl + 8 * a] = acc[a][b];
             acc[a][b] = mk(double(0), double(0));
           }
       });
 
   // Phase 2: the cluster transform with conjugate phases, the right G0 and the delta term.
-  const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
   const double beta = dims.beta;
   double2* out = G + g_sector_stride * (2 * sd.slot + sd.spin);
+  if constexpr (L > 0) {
+    for (int wl = 2 * warp; wl < WT; wl += 2 * T::kWarps) {
+      tile.template fftLines<-1>(fft, wl);
+      const int k = lane % 16;
+#pragma unroll 4
+      for (int i = 0; i < kTileR; ++i) {
+        const int e = 2 * i + lane / 16, w2 = w0 + wl + e / kTileR, row = row0 + e % kTileR;
+        if (w2 >= nw_ext || row >= D)
+          continue;
+        const int w1 = row / 16, r = row % 16;
+        double2 v = tile.Z[k * T::kSums + wl * kTileR + e];
+        if (w1 == w2 && r == k) {
+          const double2 dl = g0s[k + nc * w2];
+          v.x = fma(beta, dl.x, v.x);
+          v.y = fma(beta, dl.y, v.y);
+        }
+        out[((static_cast<long>(w1) * nw_ext + w2) * 16 + r) * 16 + k] = v;
+      }
+    }
+    return;
+  }
   const int k_tasks = (nc + kTaskK<NB> - 1) / kTaskK<NB>;
   for (int task = warp; task < WT * k_tasks; task += T::kWarps) {
     const int wl = task % WT, k0 = task / WT * kTaskK<NB>, w2 = w0 + wl;
@@ -499,6 +585,42 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
 // ------------------------------------------------------------------------------------------------
 // Host launchers
 // ------------------------------------------------------------------------------------------------
+ColFft clusterFft4(int nb, int nc, const double* r_vecs, const double* k_vecs) {
+  ColFft f{};
+  if (nb != 1 || nc != 16)
+    return f;
+  constexpr double tol = 4e-15;  // rounding of 2 pi m / 4 alone: the phases are the FFT's to FP64
+  int site[16], mom[16];
+  std::fill(site, site + 16, -1);
+  std::fill(mom, mom + 16, -1);
+  f.r0 = -1;
+  for (int i = 0; i < nc; ++i) {
+    const double c[4] = {r_vecs[2 * i], r_vecs[2 * i + 1], k_vecs[2 * i] * (2 / M_PI), k_vecs[2 * i + 1] * (2 / M_PI)};
+    int g[4];
+    for (int j = 0; j < 4; ++j) {
+      const long n = std::lround(c[j]);
+      if (!(std::abs(c[j] - n) <= (j < 2 ? 0 : tol)))
+        return ColFft{};
+      g[j] = int(n & 3);
+    }
+    int &s = site[g[0] + 4 * g[1]], &m = mom[g[2] + 4 * g[3]];
+    if (s >= 0 || m >= 0)
+      return ColFft{};
+    s = m = i;
+    if (c[0] == 0 && c[1] == 0)
+      f.r0 = i;
+  }
+  if (f.r0 < 0)
+    return ColFft{};
+  for (int g = 0; g < 16; ++g) {
+    f.rmap[g] = static_cast<unsigned char>(site[g]);
+    f.kmap[g] = static_cast<unsigned char>(mom[g]);
+  }
+  f.on = 1;
+  f.L = 4;
+  return f;
+}
+
 void launchTwiddles(const FrontendArgs& a, cudaStream_t stream) {
   const dim3 grid(a.n_max, a.n_sectors);
   twiddleKernel<<<grid, 128, 0, stream>>>(a.sectors, a.tau, a.perm_r, a.Tr, a.dims.nw_ext, a.dims.beta);
@@ -523,33 +645,42 @@ size_t frontendSmemRequirement(const TpDims& d, int /*n_max*/, bool fp64) {
   return std::max(row, col);
 }
 
+static bool fft4(const FrontendArgs& a) {
+  return a.dims.nb == 1 && a.fft.on && a.fft.L == 4;
+}
+
 // Frequencies per CTA, 16 or 8, which the tuner chooses between: every element is the same sum in the
 // same order either way.  8 alone where 16 does not fit in shared memory.
 static int tileWidth(const FrontendArgs& a, const char* family, LaunchTuner::Pick& pk, cudaStream_t stream) {
-  const bool wide = Tile<16>::bytes(a.dims) <= 227 * 1024;
+  const bool wide = (fft4(a) ? Tile<16, 4>::bytes(a.dims) : Tile<16, 0>::bytes(a.dims)) <= 227 * 1024;
   pk = tunePick(a.tuner, tuneKey(family, a.dims.nb, a.dims.nc, a.dims.nw_ext, a.n_max, a.n_sectors, 8),
                 wide ? 2 : 1, stream);
   return wide && pk.choice == 0 ? 16 : 8;
 }
 
-template <int WT, typename Kernel, typename... Args>
+template <int WT, int L, typename Kernel, typename... Args>
 static void launchTile(Kernel k, const TpDims& d, int tiles, int sectors, cudaStream_t stream, Args... args) {
-  const size_t smem = Tile<WT>::bytes(d);
+  const size_t smem = Tile<WT, L>::bytes(d);
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          int(cudaSharedmemCarveoutMaxShared)));
-  k<<<dim3(tiles, ceil_div(d.nw_ext, WT), sectors), Tile<WT>::kThreads, smem, stream>>>(d, args...);
+  k<<<dim3(tiles, ceil_div(d.nw_ext, WT), sectors), Tile<WT, L>::kThreads, smem, stream>>>(d, args...);
   DCAACC_LAUNCH_CHECK();
 }
 
 template <int WT>
 static void launchRowWT(const FrontendArgs& a, double2* Xp, cudaStream_t stream) {
-  const int nb = a.dims.nb;
-  auto k = nb == 1   ? rowTransformKernel<WT, 1>
-           : nb == 2 ? rowTransformKernel<WT, 2>
-           : nb == 3 ? rowTransformKernel<WT, 3> : rowTransformKernel<WT, 0>;
-  launchTile<WT>(k, a.dims, ceil_div(a.n_max, kTileR), a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
-                       a.row_start, a.Tr, a.Fb, a.G0, Xp);
+  const int nb = a.dims.nb, tiles = ceil_div(a.n_max, kTileR);
+  if (fft4(a)) {
+    launchTile<WT, 4>(rowTransformKernel<WT, 4, 1>, a.dims, tiles, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
+                      a.row_start, a.Tr, a.Fb, a.G0, a.fft, Xp);
+    return;
+  }
+  auto k = nb == 1   ? rowTransformKernel<WT, 0, 1>
+           : nb == 2 ? rowTransformKernel<WT, 0, 2>
+           : nb == 3 ? rowTransformKernel<WT, 0, 3> : rowTransformKernel<WT, 0, 0>;
+  launchTile<WT, 0>(k, a.dims, tiles, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c, a.row_start, a.Tr, a.Fb, a.G0,
+                    a.fft, Xp);
 }
 
 void launchRowTransform(const FrontendArgs& a, double2* Xp, cudaStream_t stream) {
@@ -564,14 +695,18 @@ void launchRowTransform(const FrontendArgs& a, double2* Xp, cudaStream_t stream)
 }
 
 template <int WT>
-static void launchColWT(const FrontendArgs& a, const double2* Xp, double2* G, long g_sector_stride,
-                        cudaStream_t stream) {
-  const int nb = a.dims.nb;
-  auto k = nb == 1   ? colTransformKernel<WT, 1>
-           : nb == 2 ? colTransformKernel<WT, 2>
-           : nb == 3 ? colTransformKernel<WT, 3> : colTransformKernel<WT, 0>;
-  launchTile<WT>(k, a.dims, ceil_div(long(a.dims.R) * a.dims.nw_ext, kTileR), a.n_sectors, stream, a.sectors,
-                       a.col_start, a.Tc, a.Fb, a.G0, Xp, G, g_sector_stride);
+static void launchColWT(const FrontendArgs& a, const double2* Xp, double2* G, long g_sector_stride, cudaStream_t stream) {
+  const int nb = a.dims.nb, tiles = ceil_div(long(a.dims.R) * a.dims.nw_ext, kTileR);
+  if (fft4(a)) {
+    launchTile<WT, 4>(colTransformKernel<WT, 4, 1>, a.dims, tiles, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb,
+                      a.G0, a.fft, Xp, G, g_sector_stride);
+    return;
+  }
+  auto k = nb == 1   ? colTransformKernel<WT, 0, 1>
+           : nb == 2 ? colTransformKernel<WT, 0, 2>
+           : nb == 3 ? colTransformKernel<WT, 0, 3> : colTransformKernel<WT, 0, 0>;
+  launchTile<WT, 0>(k, a.dims, tiles, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb, a.G0, a.fft, Xp, G,
+                    g_sector_stride);
 }
 
 void launchColTransform(const FrontendArgs& a, const double2* Xp, double2* G,

@@ -10,6 +10,16 @@
 
 namespace dcaacc {
 
+// The cluster transform of an L x L square cluster (L = 4 or 6) as a 2D FFT: grid point g = a + L b
+// is site rmap[g] (coordinates (a, b)) and momentum kmap[g] (2 pi (a, b) / L); r0 is the site at
+// the origin.  Set up on the host when the cluster's phase table has exactly that structure.
+struct ColFft {
+  int on;
+  int r0;
+  int L;
+  unsigned char rmap[36], kmap[36];
+};
+
 struct FrontendArgs {
   TpDims dims;
   const SectorDesc* sectors;  // [n_sectors], device
@@ -25,7 +35,11 @@ struct FrontendArgs {
   const double2* Fb;          // (r, k, b): e^{i k (r + a_b)}, nb * Nc * Nc
   const double2* G0;          // (b1, b2, k, w, s) over the extended mesh
   LaunchTuner* tuner;         // launch-shape tuner (null: the built-in shapes)
+  ColFft fft;                 // FP64 front-end: the cluster transform as an FFT, when fft.on
 };
+
+// The FFT of one band on a 4 x 4 cluster with integer sites and momenta 2 pi (m, n) / 4 (off otherwise).
+ColFft clusterFft4(int nb, int nc, const double* r_vecs, const double* k_vecs);
 
 void launchTwiddles(const FrontendArgs& a, cudaStream_t stream);
 
@@ -49,16 +63,6 @@ struct FrontTcShape {
   int n_sectors;
   size_t pr_elems, mb_elems, ac_elems, bq_elems;  // FP16 elements of P, M, X' and Q planes
 };
-// The cluster transform of an L x L square cluster (L = 4 or 6) as a 2D FFT: grid point g = a + L b
-// is site rmap[g] (coordinates (a, b)) and momentum kmap[g] (2 pi (a, b) / L); r0 is the site at
-// the origin.  Set up on the host when the cluster's phase table has exactly that structure.
-struct ColFft {
-  int on;
-  int r0;
-  int L;
-  unsigned char rmap[36], kmap[36];
-};
-
 // ---- FP32 front-end of the mixed path, factored by orbital (tp_frontend32.cu) ----
 struct Front32Workspace {
   // Each of T2, T4 and X is followed by kFront32Pad vertices' worth of memory that copies may run into.
