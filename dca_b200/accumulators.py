@@ -230,6 +230,7 @@ class TpAccumulator:
         _check(N.lib.dcaacc_tp_create(ctypes.byref(cfg), g0.view(np.float64).ctypes.data_as(
             ctypes.POINTER(ctypes.c_double)), ctypes.byref(self._h)))
         self._g4: Optional[List[np.ndarray]] = None
+        self._g4_arrays: List[np.ndarray] = []
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -306,13 +307,18 @@ class TpAccumulator:
     def finalize(self):
         _check(N.lib.dcaacc_tp_finalize(self._h))
         size = N.lib.dcaacc_tp_g4_size(self._h)
-        out = []
+        self._g4 = None
+        # The arrays of an earlier result are used again when nothing else refers to them (or to a view of
+        # them): memory that has been touched takes the copy several times as fast as new memory.
+        held = self._g4_arrays
         for c in range(len(self.parameters.channels)):
-            g = np.empty(size, np.complex128)
-            _check(N.lib.dcaacc_tp_get_g4(self._h, c, g.view(np.float64).ctypes.data_as(
+            if c == len(held):
+                held.append(np.empty(size, np.complex128))
+            elif sys.getrefcount(held[c]) > 2:  # the list's and the call's own references
+                held[c] = np.empty(size, np.complex128)
+            _check(N.lib.dcaacc_tp_get_g4(self._h, c, held[c].view(np.float64).ctypes.data_as(
                 ctypes.POINTER(ctypes.c_double)), size))
-            out.append(g)
-        self._g4 = out
+        self._g4 = list(held)
 
     def get_G4(self) -> List[np.ndarray]:
         if self._g4 is None:

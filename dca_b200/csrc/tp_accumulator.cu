@@ -522,6 +522,10 @@ void TpAccumulator::shareG4(TpAccumulator& owner) {
     invalid("sharing G4 requires both accumulators on the same device");
   process();
   owner.process();
+  if (finalized_)
+    keepG4();
+  if (owner.finalized_)
+    owner.keepG4();
   // What this handle has accumulated so far moves into the shared G4 (with its sign sum, which
   // stays with this handle), so no measurement is dropped with the released buffers.
   if (n_meas_ > 0) {
@@ -980,17 +984,28 @@ void TpAccumulator::finalize() {
   if (finalized_)
     return;
   process();
-  for (size_t c = 0; c < g4().size(); ++c) {
-    if (dims_.half_g4)  // the entries with w1 < Nw / 2 from their mirrors
-      launchG4Mirror(g4()[c].get(), dims_, q_mirror_d_.get(), wq_mirror_d_.get(), stream_);
-    G4_host_[c].resize(g4_size_);
-    DCAACC_CUDA_CHECK(cudaMemcpyAsync(G4_host_[c].data(), g4()[c].get(), g4()[c].bytes(),
-                                      cudaMemcpyDeviceToHost, stream_));
-  }
+  if (dims_.half_g4)  // the entries with w1 < Nw / 2 from their mirrors
+    for (auto& g : g4())
+      launchG4Mirror(g.get(), dims_, q_mirror_d_.get(), wq_mirror_d_.get(), stream_);
   DCAACC_CUDA_CHECK(cudaStreamSynchronize(stream_));
   checkDeviceError();
+  for (auto& h : G4_host_)
+    h.clear();
+  if (g4Shared())  // the other handles may go on
+    keepG4();
   finalized_ = true;
   ready_ = false;
+}
+
+// The finalized G4 stays on the device, where get_g4 reads it, until something is about to change it.
+void TpAccumulator::keepG4() {
+  for (size_t c = 0; c < g4().size(); ++c)
+    if (G4_host_[c].empty()) {
+      G4_host_[c].resize(g4_size_);
+      DCAACC_CUDA_CHECK(cudaMemcpyAsync(G4_host_[c].data(), g4()[c].get(), g4()[c].bytes(), cudaMemcpyDeviceToHost,
+                                        stream_));
+    }
+  DCAACC_CUDA_CHECK(cudaStreamSynchronize(stream_));
 }
 
 void TpAccumulator::checkDeviceError() {
@@ -1010,7 +1025,12 @@ void TpAccumulator::getG4(int channel, double* out, size_t count) const {
     invalid("channel index out of range");
   if (count != g4_size_)
     invalid("output size does not match the G4 size");
-  std::memcpy(out, G4_host_[channel].data(), 16 * count);
+  if (!G4_host_[channel].empty()) {
+    std::memcpy(out, G4_host_[channel].data(), 16 * count);
+    return;
+  }
+  DCAACC_CUDA_CHECK(cudaMemcpyAsync(out, g4()[channel].get(), 16 * count, cudaMemcpyDeviceToHost, stream_));
+  DCAACC_CUDA_CHECK(cudaStreamSynchronize(stream_));
 }
 
 void TpAccumulator::sumTo(TpAccumulator& other) {
@@ -1022,6 +1042,8 @@ void TpAccumulator::sumTo(TpAccumulator& other) {
     invalid("sumTo requires both accumulators on the same device");
   process();
   other.process();
+  if (finalized_)
+    keepG4();
   if (other.g4s_ == g4s_) {  // one shared G4: nothing to add (tp_accumulator_gpu.hpp:487-491)
     // but what other reads of it afterwards (finalize, peek) comes after this handle's updates.
     cudaEvent_t done;

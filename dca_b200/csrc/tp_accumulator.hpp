@@ -276,7 +276,9 @@ private:
   bool finalized_ = false;
   bool have_g_ = false;   // FP64 mode: G of the last measurement is in G64_
   uint64_t launches_ = 0;
+  // Per channel: the finalized G4, once it no longer is what the device holds (keepG4); else empty.
   std::vector<std::vector<std::complex<double>>> G4_host_;
+  void keepG4();
 
   // Stage timing: pairs of events per recorded launch group.
   struct Timed {

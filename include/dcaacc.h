@@ -159,7 +159,9 @@ int dcaacc_tp_accumulate_batch(dcaacc_tp* acc, int32_t n_meas, const dcaacc_sect
 /* Processes queued measurements now (mixed mode).  No-op when nothing is queued. */
 int dcaacc_tp_flush(dcaacc_tp* acc);
 
-/* finalize() — tp_accumulator_gpu.hpp:471-484: flushes, then copies G4 to the host side of the handle. */
+/* finalize() — tp_accumulator_gpu.hpp:471-484: flushes and completes G4, which get_g4 then returns until the
+ * next reset (it stays on the device, and moves to the host side of the handle only when something is
+ * about to change it there: a sum_to, a G4 shared with other handles). */
 int dcaacc_tp_finalize(dcaacc_tp* acc);
 
 /* get_G4()[channel] — tp_accumulator_gpu.hpp:503-510.  Copies G4 of one channel (complex FP64,
