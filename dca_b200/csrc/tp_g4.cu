@@ -45,20 +45,23 @@ __device__ inline cplx_t<AT> ldG(const GT* p) {
   return mk(static_cast<AT>(v.x), static_cast<AT>(v.y));
 }
 
-template <typename GT, typename AT, int EPT>
+// NB: bands (1, 2, 3; 0 for any number).  A tile's entry index is decomposed with 32-bit divisions, by constants
+// where NB gives them: with 64-bit ones at run time the kernel was bound by that arithmetic (FP64, three bands on
+// 8 sites, Nw = 16, one q, two frequency transfers, one measurement: 134 -> 92 us with 32-bit ones).
+template <typename GT, typename AT, int EPT, int NB>
 __global__ void __launch_bounds__(256)
 updateG4Kernel(const TpDims dims, const GT* __restrict__ G, long g_sector_stride,
                const int* __restrict__ signs, int n_slots, const int* __restrict__ k_add,
                const int* __restrict__ k_sub, const int* __restrict__ q_list,
                const int* __restrict__ wex_list, double2* const* __restrict__ G4, bool atomic) {
   using C = cplx_t<AT>;
-  const int nb = dims.nb, nc = dims.nc, nw = dims.nw, nw_ext = dims.nw_ext, R = dims.R;
+  const int nb = NB ? NB : dims.nb, nc = dims.nc, nw = dims.nw, nw_ext = dims.nw_ext, R = dims.R;
   const int w1 = blockIdx.x, w2 = blockIdx.y, iwq = blockIdx.z;
   const int wex = wex_list[iwq];
   const int ext = dims.ext;
-  const int nb2 = nb * nb, nb4 = nb2 * nb2;
-  const int inner = nb4 * nc;                 // (b1, b2, b3, b4, k1)
-  const long per_tile = static_cast<long>(inner) * nc * dims.nq;
+  const unsigned nb2 = nb * nb, nb4 = nb2 * nb2;
+  const unsigned inner = nb4 * nc;                         // (b1, b2, b3, b4, k1)
+  const unsigned per_tile = inner * nc * dims.nq;          // the host checks that it fits
   const long blk_stride = static_cast<long>(R) * R;
 
   // Extended frequency indices of the blocks this tile reads.
@@ -77,7 +80,7 @@ updateG4Kernel(const TpDims dims, const GT* __restrict__ G, long g_sector_stride
   const long s_wq = s_q * dims.nq;
   const long tile_base = w1 * s_w1 + w2 * s_w2 + iwq * s_wq;
 
-  for (long chunk = 0; chunk < per_tile; chunk += static_cast<long>(EPT) * blockDim.x) {
+  for (unsigned chunk = 0; chunk < per_tile; chunk += EPT * 256) {
     C acc[EPT][kMaxChannels];
 #pragma unroll
     for (int e = 0; e < EPT; ++e)
@@ -91,13 +94,12 @@ updateG4Kernel(const TpDims dims, const GT* __restrict__ G, long g_sector_stride
       const GT* G1s = G0s + g_sector_stride;
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
-        const long idx = chunk + threadIdx.x + static_cast<long>(e) * blockDim.x;
+        const unsigned idx = chunk + threadIdx.x + e * 256;
         if (idx >= per_tile)
           break;
-        const int in = static_cast<int>(idx % inner);
-        const int outer = static_cast<int>(idx / inner);  // k2 + nc * q
-        const int b1 = in % nb, b2 = (in / nb) % nb, b3 = (in / nb2) % nb, b4 = (in / (nb2 * nb)) % nb;
-        const int k1 = in / nb4;
+        const unsigned in = idx % inner, outer = idx / inner;  // outer: k2 + nc * q
+        const unsigned k1 = in / nb4, bands = in % nb4;
+        const int b1 = bands % nb, b2 = bands / nb % nb, b3 = bands / nb2 % nb, b4 = bands / (nb2 * nb);
         const int k2 = outer % nc, iq = outer / nc;
         const int q = q_list[iq];
         const int k1q = k_add[k1 + nc * q], k2q = k_add[k2 + nc * q];
@@ -153,12 +155,11 @@ updateG4Kernel(const TpDims dims, const GT* __restrict__ G, long g_sector_stride
     // One read-modify-write of the FP64 running sum per entry and channel.
 #pragma unroll
     for (int e = 0; e < EPT; ++e) {
-      const long idx = chunk + threadIdx.x + static_cast<long>(e) * blockDim.x;
+      const unsigned idx = chunk + threadIdx.x + e * 256;
       if (idx >= per_tile)
         break;
-      const int in = static_cast<int>(idx % inner);
-      const int outer = static_cast<int>(idx / inner);
-      const int k2 = outer % nc, iq = outer / nc;
+      const unsigned in = idx % inner, outer = idx / inner;
+      const unsigned k2 = outer % nc, iq = outer / nc;
       const long g4i = tile_base + in + k2 * s_k2 + iq * s_q;
 #pragma unroll
       for (int c = 0; c < kMaxChannels; ++c) {
@@ -976,16 +977,16 @@ int launchUpdateG4(const G4Args& a, const GT* G, long g_sector_stride, cudaStrea
       return 1;
     }
   }
-  if constexpr (std::is_same_v<GT, double2>) {
-    updateG4Kernel<double2, double, 4><<<grid, 256, 0, stream>>>(
-        a.dims, G, g_sector_stride, a.signs, a.n_slots, a.k_add, a.k_sub, a.q_list, a.wex_list,
-        a.G4, a.atomic);
-  }
-  else {
-    updateG4Kernel<float2, float, 8><<<grid, 256, 0, stream>>>(
-        a.dims, G, g_sector_stride, a.signs, a.n_slots, a.k_add, a.k_sub, a.q_list, a.wex_list,
-        a.G4, a.atomic);
-  }
+  const TpDims& d = a.dims;
+  if (size_t(d.nb) * d.nb * d.nb * d.nb * d.nc * d.nc * d.nq >= (size_t(1) << 32) - 8 * 256)
+    throw Error(3, "more than 2^32 G4 entries per pair of frequencies");
+  using AT = std::conditional_t<std::is_same_v<GT, double2>, double, float>;
+  constexpr int EPT = std::is_same_v<GT, double2> ? 4 : 8;
+  auto k = d.nb == 1   ? updateG4Kernel<GT, AT, EPT, 1>
+           : d.nb == 2 ? updateG4Kernel<GT, AT, EPT, 2>
+           : d.nb == 3 ? updateG4Kernel<GT, AT, EPT, 3> : updateG4Kernel<GT, AT, EPT, 0>;
+  k<<<grid, 256, 0, stream>>>(d, G, g_sector_stride, a.signs, a.n_slots, a.k_add, a.k_sub, a.q_list, a.wex_list, a.G4,
+                              a.atomic);
   DCAACC_LAUNCH_CHECK();
   return 1;
 }
