@@ -103,7 +103,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
         for (int k = 0; k < nc; ++k)
           kneg.push_back(k_sub_[k + nc * z]);
     }
-  bool mirror_ok = !kneg.empty();
+  bool mirror_ok = !kneg.empty(), mirror_exact = false;
   for (size_t k = 0; k < kneg.size(); ++k)
     mirror_ok = mirror_ok && kneg[kneg[k]] == int(k);
   const long R = dims_.R;
@@ -147,6 +147,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
             dev = std::max(dev, std::hypot(a.x - b.x, a.y + b.y));
           }
       mirror_ok = dev <= 1e-12 * mx;
+      mirror_exact = dev <= 8.9e-16 * mx;  // four ulps
     }
     else {
       mirror_ok = false;
@@ -226,6 +227,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
         for (int r = 0; r < nc; ++r) {
           const double2 a = fb[size_t(k) * nc + r], b = fb[size_t(kneg[k]) * nc + r];
           mirror_ok = mirror_ok && std::hypot(a.x - b.x, a.y + b.y) <= 1e-12;
+          mirror_exact = mirror_exact && std::hypot(a.x - b.x, a.y + b.y) <= 4e-15;
         }
   }
   fft64_ = clusterFft4(nb, nc, c.r_vecs, c.k_vecs);
@@ -363,25 +365,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
         dims_.half_g = 1;
         for (int k = 0; k < nc; ++k)
           dims_.kneg[k] = static_cast<unsigned char>(kneg[k]);
-        // Half G4 when the transfer lists are closed under negation.
-        std::vector<int> qm(q_list_.size(), -1), wm(wex_list_.size(), -1);
-        for (size_t i = 0; i < q_list_.size(); ++i)
-          for (size_t j = 0; j < q_list_.size(); ++j)
-            if (q_list_[j] == kneg[q_list_[i]])
-              qm[i] = int(j);
-        for (size_t i = 0; i < wex_list_.size(); ++i)
-          for (size_t j = 0; j < wex_list_.size(); ++j)
-            if (wex_list_[j] == -wex_list_[i])
-              wm[i] = int(j);
-        const bool closed = std::count(qm.begin(), qm.end(), -1) == 0 && std::count(wm.begin(), wm.end(), -1) == 0;
-        if (closed && nw % 2 == 0) {
-          dims_.half_g4 = 1;
-          upload_ints(q_mirror_d_, qm);
-          upload_ints(wq_mirror_d_, wm);
-          // Device window for reads of the running G4 (peek), whose lower half comes from the
-          // mirror: allocated now, so that reads of up to kPeekWindow entries between batches
-          // neither allocate nor synchronise.
-          peek_d_.alloc(kPeekWindow);
+        if (nw % 2 == 0 && mirrorTransfers(kneg)) {
           // Tiles (w1, w2) with w1 >= Nw / 2, each next to the tile that reads its B block as A:
           // (w2, w1) if w2 >= Nw / 2, else the mirror (Nw - 1 - w2, Nw - 1 - w1).
           std::vector<char> seen(size_t(nw) * nw, 0);
@@ -415,6 +399,15 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
       Tc_d_.alloc(n_vtx * nw_ext);
     X64_.alloc(x_elems);
     G64_.alloc(g_elems);
+    // Half G4 in FP64 too: particle-hole channels of one band whose inputs are mirror-symmetric to the last
+    // few bits (so that an entry and its mirror agree to rounding), transfers closed under negation.
+    const char* full_env = std::getenv("DCAACC_TP_FULL_G");
+    if (!(full_env && std::strcmp(full_env, "1") == 0) && mirror_ok && mirror_exact && nb == 1 && nw % 2 == 0 &&
+        phChannels(dims_).n_channels == c.n_channels) {
+      for (int k = 0; k < nc; ++k)
+        dims_.kneg[k] = static_cast<unsigned char>(kneg[k]);
+      mirrorTransfers(kneg);
+    }
   }
   for (auto& h : hstage_) {
     h.sectors.alloc(n_sec);
@@ -434,6 +427,47 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   if ((!mixed_ || simt_only_) && frontendSmemRequirement(dims_, max_order_, !mixed_) > 227 * 1024)
     invalid("max_order too large for the front-end's shared-memory tiles");
   G4_host_.assign(c.n_channels, {});
+}
+
+// Half G4 (dims_.half_g4) when the transfer lists are closed under negation: their negatives' positions, and a
+// device window for reads of the running G4 (peek), whose lower half comes from the mirror, allocated now
+// so that reads of up to kPeekWindow entries between batches neither allocate nor synchronise.
+bool TpAccumulator::mirrorTransfers(const std::vector<int>& kneg) {
+  std::vector<int> qm(q_list_.size(), -1), wm(wex_list_.size(), -1);
+  for (size_t i = 0; i < q_list_.size(); ++i)
+    for (size_t j = 0; j < q_list_.size(); ++j)
+      if (q_list_[j] == kneg[q_list_[i]])
+        qm[i] = int(j);
+  for (size_t i = 0; i < wex_list_.size(); ++i)
+    for (size_t j = 0; j < wex_list_.size(); ++j)
+      if (wex_list_[j] == -wex_list_[i])
+        wm[i] = int(j);
+  if (std::count(qm.begin(), qm.end(), -1) || std::count(wm.begin(), wm.end(), -1))
+    return false;
+  dims_.half_g4 = 1;
+  q_mirror_d_.alloc(qm.size());
+  DCAACC_CUDA_CHECK(cudaMemcpy(q_mirror_d_.get(), qm.data(), q_mirror_d_.bytes(), cudaMemcpyHostToDevice));
+  wq_mirror_d_.alloc(wm.size());
+  DCAACC_CUDA_CHECK(cudaMemcpy(wq_mirror_d_.get(), wm.data(), wq_mirror_d_.bytes(), cudaMemcpyHostToDevice));
+  peek_d_.alloc(kPeekWindow);
+  return true;
+}
+
+// An FP64 handle's G4 (and that of the FP64 handles sharing it) completed from its mirror; all of it is
+// accumulated from then on.
+void TpAccumulator::completeG4() {
+  if (mixed_ || !dims_.half_g4)
+    return;
+  std::lock_guard<std::mutex> lock(g4s_->m);
+  for (TpAccumulator* u : g4s_->users)
+    DCAACC_CUDA_CHECK(cudaStreamSynchronize(u->stream_));
+  for (auto& g : g4())
+    launchG4Mirror(g.get(), dims_, q_mirror_d_.get(), wq_mirror_d_.get(), stream_);
+  DCAACC_CUDA_CHECK(cudaStreamSynchronize(stream_));
+  for (TpAccumulator* u : g4s_->users) {
+    u->dims_.half_g4 = 0;
+    u->releaseGraphs();  // the mode is a kernel argument
+  }
 }
 
 TpAccumulator::~TpAccumulator() {
@@ -516,10 +550,17 @@ bool TpAccumulator::sameG4(const TpAccumulator& o) const {
 void TpAccumulator::shareG4(TpAccumulator& owner) {
   if (&owner == this || owner.g4s_ == g4s_)
     return;
-  if (!sameG4(owner) || owner.dims_.half_g4 != dims_.half_g4)
-    invalid("accumulators with different G4 shapes, transfers, channels, beta or mirror modes cannot share G4");
+  if (!sameG4(owner))
+    invalid("accumulators with different G4 shapes, transfers, channels or beta cannot share G4");
   if (owner.device_ != device_)
     invalid("sharing G4 requires both accumulators on the same device");
+  // FP64 handles give up the half G4 where the other handle has no equal one (mixed precision, G0 of less symmetry).
+  if (mixed_ != owner.mixed_ || owner.dims_.half_g4 != dims_.half_g4) {
+    completeG4();
+    owner.completeG4();
+  }
+  if (owner.dims_.half_g4 != dims_.half_g4)
+    invalid("accumulators with different G4 shapes, transfers, channels, beta or mirror modes cannot share G4");
   process();
   owner.process();
   if (finalized_)
@@ -1187,14 +1228,13 @@ void TpAccumulator::peekG4(int channel, size_t offset, size_t count, double* out
     invalid("window outside G4");
   process();
   const double2* src = g4()[channel].get() + offset;
-  if (dims_.half_g4) {  // entries with w1 < Nw / 2 come from their mirrors
-    if (peek_d_.size() < count) {
-      DCAACC_CUDA_CHECK(cudaStreamSynchronize(stream_));  // earlier reads may still use the window
-      peek_d_.alloc(count);
-    }
+  if (dims_.half_g4 && count <= peek_d_.size()) {  // entries with w1 < Nw / 2 come from their mirrors
     launchG4Window(g4()[channel].get(), dims_, q_mirror_d_.get(), wq_mirror_d_.get(), offset, count, peek_d_.get(),
                    stream_);
     src = peek_d_.get();
+  }
+  else if (dims_.half_g4) {  // a large window: filled in place, where the update never reads them
+    launchG4Mirror(g4()[channel].get(), dims_, q_mirror_d_.get(), wq_mirror_d_.get(), stream_);
   }
   DCAACC_CUDA_CHECK(cudaMemcpyAsync(out, src, 16 * count, cudaMemcpyDeviceToHost, stream_));
   if (wait)

@@ -122,7 +122,7 @@ public:
   void synchronize();
   size_t deviceFingerprint() const;
   int mirrorMode() const {
-    return (dims_.half_g ? 1 : 0) | (dims_.half_g4 ? 2 : 0);
+    return mixed_ ? (dims_.half_g ? 1 : 0) | (dims_.half_g4 ? 2 : 0) : 0;
   }
   uint64_t kernelLaunches() const {
     return launches_;
@@ -279,6 +279,8 @@ private:
   // Per channel: the finalized G4, once it no longer is what the device holds (keepG4); else empty.
   std::vector<std::vector<std::complex<double>>> G4_host_;
   void keepG4();
+  bool mirrorTransfers(const std::vector<int>& kneg);
+  void completeG4();
 
   // Stage timing: pairs of events per recorded launch group.
   struct Timed {

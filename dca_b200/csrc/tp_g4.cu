@@ -56,7 +56,7 @@ updateG4Kernel(const TpDims dims, const GT* __restrict__ G, long g_sector_stride
                const int* __restrict__ wex_list, double2* const* __restrict__ G4, bool atomic) {
   using C = cplx_t<AT>;
   const int nb = NB ? NB : dims.nb, nc = dims.nc, nw = dims.nw, nw_ext = dims.nw_ext, R = dims.R;
-  const int w1 = blockIdx.x, w2 = blockIdx.y, iwq = blockIdx.z;
+  const int w1 = blockIdx.x + dims.nw - gridDim.x, w2 = blockIdx.y, iwq = blockIdx.z;  // half G4: w1 >= Nw / 2
   const int wex = wex_list[iwq];
   const int ext = dims.ext;
   const unsigned nb2 = nb * nb, nb4 = nb2 * nb2;
@@ -204,7 +204,7 @@ updateG4StagedKernel(const TpDims dims, const GT* __restrict__ G, long g_sector_
   using C = cplx_t<AT>;
   static_assert(NCH >= 1 && NCH <= kStagedMaxCh, "channels");
   const int nb = dims.nb, nc = dims.nc, nw = dims.nw, nw_ext = dims.nw_ext, R = dims.R;
-  const int w1 = blockIdx.x, w2 = blockIdx.y, iwq = blockIdx.z;
+  const int w1 = blockIdx.x + dims.nw - gridDim.x, w2 = blockIdx.y, iwq = blockIdx.z;  // half G4: w1 >= Nw / 2
   const int wex = wex_list[iwq];
   const int ext = dims.ext;
   const int nb2 = nb * nb, nb4 = nb2 * nb2;
@@ -432,7 +432,7 @@ updateG4SinglebandPH(const TpDims dims, const GT* __restrict__ G, long g_sector_
                      int* __restrict__ err) {
   using C = cplx_t<AT>;
   const int nc = dims.nc, nw = dims.nw, nw_ext = dims.nw_ext, R = dims.R, nq = dims.nq;
-  const int w1 = blockIdx.x, w2 = blockIdx.y;
+  const int w1 = blockIdx.x + nw - gridDim.x, w2 = blockIdx.y;  // half G4: w1 >= Nw / 2
   const int n_qchunks = (nq + q_chunk - 1) / q_chunk;
   const int iwq = blockIdx.z / n_qchunks, q0 = (blockIdx.z % n_qchunks) * q_chunk;
   const int wex = wex_list[iwq];
@@ -628,7 +628,8 @@ updateG4SinglebandStream(const TpDims dims, const GT* __restrict__ G, long g_sec
   constexpr int stage_elems = 2 * (blkA + 3 * blk);  // per spin: A (padded), B, C, E
   constexpr int QSTEP = 256 / (NC * NC);             // transfers between a thread's entries
   const int nw = dims.nw, nw_ext = dims.nw_ext, nq = dims.nq, ext = dims.ext;
-  const int n_tiles = nw * nw * dims.nwq;
+  const int nw1 = dims.half_g4 ? nw / 2 : nw, w1_lo = nw - nw1;  // half G4: w1 >= Nw / 2
+  const int n_tiles = nw1 * nw * dims.nwq;
   const int t = threadIdx.x;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);  // [2]
@@ -650,7 +651,7 @@ updateG4SinglebandStream(const TpDims dims, const GT* __restrict__ G, long g_sec
   // Warp 0 issues a tile's copies: per spin, A row by row (padded), then B, C, E whole.
   constexpr uint32_t row_bytes = R * sizeof(GT), blk_bytes = row_bytes * R;
   auto issue = [&](int tile, int st) {
-    const int w1 = tile % nw, w2 = (tile / nw) % nw, iwq = tile / (nw * nw);
+    const int w1 = w1_lo + tile % nw1, w2 = (tile / nw1) % nw, iwq = tile / (nw1 * nw);
     const int wex = wex_list[iwq];
     const int w1e = w1 + ext, w2e = w2 + ext, w1x = w1e + wex, w2x = w2e + wex;
     const long bA = (static_cast<long>(w1e) * nw_ext + w2e) * blk, bB = (static_cast<long>(w2x) * nw_ext + w1x) * blk,
@@ -712,7 +713,7 @@ updateG4SinglebandStream(const TpDims dims, const GT* __restrict__ G, long g_sec
       __syncwarp();
       issue(tile + gridDim.x, st ^ 1);
     }
-    const int w1 = tile % nw, w2 = (tile / nw) % nw, iwq = tile / (nw * nw);
+    const int w1 = w1_lo + tile % nw1, w2 = (tile / nw1) % nw, iwq = tile / (nw1 * nw);
     const long base = static_cast<long>(w1) * NC + w2 * s_w2 + iwq * s_wq + own;
     const bool ok = mbarWait(&bar[st], (it >> 1) & 1, err);
     if (!__syncthreads_and(ok)) {
@@ -794,10 +795,11 @@ updateG4SinglebandGather(const TpDims dims, const GT* __restrict__ G, long g_sec
                          double2* const* __restrict__ G4, bool atomic) {
   using C = cplx_t<AT>;
   const int nc = dims.nc, nw = dims.nw, nw_ext = dims.nw_ext, blk = nc * nc;
+  const int nw1 = dims.half_g4 ? nw / 2 : nw;  // half G4: w1 >= Nw / 2
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= blk * nw * nw)
+  if (e >= blk * nw1 * nw)
     return;
-  const int k1 = e % nc, k2 = e / nc % nc, w1 = e / blk % nw, w2 = e / blk / nw;
+  const int k1 = e % nc, k2 = e / nc % nc, w1 = nw - nw1 + e / blk % nw1, w2 = e / blk / nw1;
   const int iq = blockIdx.y, iwq = blockIdx.z;
   const int q = q_list[iq], wex = wex_list[iwq];
   const int k1q = k_add[k1 + nc * q], k2q = k_add[k2 + nc * q];
@@ -834,6 +836,11 @@ updateG4SinglebandGather(const TpDims dims, const GT* __restrict__ G, long g_sec
 }
 
 }  // namespace
+
+// Row frequencies w1 that the update runs: half G4 (particle-hole, one band) the upper half.
+static int g4Rows(const TpDims& d) {
+  return d.half_g4 ? d.nw / 2 : d.nw;
+}
 
 template <typename GT>
 static bool singlebandPHApplies(const TpDims& d) {
@@ -882,7 +889,7 @@ static bool launchSinglebandPH(const G4Args& a, const GT* G, long g_sector_strid
   auto k = updateG4SinglebandPH<GT, AT, KT, QFAST, PREFETCH, MAXT, MINB>;
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int n_qchunks = (d.nq + q_chunk - 1) / q_chunk;
-  const dim3 grid(d.nw, d.nw, d.nwq * n_qchunks);
+  const dim3 grid(g4Rows(d), d.nw, d.nwq * n_qchunks);
   k<<<grid, threads, smem, stream>>>(d, G, g_sector_stride, a.signs, a.n_slots, a.k_add, a.q_list,
                                      a.wex_list, a.G4, a.atomic, q_chunk, n_kc, a.err);
   DCAACC_LAUNCH_CHECK();
@@ -903,7 +910,7 @@ static bool launchSinglebandStream(const G4Args& a, const GT* G, long g_sector_s
   auto k = d.nc == 16 ? updateG4SinglebandStream<GT, AT, 16>
            : d.nc == 8 ? updateG4SinglebandStream<GT, AT, 8> : updateG4SinglebandStream<GT, AT, 4>;
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  const long tiles = long(d.nw) * d.nw * d.nwq;
+  const long tiles = long(g4Rows(d)) * d.nw * d.nwq;
   const int grid = int(std::max(1L, std::min<long>(tiles, (sizeof(GT) == 16 ? 2L : 3L) * a.n_sm)));
   k<<<grid, 256, smem, stream>>>(d, G, g_sector_stride, a.signs, a.k_add, a.q_list, a.wex_list, a.G4, a.atomic,
                                  a.err);
@@ -916,7 +923,7 @@ constexpr int kGatherMaxQ = 2;
 template <typename GT>
 static bool launchSinglebandGather(const G4Args& a, const GT* G, long g_sector_stride, cudaStream_t stream) {
   const TpDims& d = a.dims;
-  const long entries = long(d.nc) * d.nc * d.nw * d.nw;
+  const long entries = long(d.nc) * d.nc * g4Rows(d) * d.nw;
   if (a.n_slots != 1 || d.nq > kGatherMaxQ || d.n_channels > 2 || !singlebandPHApplies<GT>(d) || entries > (1L << 31) - 256)
     return false;
   using AT = std::conditional_t<std::is_same_v<GT, double2>, double, float>;
@@ -946,7 +953,7 @@ int launchUpdateG4(const G4Args& a, const GT* G, long g_sector_stride, cudaStrea
     if (done)
       return 1;
   }
-  const dim3 grid(a.dims.nw, a.dims.nw, a.dims.nwq);
+  const dim3 grid(g4Rows(a.dims), a.dims.nw, a.dims.nwq);
   // Batches: the staged kernel (a single measurement reads each block element a few times only, and
   // the direct gathers of updateG4Kernel cost less than staging).
   if (a.n_slots >= 2 && a.dims.n_channels <= kStagedMaxCh && (size_t(a.dims.R) * a.dims.R * sizeof(GT)) % 16 == 0) {
