@@ -40,32 +40,18 @@
 
 #include "async_copy.cuh"
 #include "common.cuh"
+#include "packed.cuh"
 #include "tp_frontend.hpp"
 
 namespace dcaacc {
 
 namespace {
 
-using Pair = unsigned long long;  // two packed FP32
-
 constexpr int kLong = 32;  // rows of G or columns of M per tile
 constexpr int kRing = 4;   // ring slots per warp
 constexpr int kColV = 2;   // vertices per ring slot, column step
 constexpr int kRowV = 4;   // ... row step (M is read four sorted rows at a time)
 
-__device__ inline Pair pairOf(float a, float b) {
-  Pair p;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
-  return p;
-}
-__device__ inline float2 floatsOf(Pair p) {
-  float2 v;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(p));
-  return v;
-}
-__device__ inline void fma2(Pair& c, Pair a, Pair b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
 // Shared memory by 32-bit address: an immediate offset per access and no generic addressing.
 template <int OFF = 0>
 __device__ inline Pair lds64(uint32_t a) {
@@ -82,20 +68,6 @@ __device__ inline ulonglong2 lds128(uint32_t a) {
 template <int OFF = 0>
 __device__ inline void sts64(uint32_t a, Pair v) {
   asm volatile("st.shared.b64 [%0+%1], %2;" ::"r"(a), "n"(OFF), "l"(v) : "memory");
-}
-__device__ inline Pair add2(Pair a, Pair b) {
-  Pair c;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
-  return c;
-}
-__device__ inline Pair mul2(Pair a, Pair b) {
-  Pair c;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(c) : "l"(a), "l"(b));
-  return c;
-}
-__device__ inline Pair sub2(Pair a, Pair b) {  // exact: b times -1
-  fma2(a, b, pairOf(-1.f, -1.f));
-  return a;
 }
 __device__ inline void cpAsync16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");

@@ -17,10 +17,15 @@
 // FP64 running sum with one read-modify-write, as in the staged kernel, spread over the next pass;
 // the band indices follow its G layout (element (b3, k1; b1, k2) of the A block, (b4, q - k1;
 // b2, q - k2) of the P block).
+//
+// Bound by the FP32 pipe's multiply-adds.  They are packed pairs, which leave half the issue slots to the
+// shared-memory reads: 8 sites, three bands, Nw = 16, all transfers, four frequency transfers, a batch of 32
+// takes 1.18 ms instead of 1.23.
 #include <cuda_runtime.h>
 
 #include "async_copy.cuh"
 #include "common.cuh"
+#include "packed.cuh"
 #include "tp_g4.hpp"
 #include "tp_layout.hpp"
 
@@ -138,14 +143,14 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
     const int aoff = NB * k1 * R + NB * k2;          // element (b1, b3) at + b3 R + b1
     const int poff = (b4 + NB * qk1) * R + NB * qk2;  // element b2 at + b2
     const long g4o = NB3 * b4 + static_cast<long>(NB4) * k1 + k2 * s_k2 + iq * s_q;
-    float2 acc[NB][NB][NB];  // [b1][b2][b3]
+    Pair acc[NB][NB][NB];  // [b1][b2][b3]
 #pragma unroll
     for (int b1 = 0; b1 < NB; ++b1)
 #pragma unroll
       for (int b2 = 0; b2 < NB; ++b2)
 #pragma unroll
         for (int b3 = 0; b3 < NB; ++b3)
-          acc[b1][b2][b3] = make_float2(0.f, 0.f);
+          acc[b1][b2][b3] = 0;
 
     for (int slot = 0; slot < n_slots; ++slot, ++step) {
       const int st = static_cast<int>(step % kPPStages);
@@ -169,22 +174,30 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
       const float2* P1 = A0 + 3 * blk;
       if (live) {
         const float hs = 0.5f * static_cast<float>(sgn[slot]);
-        float2 p0[NB], p1[NB];  // s/2 P_sigma(b4, q - k1; b2, q - k2)
+        // s/2 P_sigma(b4, q - k1; b2, q - k2), its parts doubled: a p = (ax, ay) px + (-ay, ax) py.
+        Pair p0x[NB], p0y[NB], p1x[NB], p1y[NB];
 #pragma unroll
         for (int b2 = 0; b2 < NB; ++b2) {
           const float2 x0 = P0[poff + b2], x1 = P1[poff + b2];
-          p0[b2] = make_float2(hs * x0.x, hs * x0.y);
-          p1[b2] = make_float2(hs * x1.x, hs * x1.y);
+          p0x[b2] = pairOf(hs * x0.x, hs * x0.x);
+          p0y[b2] = pairOf(hs * x0.y, hs * x0.y);
+          p1x[b2] = pairOf(hs * x1.x, hs * x1.x);
+          p1y[b2] = pairOf(hs * x1.y, hs * x1.y);
         }
 #pragma unroll
         for (int b3 = 0; b3 < NB; ++b3)
 #pragma unroll
           for (int b1 = 0; b1 < NB; ++b1) {
             const float2 a0 = A0[aoff + b3 * R + b1], a1 = A1[aoff + b3 * R + b1];
+            const Pair a00 = pairOf(a0.x, a0.y), a01 = pairOf(-a0.y, a0.x);
+            const Pair a10 = pairOf(a1.x, a1.y), a11 = pairOf(-a1.y, a1.x);
 #pragma unroll
             for (int b2 = 0; b2 < NB; ++b2) {
-              cfma(acc[b1][b2][b3], a0, p1[b2]);
-              cfma(acc[b1][b2][b3], a1, p0[b2]);
+              Pair& c = acc[b1][b2][b3];
+              fma2(c, a00, p1x[b2]);
+              fma2(c, a01, p1y[b2]);
+              fma2(c, a10, p0x[b2]);
+              fma2(c, a11, p0y[b2]);
             }
           }
       }
@@ -214,7 +227,7 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
         for (int b2 = 0; b2 < NB; ++b2)
 #pragma unroll
           for (int b1 = 0; b1 < NB; ++b1)
-            fb[(b1 + NB * b2 + NB2 * b3) * kPPThreads + t] = acc[b1][b2][b3];
+            fb[(b1 + NB * b2 + NB2 * b3) * kPPThreads + t] = floatsOf(acc[b1][b2][b3]);
       pend = g4o;
       fe = 0;
     }
