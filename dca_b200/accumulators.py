@@ -397,7 +397,7 @@ class TpAccumulator:
         return {name: (ms[i], cnt[i]) for i, name in enumerate(self.STAGES)}
 
     def set_graphs(self, on: bool = True):
-        """Replay each batch shape's kernel sequence from a CUDA graph (mixed path; on by default)."""
+        """Replay each batch shape's kernel sequence from a CUDA graph (on by default)."""
         _check(N.lib.dcaacc_tp_set_graphs(self._h, int(on)))
 
     def graph_stats(self):

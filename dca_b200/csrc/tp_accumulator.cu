@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "tp_frontend.hpp"
 #include "tp_g4.hpp"
@@ -257,32 +258,29 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   const size_t n_sec = 2 * size_t(max_batch_);
   const size_t n_vtx = n_sec * max_order_;
   const size_t n_orb1 = dims_.n_orb + 1;
+  {
+    Inputs none{};
+    inputs_bytes_ = placeInputs(none, nullptr);
+  }
   for (auto& d : dstage_) {
-    d.sectors.alloc(n_sec);
-    d.tau.alloc(n_vtx);
-    d.vb_r.alloc(n_vtx);
-    d.vs_r.alloc(n_vtx);
-    if (non_density_) {
-      d.vb_c.alloc(n_vtx);
-      d.vs_c.alloc(n_vtx);
-    }
+    d.inputs_mem.alloc(inputs_bytes_);
+    placeInputs(d.in, d.inputs_mem.get());
     d.perm_r.alloc(n_vtx);
     d.rstart.alloc(n_sec * n_orb1);
     if (non_density_) {
       d.perm_c.alloc(n_vtx);
       d.cstart.alloc(n_sec * n_orb1);
     }
-    d.signs.alloc(max_batch_);
     d.M.alloc(n_sec * size_t(max_order_) * max_order_);
   }
   // Launch-shape tuning (launch_tuner.hpp), unless DCAACC_TUNE=0 keeps the built-in shapes.
+  const char* graphs_env = std::getenv("DCAACC_TP_GRAPHS");
+  graphs_on_ = !(graphs_env && std::strcmp(graphs_env, "0") == 0);
   const char* tune_env = std::getenv("DCAACC_TUNE");
   tuner_.setEnabled(!(tune_env && std::strcmp(tune_env, "0") == 0));
   const size_t x_elems = n_sec * size_t(R) * max_order_ * nw_ext;
   const size_t g_elems = n_sec * size_t(g_sector_stride_);
   if (mixed_) {
-    const char* graphs_env = std::getenv("DCAACC_TP_GRAPHS");
-    graphs_on_ = !(graphs_env && std::strcmp(graphs_env, "0") == 0);
     // DCAACC_TP_SIMT_ONLY=1 selects the all-SIMT G4 kernels and the whole of G (kept to compare both paths).
     const char* simt_env = std::getenv("DCAACC_TP_SIMT_ONLY");
     simt_only_ = simt_env && std::strcmp(simt_env, "1") == 0;
@@ -410,15 +408,8 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     }
   }
   for (auto& h : hstage_) {
-    h.sectors.alloc(n_sec);
-    h.tau.alloc(n_vtx);
-    h.vb_r.alloc(n_vtx);
-    h.vs_r.alloc(n_vtx);
-    if (non_density_) {
-      h.vb_c.alloc(n_vtx);
-      h.vs_c.alloc(n_vtx);
-    }
-    h.signs.alloc(max_batch_);
+    h.inputs_mem.alloc(inputs_bytes_);
+    placeInputs(h.in, h.inputs_mem.get());
     DCAACC_CUDA_CHECK(cudaEventRecord(h.uploaded, copy_stream_));
   }
   for (auto& d : dstage_)
@@ -427,6 +418,26 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   if ((!mixed_ || simt_only_) && frontendSmemRequirement(dims_, max_order_, !mixed_) > 227 * 1024)
     invalid("max_order too large for the front-end's shared-memory tiles");
   G4_host_.assign(c.n_channels, {});
+}
+
+size_t TpAccumulator::placeInputs(Inputs& in, unsigned char* base) const {
+  const size_t n_sec = 2 * size_t(max_batch_), n_vtx = n_sec * max_order_;
+  size_t off = 0;
+  auto take = [&](auto*& p, size_t n) {
+    using T = std::remove_reference_t<decltype(*p)>;
+    p = base ? reinterpret_cast<T*>(base + off) : nullptr;
+    off = (off + n * sizeof(T) + 15) / 16 * 16;
+  };
+  take(in.sectors, n_sec);
+  take(in.signs, max_batch_);
+  take(in.tau, n_vtx);
+  take(in.vb_r, n_vtx);
+  take(in.vs_r, n_vtx);
+  if (non_density_) {
+    take(in.vb_c, n_vtx);
+    take(in.vs_c, n_vtx);
+  }
+  return off;
 }
 
 // Half G4 (dims_.half_g4) when the transfer lists are closed under negation: their negatives' positions, and a
@@ -707,13 +718,13 @@ void TpAccumulator::stage(const dcaacc_sector* sec, int sign, bool m_f32) {
     // The vertices as given; the device sorts them by orbital (tp_sort.cu): the row side by the
     // right band / site, the column side of non-density-density models by the left ones
     // (cached_ndft_base.hpp:97-103).
-    std::copy_n(x.right_band, n, hs().vb_r.get() + vtx_off);
-    std::copy_n(x.right_site, n, hs().vs_r.get() + vtx_off);
+    std::copy_n(x.right_band, n, hs().in.vb_r + vtx_off);
+    std::copy_n(x.right_site, n, hs().in.vs_r + vtx_off);
     if (non_density_) {
-      std::copy_n(x.left_band, n, hs().vb_c.get() + vtx_off);
-      std::copy_n(x.left_site, n, hs().vs_c.get() + vtx_off);
+      std::copy_n(x.left_band, n, hs().in.vb_c + vtx_off);
+      std::copy_n(x.left_site, n, hs().in.vs_c + vtx_off);
     }
-    std::copy_n(x.tau, n, hs().tau.get() + vtx_off);
+    std::copy_n(x.tau, n, hs().in.tau + vtx_off);
 
     const double* Mptr = x.M;
     int ldm = std::max(x.ldm, 1);
@@ -754,12 +765,12 @@ void TpAccumulator::stage(const dcaacc_sector* sec, int sign, bool m_f32) {
     d.slot = slot;
     d.m_f32 = m_f32 ? 1 : 0;
     d.x_off = x_used_;
-    hs().sectors[sidx] = d;
+    hs().in.sectors[sidx] = d;
     x_used_ += long(dims_.R) * n * dims_.nw_ext;
     vtx_used_ += n;
     n_max_batch_ = std::max(n_max_batch_, n);
   }
-  hs().signs[slot] = sign;
+  hs().in.signs[slot] = sign;
   ++slots_;
 }
 
@@ -781,15 +792,20 @@ void TpAccumulator::process() {
     if (bytes)
       DCAACC_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, copy_stream_));
   };
-  h2d(ds.sectors.get(), hs().sectors.get(), sizeof(SectorDesc) * n_sec);
-  h2d(ds.tau.get(), hs().tau.get(), sizeof(double) * vtx_used_);
-  h2d(ds.vb_r.get(), hs().vb_r.get(), sizeof(int) * vtx_used_);
-  h2d(ds.vs_r.get(), hs().vs_r.get(), sizeof(int) * vtx_used_);
-  if (non_density_) {
-    h2d(ds.vb_c.get(), hs().vb_c.get(), sizeof(int) * vtx_used_);
-    h2d(ds.vs_c.get(), hs().vs_c.get(), sizeof(int) * vtx_used_);
+  if (inputs_bytes_ <= kOneCopyBytes) {
+    h2d(ds.inputs_mem.get(), hs().inputs_mem.get(), inputs_bytes_);
   }
-  h2d(ds.signs.get(), hs().signs.get(), sizeof(int) * slots_);
+  else {
+    h2d(ds.in.sectors, hs().in.sectors, sizeof(SectorDesc) * n_sec);
+    h2d(ds.in.tau, hs().in.tau, sizeof(double) * vtx_used_);
+    h2d(ds.in.vb_r, hs().in.vb_r, sizeof(int) * vtx_used_);
+    h2d(ds.in.vs_r, hs().in.vs_r, sizeof(int) * vtx_used_);
+    if (non_density_) {
+      h2d(ds.in.vb_c, hs().in.vb_c, sizeof(int) * vtx_used_);
+      h2d(ds.in.vs_c, hs().in.vs_c, sizeof(int) * vtx_used_);
+    }
+    h2d(ds.in.signs, hs().in.signs, sizeof(int) * slots_);
+  }
   DCAACC_CUDA_CHECK(cudaEventRecord(hs().uploaded, copy_stream_));
   DCAACC_CUDA_CHECK(cudaStreamWaitEvent(stream_, hs().uploaded, 0));
   const int set = hset_;
@@ -797,10 +813,10 @@ void TpAccumulator::process() {
 
   FrontendArgs fa{};
   fa.dims = dims_;
-  fa.sectors = ds.sectors.get();
+  fa.sectors = ds.in.sectors;
   fa.n_sectors = n_sec;
   fa.n_max = n_max_batch_;
-  fa.tau = ds.tau.get();
+  fa.tau = ds.in.tau;
   fa.perm_r = ds.perm_r.get();
   fa.perm_c = non_density_ ? ds.perm_c.get() : ds.perm_r.get();
   fa.row_start = ds.rstart.get();
@@ -811,14 +827,13 @@ void TpAccumulator::process() {
   fa.G0 = G0_.get();
   fa.tuner = &tuner_;
   fa.fft = fft64_;
-  // Mixed path: the launch shapes take the order bound in steps of 128; every kernel reads each
-  // sector's own order, so the results do not depend on it, and batches of similar orders share one
-  // captured graph.
-  if (mixed_ && n_max_batch_ > 0)
+  // The launch shapes take the order bound in steps of 128; every kernel reads each sector's own order,
+  // so the results do not depend on it, and batches of similar orders share one captured graph.
+  if (n_max_batch_ > 0)
     fa.n_max = (n_max_batch_ + 127) / 128 * 128;
   G4Args ga{};
   ga.dims = dims_;
-  ga.signs = ds.signs.get();
+  ga.signs = ds.in.signs;
   ga.n_slots = slots_;
   ga.k_add = k_add_d_.get();
   ga.k_sub = k_sub_d_.get();
@@ -844,7 +859,7 @@ void TpAccumulator::process() {
   ga.wait_limit = wait_limit_;
   ga.fault_stop_step = fault_stop_step_;
 
-  const bool graphable = graphs_on_ && mixed_ && !simt_only_ && !timing_ && n_max_batch_ > 0 && stream_ != nullptr &&
+  const bool graphable = graphs_on_ && !simt_only_ && !timing_ && n_max_batch_ > 0 && stream_ != nullptr &&
                          stream_ != cudaStreamLegacy && stream_ != cudaStreamPerThread;
   if (graphable)
     launches_ += launchBatchGraph(set, fa, ga, ds);
@@ -867,11 +882,11 @@ int TpAccumulator::launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStag
     timeBegin(DCAACC_STAGE_TWIDDLE, &b);
     // Vertex order and orbital runs of every sector (sortConfiguration), row side and, for
     // non-density-density models, column side.
-    launchSortVertices(fa.sectors, fa.n_sectors, ds.vb_r.get(), ds.vs_r.get(), dims_.nb, dims_.n_orb,
+    launchSortVertices(fa.sectors, fa.n_sectors, ds.in.vb_r, ds.in.vs_r, dims_.nb, dims_.n_orb,
                        ds.perm_r.get(), ds.rstart.get(), ds.orb_r.get(), stream_);
     launched += 1;
     if (non_density_) {
-      launchSortVertices(fa.sectors, fa.n_sectors, ds.vb_c.get(), ds.vs_c.get(), dims_.nb, dims_.n_orb,
+      launchSortVertices(fa.sectors, fa.n_sectors, ds.in.vb_c, ds.in.vs_c, dims_.nb, dims_.n_orb,
                          ds.perm_c.get(), ds.cstart.get(), ds.orb_c.get(), stream_);
       launched += 1;
     }
@@ -1263,9 +1278,8 @@ size_t TpAccumulator::deviceFingerprint() const {
   for (const auto& g : g4())  // a shared G4 is counted by every handle that shares it
     b += g.bytes();
   for (const auto& d : dstage_)
-    b += d.vb_r.bytes() + d.vs_r.bytes() + d.vb_c.bytes() + d.vs_c.bytes() +
-         d.sectors.bytes() + d.tau.bytes() + d.M.bytes() + d.perm_r.bytes() + d.perm_c.bytes() +
-         d.rstart.bytes() + d.cstart.bytes() + d.signs.bytes() + d.orb_r.bytes() + d.orb_c.bytes();
+    b += d.inputs_mem.bytes() + d.M.bytes() + d.perm_r.bytes() + d.perm_c.bytes() + d.rstart.bytes() + d.cstart.bytes() +
+         d.orb_r.bytes() + d.orb_c.bytes();
   return b;
 }
 

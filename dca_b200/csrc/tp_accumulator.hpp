@@ -196,18 +196,28 @@ private:
   // Batch workspace.
   // Per-batch device inputs, double-buffered like the pinned staging below: batch k + 1 is uploaded
   // on copy_stream_ while batch k's kernels run on stream_ (events order the reuse of a set).
+  // A batch's uploaded inputs, in one buffer with the same layout on both sides, so that one copy moves a
+  // small batch's (kOneCopyBytes; for larger ones the used parts are copied one by one).
+  struct Inputs {
+    SectorDesc* sectors;
+    double* tau;
+    int *signs, *vb_r, *vs_r, *vb_c, *vs_c;  // signs; per-vertex band and site of the row / column side
+  };
+  size_t placeInputs(Inputs& in, unsigned char* base) const;  // returns the bytes; base may be null
+  size_t inputs_bytes_ = 0;
+  static constexpr size_t kOneCopyBytes = 64 << 10;
   struct DevStage {
-    DevBuf<SectorDesc> sectors;
-    DevBuf<double> tau, M;  // M: host-resident sectors' matrices, copied in
-    DevBuf<int> vb_r, vs_r, vb_c, vs_c;  // per-vertex band and site of the row / column side (uploaded)
-    DevBuf<int> perm_r, perm_c, rstart, cstart, signs, orb_r, orb_c;  // sorted on the device
+    DevBuf<unsigned char> inputs_mem;
+    Inputs in{};
+    DevBuf<double> M;  // host-resident sectors' matrices, copied in
+    DevBuf<int> perm_r, perm_c, rstart, cstart, orb_r, orb_c;  // sorted on the device
     cudaEvent_t consumed = nullptr;  // the kernels that read this set have completed
   };
   DevStage dstage_[2];
   cudaStream_t copy_stream_ = nullptr;
   int launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStage& ds);
   int launchBatchGraph(int set, const FrontendArgs& fa, const G4Args& ga, DevStage& ds);
-  // CUDA graphs of the tensor-core path's batch sequence (launchBatchGraph).
+  // CUDA graphs of the batch sequence (launchBatchGraph).
   struct BatchGraph {
     int set, slots, n_max;  // key: device input set, batch size, order bound
     bool clean;             // a batch of this key ran eagerly without launch-shape probes
@@ -247,9 +257,8 @@ private:
   // Pinned staging of the batch being assembled, double-buffered: the host fills one set while the
   // uploads from the other (queued behind the previous batch's kernels) are still pending.
   struct HostStage {
-    PinBuf<SectorDesc> sectors;
-    PinBuf<double> tau;
-    PinBuf<int> vb_r, vs_r, vb_c, vs_c, signs;
+    PinBuf<unsigned char> inputs_mem;
+    Inputs in{};
     cudaEvent_t uploaded = nullptr;  // the uploads from this set have completed
   };
   HostStage hstage_[2];

@@ -228,7 +228,7 @@ enum { DCAACC_STAGE_TWIDDLE = 0, DCAACC_STAGE_ROW = 1, DCAACC_STAGE_COL = 2, DCA
 int dcaacc_tp_enable_timing(dcaacc_tp* acc, int32_t on);
 int dcaacc_tp_stage_times(dcaacc_tp* acc, double* ms, uint64_t* launches, int32_t n_stages);
 
-/* CUDA graphs of the mixed path's per-batch kernel sequence (no reference counterpart; the
+/* CUDA graphs of the per-batch kernel sequence (a measurement's in FP64; no reference counterpart; the
  * reference launches each kernel from the host per measurement).  On by default (environment
  * DCAACC_TP_GRAPHS=0 turns them off at creation); used only on a non-default stream and while
  * stage timing is off.  A batch shape's first batch runs eagerly, its second is captured, later
