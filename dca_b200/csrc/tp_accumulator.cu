@@ -89,6 +89,11 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   n_sp_ = c.n_sp_freq;
   k_add_.assign(c.k_add, c.k_add + nc * nc);
   k_sub_.assign(c.k_sub, c.k_sub + nc * nc);
+  // 6 x 6 grid of momenta, the zero momentum at any place: b - a component by component from k_0 - k_0.
+  grid6_ = nc == 36;
+  for (int a = 0; a < nc && grid6_; ++a)
+    for (int b = 0; b < nc && grid6_; ++b)
+      grid6_ = k_sub_[a + nc * b] == (b % 6 - a % 6 + k_sub_[0] % 6 + 6) % 6 + 6 * ((b / 6 - a / 6 + k_sub_[0] / 6 + 6) % 6);
   q_list_.assign(c.k_ex, c.k_ex + c.n_k_ex);
   wex_list_.assign(c.w_ex, c.w_ex + c.n_w_ex);
   g4_size_ = size_t(nb) * nb * nb * nb * nc * nc * nw * nw * c.n_k_ex * c.n_w_ex;
@@ -285,12 +290,15 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     const char* simt_env = std::getenv("DCAACC_TP_SIMT_ONLY");
     simt_only_ = simt_env && std::strcmp(simt_env, "1") == 0;
     G32_.alloc(g_elems);
-    // Front-end: factored by orbital in FP32 (tp_frontend32.cu) for one band on a 4x4 or 6x6 cluster, where the
-    // factoring saves 16 or 36 times the flops and the cluster transform is an FFT (a batch of 64, Nw = 64: 0.47
-    // against 0.66 ms; 6x6, Nw = 32, batch of 128: 4.0 against 8.7 ms); dense tensor-core products
-    // (tp_frontend_tc.cu) elsewhere (8 sites, one band, Nw = 24 + 2, batch of 32: 0.085 against 0.093 ms;
-    // three bands on 8 sites take 0.50 against 0.37 ms, but beside the FP32-bound pairing update of
-    // another batch the tensor cores' are the cheaper ones).  DCAACC_TP_FACTORED_COL selects the
+    // Front-end: factored by orbital in FP32 (tp_frontend32.cu) or dense tensor-core products (tp_frontend_tc.cu).
+    // One band: FP32 on a 4x4 or 6x6 cluster, where the factoring saves 16 or 36 times the flops and the cluster
+    // transform is an FFT (a batch of 64, Nw = 64: 0.47 against 0.66 ms; 6x6, Nw = 32, batch of 128: 2.3 against
+    // 8.4 ms), and up to 8 sites (8 sites, Nw = 24 + 2, 0.094 against 0.091 ms, and 0.23 against 0.29 for a batch
+    // of 64 with n up to 400), whose G4 is then off by 1.6e-7 of the 64-bit sums instead of 4.3e-7.  With the
+    // matrix transform 16 sites take 0.87 against 0.68 ms: there, and for 36 sites, only where the G4 kernels of
+    // transfer subsets or of the transverse and pairing channels follow, whose sums add to the error.
+    // Three bands on 8 sites take 0.37 ms in FP32 and 0.50 on the tensor cores, but beside the FP32-bound pairing
+    // update of another batch the tensor cores' are the cheaper ones.  DCAACC_TP_FACTORED_COL selects the
     // tensor-core front-end with one of its column steps: 0 the dense GEMM; 1 one band, 4x4 or
     // 6x6 cluster: factored by orbital on mma.sync or the CUDA cores (DCAACC_TP_COL_FFT=0: with the
     // matrix transform instead of the FFT); 2 one band, 4x4: factored with the sums in tensor memory.
@@ -301,7 +309,9 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     const bool fact_off = fact_env && std::strcmp(fact_env, "0") == 0;
     const bool fact_on = fact_env && std::strcmp(fact_env, "1") == 0;
     const bool fact_tc = fact_env && std::strcmp(fact_env, "2") == 0;
-    front32_ = simt_only_ || (!fact_off && !fact_on && !fact_tc && fft.on && front32Applies(dims_, max_order_));
+    const bool ph_all = phChannels(dims_).n_channels == c.n_channels && allTransfers();
+    const bool factored = nb == 1 && (fft.on || nc <= 8 || ((nc == 16 || nc == 36) && !ph_all));
+    front32_ = simt_only_ || (!fact_off && !fact_on && !fact_tc && factored && front32Applies(dims_, max_order_));
     tc_front_ = !front32_;
     if (front32_) {
       const size_t Kr = (size_t(max_order_) + 63) / 64 * 64;
@@ -438,6 +448,14 @@ size_t TpAccumulator::placeInputs(Inputs& in, unsigned char* base) const {
     take(in.vs_c, n_vtx);
   }
   return off;
+}
+
+bool TpAccumulator::allTransfers() const {
+  std::vector<char> seen(dims_.nc, 0);
+  int distinct = 0;
+  for (int q : q_list_)
+    distinct += seen[q]++ == 0;
+  return distinct == dims_.nc && int(q_list_.size()) == dims_.nc;
 }
 
 // Half G4 (dims_.half_g4) when the transfer lists are closed under negation: their negatives' positions, and a
@@ -844,13 +862,8 @@ void TpAccumulator::process() {
   ga.simt_only = simt_only_;
   ga.atomic = atomic_;
   ga.err = err_d_.get();
-  {
-    std::vector<int> seen(dims_.nc, 0);
-    int distinct = 0;
-    for (int q : q_list_)
-      distinct += seen[q]++ == 0;
-    ga.q_all = distinct == dims_.nc && int(q_list_.size()) == dims_.nc;
-  }
+  ga.q_all = allTransfers();
+  ga.grid6 = grid6_;
   ga.disc = have_disc_ ? &disc_ws_ : nullptr;
   ga.gmax = gmax_d_.get();  // null in FP64 and all-SIMT runs
   ga.tile_order = dims_.half_g4 ? tile_order_d_.get() : nullptr;

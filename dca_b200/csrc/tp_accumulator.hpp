@@ -162,6 +162,8 @@ private:
   int max_batch_ = 1, max_order_ = 1;
   int n_sp_ = 0;
   std::vector<int> k_add_, k_sub_, q_list_, wex_list_;
+  bool grid6_ = false;  // G4Args::grid6
+  bool allTransfers() const;  // q_list_ is a permutation of the cluster momenta
   size_t g4_size_ = 0;
   long g_sector_stride_ = 0;  // complex elements of one (slot, spin) G
 

@@ -26,6 +26,7 @@ struct G4Args {
   int* err;             // device error word (async_copy.cuh kErr* bits)
   bool simt_only = false;         // no tensor-core terms (mixed path, comparisons)
   bool q_all = false;             // q_list is a permutation of all Nc cluster momenta
+  bool grid6 = false;             // 6 x 6 momenta, index x + 6 y; differences component by component
   const struct DiscWorkspace* disc = nullptr;  // tensor-core disconnected-term workspace (or null)
   const int* gmax = nullptr;  // [2 slot + spin] largest |G| of each sector as float bits (or null)
   int n_sm = 0;               // multiprocessors (persistent grids)
@@ -81,6 +82,10 @@ const float2* launchDiscGemm(const G4Args& a, const float2* G, long g_sector_str
 bool directTcApplies(const G4Args& a);
 void launchDirectTc(const G4Args& a, const float2* G, long g_sector_stride, const float2* disc, int n_sm,
                     cudaStream_t stream);
+
+// The same for Nc = 36 on a 6 x 6 grid of momenta (tp_g4_mma36.cu).
+bool directTc36Applies(const G4Args& a);
+void launchDirectTc36(const G4Args& a, const float2* G, long g_sector_stride, const float2* disc, cudaStream_t stream);
 
 // half_g4: G4 entries with w1 < Nw / 2 := conj of their mirror (-k1 w1', -k2 w2', -q, -wq);
 // q_mirror[iq] / wq_mirror[iwq] are the positions of -q / -wq in the transfer lists.

@@ -1126,6 +1126,8 @@ int launchForNc(const G4Args& a, const float2* G, long stride, cudaStream_t s) {
       return 0;
     if (NC == 16 && directTcApplies(p))
       launchDirectTc(p, G, stride, disc, p.n_sm, s);
+    else if (NC == 36 && directTc36Applies(p))
+      launchDirectTc36(p, G, stride, disc, s);
     else if (NC == 36 && p.q_all)
       launchOuterSplit(p, G, stride, disc, s);
     else

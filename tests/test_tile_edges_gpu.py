@@ -14,7 +14,8 @@ FP64_TOL, MIXED_TOL, SP_TOL = 1e-12, 1e-6, 1e-9
 
 CLUSTERS = {"2x1": W.make_cluster((2, 0), (0, 1)), "3x2": W.make_cluster((3, 0), (0, 2)),
             "2x2": W.square_cluster(2), "betts8": W.betts8_cluster(), "4x4": W.square_cluster(4),
-            "5x5": W.square_cluster(5), "6x6": W.square_cluster(6)}
+            "8x2": W.make_cluster((8, 0), (0, 2)), "5x5": W.square_cluster(5), "6x6": W.square_cluster(6),
+            "9x4": W.make_cluster((9, 0), (0, 4))}
 
 
 def _g0(rng, nb, cl, n_sp):
@@ -67,6 +68,8 @@ def _compare(oracle_lib, g0, measurements, params, tol):
     ("betts8", 3, 3, [0, 2], [(47, 18), (5, 100)]),   # three bands, rows not a multiple of the tile
     ("4x4", 1, 5, [0], [(1, 33), (130, 7)]),          # 4 x 4 FFT, 10 frequencies, most orbitals empty
     ("5x5", 1, 2, [0], [(40, 70), (2, 25)]),          # 25 sites: matrix transform
+    ("8x2", 1, 4, [0], [(40, 21), (97, 5)]),          # 16 and 36 sites without the FFT, half of G
+    ("9x4", 1, 2, [0], [(40, 21), (97, 5)]),
     ("6x6", 1, 3, [0], [(40, 0), (97, 5)]),           # 6 x 6 FFT, 6 frequencies
 ])
 def test_front_end_tiles(oracle_lib, precision, tol, cluster, nb, nw_half, w_ex, orders):
@@ -103,6 +106,38 @@ def test_all_transfers_all_channels(oracle_lib, cluster):
     k_ex = list(rng.permutation(cl.nc))
     params = _params(1, cl, 2, 8, [3, 4, 1, 2], k_ex, [0, 1], orders, precision=1, max_batch=3)
     _compare(oracle_lib, _g0(rng, 1, cl, 8), _measurements(rng, 1, cl.nc, orders), params, MIXED_TOL)
+
+
+@pytest.mark.parametrize("n_meas,max_batch,channels", [(32, 32, [2, 3]), (37, 37, [2]), (41, 33, [3])])
+def test_large_cluster_all_transfers(oracle_lib, n_meas, max_batch, channels):
+    """6x6, every transfer in another order, batches that do and do not fill the steps of eight measurements."""
+    rng = np.random.default_rng(9)
+    cl = CLUSTERS["6x6"]
+    orders = [(int(a), int(b)) for a, b in rng.integers(0, 30, (n_meas, 2))]
+    params = _params(1, cl, 2, 6, channels, list(rng.permutation(36)), [0], orders, precision=1, max_batch=max_batch)
+    _compare(oracle_lib, _g0(rng, 1, cl, 6), _measurements(rng, 1, cl.nc, orders), params, MIXED_TOL)
+
+
+def test_fp64_graphs():
+    """FP64 with and without captured graphs, orders on both sides of the launch shapes' steps of 128."""
+    from dca_b200.accumulators import TpAccumulator
+    rng = np.random.default_rng(10)
+    cl = CLUSTERS["2x2"]
+    orders = [(3, 128), (129, 0), (1, 127), (130, 140), (128, 128), (5, 7), (200, 129), (0, 0), (17, 2)]
+    params = _params(1, cl, 2, 6, [2, 4], [1, 3], [0, 1], orders)
+    measurements, got = _measurements(rng, 1, cl.nc, orders), []
+    for graphs in (True, False):
+        acc = TpAccumulator(_g0(rng, 1, cl, 6), params)
+        acc.set_graphs(graphs)
+        for _ in range(2):
+            acc.resetAccumulation(0)
+            for m in measurements:
+                acc.accumulate([s.M for s in m.sectors], list(m.sectors), m.sign)
+        acc.finalize()
+        assert (acc.graph_stats()[0] > 0) == graphs
+        got.append(acc.get_G4())
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("cluster,nb,n_sp,orders", [
