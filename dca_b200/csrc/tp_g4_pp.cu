@@ -11,17 +11,21 @@
 // G(w1; w2) and nb of the P block G(m1; m2) and does nb^3 complex FMAs (27 per 12 reads for three
 // bands), where the generic staged kernel (tp_g4.cu) reads two elements per entry.  CTA = one
 // (w1, w2, wq) tile; per measurement the two spins' A and P blocks (R x R each, R = nb Nc) arrive in
-// shared memory by the bulk-copy engine through a four-stage ring.  Items (k1, k2, q, b4) are
+// shared memory by the bulk-copy engine, two measurements a stage, through a three-stage ring.  Items (k1, k2, q, b4) are
 // numbered q fastest, then k2, so that the A reads of a warp are broadcasts; items beyond the
 // CTA's threads take further passes over the batch.  The batch sum of each entry goes into the
-// FP64 running sum with one read-modify-write, as in the staged kernel, spread over the next pass;
-// the band indices follow its G layout (element (b3, k1; b1, k2) of the A block, (b4, q - k1;
+// FP64 running sum with one read-modify-write, as in the staged kernel, spread over the next pass and in
+// G4's order: for fixed (k2, q) the entries of a pass's items are one run of G4, so a pass's sums are
+// exchanged through shared memory and consecutive lanes take consecutive entries.  The band indices follow its G layout (element (b3, k1; b1, k2) of the A block, (b4, q - k1;
 // b2, q - k2) of the P block).
 //
-// Bound by the FP32 pipe's multiply-adds.  They are packed pairs, which leave half the issue slots to the
-// shared-memory reads: 8 sites, three bands, Nw = 16, all transfers, four frequency transfers, a batch of 32
-// takes 1.18 ms instead of 1.23.
+// Bound by the FP32 pipe's multiply-adds (45 % of its cycles, 46 % of the issue slots; sixteen warps of 128
+// registers hide only part of the shared-memory and G4 latencies).  They are packed pairs, at half the scalar
+// ones' issue slots.  8 sites, three bands, Nw = 16, all transfers, four frequency transfers, a batch of 32: 1.23 ms
+// with scalar multiply-adds, 1.18 packed, 0.83 with G4 read and written in runs and two measurements a stage.
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "async_copy.cuh"
 #include "common.cuh"
@@ -34,7 +38,9 @@ namespace dcaacc {
 namespace {
 
 constexpr int kPPThreads = 512;
-constexpr int kPPStages = 4;  // ring of per-measurement block sets: copies run three steps ahead
+constexpr int kPPStages = 3;  // ring of block sets: copies run two steps ahead
+constexpr int kPPMeas = 2;    // measurements per stage
+constexpr int kPPPitch = kPPThreads + 1;  // row of the batch sums in shared memory (distinct banks along the entries)
 
 template <int NB, int NC>
 __global__ void __launch_bounds__(kPPThreads, 1)
@@ -51,7 +57,8 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
   constexpr long blk = static_cast<long>(R) * R;
   const int n_items = nc * nc * nq * NB;
   const int n_passes = (n_items + kPPThreads - 1) / kPPThreads;
-  const long n_steps = static_cast<long>(n_passes) * n_slots;
+  const int pass_steps = (n_slots + kPPMeas - 1) / kPPMeas;
+  const int n_steps = n_passes * pass_steps;
   const int m1 = wex + nw - 1 - w1 + ext, m2 = wex + nw - 1 - w2 + ext;
   const long offA = (static_cast<long>(w1 + ext) * nw_ext + w2 + ext) * blk;
   const long offP = (static_cast<long>(m1) * nw_ext + m2) * blk;
@@ -59,18 +66,19 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw);     // [kPPStages] a stage's copies landed
   uint64_t* empty = bar + kPPStages;                         // [kPPStages] every warp is done with it
-  float2* stage = reinterpret_cast<float2*>(smem_raw + 64);  // [kPPStages][spin][A, P][R * R]
+  float2* stage = reinterpret_cast<float2*>(smem_raw + 64);  // [kPPStages][kPPMeas][spin][A, P][R * R]
   const uint32_t blk_bytes = static_cast<uint32_t>(blk * sizeof(float2));
-  auto issue = [&](long step) {
-    const int st = static_cast<int>(step % kPPStages);
-    const int slot = static_cast<int>(step % n_slots);
-    float2* dst = stage + st * 4 * blk;
-    mbarArriveExpectTx(&bar[st], 4 * blk_bytes);
-    for (int s = 0; s < 2; ++s) {
-      const float2* src = G + g_sector_stride * (2 * slot + s);
-      bulkCopyG2S(dst + (2 * s) * blk, src + offA, blk_bytes, &bar[st]);
-      bulkCopyG2S(dst + (2 * s + 1) * blk, src + offP, blk_bytes, &bar[st]);
-    }
+  auto issue = [&](int step) {
+    const int st = step % kPPStages;
+    const int m0 = step % pass_steps * kPPMeas, n = min(kPPMeas, n_slots - m0);
+    mbarArriveExpectTx(&bar[st], n * 4 * blk_bytes);
+    for (int m = 0; m < n; ++m)
+      for (int s = 0; s < 2; ++s) {
+        float2* dst = stage + ((st * kPPMeas + m) * 4 + 2 * s) * blk;
+        const float2* src = G + g_sector_stride * (2 * (m0 + m) + s);
+        bulkCopyG2S(dst, src + offA, blk_bytes, &bar[st]);
+        bulkCopyG2S(dst + blk, src + offP, blk_bytes, &bar[st]);
+      }
   };
   const int t = threadIdx.x;
   const int lane = t % 32;
@@ -83,7 +91,7 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
   }
   __syncthreads();
   if (t == 0)
-    for (long i = 0; i < kPPStages && i < n_steps; ++i)
+    for (int i = 0; i < kPPStages && i < n_steps; ++i)
       issue(i);
 
   // G4 strides: entry (b1, b2, b3, b4) + nb^4 (k1 + Nc (w1 + Nw (k2 + Nc (w2 + Nw (q + Nq wq))))).
@@ -91,16 +99,37 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
              s_wq = s_q * nq;
   double2* g4t = G4[0] + w1 * s_w1 + w2 * s_w2 + iwq * s_wq;
   const uint32_t limit = wait_limit ? wait_limit : kWaitLimit;
-  // A pass's batch sums wait in shared memory ([entry][thread]) and go into the FP64 running sum
-  // one entry per measurement step of the next pass, so that the read-modify-write latency hides
-  // behind that step's FMAs (the last pass's sums go at the end).
-  float2* fb = stage + kPPStages * 4 * blk;
-  int* sgn = reinterpret_cast<int*>(fb + NB3 * kPPThreads);  // [n_slots] the measurements' signs
+  // A pass's batch sums wait in shared memory ([entry of an item][item]) and go into the FP64 running sum
+  // one entry a thread per measurement of the next pass, so that the read-modify-write latency hides
+  // behind that measurement's FMAs (the last pass's sums go at the end).  In G4, the entries of (b4, k1)
+  // follow one another for fixed (k2, q): entry j of run r, r = q + Nq k2, j = b + nb^3 (item / (Nq Nc) - bk0).
+  float2* fb = stage + kPPStages * kPPMeas * 4 * blk;
+  const int n_runs = nq * nc;
+  long* run_off = reinterpret_cast<long*>(fb + NB3 * kPPPitch + (NB3 * kPPPitch) % 2);  // [n_runs]
+  int* sgn = reinterpret_cast<int*>(run_off + n_runs);  // [n_slots] the measurements' signs
   for (int i = t; i < n_slots; i += kPPThreads)
     sgn[i] = signs[i];
+  for (int r = t; r < n_runs; r += kPPThreads)
+    run_off[r] = r / nq * s_k2 + r % nq * s_q;
   __syncthreads();  // the signs are in place before any warp's first step
-  long pend = -1;  // G4 offset of this thread's pending item
-  int fe = NB3;    // its next entry to write
+  // The pending pass: offset of an item's place from its (b4, k1) and run, number of items, first (b4, k1), run
+  // length, and a thread's step from one of its entries to the next one.
+  struct Pending {
+    int place, count, bk0, run, dr, dj;
+  };
+  auto pendingOf = [&](int pass) {
+    Pending p;
+    const int item0 = kPPThreads * pass;
+    p.count = min(kPPThreads, n_items - item0);
+    p.bk0 = item0 / n_runs;
+    p.place = p.bk0 * n_runs - item0;
+    p.run = NB3 * ((item0 + p.count - 1) / n_runs - p.bk0 + 1);
+    p.dr = kPPThreads / p.run;
+    p.dj = kPPThreads - p.dr * p.run;
+    return p;
+  };
+  volatile Pending* pend = reinterpret_cast<volatile Pending*>(sgn + n_slots);  // in shared memory: registers are short
+  int fr = n_runs, fj = 0;  // this thread's next entry
   auto flushEntry = [&](double2* dst, float2 v, double2 old) {
     if (atomic) {
       atomicAdd(&dst->x, static_cast<double>(v.x));
@@ -112,26 +141,42 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
       *dst = old;
     }
   };
-  auto entryPtr = [&](int e) {  // e = b1 + nb b2 + nb^2 b3: consecutive entries are contiguous
-    return g4t + pend + e;
-  };
-  auto flushRest = [&]() {
-    if (pend >= 0 && fe == 0 && !atomic) {  // a whole item: all reads before the writes
-      double2 old[NB3];
-#pragma unroll
-      for (int e = 0; e < NB3; ++e)
-        old[e] = *entryPtr(e);
-#pragma unroll
-      for (int e = 0; e < NB3; ++e)
-        flushEntry(entryPtr(e), fb[e * kPPThreads + t], old[e]);
-      fe = NB3;
+  // The next pending entry of this thread: its place in G4 (null: not of this pass) and its sum.
+  auto nextEntry = [&](float2& v) -> double2* {
+    const int kb = fj / NB3, place = kb * n_runs + fr + pend->place;
+    double2* dst = nullptr;
+    if (place >= 0 && place < pend->count) {
+      v = fb[(fj - NB3 * kb) * kPPPitch + place];
+      dst = g4t + run_off[fr] + NB3 * pend->bk0 + fj;
     }
-    for (; pend >= 0 && fe < NB3; ++fe) {
-      double2* dst = entryPtr(fe);
-      flushEntry(dst, fb[fe * kPPThreads + t], atomic ? make_double2(0., 0.) : *dst);
+    fr += pend->dr;
+    fj += pend->dj;
+    if (fj >= pend->run) {
+      fj -= pend->run;
+      ++fr;
+    }
+    return dst;
+  };
+  auto flushRest = [&](auto in_flight) {
+    constexpr int kRest = decltype(in_flight)::value;  // entries
+    while (fr < n_runs) {
+      double2* dst[kRest];
+      float2 v[kRest];
+      double2 old[kRest];
+#pragma unroll
+      for (int u = 0; u < kRest; ++u) {
+        dst[u] = fr < n_runs ? nextEntry(v[u]) : nullptr;
+        if (dst[u] && !atomic)
+          old[u] = *dst[u];
+      }
+#pragma unroll
+      for (int u = 0; u < kRest; ++u)
+        if (dst[u])
+          flushEntry(dst[u], v[u], old[u]);
     }
   };
-  long step = 0;
+  int step = 0, st = 0;
+  uint32_t phase = 0;
   bool ok = true;
   for (int pass = 0; pass < n_passes; ++pass) {
     const int item = t + kPPThreads * pass;
@@ -142,7 +187,6 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
     const int qk1 = k_sub[k1 + nc * q], qk2 = k_sub[k2 + nc * q];
     const int aoff = NB * k1 * R + NB * k2;          // element (b1, b3) at + b3 R + b1
     const int poff = (b4 + NB * qk1) * R + NB * qk2;  // element b2 at + b2
-    const long g4o = NB3 * b4 + static_cast<long>(NB4) * k1 + k2 * s_k2 + iq * s_q;
     Pair acc[NB][NB][NB];  // [b1][b2][b3]
 #pragma unroll
     for (int b1 = 0; b1 < NB; ++b1)
@@ -152,28 +196,21 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
         for (int b3 = 0; b3 < NB; ++b3)
           acc[b1][b2][b3] = 0;
 
-    for (int slot = 0; slot < n_slots; ++slot, ++step) {
-      const int st = static_cast<int>(step % kPPStages);
-      // One pending entry of the previous pass: its FP64 value is read here, written after the FMAs.
+    // One measurement; one pending entry of the previous pass is read before it and written after it.
+    auto measure = [&](const float2* A0, int sign) {
       double2* fdst = nullptr;
       float2 fv = make_float2(0.f, 0.f);
       double2 fold = make_double2(0., 0.);
-      if (pend >= 0 && fe < NB3) {
-        fdst = entryPtr(fe);
-        fv = fb[fe * kPPThreads + t];
-        if (!atomic)
+      if (fr < n_runs) {
+        fdst = nextEntry(fv);
+        if (fdst && !atomic)
           fold = *fdst;
       }
-      const uint32_t phase = static_cast<uint32_t>((step / kPPStages) & 1);
-      ok = __all_sync(0xffffffffu, mbarWait(&bar[st], phase, err, limit));
-      if (!ok)
-        break;
-      const float2* A0 = stage + st * 4 * blk;
       const float2* P0 = A0 + blk;
       const float2* A1 = A0 + 2 * blk;
       const float2* P1 = A0 + 3 * blk;
       if (live) {
-        const float hs = 0.5f * static_cast<float>(sgn[slot]);
+        const float hs = 0.5f * static_cast<float>(sign);
         // s/2 P_sigma(b4, q - k1; b2, q - k2), its parts doubled: a p = (ax, ay) px + (-ay, ax) py.
         Pair p0x[NB], p0y[NB], p1x[NB], p1y[NB];
 #pragma unroll
@@ -201,25 +238,37 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
             }
           }
       }
-      if (fdst) {
+      if (fdst)
         flushEntry(fdst, fv, fold);
-        ++fe;
-      }
+    };
+    for (int slot = 0; slot < n_slots; slot += kPPMeas, ++step) {
+      ok = __all_sync(0xffffffffu, ok && mbarWait(&bar[st], phase, err, limit));
+      if (!ok)
+        break;
+      const float2* S = stage + st * (kPPMeas * 4 * blk);
+#pragma unroll 1
+      for (int m = 0; m < kPPMeas && slot + m < n_slots; ++m)
+        measure(S + m * 4 * blk, sgn[slot + m]);
       __syncwarp();
       if (lane == 0)
         mbarArrive(&empty[st]);  // release: this warp's reads of the stage are done
       if (t == 0 && step + kPPStages < n_steps) {
-        if (!mbarWait(&empty[st], phase, err, limit)) {
-          ok = false;  // the other warps see the missing copies as a timeout of their own
-          break;
+        // Out of time: the vote above ends this warp's loop, the others time out on the missing copies.
+        ok = mbarWait(&empty[st], phase, err, limit);
+        if (ok) {
+          fenceProxyAsync();
+          issue(step + kPPStages);
         }
-        fenceProxyAsync();
-        issue(step + kPPStages);
+      }
+      if (++st == kPPStages) {
+        st = 0;
+        phase ^= 1;
       }
     }
     if (__syncthreads_or(!ok))
       return;  // uniform bail-out; the host reports the error word
-    flushRest();  // batches shorter than nb^3 measurements leave entries of the previous pass
+    flushRest(std::integral_constant<int, 2>{});  // batches shorter than the entries a thread leave some of the previous pass
+    __syncthreads();
     if (live) {
 #pragma unroll
       for (int b3 = 0; b3 < NB; ++b3)
@@ -227,15 +276,22 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
         for (int b2 = 0; b2 < NB; ++b2)
 #pragma unroll
           for (int b1 = 0; b1 < NB; ++b1)
-            fb[(b1 + NB * b2 + NB2 * b3) * kPPThreads + t] = floatsOf(acc[b1][b2][b3]);
-      pend = g4o;
-      fe = 0;
+            fb[(b1 + NB * b2 + NB2 * b3) * kPPPitch + t] = floatsOf(acc[b1][b2][b3]);
     }
-    else {
-      pend = -1;
+    if (t == 0) {
+      const Pending p = pendingOf(pass);
+      pend->place = p.place;
+      pend->count = p.count;
+      pend->bk0 = p.bk0;
+      pend->run = p.run;
+      pend->dr = p.dr;
+      pend->dj = p.dj;
     }
+    __syncthreads();
+    fr = t / pend->run;
+    fj = t - fr * pend->run;
   }
-  flushRest();
+  flushRest(std::integral_constant<int, 9>{});
 }
 
 }  // namespace
@@ -245,9 +301,10 @@ bool launchUpdateG4PPMultiband(const G4Args& a, const float2* G, long g_sector_s
   if (d.n_channels != 1 || d.channels[0] != 4 /* PARTICLE_PARTICLE_UP_DOWN */ || d.nb != 3 || d.half_g4 || d.half_g ||
       a.n_slots < 1 || (d.nc != 4 && d.nc != 8))
     return false;
-  const size_t smem = 64 + kPPStages * 4 * size_t(d.R) * d.R * sizeof(float2) +
-                      27 * size_t(kPPThreads) * sizeof(float2) + sizeof(int) * size_t(a.n_slots);
-  if (smem > 220 * 1024)
+  const size_t smem = 64 + kPPStages * kPPMeas * 4 * size_t(d.R) * d.R * sizeof(float2) +
+                      (27 * size_t(kPPPitch) + 1) * sizeof(float2) + sizeof(long) * size_t(d.nq) * d.nc +
+                      sizeof(int) * (size_t(a.n_slots) + 6);
+  if (smem > 227 * 1024)
     return false;
   auto k = d.nc == 4 ? updateG4PPMultibandKernel<3, 4> : updateG4PPMultibandKernel<3, 8>;
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));

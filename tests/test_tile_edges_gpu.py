@@ -118,6 +118,19 @@ def test_large_cluster_all_transfers(oracle_lib, n_meas, max_batch, channels):
     _compare(oracle_lib, _g0(rng, 1, cl, 6), _measurements(rng, 1, cl.nc, orders), params, MIXED_TOL)
 
 
+@pytest.mark.parametrize("cluster,k_ex,n_meas,max_batch", [
+    ("betts8", [5], 1, 1), ("betts8", [1, 6, 3], 35, 35), ("betts8", [7, 2, 0, 4, 1, 6, 3, 5], 4, 3),
+    ("2x2", [2], 31, 31), ("2x2", [3, 0, 1, 2], 2, 2)])
+def test_three_band_pairing(oracle_lib, cluster, k_ex, n_meas, max_batch):
+    """Items that do and do not fill the passes of 512, runs cut by a pass, batches shorter and longer than the
+    27 entries of an item, odd ones against the two measurements of a stage."""
+    rng = np.random.default_rng(11)
+    cl = CLUSTERS[cluster]
+    orders = [(int(a), int(b)) for a, b in rng.integers(0, 25, (n_meas, 2))]
+    params = _params(3, cl, 2, 7, [W.PP_UP_DOWN], k_ex, [0, 1], orders, precision=1, max_batch=max_batch)
+    _compare(oracle_lib, _g0(rng, 3, cl, 7), _measurements(rng, 3, cl.nc, orders), params, MIXED_TOL)
+
+
 def test_fp64_graphs():
     """FP64 with and without captured graphs, orders on both sides of the launch shapes' steps of 128."""
     from dca_b200.accumulators import TpAccumulator
