@@ -420,7 +420,7 @@ updateG4SinglebandFew(const TpDims dims, const float2* __restrict__ G, long g_se
   for (int m = 0; m < n_slots; ++m) {
     const int st = m % DEPTH;
     const float half = (MODE == kPairing ? 0.5f : -0.5f) * static_cast<float>(__ldg(signs + m));
-    ok = __all_sync(warp_mask, mbarWait(&full[st], (m / DEPTH) & 1, err));
+    ok = __all_sync(warp_mask, ok && mbarWait(&full[st], (m / DEPTH) & 1, err));
     if (!ok)
       break;
     const float2* Sm = stage + st * 4 * BLK;
@@ -444,11 +444,10 @@ updateG4SinglebandFew(const TpDims dims, const float2* __restrict__ G, long g_se
     if (lane == 0)
       mbarArrive(&empty[st]);  // release: this warp's reads of the stage are done
     if (t == 0 && m + DEPTH < n_slots) {
-      if (!mbarWait(&empty[st], (m / DEPTH) & 1, err)) {
-        ok = false;  // the other warps see the missing copy as a timeout of their own
-        break;
-      }
-      issue(m + DEPTH);
+      // Out of time: the vote above ends this warp's loop, the others time out on the missing copy.
+      ok = mbarWait(&empty[st], (m / DEPTH) & 1, err);
+      if (ok)
+        issue(m + DEPTH);
     }
   }
   if (__syncthreads_or(!ok))
@@ -603,7 +602,7 @@ updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_
   for (int m = 0; m < n_slots; ++m) {
     const int st = m % DEPTH;
     const int sg_next = m + 1 < n_slots ? signs[m + 1] : 1;
-    ok = __all_sync(0xffffffffu, mbarWait(&full[st], (m / DEPTH) & 1, err));
+    ok = __all_sync(0xffffffffu, ok && mbarWait(&full[st], (m / DEPTH) & 1, err));
     if (!ok)
       break;
     const float2* S = stage + st * 4 * BLK;
@@ -644,11 +643,10 @@ updateG4SinglebandOuter(const TpDims dims, const float2* __restrict__ G, long g_
     if (lane == 0)
       mbarArrive(&empty[st]);  // release: this warp's reads of the stage are done
     if (t == 0 && m + DEPTH < n_slots) {
-      if (!mbarWait(&empty[st], (m / DEPTH) & 1, err)) {
-        ok = false;  // the other warps see the missing copy as a timeout of their own
-        break;
-      }
-      issue(m + DEPTH);
+      // Out of time: the vote above ends this warp's loop, the others time out on the missing copy.
+      ok = mbarWait(&empty[st], (m / DEPTH) & 1, err);
+      if (ok)
+        issue(m + DEPTH);
     }
   }
   if (__syncthreads_or(!ok))
@@ -871,7 +869,7 @@ updateG4SinglebandOuterSplit(const TpDims dims, const float2* __restrict__ G, lo
     const float ia = mir_a ? -1.f : 1.f;
     for (int m = 0; m < n_slots; ++m) {
       const int st = m % DEPTH;
-      ok = __all_sync(0xffffffffu, mbarWait(&full[st], (m / DEPTH) & 1, err));
+      ok = __all_sync(0xffffffffu, ok && mbarWait(&full[st], (m / DEPTH) & 1, err));
       if (!ok)
         break;
       const float ns = -static_cast<float>(sgn[m]);
@@ -906,11 +904,10 @@ updateG4SinglebandOuterSplit(const TpDims dims, const float2* __restrict__ G, lo
       if (lane == 0)
         mbarArrive(&empty[st]);  // release: this warp's reads of the stage are done
       if (t == 0 && m + DEPTH < n_slots) {
-        if (!mbarWait(&empty[st], (m / DEPTH) & 1, err)) {
-          ok = false;  // the other warps see the missing copy as a timeout of their own
-          break;
-        }
-        issue(m + DEPTH);
+        // Out of time: the vote above ends this warp's loop, the others time out on the missing copy.
+        ok = mbarWait(&empty[st], (m / DEPTH) & 1, err);
+        if (ok)
+          issue(m + DEPTH);
       }
     }
   };
