@@ -6,20 +6,24 @@
 // Eight measurements (one K step of the m16n8k16 MMA: eight measurements x two spins) of a tile's whole
 // blocks are 332 KB, more than an SM's shared memory.  But the elements with a given d_y = (k1 - k2)_y are, in
 // each row k1, one run of six consecutive columns, and every element belongs to one d.  So a CTA takes the
-// six d of one d_y and stages 48 bytes of each row, a sixth of the blocks (55 KB per K step, three steps
-// deep), and over the six CTAs of a tile each element is staged and split into FP16 once.
+// six d of one d_y and stages 48 bytes of each row, a sixth of the blocks (55 KB per K step, two steps
+// deep).  It takes the columns l1 of the first four l1_y or those of the other two (which are the B elements of
+// four or two rows lr_y); the twelve CTAs of a tile run next to each other, and two fit on an SM, so that one
+// multiplies while the other adds its sums to G4 or waits for its first copies.
 //
-// Twelve warps, two per d: rows k1 as three 16-row tiles, columns l1 as five 8-column tiles, three for one
-// warp and two for the other (48 x 40 of 36 x 36 used).  Operands, product order and promotion are those of
-// tp_g4_mma.cu: x = 2^e (hi + lo), lo*hi, hi*lo, hi*hi per real product, each step's chain from zero,
-// promoted into FP32 registers with 2^-2e, e from the step's largest |G| (gmax).  The sums leave through a
-// table [q][k2][k1_x], in runs of six consecutive k1 of G4 (96 bytes) and of the disconnected terms.
+// Six warps, one per d: rows k1 as three 16-row tiles, columns l1 as three 8-column tiles, or as two (48 x 40
+// of 36 x 36 used).  Operands, product order and promotion are those of tp_g4_mma.cu: x = 2^e (hi + lo), lo*hi,
+// hi*lo, hi*hi per real product, each step's chain from zero, promoted into FP32 registers with 2^-2e, e from the
+// step's largest |G| (gmax).  The sums leave through a table [line][k2][k1_x] (a line is a transfer for each k2), in runs of six consecutive k1 of G4
+// (96 bytes) and of the disconnected terms.
 //
 // Half G: a block of the lower frequency half is read as the conjugate of its mirror with k -> -k (whole
 // runs again).  Half G4: only the tiles of tile_order run.
 //
-// Bound by the fragment reads and the FP16 splits.  Nw = 32, half G and half G4, a batch of 128 measurements:
-// 1.65 ms, against 2.33 ms on the FP32 pipe (updateG4SinglebandOuterSplit).
+// Bound by latencies: the tensor pipe is busy for a quarter of the time, a quarter of it goes to the sums' way
+// into G4 (0.42 ms, 0.14 at the memory's rate), the rest to fragment reads and FP16 splits.  Nw = 32, half G and
+// half G4, a batch of 128 measurements: 1.59 ms; 1.65 with one CTA of twelve warps on an SM (a batch of 32: 0.71
+// and 0.69); 2.13 (0.74) on the FP32 pipe (updateG4SinglebandOuterSplit).
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -39,17 +43,17 @@ constexpr uint32_t kRowBytes = kL * sizeof(float2);     // 48: one run of a row
 constexpr uint32_t kPartBytes = kNc * kRowBytes;        // 1,728: A or B of one spin
 constexpr uint32_t kSlotBytes = 4 * kPartBytes + 32;    // A0 B0 A1 B1 of a measurement + bank skew
 constexpr uint32_t kStageBytes = kMeasPerStep * kSlotBytes;
-constexpr int kStages = 3;
-constexpr int kWarps = 2 * kL, kThreads = 32 * kWarps;  // two warps per d
+constexpr int kStages = 2;
+constexpr int kWarps = kL, kThreads = 32 * kWarps;      // a warp per d
 constexpr int kChunks = 4 * kNc * 3;                    // 16-byte copies of a measurement
-constexpr int kCopies = kMeasPerStep * kChunks / kThreads;
-static_assert(kMeasPerStep * kChunks % kThreads == 0, "copies per thread");
+constexpr int kCopies = (kChunks + kThreads - 1) / kThreads;
+constexpr int kSplitY = 4, kSplitCol = kSplitY * kL;    // l1_y, l1 of the CTA with three column tiles
 constexpr int kMaxSteps = 32;  // batches of up to 256 measurements
 // ... and from 32 on: the split operands' error does not depend on the batch, that of the FP32 chain does.  G4
 // against 64 bits, n 100..500: 2.6e-7 at any batch, against 2.4e-7 (12 measurements), 2.7 (24), 2.8 (32) and
 // 3.0 (64) in FP32; n < 60: 1.2e-7 against 1.2 (12), 1.6 (24), 1.8 (32) and 2.5.
 constexpr int kMinSlots = 32;
-constexpr uint32_t kTableBytes = kBlk * kL * sizeof(float2);
+constexpr uint32_t kTableBytes = kSplitCol * kNc * kL * sizeof(float2);
 static_assert(kTableBytes <= kStages * kStageBytes, "the flush table reuses the stages");
 constexpr uint32_t kOffExp = kStages * kStageBytes;
 constexpr uint32_t kOffRun = kOffExp + 4 * kMaxSteps;    // [2][36] source offset of a row's run (A, B)
@@ -58,7 +62,8 @@ constexpr uint32_t kOffKneg = kOffKsub + kBlk;           // k -> -k
 constexpr uint32_t kOffQinv = kOffKneg + kNc;            // q -> its position in q_list
 constexpr uint32_t kOffSigns = kOffQinv + kNc;           // [m]
 constexpr size_t kSmem = kOffSigns + kMaxSteps * kMeasPerStep;
-static_assert(kSmem <= 227 * 1024, "shared memory per CTA");
+static_assert(kPartBytes == 16 * 3 * kNc, "chunk order");
+static_assert(kSmem <= 113 * 1024, "shared memory per CTA");
 constexpr int kExpMax = 60;  // |e| <= 60 keeps 2^{+-2e} a normal FP32 number
 constexpr int kMaxCh = 2;
 
@@ -165,21 +170,22 @@ __device__ __forceinline__ void stepMma(const unsigned char* S, const int (&oa)[
   }
 }
 
-// Barrier of the whole CTA, met by the two kinds of warps at different places of the code.
-__device__ inline void ctaSync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
-}
-
 struct Tables {
   const int* step_exp;
-  const unsigned char *ksub, *kneg, *qinv;
+  const unsigned char *ksub, *kneg;
   const signed char* sgn;
 };
 
-// The batch loop of a warp with NT column tiles from n0 on, and its part of the flush table.
-template <int NT, typename Advance>
-__device__ __forceinline__ void batchProduct(unsigned char* smem, const Tables& tb, int d, int n0, bool mir_a, bool mir_b,
+// The table's line of entry (k1, l1): the l1 that belongs to the first k1 of its run and the same q = l1 - k1.
+__device__ inline int lineOf(const Tables& tb, int k1, int l1) {
+  return tb.ksub[tb.kneg[k1 / kL * kL] + kNc * tb.ksub[k1 + kNc * l1]];
+}
+
+// The batch loop of a warp: columns l1 from 8 N0 on, NT tiles of 8, and its part of the flush table.
+template <int NT, int N0, typename Advance>
+__device__ __forceinline__ void batchProduct(unsigned char* smem, const Tables& tb, int d, bool mir_a, bool mir_b,
                                              int n_slots, Advance advance) {
+  constexpr int n0 = N0;
   const int lane = threadIdx.x % 32, g = lane >> 2, t4 = lane & 3;
   // Element (k1, k2 = k1 - d) of A: staged row k1, column k2_x of the run (mirrored: (-k2)_x); element
   // (lr = l1 - d, l1) of B: staged row lr, column l1_x (mirrored: (-l1)_x).
@@ -214,7 +220,7 @@ __device__ __forceinline__ void batchProduct(unsigned char* smem, const Tables& 
     else
       stepMma<NT, false>(S, oa, ob, a4, blast, t4, m0, n_slots, tb.sgn, pow2(e), pow2(-2 * e), ca, cb, re, im);
   }
-  ctaSync();  // every warp is done with the stages
+  __syncthreads();  // every warp is done with the stages
   float2* table = reinterpret_cast<float2*>(smem);
 #pragma unroll
   for (int mt = 0; mt < 3; ++mt)
@@ -224,13 +230,13 @@ __device__ __forceinline__ void batchProduct(unsigned char* smem, const Tables& 
       for (int k = 0; k < 4; ++k) {
         const int k1 = 16 * mt + g + 8 * (k >> 1), l1 = 8 * (n0 + n) + 2 * t4 + (k & 1);
         if (k1 < kNc && l1 < kNc)
-          table[(tb.qinv[tb.ksub[k1 + kNc * l1]] * kNc + tb.ksub[d + kNc * k1]) * kL + k1 % kL] =
+          table[((lineOf(tb, k1, l1) - 8 * N0) * kNc + tb.ksub[d + kNc * k1]) * kL + k1 % kL] =
               make_float2(re[mt][n][k], im[mt][n][k]);
       }
-  ctaSync();
+  __syncthreads();
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 2)
 updateG4DirectMma36(const TpDims dims, const float2* __restrict__ G, long g_sector_stride,
                     const int* __restrict__ signs, int n_slots, const int* __restrict__ k_sub,
                     const int* __restrict__ q_list, const int* __restrict__ wex_list, const int* __restrict__ gmax,
@@ -245,7 +251,9 @@ updateG4DirectMma36(const TpDims dims, const float2* __restrict__ G, long g_sect
   signed char* sgn = reinterpret_cast<signed char*>(smem + kOffSigns);
   const int t = threadIdx.x, warp = t / 32, lane = t % 32;
   const int nw = dims.nw, nw_ext = dims.nw_ext, nq = dims.nq, n_ch = dims.n_channels;
-  const int dy = blockIdx.x % kL, tile = blockIdx.x / kL;  // the six CTAs of a tile run next to each other
+  const int part = blockIdx.x % (2 * kL), tile = blockIdx.x / (2 * kL);  // the twelve CTAs of a tile run next to each other
+  const int dy = part >> 1;
+  const bool wide = (part & 1) == 0;  // columns l1 < 24, or the others
   const int per_wq = tile_order ? nw * nw / 2 : nw * nw;
   int w1, w2;
   if (tile_order) {
@@ -300,25 +308,32 @@ updateG4DirectMma36(const TpDims dims, const float2* __restrict__ G, long g_sect
   }
   __syncthreads();
 
-  // This thread's copies of a step: 16-byte chunk c of measurement c / kChunks, part A0 B0 A1 B1, row, third.
-  long src[kCopies];
-  uint32_t dst[kCopies];
+  // This thread's copies of a measurement, 16-byte chunk t + kThreads i: part A0 B0 A1 B1, row, third; without
+  // the B rows lr = l1 - d of the other columns l1.
+  int src[kCopies];  // element of its block, or -1
 #pragma unroll
   for (int i = 0; i < kCopies; ++i) {
-    const int c = t + kThreads * i, m = c / kChunks, rem = c % kChunks;
-    const int part = rem / (3 * kNc), row = rem % (3 * kNc) / 3, third = rem % 3;
-    src[i] = g_sector_stride * (2 * m + (part >> 1)) + ((part & 1) ? b_B + run[kNc + row] : b_A + run[row]) + 2 * third;
-    dst[i] = smemAddr(smem) + m * kSlotBytes + part * kPartBytes + row * kRowBytes + 16 * third;
+    const int c = t + kThreads * i, p = c / (3 * kNc) % 4, row = c % (3 * kNc) / 3, third = c % 3;
+    const int l1 = ksub[kneg[kL * dy] + kNc * row];  // row + d: y of the columns that read this row of B
+    const bool need = c < kChunks && (!(p & 1) || (l1 < kSplitCol) == wide);
+    src[i] = !need ? -1 : (p & 1) ? run[kNc + row] + 2 * third : run[row] + 2 * third;
   }
   auto copyStep = [&](int step) {
     if (step < n_steps) {
+      const uint32_t to = smemAddr(smem) + step % kStages * kStageBytes + 16 * t;  // chunks lie in order
+      const int n = min(kMeasPerStep, n_slots - step * kMeasPerStep);
       const float2* base = G + g_sector_stride * (2 * kMeasPerStep * static_cast<long>(step));
-      const uint32_t st = step % kStages * kStageBytes;
-      const int left = (n_slots - step * kMeasPerStep) * kChunks;
 #pragma unroll
-      for (int i = 0; i < kCopies; ++i)
-        if (t + kThreads * i < left)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst[i] + st), "l"(base + src[i]) : "memory");
+      for (int i = 0; i < kCopies; ++i) {
+        if (src[i] < 0)
+          continue;
+        const int p = (t + kThreads * i) / (3 * kNc);
+        const float2* from = base + (p >> 1) * g_sector_stride + ((p & 1) ? b_B : b_A) + src[i];
+        for (int m = 0; m < n; ++m)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16 * kThreads * i + m * kSlotBytes),
+                       "l"(from + 2 * m * g_sector_stride)
+                       : "memory");
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -326,42 +341,43 @@ updateG4DirectMma36(const TpDims dims, const float2* __restrict__ G, long g_sect
     copyStep(s);
   auto advance = [&](int step) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
-    ctaSync();
+    __syncthreads();
     copyStep(step + kStages - 1);
   };
-  const Tables tb{step_exp, ksub, kneg, qinv, sgn};
-  const int d = kL * dy + warp / 2;
-  if (warp % 2 == 0)
-    batchProduct<3>(smem, tb, d, 0, mir_a, mir_b, n_slots, advance);
+  const Tables tb{step_exp, ksub, kneg, sgn};
+  const int d = kL * dy + warp;
+  if (wide)
+    batchProduct<3, 0>(smem, tb, d, mir_a, mir_b, n_slots, advance);
   else
-    batchProduct<2>(smem, tb, d, 3, mir_a, mir_b, n_slots, advance);
+    batchProduct<2, 3>(smem, tb, d, mir_a, mir_b, n_slots, advance);
 
-  // Flush: k1_x fastest, then k2, then the transfer; U entries' loads in flight.
+  // Flush: k1_x fastest, then k2, then the line; U entries' loads in flight.
   const float2* table = reinterpret_cast<const float2*>(smem);
+  const int line0 = wide ? 0 : kSplitCol, entries = (wide ? kSplitCol : kNc - kSplitCol) * kNc * kL;
   const long M = static_cast<long>(kNc) * nw;
   const long s_w1 = kNc, s_k2 = s_w1 * nw, s_w2 = s_k2 * kNc, s_q = s_w2 * nw, s_wq = s_q * nq;
-  constexpr int U = 7, kEntries = kBlk * kL;
+  constexpr int U = 9;
   for (int c = 0; c < n_ch; ++c)
-    for (int base = t; base < kEntries; base += U * kThreads) {
+    for (int base = t; base < entries; base += U * kThreads) {
       double2 o[U];
       float2 v[U];
       long at[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int idx = min(base + u * kThreads, kEntries - 1);
-        const int kx = idx % kL, k2 = idx / kL % kNc, qi = idx / (kL * kNc);
+        const int idx = min(base + u * kThreads, entries - 1);
+        const int kx = idx % kL, k2 = idx / kL % kNc, l1 = line0 + idx / (kL * kNc);
         // k1 = k2 + d has y = (k2 + d)_y; the run's x are those of the table.
-        const int k1 = ksub[kneg[kL * dy] + kNc * k2] / kL * kL + kx;
-        at[u] = k1 + w1 * s_w1 + k2 * s_k2 + w2 * s_w2 + qi * s_q + iwq * s_wq;
+        const int k1 = ksub[kneg[kL * dy] + kNc * k2] / kL * kL, qi = qinv[ksub[k1 + kNc * l1]];
+        at[u] = k1 + kx + w1 * s_w1 + k2 * s_k2 + w2 * s_w2 + qi * s_q + iwq * s_wq;
         const float2 dv = __ldg(disc + ((static_cast<long>(iwq * nq + qi) * n_ch + c) * M + k2 +
-                                        static_cast<long>(kNc) * w2) * M + k1 + static_cast<long>(kNc) * w1);
+                                        static_cast<long>(kNc) * w2) * M + k1 + kx + static_cast<long>(kNc) * w1);
         const float2 x = table[idx];
         v[u] = make_float2(x.x + dv.x, x.y + dv.y);
         o[u] = atomic ? make_double2(0., 0.) : G4[c][at[u]];
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        if (base + u * kThreads >= kEntries)
+        if (base + u * kThreads >= entries)
           continue;
         double2* p = G4[c] + at[u];
         if (atomic) {
@@ -386,7 +402,7 @@ void launchDirectTc36(const G4Args& a, const float2* G, long g_sector_stride, co
   const TpDims& d = a.dims;
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(updateG4DirectMma36, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem)));
   const long tiles = long(d.nw) * d.nw * d.nwq / (a.tile_order ? 2 : 1);  // half G4: w1 >= Nw / 2 only
-  updateG4DirectMma36<<<static_cast<unsigned>(tiles * kL), kThreads, kSmem, stream>>>(
+  updateG4DirectMma36<<<static_cast<unsigned>(tiles * 2 * kL), kThreads, kSmem, stream>>>(
       d, G, g_sector_stride, a.signs, a.n_slots, a.k_sub, a.q_list, a.wex_list, a.gmax, a.tile_order, disc, a.G4, a.atomic);
   DCAACC_LAUNCH_CHECK();
 }
