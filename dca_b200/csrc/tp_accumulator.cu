@@ -415,6 +415,8 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
       for (int k = 0; k < nc; ++k)
         dims_.kneg[k] = static_cast<unsigned char>(kneg[k]);
       mirrorTransfers(kneg);
+      // Half of G where every measurement goes to the kernel that reads it mirrored.
+      dims_.half_g = max_batch_ == 1 && singlebandGatherApplies(dims_);
     }
   }
   for (auto& h : hstage_) {
@@ -1181,7 +1183,7 @@ void TpAccumulator::getG(int spin, double* out, size_t count) const {
   const size_t total = size_t(g_sector_stride_);
   if (count != total)
     invalid("output size does not match the G size");
-  std::vector<double2> blk(total);
+  std::vector<double2> blk(total);  // with half G, of the upper frequency half alone
   DCAACC_CUDA_CHECK(cudaStreamSynchronize(stream_));
   DCAACC_CUDA_CHECK(cudaMemcpy(blk.data(), G64_.get() + size_t(spin) * g_sector_stride_,
                                sizeof(double2) * total, cudaMemcpyDeviceToHost));
@@ -1192,9 +1194,11 @@ void TpAccumulator::getG(int spin, double* out, size_t count) const {
         for (int cc = 0; cc < R; ++cc) {
           const int b1 = r % nb, k1 = r / nb, b2 = cc % nb, k2 = cc / nb;
           const size_t o = b1 + nb * (b2 + nb * (k1 + nc * (k2 + size_t(nc) * (wr + size_t(nwe) * wc))));
-          const double2 v = blk[((size_t(wr) * nwe + wc) * R + r) * R + cc];
+          const bool mirror = dims_.half_g && 2 * wr < nwe;
+          const double2 v = mirror ? blk[((size_t(nwe - 1 - wr) * nwe + nwe - 1 - wc) * R + dims_.kneg[r]) * R + dims_.kneg[cc]]
+                                   : blk[((size_t(wr) * nwe + wc) * R + r) * R + cc];
           out[2 * o] = v.x;
-          out[2 * o + 1] = v.y;
+          out[2 * o + 1] = mirror ? -v.y : v.y;
         }
 }
 

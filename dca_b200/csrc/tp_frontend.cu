@@ -25,8 +25,12 @@
 // reads 2 + WT/4 elements for 2 WT/4 complex multiply-adds.  Phase 2: 4 x 2 sums a lane over the
 // sites, or on a 4 x 4 cluster an FFT (a fifth of the matrix's FP64 operations, which were more than
 // phase 1's), one (row, frequency) pair a thread.  Both phases are bound by the FP64 pipe.  The earlier kernels gave a thread one sum, that
-// is two shared-memory reads per multiply-add, and a whole CTA one orbital at a time:
-// FRONT_BEFORE_AFTER
+// is two shared-memory reads per multiply-add, and a whole CTA one orbital at a time.  One measurement, 4x4,
+// Nw = 64, n 100..300: row step 42 -> 17 us, 14 with the FFT; column step 151 -> 41, 28 with the FFT.  The FFT's
+// phases are exact; those of momenta rounded to 2 pi m / 4 +- 2e-15 are off by 3e-15, and so is a G from them.
+//
+// Half G (dims.half_g; mirror-symmetric inputs, a G4 kernel that reads mirrored blocks): the rows with
+// w1 >= NwExt / 2 alone, in both steps: 28 -> 16 and 14 -> 13 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -248,7 +252,7 @@ struct Tile {
 template <int NB>
 constexpr int kTaskK = NB == 1 ? 16 : 8;
 
-// Row transform.  grid (ceil(n_max / 16), ceil(NwExt / WT), n_sectors).  NB: bands (1, 2 or 3), 0 for
+// Row transform.  grid (ceil(n_max / 16), ceil(frequencies / WT), n_sectors).  NB: bands (1, 2 or 3), 0 for
 // any number.
 template <int WT, int L, int NB>
 __global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
@@ -260,7 +264,8 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const __grid_constant__ ColFft fft, double2* __restrict__ Xp) {
   using T = Tile<WT, L>;
   const SectorDesc sd = sectors[blockIdx.z];
-  const int n = sd.n, j0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
+  // Half G: the frequencies from NwExt / 2 on.
+  const int n = sd.n, j0 = blockIdx.x * kTileR, w0 = (dims.half_g ? dims.nw_ext / 2 : 0) + blockIdx.y * WT;
   if (j0 >= n)
     return;
   const int nw_ext = dims.nw_ext, R = dims.R, nb = NB ? NB : dims.nb, nc = dims.nc;
@@ -417,8 +422,8 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   }
 }
 
-// Column transform + G epilogue.  grid (ceil(D / 16), ceil(NwExt / WT), n_sectors); the rows of a tile
-// are 16 consecutive (w1, r).
+// Column transform + G epilogue.  grid (ceil(rows / 16), ceil(NwExt / WT), n_sectors); the rows of a tile
+// are 16 consecutive (w1, r), with half G those from D / 2 on.
 template <int WT, int L, int NB>
 __global__ void __launch_bounds__(kTileR* WT, WT == 16 ? 2 : 4)
 colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
@@ -430,7 +435,7 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   using T = Tile<WT, L>;
   const SectorDesc sd = sectors[blockIdx.z];
   const int nw_ext = dims.nw_ext, R = dims.R, nb = NB ? NB : dims.nb, nc = dims.nc;
-  const int D = R * nw_ext, row0 = blockIdx.x * kTileR, w0 = blockIdx.y * WT;
+  const int D = R * nw_ext, row0 = (dims.half_g ? D / 2 : 0) + blockIdx.x * kTileR, w0 = blockIdx.y * WT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
   T tile(smem_raw, dims, Fb, col_start + sd.orb_off, fft,
@@ -659,27 +664,27 @@ static int tileWidth(const FrontendArgs& a, const char* family, LaunchTuner::Pic
 }
 
 template <int WT, int L, typename Kernel, typename... Args>
-static void launchTile(Kernel k, const TpDims& d, int tiles, int sectors, cudaStream_t stream, Args... args) {
+static void launchTile(Kernel k, const TpDims& d, int tiles, int freqs, int sectors, cudaStream_t stream, Args... args) {
   const size_t smem = Tile<WT, L>::bytes(d);
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   DCAACC_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                                          int(cudaSharedmemCarveoutMaxShared)));
-  k<<<dim3(tiles, ceil_div(d.nw_ext, WT), sectors), Tile<WT, L>::kThreads, smem, stream>>>(d, args...);
+  k<<<dim3(tiles, ceil_div(freqs, WT), sectors), Tile<WT, L>::kThreads, smem, stream>>>(d, args...);
   DCAACC_LAUNCH_CHECK();
 }
 
 template <int WT>
 static void launchRowWT(const FrontendArgs& a, double2* Xp, cudaStream_t stream) {
-  const int nb = a.dims.nb, tiles = ceil_div(a.n_max, kTileR);
+  const int nb = a.dims.nb, tiles = ceil_div(a.n_max, kTileR), freqs = a.dims.nw_ext / (a.dims.half_g ? 2 : 1);
   if (fft4(a)) {
-    launchTile<WT, 4>(rowTransformKernel<WT, 4, 1>, a.dims, tiles, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
+    launchTile<WT, 4>(rowTransformKernel<WT, 4, 1>, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
                       a.row_start, a.Tr, a.Fb, a.G0, a.fft, Xp);
     return;
   }
   auto k = nb == 1   ? rowTransformKernel<WT, 0, 1>
            : nb == 2 ? rowTransformKernel<WT, 0, 2>
            : nb == 3 ? rowTransformKernel<WT, 0, 3> : rowTransformKernel<WT, 0, 0>;
-  launchTile<WT, 0>(k, a.dims, tiles, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c, a.row_start, a.Tr, a.Fb, a.G0,
+  launchTile<WT, 0>(k, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c, a.row_start, a.Tr, a.Fb, a.G0,
                     a.fft, Xp);
 }
 
@@ -696,16 +701,17 @@ void launchRowTransform(const FrontendArgs& a, double2* Xp, cudaStream_t stream)
 
 template <int WT>
 static void launchColWT(const FrontendArgs& a, const double2* Xp, double2* G, long g_sector_stride, cudaStream_t stream) {
-  const int nb = a.dims.nb, tiles = ceil_div(long(a.dims.R) * a.dims.nw_ext, kTileR);
+  const int nb = a.dims.nb, freqs = a.dims.nw_ext;
+  const int tiles = ceil_div(long(a.dims.R) * freqs / (a.dims.half_g ? 2 : 1), kTileR);
   if (fft4(a)) {
-    launchTile<WT, 4>(colTransformKernel<WT, 4, 1>, a.dims, tiles, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb,
+    launchTile<WT, 4>(colTransformKernel<WT, 4, 1>, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb,
                       a.G0, a.fft, Xp, G, g_sector_stride);
     return;
   }
   auto k = nb == 1   ? colTransformKernel<WT, 0, 1>
            : nb == 2 ? colTransformKernel<WT, 0, 2>
            : nb == 3 ? colTransformKernel<WT, 0, 3> : colTransformKernel<WT, 0, 0>;
-  launchTile<WT, 0>(k, a.dims, tiles, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb, a.G0, a.fft, Xp, G,
+  launchTile<WT, 0>(k, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb, a.G0, a.fft, Xp, G,
                     g_sector_stride);
 }
 

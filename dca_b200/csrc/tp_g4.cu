@@ -786,7 +786,7 @@ updateG4SinglebandStream(const TpDims dims, const GT* __restrict__ G, long g_sec
 //
 // With few transfers an entry costs more G than G4 traffic and a tile is 256 entries: the streaming kernel's
 // persistent CTAs wait out a load round trip per tile for it, this one has all of an SM's threads in flight.
-// 4x4, Nw = 64, one transfer, FP64: 36 -> 19 us per measurement.
+// 4x4, Nw = 64, one transfer, FP64: 36 -> 19 us per measurement, 11 with half of G4.
 template <typename GT, typename AT>
 __global__ void __launch_bounds__(256)
 updateG4SinglebandGather(const TpDims dims, const GT* __restrict__ G, long g_sector_stride,
@@ -794,7 +794,7 @@ updateG4SinglebandGather(const TpDims dims, const GT* __restrict__ G, long g_sec
                          const int* __restrict__ q_list, const int* __restrict__ wex_list,
                          double2* const* __restrict__ G4, bool atomic) {
   using C = cplx_t<AT>;
-  const int nc = dims.nc, nw = dims.nw, nw_ext = dims.nw_ext, blk = nc * nc;
+  const int nc = dims.nc, nw = dims.nw, blk = nc * nc;
   const int nw1 = dims.half_g4 ? nw / 2 : nw;  // half G4: w1 >= Nw / 2
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= blk * nw1 * nw)
@@ -804,17 +804,23 @@ updateG4SinglebandGather(const TpDims dims, const GT* __restrict__ G, long g_sec
   const int q = q_list[iq], wex = wex_list[iwq];
   const int k1q = k_add[k1 + nc * q], k2q = k_add[k2 + nc * q];
   const int w1e = w1 + dims.ext, w2e = w2 + dims.ext, w1x = w1e + wex, w2x = w2e + wex;
-  auto at = [&](int wr, int wc, int r, int c) { return ((static_cast<long>(wr) * nw_ext + wc) * nc + r) * nc + c; };
   const GT* G1 = G + g_sector_stride;
-  const long ia = at(w1e, w2e, k1, k2), ib = at(w2x, w1x, k2q, k1q), iu = at(w1e, w1x, k1, k1q),
-             iv = at(w2x, w2e, k2q, k2);
+  bool ca, cb, cu, cv;
+  const long ia = gIndexMirrored(dims, w1e, w2e, k1, k2, ca), ib = gIndexMirrored(dims, w2x, w1x, k2q, k1q, cb),
+             iu = gIndexMirrored(dims, w1e, w1x, k1, k1q, cu), iv = gIndexMirrored(dims, w2x, w2e, k2q, k2, cv);
+  auto load = [&](const GT* g, long i, bool conj) {
+    C z = ldG<GT, AT>(g + i);
+    if (conj)
+      z.y = -z.y;
+    return z;
+  };
   const long g4i = k1 + nc * (w1 + static_cast<long>(nw) * (k2 + nc * (w2 + static_cast<long>(nw) * (iq + static_cast<long>(dims.nq) * iwq))));
   double2 old[2];
 #pragma unroll
   for (int c = 0; c < 2; ++c)
     old[c] = c < dims.n_channels && !atomic ? G4[c][g4i] : make_double2(0., 0.);
-  const C a0 = ldG<GT, AT>(G + ia), a1 = ldG<GT, AT>(G1 + ia), b0 = ldG<GT, AT>(G + ib), b1 = ldG<GT, AT>(G1 + ib);
-  const C u0 = ldG<GT, AT>(G + iu), u1 = ldG<GT, AT>(G1 + iu), v0 = ldG<GT, AT>(G + iv), v1 = ldG<GT, AT>(G1 + iv);
+  const C a0 = load(G, ia, ca), a1 = load(G1, ia, ca), b0 = load(G, ib, cb), b1 = load(G1, ib, cb);
+  const C u0 = load(G, iu, cu), u1 = load(G1, iu, cu), v0 = load(G, iv, cv), v1 = load(G1, iv, cv);
   const AT hs = AT(0.5) * static_cast<AT>(signs[0]);
   C d = cmul(a0, b0);
   cfma(d, a1, b1);
@@ -920,11 +926,16 @@ static bool launchSinglebandStream(const G4Args& a, const GT* G, long g_sector_s
 
 // Up to kGatherMaxQ transfers (the streaming kernel reuses a tile's blocks for each further one).
 constexpr int kGatherMaxQ = 2;
+bool singlebandGatherApplies(const TpDims& d) {
+  return d.nq <= kGatherMaxQ && d.n_channels <= 2 && singlebandPHApplies<double2>(d) &&
+         long(d.nc) * d.nc * d.nw * d.nw <= (1L << 31) - 256;
+}
+
 template <typename GT>
 static bool launchSinglebandGather(const G4Args& a, const GT* G, long g_sector_stride, cudaStream_t stream) {
   const TpDims& d = a.dims;
   const long entries = long(d.nc) * d.nc * g4Rows(d) * d.nw;
-  if (a.n_slots != 1 || d.nq > kGatherMaxQ || d.n_channels > 2 || !singlebandPHApplies<GT>(d) || entries > (1L << 31) - 256)
+  if (a.n_slots != 1 || !singlebandGatherApplies(d))
     return false;
   using AT = std::conditional_t<std::is_same_v<GT, double2>, double, float>;
   updateG4SinglebandGather<GT, AT><<<dim3(ceil_div(entries, 256), d.nq, d.nwq), 256, 0, stream>>>(

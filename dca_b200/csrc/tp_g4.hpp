@@ -77,6 +77,10 @@ size_t discScratchBytes(const TpDims& d, int max_batch);
 void discInit(DiscWorkspace& w, const TpDims& d, int max_batch, void* mem, size_t bytes);
 const float2* launchDiscGemm(const G4Args& a, const float2* G, long g_sector_stride, cudaStream_t stream);
 
+// Single measurements of these sizes take the kernel that reads its operands straight from G, and mirrored ones
+// with half G (tp_g4.cu, updateG4SinglebandGather).
+bool singlebandGatherApplies(const TpDims& d);
+
 // Tensor-core direct term (tp_g4_mma.cu): one band, Nc = 16, all momentum transfers, with the
 // disconnected terms precomputed (disc) and the per-sector maxima of G recorded by the column step.
 bool directTcApplies(const G4Args& a);

@@ -27,12 +27,12 @@ struct TpDims {
   int n_channels;
   int channels[kMaxChannels];
   double beta;
-  // Mixed path, one band, Nc <= kMaxMirrorNc: G rows of the lower frequency half (w1 < nw_ext / 2)
+  // One band (mixed path: Nc = 16, 36; FP64: where singlebandGatherApplies): G rows of the lower frequency half (w1 < nw_ext / 2)
   // are not computed; G(k1 w1; k2 w2) = conj G(-k1 w1'; -k2 w2') with w' = nw_ext - 1 - w (real M
   // and G0(-k, -w) = conj G0(k, w)), and the consumers read that mirror instead.
   int half_g;
   unsigned char kneg[64];  // index of -k (half_g only; Nc <= kMaxKneg)
-  // With half_g (or in FP64, where all of G is computed, with inputs symmetric to rounding), and momentum
+  // With half_g (or in FP64 with inputs symmetric to rounding), and momentum
   // and frequency transfers closed under negation, G4 itself obeys
   // G4(-k1 w1', -k2 w2', -q, -wq) = conj G4(k1 w1, k2 w2, q, wq) (w' = Nw - 1 - w): the update
   // accumulates the frequency tiles with w1 >= Nw / 2 only and the rest is filled from them when

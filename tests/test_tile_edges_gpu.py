@@ -131,6 +131,29 @@ def test_three_band_pairing(oracle_lib, cluster, k_ex, n_meas, max_batch):
     _compare(oracle_lib, _g0(rng, 3, cl, 7), _measurements(rng, 3, cl.nc, orders), params, MIXED_TOL)
 
 
+@pytest.mark.parametrize("cluster,w_ex,channels", [("2x1", [0, 2], [3]), ("3x2", [0], [2]), ("4x4", [-1, 1], [2, 3])])
+def test_fp64_half_g(monkeypatch, cluster, w_ex, channels):
+    """FP64, one transfer: G4 and G with half of G against all of it.  The two halves come from different
+    terms' roundings of one sum: a few ulps of the largest entries."""
+    from dca_b200.accumulators import TpAccumulator
+    rng = np.random.default_rng(12)
+    cl = CLUSTERS[cluster]
+    orders = [(33, 7), (0, 18)]
+    params = _params(1, cl, 3, 9, channels, [cl.nc - 1], w_ex, orders)
+    measurements, got = _measurements(rng, 1, cl.nc, orders), []
+    for full in ("0", "1"):
+        monkeypatch.setenv("DCAACC_TP_FULL_G", full)
+        acc = TpAccumulator(_g0(rng, 1, cl, 9), params)
+        acc.resetAccumulation(0)
+        for m in measurements:
+            acc.accumulate([s.M for s in m.sectors], list(m.sectors), m.sign)
+        gs = [acc.get_G(spin) for spin in range(2)]
+        acc.finalize()
+        got.append(gs + acc.get_G4())
+    for a, b in zip(*got):
+        assert rel_err(a, b) <= FP64_TOL
+
+
 def test_fp64_graphs():
     """FP64 with and without captured graphs, orders on both sides of the launch shapes' steps of 128."""
     from dca_b200.accumulators import TpAccumulator
