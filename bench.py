@@ -559,6 +559,8 @@ def run_ours(args, world, rank, local):
     g4_sec = stages["update_g4"][0] / args.steps / 1e3  # the stage's time per batch
     g4_paths = {"direct_tc": "discPlanesKernel + frontGemmKernel<2> (disconnected terms) + updateG4DirectMma "
                              "(direct term, G4 flush)",
+                "direct_tc36": "discPlanesKernel + frontGemmKernel<2> (disconnected terms) + "
+                               "updateG4DirectMma36 (direct term, G4 flush)",
                 "split36": "discPlanesKernel + frontGemmKernel<2> (disconnected terms) + "
                            "updateG4SinglebandOuterSplit (direct term, G4 flush)",
                 "staged": "updateG4StagedKernel (all terms, G blocks staged in shared memory)",
@@ -569,13 +571,15 @@ def run_ours(args, world, rank, local):
     # Column step and G4 kernels as the accumulator selects them (environment switches included).
     half_any = bool(mirror & 1) or bool(mirror & 2)
     col_env = os.environ.get("DCAACC_TP_FACTORED_COL")
-    factorable = nb == 1 and nc == 16 and not fp64_main and not simt
-    col_tc = factorable and col_env not in ("0", "1") and os.environ.get("DCAACC_TP_COL_FFT") != "0"
-    factored_col = factorable and (col_tc or (col_env == "1" and os.environ.get("DCAACC_TP_COL_FFT") != "0"))
+    fft_on = os.environ.get("DCAACC_TP_COL_FFT") != "0"
+    # One band: both steps factored by orbital in FP32 unless the tensor-core front-end is asked for.
+    front32 = not fp64_main and (simt or (nb == 1 and (nc <= 8 or fft_on) and col_env not in ("0", "1", "2")))
+    factorable = nb == 1 and nc == 16 and not fp64_main and not front32
+    col_tc = factorable and col_env == "2" and fft_on
+    factored_col = factorable and (col_tc or (col_env == "1" and fft_on))
     # 6 x 6 cluster with DCAACC_TP_FACTORED_COL=1: the column step factored on the CUDA cores with the
     # 6 x 6 FFT.
-    wide_col = (nb == 1 and nc == 36 and not fp64_main and not simt and col_env == "1"
-                and os.environ.get("DCAACC_TP_COL_FFT") != "0")
+    wide_col = nb == 1 and nc == 36 and not fp64_main and not simt and col_env == "1" and fft_on
     factored_col = factored_col or wide_col
     if fp64_main:
         g4_path = "stream" if nb == 1 and nc * nc <= 256 and set(w.channels) <= {2, 3} else "fp64_other"
@@ -586,20 +590,22 @@ def run_ours(args, world, rank, local):
     elif nb > 1:
         g4_path = "staged"
     elif nc == 36:
-        g4_path = "split36"
+        g4_path = "direct_tc36" if B >= 32 else "split36"
     else:
         g4_path = "direct_tc"
     stage_kernels = {"update_g4": {"direct_tc": ["discPlanesKernel", "frontGemmKernel<2>", "updateG4DirectMma"],
+                                   "direct_tc36": ["discPlanesKernel", "frontGemmKernel<2>", "updateG4DirectMma36"],
                                    "split36": ["discPlanesKernel", "frontGemmKernel<2>",
                                                "updateG4SinglebandOuterSplit"],
                                    "staged": ["updateG4StagedKernel"],
                                    "pp3": ["updateG4PPMultibandKernel"],
                                    "stream": ["updateG4SinglebandStream"]}.get(g4_path, []),
-                     "col_transform": (["colFactorTcKernel"] if col_tc else ["colFactorWideKernel"] if wide_col else
+                     "col_transform": (["colTransform32Kernel"] if front32 else ["colFactorTcKernel"] if col_tc else ["colFactorWideKernel"] if wide_col else
                                        ["colTwiddlePlanesKernel", "colFactorMmaKernel"] if factored_col
                                        else ["frontGemmKernel<1>"]),
-                     "row_transform": ["frontGemmKernel<0>"],
-                     "twiddle": (["twiddleWiKernel", "buildMOperandKernel", "buildPhaseOperandKernel"] if factored_col
+                     "row_transform": ["rowTransform32Kernel" if front32 else "frontGemmKernel<0>"],
+                     "twiddle": (["twiddle32Kernel", "sortM32Kernel"] if front32 else
+                                 ["twiddleWiKernel", "buildMOperandKernel", "buildPhaseOperandKernel"] if factored_col
                                  else ["twiddleWiKernel", "buildMOperandKernel", "buildPhasePairKernel"])}
     # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of each stage's kernels per launch of
     # the stage, from the committed ncu capture of this workload (cold caches).
@@ -632,7 +638,7 @@ def run_ours(args, world, rank, local):
     dom_ms, dom_launches = stages[dom]
     per_launch_ms = dom_ms / args.steps
     sec = per_launch_ms / 1e3
-    tc_front = not simt and not fp64_main
+    tc_front = not front32 and not fp64_main
     if dom == "update_g4":
         roof = {"kernel": "update_g4 stage: " + g4_roof["kernels"], "bound": "hbm",
                 "achieved": g4_alg_bytes / sec / 1e9, "peak": hbm_gbs, "unit": "GB/s",
@@ -684,6 +690,21 @@ def run_ours(args, world, rank, local):
             roof["memory_view"] = {"algorithmic_bytes": mem_bytes, "achieved_gbs": mem_bytes / sec / 1e9,
                                    "frac_of_hbm": mem_bytes / sec / 1e9 / hbm_gbs,
                                    "note": "X' read and G written once per launch, for the rows computed"}
+    elif dom in ("col_transform", "row_transform") and front32:
+        # FP32 front-end factored by orbital: the algorithmic flops against the FP32 pipe, and the row or column
+        # step's own bytes (M or X' in, X' or G out, for the rows computed) against HBM.
+        rows_done = 0.5 if mirror & 1 else 1.0
+        fp32_peak = 148 * 128 * 2 * 1.965e-3  # TFLOP/s, 148 SMs of 128 lanes at 1,965 MHz
+        kern = {"col_transform": "colTransform32Kernel", "row_transform": "rowTransform32Kernel"}[dom]
+        roof = {"kernel": kern + " (factored by orbital, packed FP32 multiply-adds, cluster transform, G0 factor)",
+                "bound": "fp32", "achieved": alg_flops[dom] * rows_done / sec / 1e12, "peak": fp32_peak,
+                "unit": "TFLOP/s", "algorithmic_flops": alg_flops[dom] * rows_done,
+                "peak_note": "nominal FP32 rate; algorithmic flops per spin of the reference's two-stage form, for the "
+                             "rows computed (its matrix cluster transform is an FFT here)"}
+        per = D * ns * 8.0 + D * D * 8.0 if dom == "col_transform" else ns * ns * 4.0 / rows_done + D * ns * 8.0
+        mem_bytes = per_step * rows_done * float(np.sum(per))
+        roof["memory_view"] = {"algorithmic_bytes": mem_bytes, "achieved_gbs": mem_bytes / sec / 1e9,
+                               "frac_of_hbm": mem_bytes / sec / 1e9 / hbm_gbs}
     else:
         # SIMT front-end stages are dominated by their global traffic (M / X' / G, complex of the
         # path's precision).

@@ -11,8 +11,8 @@
 //   G(rho1; k2, w2) = -(1/Nc) G0_s(k2, w2) sum_r e^{-i k2 x_r} Z(rho1, w2, r)
 //                     + beta G0_s(k2, w2) delta_{rho1, rho2}
 // whose work is 8 D NwExt n + 8 D^2 Nc flops per sector instead of 8 D^2 n (12x less on the 4x4
-// benchmark cluster).  Two kernels, both selected by DCAACC_TP_FACTORED_COL=1 (the dense tcgen05
-// GEMM stays the default, being faster on B200: see the tensor-core form below):
+// benchmark cluster).  Two kernels behind the tensor-core row step, both selected by DCAACC_TP_FACTORED_COL=1 (the
+// FP32 front-end, tp_frontend32.cu, is the default on these clusters and the faster one):
 //  - colFactorMmaKernel (4 x 4 clusters): stage A on the tensor cores, stage B as a 4 x 4 FFT;
 //  - colFactorKernel (any 16-site cluster, or DCAACC_TP_COL_FFT=0): both stages in FP32 on the
 //    CUDA cores of one CTA per (sector, 32 rows rho1, 16 frequencies w2):

@@ -1,5 +1,5 @@
 // Column step factored by orbital with the per-site sums in tensor memory (one band, 4 x 4
-// cluster, mixed path): tcgen05 form of tp_colfactor.cu's two stages,
+// cluster, mixed path, DCAACC_TP_FACTORED_COL=2): tcgen05 form of tp_colfactor.cu's two stages,
 //   Z(rho1, w2, r)  = sum_{j in site r} X'(rho1, j) conj T(w2, j)
 //   G(rho1; k2, w2) = -(1/Nc) G0_s(k2, w2) sum_r e^{-i k2 x_r} Z(rho1, w2, r) + beta G0_s delta,
 // (CachedNdft<GPU>::performFT, cached_ndft_gpu.hpp:193-252; SpaceTransform2DGpu::execute,

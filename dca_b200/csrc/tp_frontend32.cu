@@ -16,8 +16,8 @@
 // 4 D n^2 and 8 D^2 n flops three times over (split FP16) and three operand builders; grouped by
 // orbital they take 4 NwExt n^2 and 8 D NwExt n, nb Nc times fewer, which the FP32 pipe does in less
 // time.  Half G, per batch, operand builders included: 4x4, Nw = 64, n 50..400, 64 measurements 0.66 -> 0.48 ms
-// (column step 0.35, row step 0.086, sort of M 0.032); 6x6, Nw = 32, n 300..1000, 128 measurements 8.7 ->
-// 4.0 ms (2.36, 1.22, 0.43).  The G4 of a 4x4 batch is off by 2.8e-7 of the 64-bit sums instead of 5.9e-7.
+// (column step 0.35, row step 0.086, sort of M 0.032); 6x6, Nw = 32, n 300..1000, 128 measurements 8.4 (whole
+// G) -> 2.3 ms (1.19, 0.64, 0.43).  The G4 of a 4x4 batch is off by 2.8e-7 of the 64-bit sums instead of 5.9e-7.
 //
 // CTA = 32 rows of G (row step: 32 columns of M) x WT frequencies, eight or sixteen warps.
 // Phase 1: the warps take the orbitals from a counter.  A warp holds the whole 32 x WT tile, 4 x WT/4
@@ -30,7 +30,7 @@
 // Phase 2: the cluster transform of the sums in shared memory.  On an L x L cluster (L = 4, 6) an
 // FFT, one (row, frequency) pair a thread, in place; the result leaves row by row (the sums of an
 // orbital are padded by one, so that lanes along k and lanes along rows both read distinct banks).
-// Otherwise the matrix of phases, 4 x 2 sums a lane (all-SIMT runs only).  The 4x4 column step keeps the
+// Otherwise the matrix of phases, 4 x 2 sums a lane.  The 4x4 column step keeps the
 // FP32 pipe busy for a third of its time and shared memory for 60 %; two CTAs per SM (128 registers a
 // thread) leave four warps per scheduler to hide both.
 #include <cuda_runtime.h>

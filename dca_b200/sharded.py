@@ -10,8 +10,8 @@ created with that sub-list, bit for bit the full G4's entries with those transfe
 entry mixes transfers.  What crosses between ranks is each measurement's walker output (M and the
 vertex configuration, n x n real numbers per spin) rather than its G (D x D complex numbers per
 spin): every rank recomputes the G of every measurement, which on a B200 takes less time than
-moving G over NVLink would (c3: about 11 us of front-end kernels per measurement against 16.8 MB
-of FP32 G; c5: 0.34 ms against 340 MB).  Sharding trades that replicated front-end work for G4
+moving G over NVLink would (c3: about 7.5 us of front-end kernels per measurement against 16.8 MB
+of FP32 G).  Sharding trades that replicated front-end work for G4
 memory: each GPU holds 1/n_ranks of G4 and of its FP64 read-modify-write traffic.  For the
 benchmark configurations, whose G4 fits on one GPU, independent replicas (replicas.py) are faster.
 

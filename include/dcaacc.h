@@ -54,8 +54,8 @@ enum {
 enum {
   /* FP64 everywhere (the reference's double TP accumulation, mc_options.hpp.in TPAccumulationPrecision). */
   DCAACC_PRECISION_FP64 = 0,
-  /* Mixed: the NDFT and cluster transform on the tensor cores in split-BF16 with FP32 accumulation,
-   * G in FP32, per-batch G4 partial sums in FP32, running G4 in FP64. */
+  /* Mixed: the NDFT and cluster transform in FP32 (one band) or on the tensor cores in split FP16 with FP32
+   * accumulation, G in FP32, per-batch G4 partial sums in FP32, running G4 in FP64. */
   DCAACC_PRECISION_MIXED = 1
 };
 
