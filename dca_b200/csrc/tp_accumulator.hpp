@@ -122,7 +122,7 @@ public:
   void synchronize();
   size_t deviceFingerprint() const;
   int mirrorMode() const {
-    return mixed_ ? (dims_.half_g ? 1 : 0) | (dims_.half_g4 ? 2 : 0) : 0;
+    return (dims_.half_g ? 1 : 0) | (dims_.half_g4 ? 2 : 0);
   }
   uint64_t kernelLaunches() const {
     return launches_;

@@ -212,9 +212,10 @@ int dcaacc_tp_get_g4_normalized(const dcaacc_tp* acc, int32_t channel, double* o
  * allocation-free entry point's static scratch array. */
 size_t dcaacc_tp_static_device_fingerprint(void);
 
-/* Which mirror symmetries the mixed path uses (no reference counterpart; monitoring): bit 0, only
+/* Which mirror symmetries the handle uses (no reference counterpart; monitoring): bit 0, only
  * the upper frequency half of G is computed (real M and G0(-k,-w) = conj G0(k,w)); bit 1, only
- * the G4 tiles with w1 >= Nw/2 are accumulated and the rest is their conjugated mirror. */
+ * the G4 tiles with w1 >= Nw/2 are accumulated and the rest is their conjugated mirror.  FP64 handles
+ * use them where G0 is symmetric to a few ulps, mixed ones to 1e-12. */
 int32_t dcaacc_tp_mirror_mode(const dcaacc_tp* acc);
 
 /* Stage timers, the counterpart of the reference's Profiler scopes in the accumulator

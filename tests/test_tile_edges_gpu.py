@@ -131,19 +131,33 @@ def test_three_band_pairing(oracle_lib, cluster, k_ex, n_meas, max_batch):
     _compare(oracle_lib, _g0(rng, 3, cl, 7), _measurements(rng, 3, cl.nc, orders), params, MIXED_TOL)
 
 
-@pytest.mark.parametrize("cluster,w_ex,channels", [("2x1", [0, 2], [3]), ("3x2", [0], [2]), ("4x4", [-1, 1], [2, 3])])
-def test_fp64_half_g(monkeypatch, cluster, w_ex, channels):
-    """FP64, one transfer: G4 and G with half of G against all of it.  The two halves come from different
+def _symmetric(cl, g0):
+    """g0 with G0(-k, -w) = conj G0(k, w) to the bit."""
+    identity = [z for z in range(cl.nc) if np.array_equal(cl.k_add[z], np.arange(cl.nc))][0]
+    minus = cl.k_sub[:, identity]
+    return 0.5 * (g0 + np.conj(g0[::-1][:, minus]))
+
+
+@pytest.mark.parametrize("cluster,k_ex,w_ex,channels,mode", [
+    ("2x1", [1], [0, 2], [3], 1),      # frequency transfers not closed under negation: half of G alone
+    ("3x2", [5], [0], [2], 1),         # nor is this momentum transfer
+    ("3x2", [5, 3], [0], [2], 3),      # each the other's negative
+    ("4x4", [15], [-1, 1], [2, 3], 3),
+    ("3x2", [0, 1, 2, 3, 4, 5], [0], [3, 2], 2)])  # half of G4 alone: with this many transfers the update reads all of G
+def test_fp64_half_g(monkeypatch, cluster, k_ex, w_ex, channels, mode):
+    """FP64: G4 and G with half of G or G4 against all of it.  The two halves come from different
     terms' roundings of one sum: a few ulps of the largest entries."""
     from dca_b200.accumulators import TpAccumulator
     rng = np.random.default_rng(12)
     cl = CLUSTERS[cluster]
     orders = [(33, 7), (0, 18)]
-    params = _params(1, cl, 3, 9, channels, [cl.nc - 1], w_ex, orders)
+    params = _params(1, cl, 3, 9, channels, k_ex, w_ex, orders)
+    g0 = _symmetric(cl, _g0(rng, 1, cl, 9))
     measurements, got = _measurements(rng, 1, cl.nc, orders), []
     for full in ("0", "1"):
         monkeypatch.setenv("DCAACC_TP_FULL_G", full)
-        acc = TpAccumulator(_g0(rng, 1, cl, 9), params)
+        acc = TpAccumulator(g0, params)
+        assert acc.mirror_mode() == (0 if full == "1" else mode)
         acc.resetAccumulation(0)
         for m in measurements:
             acc.accumulate([s.M for s in m.sectors], list(m.sectors), m.sign)
@@ -152,6 +166,17 @@ def test_fp64_half_g(monkeypatch, cluster, w_ex, channels):
         got.append(gs + acc.get_G4())
     for a, b in zip(*got):
         assert rel_err(a, b) <= FP64_TOL
+
+
+def test_fp64_whole_g_when_not_symmetric():
+    """An asymmetry of G0 beyond rounding: the whole of G and G4."""
+    from dca_b200.accumulators import TpAccumulator
+    cl = CLUSTERS["4x4"]
+    g0 = _symmetric(cl, _g0(None, 1, cl, 9))
+    params = _params(1, cl, 3, 9, [2], [15], [0], [(1, 1)])
+    assert TpAccumulator(g0, params).mirror_mode() == 3
+    g0[9, 3, 0, 0, 0, 0] += 1e-14 * np.abs(g0).max()
+    assert TpAccumulator(g0, params).mirror_mode() == 0
 
 
 def test_fp64_graphs():
