@@ -616,6 +616,12 @@ rowTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, 
   }
 }
 
+// v + beta g, rounded once: beta and g are no FP32 numbers, and beta's rounding would be in every delta term alike.
+__device__ inline float2 addDelta(float2 v, double beta, double2 g) {
+  return make_float2(static_cast<float>(fma(beta, g.x, static_cast<double>(v.x))),
+                     static_cast<float>(fma(beta, g.y, static_cast<double>(v.y))));
+}
+
 // Column step.  grid (ceil(rows / 32), ceil(NwExt / WT), n_sectors), rows = D - row0.  gmax (or null):
 // [2 slot + spin] raised to the sector's largest |Re|, |Im| of G (float bits).
 template <int WT, int L, int NB>
@@ -702,7 +708,6 @@ colTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, 
 
   // Phase 2: cluster transform with conjugate phases, right G0, delta term.
   float2* out = G + g_sector_stride * (2 * sd.slot + sd.spin);
-  const float beta = static_cast<float>(dims.beta);
   float gabs = 0.f;
   auto note = [&](float2 v) { gabs = fmaxf(gabs, fmaxf(fabsf(v.x), fabsf(v.y))); };
   if constexpr (L > 0) {
@@ -721,7 +726,8 @@ colTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, 
           const double2 g = g0s[k1 + nc * w2];
           const uint32_t at = tile.lineAddr(wl, lane) + 8 * T::kSums * tile.slot_k[k1];
           const float2 z = floatsOf(lds64(at));
-          sts64(at, pairOf(fmaf(beta, static_cast<float>(g.x), z.x), fmaf(beta, static_cast<float>(g.y), z.y)));
+          const float2 v = addDelta(z, dims.beta, g);
+          sts64(at, pairOf(v.x, v.y));
         }
       }
       __syncwarp();
@@ -748,11 +754,8 @@ colTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, 
           return;
         const int row = row0 + t0 + l0 + 4 * i;
         const int w1 = row / R, r = row - w1 * R, k1 = r / nb;
-        if (w1 == w2 && k1 == k2) {
-          const float2 dl = to_f2(g0[(r - nb * k1) + nb * (b2 + nb * k2)]);
-          v.x = fmaf(beta, dl.x, v.x);
-          v.y = fmaf(beta, dl.y, v.y);
-        }
+        if (w1 == w2 && k1 == k2)
+          v = addDelta(v, dims.beta, g0[(r - nb * k1) + nb * (b2 + nb * k2)]);
         note(v);
         out[((static_cast<long>(w1) * nw_ext + w2) * R + r) * R + b2 + nb * k2] = v;
       };

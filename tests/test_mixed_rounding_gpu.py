@@ -43,3 +43,20 @@ def test_batch_sums_round_once_a_measurement(length, channels, transfers):
     err = rel_err(got.get_G4()[0], exact.get_G4()[0])
     print("error:", err)
     assert err <= 1.8e-7
+
+
+@pytest.mark.parametrize("cluster", [W.square_cluster(2), W.betts8_cluster(), W.square_cluster(4), W.square_cluster(6)])
+def test_delta_term_rounds_once(cluster):
+    """G = beta G0 delta (M = 0), with a beta whose rounding to FP32 is the largest there is, u: G rounded once
+    leaves 0.4 u (2 G's: 0.6 u) and their product as much again, 0.8 u = 5e-8; a rounded beta would add 2 u in every entry."""
+    beta = 4 * (1 + 2.0 ** -24)
+    rng = np.random.default_rng(4)
+    sectors = tuple(W.make_sector(rng, 1, 1, cluster.nc, beta) for _ in range(2))
+    for s in sectors:
+        s.M[:] = 0.
+    ms = [W.Measurement(1, sectors)]
+    exact = _run(cluster, 0, [W.PP_UP_DOWN], [0], ms, beta)
+    got = _run(cluster, 1, [W.PP_UP_DOWN], [0], ms, beta)
+    err = rel_err(got.get_G4()[0], exact.get_G4()[0])
+    print("error:", err)
+    assert err <= 8e-8
