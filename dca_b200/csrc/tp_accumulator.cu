@@ -484,21 +484,16 @@ bool TpAccumulator::mirrorTransfers(const std::vector<int>& kneg) {
   return true;
 }
 
-// An FP64 handle's G4 (and that of the FP64 handles sharing it) completed from its mirror; all of it is
-// accumulated from then on.
+// This handle's own half G4 (no other handle shares it) completed from its mirror; all of it is accumulated from
+// then on.
 void TpAccumulator::completeG4() {
-  if (mixed_ || !dims_.half_g4)
+  if (!dims_.half_g4)
     return;
-  std::lock_guard<std::mutex> lock(g4s_->m);
-  for (TpAccumulator* u : g4s_->users)
-    DCAACC_CUDA_CHECK(cudaStreamSynchronize(u->stream_));
   for (auto& g : g4())
     launchG4Mirror(g.get(), dims_, q_mirror_d_.get(), wq_mirror_d_.get(), stream_);
   DCAACC_CUDA_CHECK(cudaStreamSynchronize(stream_));
-  for (TpAccumulator* u : g4s_->users) {
-    u->dims_.half_g4 = 0;
-    u->releaseGraphs();  // the mode is a kernel argument
-  }
+  dims_.half_g4 = 0;
+  releaseGraphs();  // the mode is a kernel argument
 }
 
 TpAccumulator::~TpAccumulator() {
@@ -585,13 +580,15 @@ void TpAccumulator::shareG4(TpAccumulator& owner) {
     invalid("accumulators with different G4 shapes, transfers, channels or beta cannot share G4");
   if (owner.device_ != device_)
     invalid("sharing G4 requires both accumulators on the same device");
-  // FP64 handles give up the half G4 where the other handle has no equal one (mixed precision, G0 of less symmetry).
-  if (mixed_ != owner.mixed_ || owner.dims_.half_g4 != dims_.half_g4) {
-    completeG4();
-    owner.completeG4();
-  }
-  if (owner.dims_.half_g4 != dims_.half_g4)
+  // FP64 handles accumulate the whole of a G4 that they share: one whose inputs are less symmetric may join them later,
+  // and nothing can change their mode then, while they run on threads of their own.
+  const auto shared_half = [](const TpAccumulator& h) { return h.mixed_ ? h.dims_.half_g4 : 0; };
+  if (shared_half(owner) != shared_half(*this))
     invalid("accumulators with different G4 shapes, transfers, channels, beta or mirror modes cannot share G4");
+  if (!mixed_)
+    completeG4();
+  if (!owner.mixed_)
+    owner.completeG4();
   process();
   owner.process();
   if (finalized_)

@@ -122,8 +122,9 @@ int dcaacc_tp_reset(dcaacc_tp* acc);
  * (tp_accumulator_kernels.cu:677-680), zeroed once per DCA loop (callOncePerLoop,
  * tp_accumulator_gpu.hpp:271-296), and sumTo has nothing to add for it (:487-491).  Here each handle
  * owns its G4 unless share_g4 makes acc accumulate into owner's (same G4 shape, transfer lists,
- * channels, beta, mirror mode and device, else DCAACC_INVALID_ARG; what acc has accumulated so
- * far is added into owner's G4 and acc's own is released; both switch to atomic updates).
+ * channels, beta and device, and for a mixed handle that accumulates half of G4 another such one, else
+ * DCAACC_INVALID_ARG; what acc has accumulated so far is added into owner's G4 and acc's own is
+ * released; both switch to atomic updates, and FP64 handles to the whole of G4).
  * reset_loop is resetAccumulation(dca_loop): a shared G4 is zeroed only by the first handle that
  * resets for a given dca_loop, after the updates already launched on every sharing handle's
  * stream and before any later one (measurements a handle has queued but not launched, see flush,

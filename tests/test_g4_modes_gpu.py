@@ -1,0 +1,119 @@
+"""Handles that accumulate half of G4 (mirror symmetry) beside handles that accumulate all of it: sharing one G4,
+adding into each other, reads of the running and of the finalized G4.  Against the oracle, which always sums the
+whole, at the tolerances of the other GPU tests."""
+
+import numpy as np
+import pytest
+
+from helpers import rel_err
+from dca_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+FP64_TOL, MIXED_TOL = 1e-12, 1e-6
+CLUSTER = W.square_cluster(4)
+BETA, NW_HALF, N_SP, MAX_ORDER = 7.0, 4, 8, 40
+
+
+def _g0(symmetric=True):
+    """Symmetric to the bit (all hoppings real), or with a G0(k, w) of no symmetry at all."""
+    g = W.make_g0(W.Model("single", tp=-0.1), CLUSTER, BETA, 0.3, N_SP)
+    if not symmetric:
+        rng = np.random.default_rng(2)
+        g = g * (1 + 0.2 * rng.normal(size=g.shape) + 0.2j * rng.normal(size=g.shape))
+    return g
+
+
+def _params(precision=0, k_ex=range(16), channels=(W.PH_MAGNETIC, W.PH_CHARGE), max_batch=None):
+    from dca_b200.accumulators import TpParameters
+    return TpParameters(1, 16, NW_HALF, N_SP, BETA, list(channels), list(k_ex), [0], CLUSTER.r_vecs, CLUSTER.k_vecs,
+                        np.zeros((1, 2)), CLUSTER.k_add, CLUSTER.k_sub, CLUSTER.r_sub, max_order=MAX_ORDER,
+                        precision=precision, max_batch=max_batch or (2 if precision else 1))
+
+
+def _measurements(count, seed):
+    rng = np.random.default_rng(seed)
+    return [W.Measurement(-1 if i % 3 == 2 else 1,
+                          tuple(W.make_sector(rng, int(n), 1, 16, BETA) for n in rng.integers(5, MAX_ORDER, 2)))
+            for i in range(count)]
+
+
+def _feed(acc, measurements):
+    for m in measurements:
+        acc.accumulate([s.M for s in m.sectors], list(m.sectors), m.sign)
+
+
+class _Fed:
+    """A handle and the oracle of everything that it has been fed."""
+
+    def __init__(self, oracle_lib, symmetric=True, **kw):
+        from dca_b200.accumulators import TpAccumulator
+        self.acc = TpAccumulator(_g0(symmetric), _params(**kw))
+        self.acc.resetAccumulation(0)
+        self.ora = oracle_lib.OracleTp(_g0(symmetric), _params(**kw))
+
+    def feed(self, count, seed):
+        for a in (self.acc, self.ora):
+            _feed(a, _measurements(count, seed))
+        return self
+
+    def want(self):
+        return [np.array(g) for g in self.ora.get_G4()]
+
+
+def _total(*fed):
+    return [sum(gs) for gs in zip(*(f.want() for f in fed))]
+
+
+def _check(acc, want, tol):
+    acc.finalize()
+    for got, ref in zip(acc.get_G4(), want):
+        assert rel_err(got, ref) <= tol
+
+
+def _tol(*kinds):
+    return MIXED_TOL if any(k.get("precision") for k in kinds) else FP64_TOL
+
+
+HALF, FULL = dict(), dict(symmetric=False)                            # FP64
+MIXED_HALF, MIXED_FULL = dict(precision=1), dict(precision=1, symmetric=False)
+
+
+def test_modes(oracle_lib):
+    """The four kinds of handle that the tests below combine."""
+    for kind, mode in ((HALF, 2), (FULL, 0), (MIXED_HALF, 3), (MIXED_FULL, 0)):
+        assert _Fed(oracle_lib, **kind).acc.mirror_mode() == mode
+
+
+@pytest.mark.parametrize("first,second", [(HALF, HALF), (HALF, FULL), (FULL, HALF), (HALF, MIXED_FULL), (MIXED_FULL, HALF),
+                                          (MIXED_HALF, MIXED_HALF)])
+def test_shared_g4_of_two_kinds(oracle_lib, first, second):
+    """Measurements before and after the two share a G4, and a third handle that joins later: the others' modes
+    stay as they are, and every contribution arrives."""
+    a, b = _Fed(oracle_lib, **first).feed(2, 1), _Fed(oracle_lib, **second).feed(2, 2)
+    b.acc.share_G4_with(a.acc)
+    modes = a.acc.mirror_mode(), b.acc.mirror_mode()
+    a.feed(2, 3)
+    b.feed(1, 4)
+    joiner = first if first is MIXED_HALF else FULL
+    c = _Fed(oracle_lib, **joiner).feed(1, 5)
+    c.acc.share_G4_with(a.acc)
+    assert (a.acc.mirror_mode(), b.acc.mirror_mode()) == modes
+    for fed, seed in ((a, 6), (b, 7), (c, 8)):
+        fed.feed(2, seed)
+    b.acc.sumTo(a.acc)
+    c.acc.sumTo(a.acc)
+    _check(a.acc, _total(a, b, c), _tol(first, second))
+
+
+@pytest.mark.parametrize("owner,joiner", [(HALF, MIXED_HALF), (MIXED_HALF, HALF), (FULL, MIXED_HALF)])
+def test_refused_share_changes_nothing(oracle_lib, owner, joiner):
+    """A mixed handle with half of G4 shares with handles of its own kind alone."""
+    from dca_b200.accumulators import LogicError
+    a, b = _Fed(oracle_lib, **owner).feed(2, 1), _Fed(oracle_lib, **joiner).feed(2, 2)
+    modes = a.acc.mirror_mode(), b.acc.mirror_mode()
+    with pytest.raises(LogicError):
+        b.acc.share_G4_with(a.acc)
+    assert (a.acc.mirror_mode(), b.acc.mirror_mode()) == modes
+    for fed, kind in ((a, owner), (b, joiner)):
+        _check(fed.feed(1, 3).acc, fed.want(), _tol(kind))
