@@ -236,6 +236,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
           mirror_exact = mirror_exact && std::hypot(a.x - b.x, a.y + b.y) <= 4e-15;
         }
   }
+  mirror_ok_ = mirror_ok;
   fft64_ = clusterFft4(nb, nc, c.r_vecs, c.k_vecs);
   auto upload_ints = [](DevBuf<int>& d, const std::vector<int>& h) {
     d.alloc(h.size());
@@ -1108,6 +1109,14 @@ void TpAccumulator::sumTo(TpAccumulator& other) {
     invalid("sumTo between accumulators of different G4 shapes, transfers, channels or beta");
   if (other.device_ != device_)
     invalid("sumTo requires both accumulators on the same device");
+  // A half-G4 target refills its lower half from its upper one when it is read.  What a full source adds obeys that
+  // mirror only if its G0 does (and in FP64 the two halves also differ in their last bits): else the target's G4 is
+  // completed first, and all of it accumulated from then on.
+  if (other.g4s_ != g4s_ && other.dims_.half_g4 && !dims_.half_g4 && !(other.mixed_ && mirror_ok_)) {
+    if (other.g4Shared())
+      invalid("sumTo of an accumulator without mirror symmetry into a G4 that several handles accumulate by halves");
+    other.completeG4();
+  }
   process();
   other.process();
   if (finalized_)
@@ -1132,8 +1141,7 @@ void TpAccumulator::sumTo(TpAccumulator& other) {
   DCAACC_CUDA_CHECK(cudaStreamWaitEvent(stream_, ev, 0));
   for (size_t c = 0; c < g4().size(); ++c) {
     // A half-G4 source holds only the tiles with w1 >= Nw / 2; a full-G4 target needs the rest
-    // too, so the source's lower half is filled from its mirror first.  (A full source adding into
-    // a half target is complete already: the target refills its lower half from its upper half.)
+    // too, so the source's lower half is filled from its mirror first.
     if (dims_.half_g4 && !other.dims_.half_g4) {
       launchG4Mirror(g4()[c].get(), dims_, q_mirror_d_.get(), wq_mirror_d_.get(), stream_);
       ++launches_;

@@ -163,6 +163,7 @@ private:
   int n_sp_ = 0;
   std::vector<int> k_add_, k_sub_, q_list_, wex_list_;
   bool grid6_ = false;  // G4Args::grid6
+  bool mirror_ok_ = false;  // G0 and the phases are mirror-symmetric to 1e-12
   bool allTransfers() const;  // q_list_ is a permutation of the cluster momenta
   size_t g4_size_ = 0;
   long g_sector_stride_ = 0;  // complex elements of one (slot, spin) G

@@ -176,8 +176,10 @@ size_t dcaacc_tp_g4_size(const dcaacc_tp* acc);
 /* sumTo(other) — the CPU accumulator adds its G4 into other's and clears its own
  * (tp_accumulator_cpu.hpp:896-904).  Here: other.G4 += this.G4 on the device, this.G4 = 0.  Both
  * handles must accumulate the same G4 (sizes, transfer lists, channels, beta), else
- * DCAACC_INVALID_ARG; their precisions and mirror modes may differ (a half-G4 source is completed
- * from its mirror before it is added into a full-G4 target). */
+ * DCAACC_INVALID_ARG; their precisions and mirror modes may differ.  A half-G4 source is completed from
+ * its mirror before it is added into a full-G4 target.  Under a full source, a half-G4 target is
+ * completed, and accumulates the whole of G4 from then on, when it is an FP64 one or the source is
+ * not mirror-symmetric (DCAACC_INVALID_ARG if mixed handles share that target). */
 int dcaacc_tp_sum_to(dcaacc_tp* acc, dcaacc_tp* other);
 
 /* Debug / parity: copies the last measurement's G for one spin (complex, layout

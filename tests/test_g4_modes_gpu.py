@@ -117,3 +117,34 @@ def test_refused_share_changes_nothing(oracle_lib, owner, joiner):
     assert (a.acc.mirror_mode(), b.acc.mirror_mode()) == modes
     for fed, kind in ((a, owner), (b, joiner)):
         _check(fed.feed(1, 3).acc, fed.want(), _tol(kind))
+
+
+@pytest.mark.parametrize("source,target", [(FULL, HALF), (HALF, FULL), (HALF, HALF), (MIXED_FULL, HALF), (MIXED_HALF, HALF),
+                                           (FULL, MIXED_HALF), (MIXED_FULL, MIXED_HALF), (HALF, MIXED_HALF)])
+def test_sum_to_between_kinds(oracle_lib, source, target):
+    """The target's G4 is the sum of both, whatever half of it either has accumulated, also after further
+    measurements; and so is what a read of the running G4 gives."""
+    a, b = _Fed(oracle_lib, **source).feed(3, 1), _Fed(oracle_lib, **target).feed(2, 2)
+    a.acc.sumTo(b.acc)
+    tol = _tol(source, target)
+    size = b.want()[0].size
+    for c, ref in enumerate(_total(a, b)):
+        assert rel_err(b.acc.peek_G4(c, 0, size), ref) <= tol
+    b.feed(3, 3)
+    _check(b.acc, _total(a, b), tol)
+    a.acc.finalize()
+    assert not any(np.any(g) for g in a.acc.get_G4())
+
+
+def test_sum_to_shared_half_g4(oracle_lib):
+    """Into a G4 that mixed handles accumulate by halves: only what has the mirror symmetry."""
+    from dca_b200.accumulators import LogicError
+    a, b = _Fed(oracle_lib, **MIXED_HALF).feed(2, 1), _Fed(oracle_lib, **MIXED_HALF).feed(2, 2)
+    b.acc.share_G4_with(a.acc)
+    c, d = _Fed(oracle_lib, **FULL).feed(2, 3), _Fed(oracle_lib, **HALF).feed(2, 4)
+    with pytest.raises(LogicError):
+        c.acc.sumTo(a.acc)
+    d.acc.sumTo(a.acc)
+    b.acc.sumTo(a.acc)
+    _check(a.acc, _total(a, b, d), MIXED_TOL)
+    _check(c.acc, c.want(), FP64_TOL)
