@@ -319,13 +319,10 @@ struct SpAccumulator::Impl {
   DevBuf<int> r_sub_d;
   DevBuf<double2> out_d, roots;
   // A measurement's vertices, packed (tau, row orbitals, column orbitals) so that one copy uploads
-  // them.  The pinned sets are a ring, so that the host fills the next ones while copies wait behind
-  // earlier kernels; the device set is reused in stream order.
-  static constexpr int kSets = 4;
-  PinBuf<double> vtx_h[kSets];
+  // them; the device set is reused in stream order.
+  PinBuf<double> vtx_h;
   DevBuf<double> vtx_d;
-  cudaEvent_t uploaded[kSets] = {};
-  int set = 0;
+  cudaEvent_t uploaded = nullptr;  // the last measurement's inputs, host M included, have been copied
   std::vector<double2> mrw, mrw_sqr;
   bool ready = false, finalized = false;
   uint64_t launches = 0;
@@ -399,8 +396,7 @@ SpAccumulator::SpAccumulator(const dcaacc_sp_config& c) : d_(new Impl) {
   DCAACC_CUDA_CHECK(cudaDeviceGetAttribute(&d.n_sm, cudaDevAttrMultiProcessorCount, d.device));
   DCAACC_CUDA_CHECK(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking));
   d.own_stream = true;
-  for (auto& e : d.uploaded)
-    DCAACC_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  DCAACC_CUDA_CHECK(cudaEventCreateWithFlags(&d.uploaded, cudaEventDisableTiming));
   d.coeff.alloc(cf.size());
   DCAACC_CUDA_CHECK(cudaMemcpy(d.coeff.get(), cf.data(), d.coeff.bytes(), cudaMemcpyHostToDevice));
   d.inv_phi.alloc(ip.size());
@@ -424,10 +420,8 @@ SpAccumulator::SpAccumulator(const dcaacc_sp_config& c) : d_(new Impl) {
   d.M_d.alloc(2 * size_t(d.max_order) * d.max_order);
   d.out_d.alloc(size_t(2 * nb) * (2 * nb) * nc * 2 * d.n_sp);
   d.vtx_d.alloc(2 * nv);  // per vertex one double and two ints
-  for (int i = 0; i < Impl::kSets; ++i) {
-    d.vtx_h[i].alloc(2 * nv);
-    DCAACC_CUDA_CHECK(cudaEventRecord(d.uploaded[i], d.stream));
-  }
+  d.vtx_h.alloc(2 * nv);
+  DCAACC_CUDA_CHECK(cudaEventRecord(d.uploaded, d.stream));
   if (sizeof(double) * 2 * g.n_padded > 200 * 1024 || sizeof(double) * 3 * g.n > 200 * 1024)
     throw Error(DCAACC_INVALID_ARG, "n_sp_freq too large for the shared-memory NFFT rows");
 }
@@ -435,9 +429,8 @@ SpAccumulator::SpAccumulator(const dcaacc_sp_config& c) : d_(new Impl) {
 SpAccumulator::~SpAccumulator() {
   if (d_->stream)
     cudaStreamSynchronize(d_->stream);
-  for (auto& e : d_->uploaded)
-    if (e)
-      cudaEventDestroy(e);
+  if (d_->uploaded)
+    cudaEventDestroy(d_->uploaded);
   if (d_->own_stream && d_->stream)
     cudaStreamDestroy(d_->stream);
 }
@@ -462,6 +455,9 @@ void SpAccumulator::accumulate(const dcaacc_sector* sec, double factor) {
     throw Error(DCAACC_NOT_READY, "The accumulator is already finalized.");
   if (!sec)
     throw Error(DCAACC_INVALID_ARG, "null sectors");
+  // One measurement's uploads in flight: the inputs of a call may be reused once the next one has returned.  The
+  // uploads are behind the kernel of the measurement before theirs alone, so the GPU is not idle meanwhile.
+  DCAACC_CUDA_CHECK(cudaEventSynchronize(d.uploaded));
   for (int s = 0; s < 2; ++s) {
     const auto& x = sec[s];
     if (x.n < 0 || x.n > d.max_order)
@@ -483,10 +479,7 @@ void SpAccumulator::accumulate(const dcaacc_sector* sec, double factor) {
       DCAACC_CUDA_CHECK(cudaMemsetAsync(d.f_tau_single.get(), 0, d.f_tau_single.bytes(), d.stream));
     return;
   }
-  const int set = d.set;
-  d.set = (set + 1) % Impl::kSets;
-  DCAACC_CUDA_CHECK(cudaEventSynchronize(d.uploaded[set]));  // the set's earlier copy has been made
-  double* tau = d.vtx_h[set].get();
+  double* tau = d.vtx_h.get();
   int* orb_r = reinterpret_cast<int*>(tau + vtx);
   int* orb_c = orb_r + vtx;
   SpMeasurement m{};
@@ -520,7 +513,7 @@ void SpAccumulator::accumulate(const dcaacc_sector* sec, double factor) {
   }
   DCAACC_CUDA_CHECK(cudaMemcpyAsync(d.vtx_d.get(), tau, (sizeof(double) + 2 * sizeof(int)) * vtx,
                                     cudaMemcpyHostToDevice, d.stream));
-  DCAACC_CUDA_CHECK(cudaEventRecord(d.uploaded[set], d.stream));
+  DCAACC_CUDA_CHECK(cudaEventRecord(d.uploaded, d.stream));
   // With stamping the measurement goes to its own f(tau) first, which is then added to the sum.
   double* target = d.f_tau.get();
   if (d.stamping) {

@@ -356,7 +356,8 @@ void dcaacc_sp_destroy(dcaacc_sp* acc);
 /* resetAccumulation() — sp_accumulator_gpu.hpp:146-158. */
 int dcaacc_sp_reset(dcaacc_sp* acc);
 
-/* accumulate(Ms, configs, factor) — sp_accumulator_gpu.hpp:160-195.  sectors: [2]. */
+/* accumulate(Ms, configs, factor) — sp_accumulator_gpu.hpp:160-195.  sectors: [2].  A host M may be reused
+ * once the next accumulate or synchronize has returned, a device M once synchronize has. */
 int dcaacc_sp_accumulate(dcaacc_sp* acc, const dcaacc_sector* sectors, double sign);
 
 /* finalize() — sp_accumulator_gpu.hpp:215-229, with the fold / DFT / window division of

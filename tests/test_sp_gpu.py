@@ -99,3 +99,39 @@ def test_sp_errors():
         acc.get_sign_times_M_r_w_sqr()
     with pytest.raises(LogicError):  # already finalized
         acc.accumulate([s.M for s in m.sectors], list(m.sectors), 1.0)
+
+
+def test_sp_host_inputs_after_the_next_call():
+    """A call's host M and vertices belong to the caller again when the next call has returned, also while the
+    handle's stream is behind (a wait of some 20 ms in it before the first upload; M pinned, so that nothing
+    stages it)."""
+    import ctypes
+
+    import torch
+
+    from dca_b200 import _native as N
+    from dca_b200.accumulators import SpAccumulator
+    case = case_from_workload(W.WORKLOADS["c1"], 4)
+    want = run_sp(case, sqr=False).get_sign_times_M_r_w()
+    acc = SpAccumulator(case.sp_params())
+    stream = torch.cuda.Stream()
+    assert N.lib.dcaacc_sp_set_stream(acc._h, ctypes.c_void_p(stream.cuda_stream)) == 0
+    acc.resetAccumulation()
+    pinned = [[torch.empty(s.n, s.n, dtype=torch.float64, pin_memory=True).numpy().T for s in m.sectors]
+              for m in case.measurements]
+    for i, m in enumerate(case.measurements):
+        for buf, s in zip(pinned[i], m.sectors):
+            buf[...] = s.M
+        if i == 0:
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(40_000_000)
+        acc.accumulate(pinned[i], list(m.sectors), m.sign)
+        if i:
+            for buf in pinned[i - 1]:
+                buf[...] = np.nan
+    acc.finalize()
+    assert np.array_equal(np.isnan(acc.get_sign_times_M_r_w()), np.zeros(want.shape, bool))
+    assert rel_err(acc.get_sign_times_M_r_w(), want) <= 1e-13
+    acc.synchronizeCopy()
+    torch.cuda.synchronize()
+    del acc  # before its stream
