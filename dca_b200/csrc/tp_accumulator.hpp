@@ -257,6 +257,9 @@ private:
   DevBuf<unsigned> tile_order_d_;
   DevBuf<double2> peek_d_;
   static constexpr size_t kPeekWindow = size_t(1) << 16;  // entries allocated with a half-G4 handle
+  // Half G4, unshared: what reads have filled from the mirror in place, per channel, since the last update.
+  enum Mirrored : unsigned char { kMirroredNone, kMirroredPart, kMirroredAll };
+  std::vector<unsigned char> mirrored_;
   // Pinned staging of the batch being assembled, double-buffered: the host fills one set while the
   // uploads from the other (queued behind the previous batch's kernels) are still pending.
   struct HostStage {

@@ -1055,12 +1055,12 @@ __device__ inline bool g4Mirror(const TpDims& d, const int* q_mirror, const int*
 }
 
 __global__ void g4MirrorKernel(double2* __restrict__ G4, const TpDims d, const int* __restrict__ q_mirror,
-                               const int* __restrict__ wq_mirror, size_t n) {
-  for (size_t e = blockIdx.x * size_t(blockDim.x) + threadIdx.x; e < n; e += size_t(gridDim.x) * blockDim.x) {
+                               const int* __restrict__ wq_mirror, size_t offset, size_t count) {
+  for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < count; i += size_t(gridDim.x) * blockDim.x) {
     size_t m;
-    if (g4Mirror(d, q_mirror, wq_mirror, e, m)) {
+    if (g4Mirror(d, q_mirror, wq_mirror, offset + i, m)) {
       const double2 v = G4[m];
-      G4[e] = make_double2(v.x, -v.y);
+      G4[offset + i] = make_double2(v.x, -v.y);
     }
   }
 }
@@ -1080,16 +1080,14 @@ __global__ void g4WindowKernel(const double2* __restrict__ G4, const TpDims d, c
   }
 }
 
-size_t g4Entries(const TpDims& d) {
-  return size_t(d.nb) * d.nb * d.nb * d.nb * d.nc * d.nc * d.nw * d.nw * d.nq * d.nwq;
-}
-
 }  // namespace
 
-void launchG4Mirror(double2* G4, const TpDims& d, const int* q_mirror, const int* wq_mirror, cudaStream_t stream) {
-  const size_t n = g4Entries(d);
-  const int blocks = static_cast<int>(std::min<size_t>((n + 255) / 256, 148 * 16));
-  g4MirrorKernel<<<blocks, 256, 0, stream>>>(G4, d, q_mirror, wq_mirror, n);
+void launchG4Mirror(double2* G4, const TpDims& d, const int* q_mirror, const int* wq_mirror, size_t offset, size_t count,
+                    cudaStream_t stream) {
+  if (!count)
+    return;
+  const int blocks = static_cast<int>(std::min<size_t>((count + 255) / 256, 148 * 16));
+  g4MirrorKernel<<<blocks, 256, 0, stream>>>(G4, d, q_mirror, wq_mirror, offset, count);
   DCAACC_LAUNCH_CHECK();
 }
 

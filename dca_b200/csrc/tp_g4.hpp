@@ -91,9 +91,10 @@ void launchDirectTc(const G4Args& a, const float2* G, long g_sector_stride, cons
 bool directTc36Applies(const G4Args& a);
 void launchDirectTc36(const G4Args& a, const float2* G, long g_sector_stride, const float2* disc, cudaStream_t stream);
 
-// half_g4: G4 entries with w1 < Nw / 2 := conj of their mirror (-k1 w1', -k2 w2', -q, -wq);
+// half_g4: G4 entries with w1 < Nw / 2 among count from offset on := conj of their mirror (-k1 w1', -k2 w2', -q, -wq);
 // q_mirror[iq] / wq_mirror[iwq] are the positions of -q / -wq in the transfer lists.
-void launchG4Mirror(double2* G4, const TpDims& d, const int* q_mirror, const int* wq_mirror, cudaStream_t stream);
+void launchG4Mirror(double2* G4, const TpDims& d, const int* q_mirror, const int* wq_mirror, size_t offset, size_t count,
+                    cudaStream_t stream);
 // Entries [offset, offset + count) of G4 with the mirror applied (half_g4) into out (device).
 void launchG4Window(const double2* G4, const TpDims& d, const int* q_mirror, const int* wq_mirror, size_t offset,
                     size_t count, double2* out, cudaStream_t stream);

@@ -148,3 +148,36 @@ def test_sum_to_shared_half_g4(oracle_lib):
     b.acc.sumTo(a.acc)
     _check(a.acc, _total(a, b, d), MIXED_TOL)
     _check(c.acc, c.want(), FP64_TOL)
+
+
+@pytest.mark.parametrize("kind", [HALF, MIXED_HALF])
+@pytest.mark.parametrize("shared", [False, True])
+def test_reads_of_a_running_half_g4(oracle_lib, kind, shared):
+    """Windows below and above the one that a handle keeps (65,536 entries), at both ends and between, in one
+    private or shared G4 that goes on accumulating; reads that follow one another; and the finalized G4 after them."""
+    a = _Fed(oracle_lib, **kind)
+    if shared:
+        b = _Fed(oracle_lib, **kind)
+        b.acc.share_G4_with(a.acc)
+    size = a.want()[0].size
+    for seed, (offset, count) in enumerate([(5, 100), (7, 65536), (3, 65537), (size - 70000, 70000), (1, size - 1),
+                                            (0, size), (size, 0)]):
+        a.feed(1, seed)
+        for channel in (1, 0):
+            got = a.acc.peek_G4(channel, offset, count)
+            assert got.size == count and rel_err(got, a.want()[channel][offset:offset + count]) <= _tol(kind)
+    # Several reads without an update between them, then another handle's sum, then an update.
+    c = _Fed(oracle_lib, **kind).feed(1, 20)
+    fed = [a]
+    for step in range(3):
+        if step == 1:
+            c.acc.sumTo(a.acc)
+            fed.append(c)
+        if step == 2:
+            a.feed(1, 21)
+        want = _total(*fed)[1]
+        for offset, count in [(0, 70000), (70000, 70000), (100, 50), (140000, size - 140000), (30, 90000)]:
+            assert rel_err(a.acc.peek_G4(1, offset, count), want[offset:offset + count]) <= _tol(kind)
+    _check(a.acc, _total(*fed), _tol(kind))
+    a.acc.resetAccumulation(1)
+    assert not np.any(a.acc.peek_G4(1, 0, size))
