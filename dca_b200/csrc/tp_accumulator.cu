@@ -237,7 +237,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
         }
   }
   mirror_ok_ = mirror_ok;
-  fft64_ = clusterFft4(nb, nc, c.r_vecs, c.k_vecs);
+  axes_ = clusterAxes4(nb, nc, c.r_vecs, c.k_vecs);
   auto upload_ints = [](DevBuf<int>& d, const std::vector<int>& h) {
     d.alloc(h.size());
     DCAACC_CUDA_CHECK(cudaMemcpy(d.get(), h.data(), d.bytes(), cudaMemcpyHostToDevice));
@@ -847,7 +847,7 @@ void TpAccumulator::process() {
   fa.Fb = Fb_.get();
   fa.G0 = G0_.get();
   fa.tuner = &tuner_;
-  fa.fft = fft64_;
+  fa.axes = axes_;
   // The launch shapes take the order bound in steps of 128; every kernel reads each sector's own order,
   // so the results do not depend on it, and batches of similar orders share one captured graph.
   if (n_max_batch_ > 0)

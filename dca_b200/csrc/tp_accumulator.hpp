@@ -241,7 +241,7 @@ private:
   bool have_disc_ = false;
   // Mixed mode: the FP32 front-end's twiddles and sorted M, or the tensor-core front-end's operand
   // planes and TMA descriptors (with the orbital of each vertex in row / column order).
-  ColFft fft64_{};  // FP64 front-end: the cluster transform as an FFT, where it is one
+  AxisTransform axes_{};  // FP64 front-end: the cluster transform axis by axis, where it is one
   bool front32_ = false, tc_front_ = false, simt_only_ = false;
   DevBuf<float2> T2_d_;
   DevBuf<float4> T4_d_;

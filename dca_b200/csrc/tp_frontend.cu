@@ -23,14 +23,15 @@
 // whole 16 x WT tile, 2 x WT/4 sums a lane, and streams its orbital's vertices through a ring of
 // its own in shared memory, one asynchronous 16-byte copy per lane and vertex; per vertex a lane
 // reads 2 + WT/4 elements for 2 WT/4 complex multiply-adds.  Phase 2: 4 x 2 sums a lane over the
-// sites, or on a 4 x 4 cluster an FFT (a fifth of the matrix's FP64 operations, which were more than
-// phase 1's), one (row, frequency) pair a thread.  Both phases are bound by the FP64 pipe.  The earlier kernels gave a thread one sum, that
+// sites, or on a 4 x 4 grid axis by axis (AxisTransform: 384 multiply-adds instead of 1,024, which were more than
+// phase 1's), one (row, frequency) pair a thread.  Bound by the FP64 pipe and by latencies: a measurement is one
+// partial wave of CTAs, four times as long as its FP64 operations.  The earlier kernels gave a thread one sum, that
 // is two shared-memory reads per multiply-add, and a whole CTA one orbital at a time.  One measurement, 4x4,
-// Nw = 64, n 100..300: row step 42 -> 17 us, 14 with the FFT; column step 151 -> 41, 28 with the FFT.  The FFT's
-// phases are exact; those of momenta rounded to 2 pi m / 4 +- 2e-15 are off by 3e-15, and so is a G from them.
+// Nw = 64, n 100..300: row step 42 -> 17 us, 14.5 axis by axis; column step 151 -> 41, 29 axis by axis.  An FFT (14 and
+// 27.5 us) would take momenta such as 2 pi m / 4 + 8 ulps for exact quarters: G off by 2e-15 instead of 8e-16.
 //
 // Half G (dims.half_g; mirror-symmetric inputs, a G4 kernel that reads mirrored blocks): the rows with
-// w1 >= NwExt / 2 alone, in both steps: 28 -> 16 and 14 -> 13 us.
+// w1 >= NwExt / 2 alone, in both steps: 29 -> 17 and 14.5 -> 13 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -91,15 +92,22 @@ __device__ inline void cpAsyncWait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// X[m] = sum_x e^{SIGN i pi m x / 2} z[x], in place.
-template <int SIGN>
-__device__ inline void dft4(double2& z0, double2& z1, double2& z2, double2& z3) {
-  const double2 t0 = cadd(z0, z2), t1 = csub(z0, z2), t2 = cadd(z1, z3), d = csub(z1, z3);
-  const double2 t3 = SIGN < 0 ? mk(d.y, -d.x) : mk(-d.y, d.x);
-  z0 = cadd(t0, t2);
-  z2 = csub(t0, t2);
-  z1 = cadd(t1, t3);
-  z3 = csub(t1, t3);
+// z[m] := sum_a p[m][a] z[a] (SIGN < 0: with conjugated phases), the four z S apart; p[m][0] = 1.
+template <int SIGN, int S>
+__device__ inline void axisSums(double2* z, const double2 (&p)[4][4]) {
+  const double2 in[4] = {z[0], z[S], z[2 * S], z[3 * S]};
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    double2 s = in[0];
+#pragma unroll
+    for (int a = 1; a < 4; ++a) {
+      if (SIGN < 0)
+        cfmac(s, in[a], p[m][a]);
+      else
+        cfma(s, in[a], p[m][a]);
+    }
+    z[m * S] = s;
+  }
 }
 
 // Shared memory of a tile kernel: the orbitals' sums Z[o][w][16], the warps' rings (16 bytes per
@@ -108,7 +116,7 @@ __device__ inline void dft4(double2& z0, double2& z1, double2& z2, double2& z3) 
 template <int WT, int L>
 struct Tile {
   static constexpr int kPairs = kTileR * WT;
-  static constexpr int kSums = kPairs + (L ? 1 : 0);  // stride of an orbital's sums (FFT: lanes along k, distinct banks)
+  static constexpr int kSums = kPairs + (L ? 1 : 0);  // stride of an orbital's sums (L: lanes along k, distinct banks)
   static constexpr int kThreads = kPairs;
   static constexpr int kWarps = kThreads / 32;
   static_assert(kTileR + WT <= 32, "one copy per lane and vertex");
@@ -127,10 +135,10 @@ struct Tile {
     return size_t(kWarps) * kRing * 512 + sizeof(double2) * (size_t(d.n_orb) * kSums + factors(d)) +
            sizeof(int) * (d.n_orb + 2);
   }
-  // Lays the memory out and fills the phases (FFT: factor(w, k), in slot order), the starts and the counter.
+  // Lays the memory out and fills the phases (L: factor(w, k), in slot order), the starts and the counter.
   template <typename Factor>
   __device__ Tile(unsigned char* raw, const TpDims& d, const double2* __restrict__ Fb,
-                  const int* __restrict__ orb_start, const ColFft& fft, Factor factor) {
+                  const int* __restrict__ orb_start, const AxisTransform& axes, Factor factor) {
     ring = raw;
     Z = reinterpret_cast<double2*>(raw + kWarps * kRing * 512);
     F = Z + d.n_orb * kSums;
@@ -138,7 +146,7 @@ struct Tile {
     next = start + d.n_orb + 1;
     if constexpr (L > 0) {
       for (int i = threadIdx.x; i < WT * L * L; i += kThreads)
-        F[i] = factor(i / (L * L), static_cast<int>(fft.kmap[i % (L * L)]));
+        F[i] = factor(i / (L * L), static_cast<int>(axes.kmap[i % (L * L)]));
     }
     else {
       const int kp = kPad(d);
@@ -224,26 +232,26 @@ struct Tile {
     }
   }
 
-  // FFT form of phase 2 (L = 4), for the 32 pairs of this warp from line wl on (two lines): the sums of site
+  // Phase 2 axis by axis (L = 4), for the 32 pairs of this warp from line wl on (two lines): the sums of site
   // (a, b) become factor times the transform e^{SIGN i k r}, element k in place of orbital k.
   template <int SIGN>
-  __device__ void fftLines(const ColFft& fft, int wl) const {
+  __device__ void axisLines(const AxisTransform& axes, int wl) const {
     const int lane = threadIdx.x % 32;
     double2* p = Z + wl * kTileR + lane;
     double2 z[16];
 #pragma unroll
     for (int g = 0; g < 16; ++g)
-      z[g] = p[fft.rmap[g] * kSums];
+      z[g] = p[axes.rmap[g] * kSums];
 #pragma unroll
     for (int b = 0; b < 4; ++b)
-      dft4<SIGN>(z[4 * b], z[4 * b + 1], z[4 * b + 2], z[4 * b + 3]);
+      axisSums<SIGN, 1>(z + 4 * b, axes.x);
 #pragma unroll
     for (int m = 0; m < 4; ++m)
-      dft4<SIGN>(z[m], z[m + 4], z[m + 8], z[m + 12]);
+      axisSums<SIGN, 4>(z + m, axes.y);
     const double2* f = F + (wl + lane / kTileR) * 16;
 #pragma unroll
     for (int g = 0; g < 16; ++g)
-      p[fft.kmap[g] * kSums] = cmul(f[g], z[g]);
+      p[axes.kmap[g] * kSums] = cmul(f[g], z[g]);
     __syncwarp();
   }
 };
@@ -261,7 +269,7 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const int* __restrict__ row_start, const double2* __restrict__ Tr,
                    const double2* __restrict__ Fb,  // (r, k, b): e^{i k (r + a_b)}
                    const double2* __restrict__ G0,  // (b1, b2, k, w, s)
-                   const __grid_constant__ ColFft fft, double2* __restrict__ Xp) {
+                   const __grid_constant__ AxisTransform axes, double2* __restrict__ Xp) {
   using T = Tile<WT, L>;
   const SectorDesc sd = sectors[blockIdx.z];
   // Half G: the frequencies from NwExt / 2 on.
@@ -272,8 +280,8 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
   const double norm = -1.0 / nc;
-  T tile(smem_raw, dims, Fb, row_start + sd.orb_off, fft, [&](int w, int k) {
-    const double2 g = cmul(g0s[k + nc * min(w0 + w, nw_ext - 1)], Fb[k * nc + fft.r0]);
+  T tile(smem_raw, dims, Fb, row_start + sd.orb_off, axes, [&](int w, int k) {
+    const double2 g = cmul(g0s[k + nc * min(w0 + w, nw_ext - 1)], Fb[k * nc + axes.r0]);
     return mk(norm * g.x, norm * g.y);
   });
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
@@ -337,7 +345,7 @@ rowTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   const long D = static_cast<long>(R) * nw_ext;
   if constexpr (L > 0) {
     for (int wl = 2 * warp; wl < WT; wl += 2 * T::kWarps) {
-      tile.template fftLines<1>(fft, wl);
+      tile.template axisLines<1>(axes, wl);
       const int k = lane % 16;
 #pragma unroll 4
       for (int i = 0; i < kTileR; ++i) {  // two elements of the line pair a step: j = j0 + (e % 16)
@@ -430,7 +438,7 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
                    const int* __restrict__ col_start, const double2* __restrict__ Tc,
                    const double2* __restrict__ Fb,
                    const double2* __restrict__ G0,  // (b1, b2, k, w, s)
-                   const __grid_constant__ ColFft fft, const double2* __restrict__ Xp, double2* __restrict__ G,
+                   const __grid_constant__ AxisTransform axes, const double2* __restrict__ Xp, double2* __restrict__ G,
                    long g_sector_stride) {
   using T = Tile<WT, L>;
   const SectorDesc sd = sectors[blockIdx.z];
@@ -438,8 +446,8 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   const int D = R * nw_ext, row0 = (dims.half_g ? D / 2 : 0) + blockIdx.x * kTileR, w0 = blockIdx.y * WT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const double2* g0s = G0 + static_cast<long>(sd.spin) * nw_ext * nc * nb * nb;
-  T tile(smem_raw, dims, Fb, col_start + sd.orb_off, fft,
-         [&](int w, int k) { return cmulc(g0s[k + nc * min(w0 + w, nw_ext - 1)], Fb[k * nc + fft.r0]); });
+  T tile(smem_raw, dims, Fb, col_start + sd.orb_off, axes,
+         [&](int w, int k) { return cmulc(g0s[k + nc * min(w0 + w, nw_ext - 1)], Fb[k * nc + axes.r0]); });
   const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
 
   // Phase 1: Z(o, w2, row) = sum of X'(row, j) conj T(w2, j) over the vertices j of orbital o.
@@ -488,7 +496,7 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
   double2* out = G + g_sector_stride * (2 * sd.slot + sd.spin);
   if constexpr (L > 0) {
     for (int wl = 2 * warp; wl < WT; wl += 2 * T::kWarps) {
-      tile.template fftLines<-1>(fft, wl);
+      tile.template axisLines<-1>(axes, wl);
       const int k = lane % 16;
 #pragma unroll 4
       for (int i = 0; i < kTileR; ++i) {
@@ -590,40 +598,49 @@ colTransformKernel(const TpDims dims, const SectorDesc* __restrict__ sectors,
 // ------------------------------------------------------------------------------------------------
 // Host launchers
 // ------------------------------------------------------------------------------------------------
-ColFft clusterFft4(int nb, int nc, const double* r_vecs, const double* k_vecs) {
-  ColFft f{};
+AxisTransform clusterAxes4(int nb, int nc, const double* r_vecs, const double* k_vecs) {
+  AxisTransform t{};
   if (nb != 1 || nc != 16)
-    return f;
-  constexpr double tol = 4e-15;  // rounding of 2 pi m / 4 alone: the phases are the FFT's to FP64
-  int site[16], mom[16];
-  std::fill(site, site + 16, -1);
-  std::fill(mom, mom + 16, -1);
-  f.r0 = -1;
-  for (int i = 0; i < nc; ++i) {
-    const double c[4] = {r_vecs[2 * i], r_vecs[2 * i + 1], k_vecs[2 * i] * (2 / M_PI), k_vecs[2 * i + 1] * (2 / M_PI)};
-    int g[4];
-    for (int j = 0; j < 4; ++j) {
-      const long n = std::lround(c[j]);
-      if (!(std::abs(c[j] - n) <= (j < 2 ? 0 : tol)))
-        return ColFft{};
-      g[j] = int(n & 3);
+    return t;
+  // The place of each vector on a grid of four values an axis, the sites' with 0 first: map[i + 4 j].
+  auto grid = [](const double* v, bool zero_first, double (&axis)[2][4], unsigned char* map) {
+    int used = 0, count[2] = {0, 0};
+    if (zero_first) {
+      axis[0][0] = axis[1][0] = 0;
+      count[0] = count[1] = 1;
     }
-    int &s = site[g[0] + 4 * g[1]], &m = mom[g[2] + 4 * g[3]];
-    if (s >= 0 || m >= 0)
-      return ColFft{};
-    s = m = i;
-    if (c[0] == 0 && c[1] == 0)
-      f.r0 = i;
-  }
-  if (f.r0 < 0)
-    return ColFft{};
-  for (int g = 0; g < 16; ++g) {
-    f.rmap[g] = static_cast<unsigned char>(site[g]);
-    f.kmap[g] = static_cast<unsigned char>(mom[g]);
-  }
-  f.on = 1;
-  f.L = 4;
-  return f;
+    for (int i = 0; i < 16; ++i) {
+      int at[2];
+      for (int c = 0; c < 2; ++c) {
+        const double x = v[2 * i + c];
+        int j = 0;
+        while (j < count[c] && axis[c][j] != x)
+          ++j;
+        if (j == 4 || x != x)
+          return false;
+        if (j == count[c])
+          axis[c][count[c]++] = x;
+        at[c] = j;
+      }
+      const int g = at[0] + 4 * at[1];
+      if (used & (1 << g))
+        return false;
+      used |= 1 << g;
+      map[g] = static_cast<unsigned char>(i);
+    }
+    return true;  // sixteen different places: all of them
+  };
+  double r[2][4], k[2][4];
+  if (!grid(r_vecs, true, r, t.rmap) || !grid(k_vecs, false, k, t.kmap))
+    return t;
+  for (int m = 0; m < 4; ++m)
+    for (int a = 0; a < 4; ++a) {
+      t.x[m][a] = mk(std::cos(k[0][m] * r[0][a]), std::sin(k[0][m] * r[0][a]));
+      t.y[m][a] = mk(std::cos(k[1][m] * r[1][a]), std::sin(k[1][m] * r[1][a]));
+    }
+  t.r0 = t.rmap[0];
+  t.on = 1;
+  return t;
 }
 
 void launchTwiddles(const FrontendArgs& a, cudaStream_t stream) {
@@ -650,14 +667,14 @@ size_t frontendSmemRequirement(const TpDims& d, int /*n_max*/, bool fp64) {
   return std::max(row, col);
 }
 
-static bool fft4(const FrontendArgs& a) {
-  return a.dims.nb == 1 && a.fft.on && a.fft.L == 4;
+static bool axes4(const FrontendArgs& a) {
+  return a.dims.nb == 1 && a.axes.on;
 }
 
 // Frequencies per CTA, 16 or 8, which the tuner chooses between: every element is the same sum in the
 // same order either way.  8 alone where 16 does not fit in shared memory.
 static int tileWidth(const FrontendArgs& a, const char* family, LaunchTuner::Pick& pk, cudaStream_t stream) {
-  const bool wide = (fft4(a) ? Tile<16, 4>::bytes(a.dims) : Tile<16, 0>::bytes(a.dims)) <= 227 * 1024;
+  const bool wide = (axes4(a) ? Tile<16, 4>::bytes(a.dims) : Tile<16, 0>::bytes(a.dims)) <= 227 * 1024;
   pk = tunePick(a.tuner, tuneKey(family, a.dims.nb, a.dims.nc, a.dims.nw_ext, a.n_max, a.n_sectors, 8),
                 wide ? 2 : 1, stream);
   return wide && pk.choice == 0 ? 16 : 8;
@@ -676,16 +693,16 @@ static void launchTile(Kernel k, const TpDims& d, int tiles, int freqs, int sect
 template <int WT>
 static void launchRowWT(const FrontendArgs& a, double2* Xp, cudaStream_t stream) {
   const int nb = a.dims.nb, tiles = ceil_div(a.n_max, kTileR), freqs = a.dims.nw_ext / (a.dims.half_g ? 2 : 1);
-  if (fft4(a)) {
+  if (axes4(a)) {
     launchTile<WT, 4>(rowTransformKernel<WT, 4, 1>, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c,
-                      a.row_start, a.Tr, a.Fb, a.G0, a.fft, Xp);
+                      a.row_start, a.Tr, a.Fb, a.G0, a.axes, Xp);
     return;
   }
   auto k = nb == 1   ? rowTransformKernel<WT, 0, 1>
            : nb == 2 ? rowTransformKernel<WT, 0, 2>
            : nb == 3 ? rowTransformKernel<WT, 0, 3> : rowTransformKernel<WT, 0, 0>;
   launchTile<WT, 0>(k, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.perm_r, a.perm_c, a.row_start, a.Tr, a.Fb, a.G0,
-                    a.fft, Xp);
+                    a.axes, Xp);
 }
 
 void launchRowTransform(const FrontendArgs& a, double2* Xp, cudaStream_t stream) {
@@ -703,15 +720,15 @@ template <int WT>
 static void launchColWT(const FrontendArgs& a, const double2* Xp, double2* G, long g_sector_stride, cudaStream_t stream) {
   const int nb = a.dims.nb, freqs = a.dims.nw_ext;
   const int tiles = ceil_div(long(a.dims.R) * freqs / (a.dims.half_g ? 2 : 1), kTileR);
-  if (fft4(a)) {
+  if (axes4(a)) {
     launchTile<WT, 4>(colTransformKernel<WT, 4, 1>, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb,
-                      a.G0, a.fft, Xp, G, g_sector_stride);
+                      a.G0, a.axes, Xp, G, g_sector_stride);
     return;
   }
   auto k = nb == 1   ? colTransformKernel<WT, 0, 1>
            : nb == 2 ? colTransformKernel<WT, 0, 2>
            : nb == 3 ? colTransformKernel<WT, 0, 3> : colTransformKernel<WT, 0, 0>;
-  launchTile<WT, 0>(k, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb, a.G0, a.fft, Xp, G,
+  launchTile<WT, 0>(k, a.dims, tiles, freqs, a.n_sectors, stream, a.sectors, a.col_start, a.Tc, a.Fb, a.G0, a.axes, Xp, G,
                     g_sector_stride);
 }
 

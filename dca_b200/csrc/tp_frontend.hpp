@@ -20,6 +20,16 @@ struct ColFft {
   unsigned char rmap[36], kmap[36];
 };
 
+// The cluster transform of a 4 x 4 grid of sites and momenta axis by axis: e^{i k r} = x[m][a] y[n][b] for the site
+// rmap[a + 4 b] and the momentum kmap[m + 4 n], with the phases of the caller's own sites and momenta; a = b = 0 is
+// r0, the site at the origin, whose phases are 1.
+struct AxisTransform {
+  int on;
+  int r0;
+  unsigned char rmap[16], kmap[16];
+  double2 x[4][4], y[4][4];
+};
+
 struct FrontendArgs {
   TpDims dims;
   const SectorDesc* sectors;  // [n_sectors], device
@@ -35,11 +45,11 @@ struct FrontendArgs {
   const double2* Fb;          // (r, k, b): e^{i k (r + a_b)}, nb * Nc * Nc
   const double2* G0;          // (b1, b2, k, w, s) over the extended mesh
   LaunchTuner* tuner;         // launch-shape tuner (null: the built-in shapes)
-  ColFft fft;                 // FP64 front-end: the cluster transform as an FFT, when fft.on
+  AxisTransform axes;         // FP64 front-end: the cluster transform axis by axis, when axes.on
 };
 
-// The FFT of one band on a 4 x 4 cluster with integer sites and momenta 2 pi (m, n) / 4 (off otherwise).
-ColFft clusterFft4(int nb, int nc, const double* r_vecs, const double* k_vecs);
+// On for one band and 16 sites (momenta) that are every pair of four x and four y coordinates.
+AxisTransform clusterAxes4(int nb, int nc, const double* r_vecs, const double* k_vecs);
 
 void launchTwiddles(const FrontendArgs& a, cudaStream_t stream);
 

@@ -254,7 +254,7 @@ void computeGNoAlloc(const dcaacc_tp_config& c, const double* G0_dev, const dcaa
   fa.Tc = reinterpret_cast<double2*>(base + o_tc);
   fa.Fb = reinterpret_cast<const double2*>(base + o_fb);
   fa.G0 = reinterpret_cast<const double2*>(base + o_g0);
-  fa.fft = clusterFft4(nb, nc, c.r_vecs, c.k_vecs);
+  fa.axes = clusterAxes4(nb, nc, c.r_vecs, c.k_vecs);
   double2* Xp = reinterpret_cast<double2*>(base + o_x);
   if (fa.n_max > 0) {
     launchTwiddles(fa, stream);

@@ -179,6 +179,33 @@ def test_fp64_whole_g_when_not_symmetric():
     assert TpAccumulator(g0, params).mirror_mode() == 0
 
 
+@pytest.mark.parametrize("twist", [(0.0, 0.0), (0.3, -0.7)])
+@pytest.mark.parametrize("order", ["sorted", "shuffled"])
+def test_fp64_phases_of_the_given_momenta(oracle_lib, twist, order):
+    """4x4, FP64: the phases are those of the momenta as given, here 2 pi m / 4 + 8 ulps or a twisted boundary's, not of
+    exact quarters (off by 3e-15 rms in the first case).  Between different frequencies, where G is M's part
+    alone: sums of 10 to 100 rounded terms twice over, in both codes, leave 10 u = 1.1e-15 at most."""
+    from dca_b200.accumulators import TpAccumulator
+    rng = np.random.default_rng(13)
+    cl = CLUSTERS["4x4"]
+    orders = [(120, 45)]
+    params = _params(1, cl, 5, 9, [2], [15], [0], orders)
+    params.k_vecs = cl.k_vecs + np.array(twist)
+    if order == "shuffled":
+        sites = rng.permutation(16)
+        params.r_vecs, params.r_sub = cl.r_vecs[sites], None
+    acc, ora = TpAccumulator(_g0(rng, 1, cl, 9), params), oracle_lib.OracleTp(_g0(rng, 1, cl, 9), params)
+    acc.resetAccumulation(0)
+    for m in _measurements(rng, 1, cl.nc, orders):
+        for a in (acc, ora):
+            a.accumulate([s.M for s in m.sectors], list(m.sectors), m.sign)
+    for spin in range(2):
+        got, want = (np.asarray(a.get_G(spin)).reshape(10, 10, -1) for a in (acc, ora))  # w2, w1
+        off = ~np.eye(10, dtype=bool)
+        print("error:", rel_err(got[off], want[off]))
+        assert rel_err(got[off], want[off]) <= 10 * 2.0 ** -53
+
+
 def test_fp64_graphs():
     """FP64 with and without captured graphs, orders on both sides of the launch shapes' steps of 128."""
     from dca_b200.accumulators import TpAccumulator
