@@ -295,9 +295,15 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     // One band: FP32 on a 4x4 or 6x6 cluster, where the factoring saves 16 or 36 times the flops and the cluster
     // transform is an FFT (a batch of 64, Nw = 64: 0.47 against 0.66 ms; 6x6, Nw = 32, batch of 128: 2.3 against
     // 8.4 ms), and up to 8 sites (8 sites, Nw = 24 + 2, 0.094 against 0.091 ms, and 0.23 against 0.29 for a batch
-    // of 64 with n up to 400), whose G4 is then off by 1.6e-7 of the 64-bit sums instead of 4.3e-7.  With the
-    // matrix transform 16 sites take 0.87 against 0.68 ms: there, and for 36 sites, only where the G4 kernels of
-    // transfer subsets or of the transverse and pairing channels follow, whose sums add to the error.
+    // of 64 with n up to 400), whose G4 is then off by 1.6e-7 of the 64-bit sums instead of 4.3e-7.
+    // With the matrix of phases FP32 is the more precise one, and the slower one as long as the orders are low.  It is
+    // taken where the tensor cores' G4 would be further off than on the kernels that had these calls before, for the
+    // disconnected terms of a transfer subset: 16 sites (8x2, Nw = 32, a batch of 32, magnetic and pairing, three transfers,
+    // n 100..400: 0.45 against 0.42 ms, off by 1.7e-7 against 3.7e-7; without magnetic or charge 0.37 against 0.34 ms,
+    // 3.4e-7 against 6.5e-7), and 36 sites with half of G (9x4, Nw = 16, magnetic, one transfer, n 300..700: 0.56 against
+    // 0.82 ms, 1.7e-7 against 4.6e-7; n 30..100: 0.31 against 0.27).  The whole of G on 36 sites is the dense
+    // product's: pairing, one transfer, 0.26 against 0.48 ms (n 30..100), 0.82 against 0.88 (n 300..700), and 0.93
+    // against 1.87 for Nw = 32, n 100..300.
     // Three bands on 8 sites take 0.37 ms in FP32 and 0.50 on the tensor cores, but beside the FP32-bound pairing
     // update of another batch the tensor cores' are the cheaper ones.  DCAACC_TP_FACTORED_COL selects the
     // tensor-core front-end with one of its column steps: 0 the dense GEMM; 1 one band, 4x4 or
@@ -310,8 +316,9 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     const bool fact_off = fact_env && std::strcmp(fact_env, "0") == 0;
     const bool fact_on = fact_env && std::strcmp(fact_env, "1") == 0;
     const bool fact_tc = fact_env && std::strcmp(fact_env, "2") == 0;
-    const bool ph_all = phChannels(dims_).n_channels == c.n_channels && allTransfers();
-    const bool factored = nb == 1 && (fft.on || nc <= 8 || ((nc == 16 || nc == 36) && !ph_all));
+    const bool ph = phChannels(dims_).n_channels == c.n_channels;
+    const bool factored = nb == 1 && (fft.on || nc <= 8 || (nc == 16 && !(ph && allTransfers())) ||
+                                      (nc == 36 && ph && !allTransfers()));
     front32_ = simt_only_ || (!fact_off && !fact_on && !fact_tc && factored && front32Applies(dims_, max_order_));
     tc_front_ = !front32_;
     if (front32_) {

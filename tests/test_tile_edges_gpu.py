@@ -179,6 +179,23 @@ def test_fp64_whole_g_when_not_symmetric():
     assert TpAccumulator(g0, params).mirror_mode() == 0
 
 
+@pytest.mark.parametrize("cluster,channels,k_ex,fp32,mode", [
+    ("8x2", [2], [15], True, 3), ("8x2", [4], [15], True, 0), ("8x2", [2, 3], list(range(16)), False, 3),
+    ("9x4", [2], [35], True, 1), ("9x4", [4], [35], False, 0), ("9x4", [2, 4], [35, 1, 2], False, 0),
+    ("9x4", [3], list(range(36)), False, 3)])
+def test_front_end_of_clusters_without_fft(oracle_lib, cluster, channels, k_ex, fp32, mode):
+    """16 and 36 sites off the square clusters: which front-end runs (the launch-shape tuner names its kernels),
+    with half of G where it applies (half of D a whole number of 128-row tiles on the tensor cores)."""
+    rng = np.random.default_rng(14)
+    cl = CLUSTERS[cluster]
+    orders = [(40, 21), (97, 5), (0, 3)]
+    nw_half = 32 if len(k_ex) == 36 else 8
+    params = _params(1, cl, nw_half, nw_half + 3, channels, k_ex, [0], orders, precision=1, max_batch=2)
+    acc = _compare(oracle_lib, _g0(rng, 1, cl, nw_half + 3), _measurements(rng, 1, cl.nc, orders), params, MIXED_TOL)
+    assert ("row32" in acc.tuning_report()) == fp32 and ("tc_row_order" in acc.tuning_report()) != fp32
+    assert acc.mirror_mode() == mode
+
+
 @pytest.mark.parametrize("twist", [(0.0, 0.0), (0.3, -0.7)])
 @pytest.mark.parametrize("order", ["sorted", "shuffled"])
 def test_fp64_phases_of_the_given_momenta(oracle_lib, twist, order):
