@@ -181,3 +181,56 @@ def test_reads_of_a_running_half_g4(oracle_lib, kind, shared):
     _check(a.acc, _total(*fed), _tol(kind))
     a.acc.resetAccumulation(1)
     assert not np.any(a.acc.peek_G4(1, 0, size))
+
+
+@pytest.mark.parametrize("kind", [HALF, FULL, MIXED_HALF])
+def test_finalized_g4_outlives_changes(oracle_lib, kind):
+    """get_G4 after finalize gives the finalized sums, read from the device or kept on the host: after a
+    sumTo that clears the device's, after a share, and while other handles add to the shared ones."""
+    import ctypes
+
+    from dca_b200 import _native as N
+
+    def read(acc, c):
+        out = np.empty(a.want()[c].size, np.complex128)
+        assert N.lib.dcaacc_tp_get_g4(acc._h, c, out.view(np.float64).ctypes.data_as(
+            ctypes.POINTER(ctypes.c_double)), out.size) == 0
+        return out
+
+    a, b, c = (_Fed(oracle_lib, **kind).feed(2, seed) for seed in (1, 2, 3))
+    want = a.want()
+    a.acc.finalize()
+    a.acc.peek_G4(0, 0, want[0].size)
+    a.acc.sumTo(b.acc)
+    for channel in range(2):
+        assert rel_err(read(a.acc, channel), want[channel]) <= _tol(kind)
+    total = _total(a, b)
+    _check(b.acc, total, _tol(kind))
+    c.acc.share_G4_with(b.acc)
+    c.feed(2, 4)
+    c.acc.synchronizeCopy()
+    for channel in range(2):
+        assert rel_err(read(b.acc, channel), total[channel]) <= _tol(kind)
+    _check(c.acc, _total(a, b, c), _tol(kind))
+
+
+def test_finalize_reuses_only_unreferenced_arrays(oracle_lib):
+    """A result that the caller still holds, whole or by a view, stays as it was; one that nothing holds is
+    the next result's memory."""
+    a = _Fed(oracle_lib)
+
+    def result(seed):
+        a.acc.resetAccumulation(seed)
+        a.feed(1, seed)
+        a.acc.finalize()
+
+    result(1)
+    kept = a.acc.get_G4()[0]
+    view = a.acc.get_G4()[1][5:9]
+    copies = kept.copy(), view.copy()
+    result(2)
+    assert not np.shares_memory(kept, a.acc.get_G4()[0]) and not np.shares_memory(view, a.acc.get_G4()[1])
+    assert np.array_equal(kept, copies[0]) and np.array_equal(view, copies[1])
+    addresses = [g.ctypes.data for g in a.acc.get_G4()]
+    result(3)
+    assert [g.ctypes.data for g in a.acc.get_G4()] == addresses

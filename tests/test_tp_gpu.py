@@ -649,9 +649,10 @@ def test_factored_column_step_matches_dense(monkeypatch, full_g, fft, mode):
 @pytest.mark.parametrize("full_g", ["0", "1"])
 def test_factored_column_step_6x6_matches_dense(monkeypatch, full_g):
     """One band, 6 x 6 cluster (Nc = 36): the column step factored by orbital on the CUDA cores with
-    the 6 x 6 FFT (DCAACC_TP_FACTORED_COL=1) against the dense tensor-core GEMM (the default) and
-    the FP64 path, with half G (mirror symmetry) and with all of G.  An empty spin sector, and a
-    measurement whose 150 vertices sit on three sites (sites of more than one 32-vertex block)."""
+    the 6 x 6 FFT (DCAACC_TP_FACTORED_COL=1) against the dense tensor-core GEMM (=0), the FP32
+    front-end (the default) and the FP64 path, with half G (mirror symmetry) and with all of G.  An
+    empty spin sector, and a measurement whose 150 vertices sit on three sites (sites of more than one
+    32-vertex block)."""
     import dataclasses
     w = _small("c5", nw_half=32, n_sp=128, n_range=(30, 150))
     case = case_from_workload(w, 6)
@@ -664,12 +665,18 @@ def test_factored_column_step_6x6_matches_dense(monkeypatch, full_g):
     monkeypatch.setenv("DCAACC_TP_FULL_G", full_g)
     monkeypatch.setenv("DCAACC_TP_FACTORED_COL", "1")
     fact = _run_timed(case, False, monkeypatch, max_batch=4)
-    monkeypatch.delenv("DCAACC_TP_FACTORED_COL")
+    monkeypatch.setenv("DCAACC_TP_FACTORED_COL", "0")
     dense = _run_timed(case, False, monkeypatch, max_batch=4)
+    monkeypatch.delenv("DCAACC_TP_FACTORED_COL")
+    fp32 = _run_timed(case, False, monkeypatch, max_batch=4)
     exact = run_gpu(case, precision=0, max_batch=1)
-    assert fact.mirror_mode() == dense.mirror_mode() == (0 if full_g == "1" else 3)
-    for f, d, want in zip(fact.get_G4(), dense.get_G4(), exact.get_G4()):
-        print("6x6 factored / dense column step, relative errors:", rel_err(f, want), rel_err(d, want))
-        assert not np.array_equal(f, d)  # two different column steps ran
+    assert "tc_col_order" in dense.tuning_report() and "col32" not in dense.tuning_report()
+    assert "col32" in fp32.tuning_report() and "tc_col_order" not in fp32.tuning_report()
+    assert "col32" not in fact.tuning_report() and "tc_col_order" not in fact.tuning_report()
+    assert fact.mirror_mode() == dense.mirror_mode() == fp32.mirror_mode() == (0 if full_g == "1" else 3)
+    for f, d, p, want in zip(fact.get_G4(), dense.get_G4(), fp32.get_G4(), exact.get_G4()):
+        print("6x6 factored / dense / FP32 column step, relative errors:", rel_err(f, want), rel_err(d, want), rel_err(p, want))
+        assert not np.array_equal(f, d)  # different column steps ran
         assert rel_err(f, want) <= MIXED_TOL
         assert rel_err(d, want) <= MIXED_TOL
+        assert rel_err(p, want) <= MIXED_TOL
