@@ -560,9 +560,11 @@ def run_ours(args, world, rank, local):
         "row_transform": per_step * float(np.sum(8.0 * nwe * ns * ns + 8.0 * nc * D * D)),
         "col_transform": per_step * float(np.sum(8.0 * nwe * nwe * n_orb * ns + 8.0 * nc * D * D + epi * D * D)),
     }
-    # (plain FP64 path: every measurement reads and writes all of G4 and reads its FP64 G)
-    g4_alg_bytes = (B * (len(w.channels) * n_g4 * 32 + 2 * D * D * 16) if fp64_main
-                    else len(w.channels) * n_g4 * 32 + B * 2 * D * D * 8)
+    # (plain FP64 path: every measurement reads and writes G4, or the half that the handle accumulates, and reads
+    # its FP64 G, or the half that is computed)
+    rows_done = 0.5 if mirror & 1 else 1.0
+    g4_alg_bytes = (B * (len(w.channels) * n_g4 * 32 * (0.5 if mirror & 2 else 1.0) + 2 * D * D * 16 * rows_done)
+                    if fp64_main else len(w.channels) * n_g4 * 32 + B * 2 * D * D * 8)
     g4_sec = stages["update_g4"][0] / args.steps / 1e3  # the stage's time per batch
     g4_paths = {"direct_tc": "discPlanesKernel + frontGemmKernel<2> (disconnected terms) + updateG4DirectMma "
                              "(direct term, G4 flush)",
@@ -574,6 +576,7 @@ def run_ours(args, world, rank, local):
                 "pp3": "updateG4PPMultibandKernel (particle-particle up-down, 27 band entries per thread)",
                 "simt": "updateG4SinglebandBatched",
                 "stream": "updateG4SinglebandStream (one measurement, G4 streamed in memory order)",
+                "gather": "updateG4SinglebandGather (one measurement, a thread per G4 entry)",
                 "fp64_other": "updateG4SinglebandPH / updateG4Kernel (one measurement)"}
     # Column step and G4 kernels as the accumulator selects them (environment switches included).
     half_any = bool(mirror & 1) or bool(mirror & 2)
@@ -589,7 +592,9 @@ def run_ours(args, world, rank, local):
     wide_col = nb == 1 and nc == 36 and not fp64_main and not simt and col_env == "1" and fft_on
     factored_col = factored_col or wide_col
     if fp64_main:
-        g4_path = "stream" if nb == 1 and nc * nc <= 256 and set(w.channels) <= {2, 3} else "fp64_other"
+        ph1 = nb == 1 and set(w.channels) <= {2, 3}
+        g4_path = ("gather" if ph1 and len(w.exchange_momenta(nc)) <= 2 else
+                   "stream" if ph1 and nc in (4, 8, 16) else "fp64_other")
     elif simt:
         g4_path = "simt"
     elif nb == 3 and tuple(w.channels) == (4,) and not half_any and os.environ.get("DCAACC_TP_PP_GENERIC") != "1":
@@ -606,7 +611,8 @@ def run_ours(args, world, rank, local):
                                                "updateG4SinglebandOuterSplit"],
                                    "staged": ["updateG4StagedKernel"],
                                    "pp3": ["updateG4PPMultibandKernel"],
-                                   "stream": ["updateG4SinglebandStream"]}.get(g4_path, []),
+                                   "stream": ["updateG4SinglebandStream"],
+                                   "gather": ["updateG4SinglebandGather"]}.get(g4_path, []),
                      "col_transform": (["colTransform32Kernel"] if front32 else ["colFactorTcKernel"] if col_tc else ["colFactorWideKernel"] if wide_col else
                                        ["colTwiddlePlanesKernel", "colFactorMmaKernel"] if factored_col
                                        else ["frontGemmKernel<1>"]),
@@ -661,7 +667,6 @@ def run_ours(args, world, rank, local):
         chunks = np.ceil(ns / 32)
         Dp = -(-D // 128) * 128
         mma_flop = 2.0 * 128 * 128 * 16
-        rows_done = 0.5 if mirror & 1 else 1.0  # half G: the upper frequency half of the rows
         if dom == "col_transform" and factored_col:
             # The orbital-factored column step (no dense product): its work is the algorithmic one
             # (plus the site-masked zeros of its MMAs), so only the algorithmic rate is reported.
@@ -700,7 +705,6 @@ def run_ours(args, world, rank, local):
     elif dom in ("col_transform", "row_transform") and front32:
         # FP32 front-end factored by orbital: the algorithmic flops against the FP32 pipe, and the row or column
         # step's own bytes (M or X' in, X' or G out, for the rows computed) against HBM.
-        rows_done = 0.5 if mirror & 1 else 1.0
         fp32_peak = 148 * 128 * 2 * 1.965e-3  # TFLOP/s, 148 SMs of 128 lanes at 1,965 MHz
         kern = {"col_transform": "colTransform32Kernel", "row_transform": "rowTransform32Kernel"}[dom]
         roof = {"kernel": kern + " (factored by orbital, packed FP32 multiply-adds, cluster transform, G0 factor)",
@@ -719,10 +723,10 @@ def run_ours(args, world, rank, local):
         cs = 16 if fp64_main else 8
         real = "double" if fp64_main else "float"
         if dom == "col_transform":
-            alg_bytes = 2 * B * (D * mean_n * cs + D * D * cs)
+            alg_bytes = 2 * B * (D * mean_n * cs + D * D * cs) * rows_done
             kern = f"colTransformKernel<{real}>"
         elif dom == "row_transform":
-            alg_bytes = 2 * B * (mean_n * mean_n * 8 + D * mean_n * cs)
+            alg_bytes = 2 * B * (mean_n * mean_n * 8 + D * mean_n * cs * rows_done)
             kern = f"rowTransformKernel<{real}>"
         else:
             alg_bytes = 2 * B * mean_n * nwe * 16
