@@ -435,8 +435,8 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   for (auto& d : dstage_)
     DCAACC_CUDA_CHECK(cudaEventRecord(d.consumed, stream_));
 
-  if ((!mixed_ || simt_only_) && frontendSmemRequirement(dims_, max_order_, !mixed_) > 227 * 1024)
-    invalid("max_order too large for the front-end's shared-memory tiles");
+  if ((!mixed_ || simt_only_) && frontendSmemRequirement(dims_, !mixed_) > 227 * 1024)
+    invalid("bands x sites too large for the front-end's shared-memory tiles");
   G4_host_.assign(c.n_channels, {});
   mirrored_.assign(c.n_channels, kMirroredNone);
 }

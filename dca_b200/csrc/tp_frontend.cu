@@ -653,9 +653,10 @@ void launchTwiddles(const FrontendArgs& a, cudaStream_t stream) {
   }
 }
 
-// The clusters that the front-end takes: per orbital 4 KB (FP64) of a 32 x 8 row tile and the phases in
-// 227 KB of shared memory, and R x R blocks of one column frequency.  (The kernels' own tiles are smaller.)
-size_t frontendSmemRequirement(const TpDims& d, int /*n_max*/, bool fp64) {
+// Which clusters the FP64 and the all-SIMT front-end take, whatever the orders: 4 KB (FP64) an orbital for 32 x 8
+// tiles, the phases, and R x R blocks of a few column frequencies within 227 KB.  The kernels' own tiles (Tile,
+// Tile32) are smaller, so that what passes fits.
+size_t frontendSmemRequirement(const TpDims& d, bool fp64) {
   const size_t real = fp64 ? sizeof(double) : sizeof(float), cplx = 2 * real;
   const size_t R = d.R, orb = d.n_orb, phases = size_t(d.nb) * d.nc * d.nc;
   const size_t row = cplx * (256 * orb + phases + 512) + real * 32 * 65 + sizeof(int) * (orb + 1);

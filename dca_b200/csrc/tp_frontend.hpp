@@ -61,7 +61,8 @@ void launchRowTransform(const FrontendArgs& a, double2* Xp, cudaStream_t stream)
 void launchColTransform(const FrontendArgs& a, const double2* Xp, double2* G, long g_sector_stride,
                         cudaStream_t stream);
 
-size_t frontendSmemRequirement(const TpDims& d, int n_max, bool fp64);
+// Bytes that decide which clusters the FP64 and the all-SIMT front-end take (227 KB at most).
+size_t frontendSmemRequirement(const TpDims& d, bool fp64);
 
 // ---- Tensor-core front-end of the mixed path (tp_frontend_tc.cu) ----
 // Workspace: split-BF16 operand planes for a batch of n_sectors sectors of order <= max_order.

@@ -139,7 +139,7 @@ void computeGNoAlloc(const dcaacc_tp_config& c, const double* G0_dev, const dcaa
   d.beta = c.beta;
   // The FP64 front-end keeps per-CTA tiles of the cluster transform in shared memory; their size
   // grows with nb * Nc (for one band it passes 227 KB above Nc = 43).
-  if (frontendSmemRequirement(d, std::max(n[0], n[1]), true) > 227 * 1024)
+  if (frontendSmemRequirement(d, true) > 227 * 1024)
     throw Error(DCAACC_INVALID_ARG, "nb * Nc too large for the FP64 front-end's shared-memory tiles "
                                     "(more than 227 KB per block)");
   // Each call uploads its sorted vertex tables from stack memory: such copies cannot be recorded

@@ -55,7 +55,9 @@ enum {
   /* FP64 everywhere (the reference's double TP accumulation, mc_options.hpp.in TPAccumulationPrecision). */
   DCAACC_PRECISION_FP64 = 0,
   /* Mixed: the NDFT and cluster transform in FP32 (one band) or on the tensor cores in split FP16 with FP32
-   * accumulation, G in FP32, per-batch G4 partial sums in FP32, running G4 in FP64. */
+   * accumulation, G in FP32, per-batch G4 partial sums in FP32, running G4 in FP64.  One band: the disconnected
+   * terms, and with all transfers the direct term on 16 sites and on 6x6 clusters (batches of 32 and more), multiply
+   * G split into two FP16 parts (22 significant bits) on the tensor cores. */
   DCAACC_PRECISION_MIXED = 1
 };
 
