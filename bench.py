@@ -257,15 +257,6 @@ CPU_WARMUP = 1  # untimed measurements per process (first-touch of the process's
 CPU_TIMED = 5   # timed measurements per process
 
 
-def reference_binary():
-    """The reference's own CPU accumulators as oracle/refbuild compiles them from its checkout, or None."""
-    from oracle import pyoracle
-    for name in (os.path.join(os.path.dirname(pyoracle.REF_BIN), "tp_ref_openblas"), pyoracle.REF_BIN):
-        if os.path.exists(name):
-            return name
-    return None
-
-
 def run_cpu_reference(w, timed, warmup, workers=None):
     """The reference's own TpAccumulator<CPU> (oracle/_ref/tp_ref_openblas, else tp_ref with its
     naive zgemm_, else the restatement oracle) in P single-threaded processes, one per core, each
@@ -274,13 +265,15 @@ def run_cpu_reference(w, timed, warmup, workers=None):
     one's end (every process's timed loop lies inside it).  Returns a dict."""
     from dca_b200 import workloads as W
     from oracle import casefile as CF
+    from oracle import pyoracle
     cl = w.cluster()
     g0 = W.make_g0(w.model, cl, w.beta, w.chemical_potential(), w.n_sp)
     g4_bytes = 16 * (w.nb ** 4) * cl.nc ** 2 * (2 * w.nw_half) ** 2 * len(w.exchange_momenta(cl.nc)) * len(
         w.exchange_frequencies()) * len(w.channels)
     P = workers or _cpu_workers(g4_bytes * 1.5 + 256e6)
-    binary = reference_binary()
-    kind = "reference" if binary else "port"
+    ref_blas = os.path.join(os.path.dirname(pyoracle.REF_BIN), "tp_ref_openblas")
+    binary = ref_blas if os.path.exists(ref_blas) else pyoracle.REF_BIN
+    kind = "reference" if os.path.exists(binary) else "port"
     n_per = warmup + timed
     with tempfile.TemporaryDirectory() as d:
         # Every worker's input is written first, then all workers start together, so that their
@@ -808,9 +801,6 @@ def run_reference_arm(args, world, rank):
     w = workload(args)
     if rank != 0:
         return None
-    if reference_binary() is None:  # the restatement oracle is this repository's code, not the reference
-        return {"impl": "reference",
-                "unavailable": "the reference's CPU accumulators are not built here (no checkout for oracle/refbuild)"}
     timed = max(1, min(args.steps, 20))
     warm = min(args.warmup, 5)
     cb = run_cpu_reference(w, timed, warm)
