@@ -810,6 +810,9 @@ def run_reference_arm(args, world, rank):
             "ms_per_step": 1e3 * cb["window_s"] / timed,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "fp64",
             "data": "synthetic (seeded; dca_b200.workloads)",
+            "code": ("the reference's own CPU accumulator" if cb["kind"] == "reference" else
+                     "this repository's restatement of the reference's CPU accumulator (kind port): the reference is "
+                     "not built here, and a ratio to this line compares with no code of the reference"),
             "config": bench_config(w, world),
             "parallelism": f"{cb['cores']} CPU processes, one per core, one measurement at a time each",
             "cpu_baseline": cb,
