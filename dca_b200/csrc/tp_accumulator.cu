@@ -120,6 +120,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
   DCAACC_CUDA_CHECK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
   own_stream_ = true;
   DCAACC_CUDA_CHECK(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking));
+  DCAACC_CUDA_CHECK(cudaStreamCreateWithFlags(&capture_stream_, cudaStreamNonBlocking));
   for (auto& h : hstage_)
     DCAACC_CUDA_CHECK(cudaEventCreateWithFlags(&h.uploaded, cudaEventDisableTiming));
   for (auto& d : dstage_)
@@ -538,6 +539,9 @@ void TpAccumulator::releaseStreamsAndEvents() {
   if (copy_stream_)
     cudaStreamDestroy(copy_stream_);
   copy_stream_ = nullptr;
+  if (capture_stream_)
+    cudaStreamDestroy(capture_stream_);
+  capture_stream_ = nullptr;
   if (own_stream_ && stream_)
     cudaStreamDestroy(stream_);
   stream_ = nullptr;
@@ -887,7 +891,7 @@ void TpAccumulator::process() {
   if (graphable)
     launches_ += launchBatchGraph(set, fa, ga, ds);
   else
-    launches_ += launchBatch(fa, ga, ds);
+    launches_ += launchBatch(fa, ga, ds, stream_);
   DCAACC_CUDA_CHECK(cudaEventRecord(ds.consumed, stream_));
   mirrored_.assign(dims_.n_channels, kMirroredNone);
   have_g_ = !mixed_;
@@ -898,8 +902,8 @@ void TpAccumulator::process() {
   n_max_batch_ = 0;
 }
 
-// The kernels of one batch, all on stream_ and nothing else (the sequence a graph captures).
-int TpAccumulator::launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStage& ds) {
+// The kernels of one batch, all on `stream` and nothing else (the sequence a graph captures).
+int TpAccumulator::launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStage& ds, cudaStream_t stream) {
   int launched = 0;
   cudaEvent_t b = nullptr;
   if (fa.n_max > 0) {
@@ -907,23 +911,23 @@ int TpAccumulator::launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStag
     // Vertex order and orbital runs of every sector (sortConfiguration), row side and, for
     // non-density-density models, column side.
     launchSortVertices(fa.sectors, fa.n_sectors, ds.in.vb_r, ds.in.vs_r, dims_.nb, dims_.n_orb,
-                       ds.perm_r.get(), ds.rstart.get(), ds.orb_r.get(), stream_);
+                       ds.perm_r.get(), ds.rstart.get(), ds.orb_r.get(), stream);
     launched += 1;
     if (non_density_) {
       launchSortVertices(fa.sectors, fa.n_sectors, ds.in.vb_c, ds.in.vs_c, dims_.nb, dims_.n_orb,
-                         ds.perm_c.get(), ds.cstart.get(), ds.orb_c.get(), stream_);
+                         ds.perm_c.get(), ds.cstart.get(), ds.orb_c.get(), stream);
       launched += 1;
     }
     int n_prep;
     if (front32_) {
-      n_prep = launchFront32Prep(fa, f32_, stream_);
+      n_prep = launchFront32Prep(fa, f32_, stream);
     }
     else if (tc_front_) {
       n_prep = launchFrontendTcPrep(fa, ftc_, ds.orb_r.get(), non_density_ ? ds.orb_c.get() : ds.orb_r.get(),
-                                    stream_);
+                                    stream);
     }
     else {
-      launchTwiddles(fa, stream_);
+      launchTwiddles(fa, stream);
       n_prep = non_density_ ? 2 : 1;
     }
     launched += n_prep;
@@ -931,24 +935,24 @@ int TpAccumulator::launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStag
   }
   timeBegin(DCAACC_STAGE_ROW, &b);
   if (tc_front_)
-    launchFrontendTcRow(fa, ftc_, err_d_.get(), stream_);
+    launchFrontendTcRow(fa, ftc_, err_d_.get(), stream);
   else if (front32_)
-    launchFront32Row(fa, f32_, stream_);
+    launchFront32Row(fa, f32_, stream);
   else
-    launchRowTransform(fa, X64_.get(), stream_);
+    launchRowTransform(fa, X64_.get(), stream);
   timeEnd(DCAACC_STAGE_ROW, b, 1);
   timeBegin(DCAACC_STAGE_COL, &b);
   int col_launches = 1;
   if (tc_front_)
-    col_launches = launchFrontendTcCol(fa, ftc_, G32_.get(), g_sector_stride_, gmax_d_.get(), err_d_.get(), stream_);
+    col_launches = launchFrontendTcCol(fa, ftc_, G32_.get(), g_sector_stride_, gmax_d_.get(), err_d_.get(), stream);
   else if (front32_)
-    launchFront32Col(fa, f32_, G32_.get(), g_sector_stride_, gmax_d_.get(), stream_);
+    launchFront32Col(fa, f32_, G32_.get(), g_sector_stride_, gmax_d_.get(), stream);
   else
-    launchColTransform(fa, X64_.get(), G64_.get(), g_sector_stride_, stream_);
+    launchColTransform(fa, X64_.get(), G64_.get(), g_sector_stride_, stream);
   timeEnd(DCAACC_STAGE_COL, b, col_launches);
   timeBegin(DCAACC_STAGE_G4, &b);
-  const int g4_launches = mixed_ ? launchUpdateG4<float2>(ga, G32_.get(), g_sector_stride_, stream_)
-                                 : launchUpdateG4<double2>(ga, G64_.get(), g_sector_stride_, stream_);
+  const int g4_launches = mixed_ ? launchUpdateG4<float2>(ga, G32_.get(), g_sector_stride_, stream)
+                                 : launchUpdateG4<double2>(ga, G64_.get(), g_sector_stride_, stream);
   timeEnd(DCAACC_STAGE_G4, b, g4_launches);
   return launched + 1 + col_launches + g4_launches;
 }
@@ -981,24 +985,26 @@ int TpAccumulator::launchBatchGraph(int set, const FrontendArgs& fa, const G4Arg
   g->last = ++graph_stamp_;
   if (!g->clean) {
     const uint64_t p0 = tuner_.probes();
-    const int n = launchBatch(fa, ga, ds);
+    const int n = launchBatch(fa, ga, ds, stream_);
     g->clean = tuner_.probes() == p0;
     return n;
   }
   if (!g->exec) {
-    DCAACC_CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeRelaxed));
+    // Captured on a stream of the handle's own: the caller's (setStream) may take other work meanwhile, from another
+    // thread or handle, which the graph would swallow.
+    DCAACC_CUDA_CHECK(cudaStreamBeginCapture(capture_stream_, cudaStreamCaptureModeRelaxed));
     int n = 0;
     cudaGraph_t graph = nullptr;
     try {
-      n = launchBatch(fa, ga, ds);
+      n = launchBatch(fa, ga, ds, capture_stream_);
     }
     catch (...) {
-      if (cudaStreamEndCapture(stream_, &graph) == cudaSuccess && graph)
+      if (cudaStreamEndCapture(capture_stream_, &graph) == cudaSuccess && graph)
         cudaGraphDestroy(graph);
       cudaGetLastError();
       throw;
     }
-    DCAACC_CUDA_CHECK(cudaStreamEndCapture(stream_, &graph));
+    DCAACC_CUDA_CHECK(cudaStreamEndCapture(capture_stream_, &graph));
     const cudaError_t e = cudaGraphInstantiate(&g->exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {

@@ -217,8 +217,8 @@ private:
     cudaEvent_t consumed = nullptr;  // the kernels that read this set have completed
   };
   DevStage dstage_[2];
-  cudaStream_t copy_stream_ = nullptr;
-  int launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStage& ds);
+  cudaStream_t copy_stream_ = nullptr, capture_stream_ = nullptr;
+  int launchBatch(const FrontendArgs& fa, const G4Args& ga, DevStage& ds, cudaStream_t stream);
   int launchBatchGraph(int set, const FrontendArgs& fa, const G4Args& ga, DevStage& ds);
   // CUDA graphs of the batch sequence (launchBatchGraph).
   struct BatchGraph {

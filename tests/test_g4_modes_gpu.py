@@ -234,3 +234,46 @@ def test_finalize_reuses_only_unreferenced_arrays(oracle_lib):
     addresses = [g.ctypes.data for g in a.acc.get_G4()]
     result(3)
     assert [g.ctypes.data for g in a.acc.get_G4()] == addresses
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_graphs_on_a_shared_stream(precision):
+    """A handle on the caller's stream captures its batches while another thread launches on the same stream: the
+    other's kernels run once each, and the handle's graphs hold its own alone."""
+    import threading
+
+    import torch
+
+    from dca_b200.accumulators import TpAccumulator
+    want = TpAccumulator(_g0(), _params(precision))
+    want.set_graphs(False)
+    got = TpAccumulator(_g0(), _params(precision))
+    stream = torch.cuda.Stream()
+    got.set_stream(stream.cuda_stream)
+    count, stop, calls = torch.zeros(1, dtype=torch.float64, device="cuda"), threading.Event(), [0]
+    torch.cuda.synchronize()
+
+    def other():
+        with torch.cuda.stream(stream):
+            while not stop.is_set():
+                count.add_(1.)
+                calls[0] += 1
+
+    thread = threading.Thread(target=other)
+    thread.start()
+    try:
+        for acc in (got, want):
+            acc.resetAccumulation(0)
+            _feed(acc, _measurements(60, 30))
+            acc.synchronizeCopy()
+    finally:
+        stop.set()
+        thread.join()
+    torch.cuda.synchronize()
+    assert got.graph_stats()[0] > 0 and got.graph_stats()[1] > 0
+    assert count.item() == calls[0]
+    for acc in (got, want):
+        acc.finalize()
+    for a, b in zip(got.get_G4(), want.get_G4()):
+        assert rel_err(a, b) <= (1e-14 if precision == 0 else 1e-7)
+    del got  # before its stream
