@@ -40,6 +40,7 @@ namespace {
 constexpr int kPPThreads = 512;
 constexpr int kPPStages = 3;  // ring of block sets: copies run two steps ahead
 constexpr int kPPMeas = 2;    // measurements per stage
+constexpr int kPPPending = 6;  // ints of the pending pass
 constexpr int kPPPitch = kPPThreads + 1;  // row of the batch sums in shared memory (distinct banks along the entries)
 
 template <int NB, int NC>
@@ -106,9 +107,10 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
   float2* fb = stage + kPPStages * kPPMeas * 4 * blk;
   const int n_runs = nq * nc;
   long* run_off = reinterpret_cast<long*>(fb + NB3 * kPPPitch + (NB3 * kPPPitch) % 2);  // [n_runs]
-  int* sgn = reinterpret_cast<int*>(run_off + n_runs);  // [n_slots] the measurements' signs
+  int* pend_mem = reinterpret_cast<int*>(run_off + n_runs);                // [kPPPending]
+  signed char* sgn = reinterpret_cast<signed char*>(pend_mem + kPPPending);  // [n_slots] the measurements' signs
   for (int i = t; i < n_slots; i += kPPThreads)
-    sgn[i] = signs[i];
+    sgn[i] = static_cast<signed char>(signs[i]);
   for (int r = t; r < n_runs; r += kPPThreads)
     run_off[r] = r / nq * s_k2 + r % nq * s_q;
   __syncthreads();  // the signs are in place before any warp's first step
@@ -128,7 +130,8 @@ updateG4PPMultibandKernel(const TpDims dims, const float2* __restrict__ G, long 
     p.dj = kPPThreads - p.dr * p.run;
     return p;
   };
-  volatile Pending* pend = reinterpret_cast<volatile Pending*>(sgn + n_slots);  // in shared memory: registers are short
+  static_assert(sizeof(Pending) == kPPPending * sizeof(int), "its place in shared memory");
+  volatile Pending* pend = reinterpret_cast<volatile Pending*>(pend_mem);  // in shared memory: registers are short
   int fr = n_runs, fj = 0;  // this thread's next entry
   auto flushEntry = [&](double2* dst, float2 v, double2 old) {
     if (atomic) {
@@ -303,7 +306,7 @@ bool launchUpdateG4PPMultiband(const G4Args& a, const float2* G, long g_sector_s
     return false;
   const size_t smem = 64 + kPPStages * kPPMeas * 4 * size_t(d.R) * d.R * sizeof(float2) +
                       (27 * size_t(kPPPitch) + 1) * sizeof(float2) + sizeof(long) * size_t(d.nq) * d.nc +
-                      sizeof(int) * (size_t(a.n_slots) + 6);
+                      sizeof(int) * kPPPending + size_t(a.n_slots);
   if (smem > 227 * 1024)
     return false;
   auto k = d.nc == 4 ? updateG4PPMultibandKernel<3, 4> : updateG4PPMultibandKernel<3, 8>;
