@@ -7,6 +7,7 @@
 #include <cstring>
 #include <string>
 #include <type_traits>
+#include <utility>
 
 #include "tp_frontend.hpp"
 #include "tp_g4.hpp"
@@ -769,6 +770,7 @@ void TpAccumulator::stage(const dcaacc_sector* sec, int sign, bool m_f32) {
         if (mcopy_bytes_ && reinterpret_cast<const char*>(mcopy_src_) + mcopy_bytes_ == reinterpret_cast<const char*>(x.M) &&
             reinterpret_cast<char*>(mcopy_dst_) + mcopy_bytes_ == reinterpret_cast<char*>(dst)) {
           mcopy_bytes_ += bytes;  // contiguous on both sides: one larger copy
+          mcopy_parts_.push_back(bytes);
           if (mcopy_bytes_ >= (size_t(8) << 20))
             flushMCopy();  // in pieces of about 8 MB, overlapping the staging of the rest
         }
@@ -777,6 +779,7 @@ void TpAccumulator::stage(const dcaacc_sector* sec, int sign, bool m_f32) {
           mcopy_src_ = x.M;
           mcopy_dst_ = dst;
           mcopy_bytes_ = bytes;
+          mcopy_parts_.assign(1, bytes);
         }
       }
       else {
@@ -807,9 +810,23 @@ void TpAccumulator::stage(const dcaacc_sector* sec, int sign, bool m_f32) {
 }
 
 void TpAccumulator::flushMCopy() {
-  if (mcopy_bytes_)
-    DCAACC_CUDA_CHECK(cudaMemcpyAsync(mcopy_dst_, mcopy_src_, mcopy_bytes_, cudaMemcpyHostToDevice, copy_stream_));
-  mcopy_bytes_ = 0;
+  const size_t bytes = std::exchange(mcopy_bytes_, 0);
+  if (!bytes)
+    return;
+  const cudaError_t e = cudaMemcpyAsync(mcopy_dst_, mcopy_src_, bytes, cudaMemcpyHostToDevice, copy_stream_);
+  if (e != cudaErrorInvalidValue || mcopy_parts_.size() == 1) {
+    DCAACC_CUDA_CHECK(e);
+    return;
+  }
+  // Matrices side by side in separately pinned memory: CUDA refuses a copy across both, so each by itself.
+  cudaGetLastError();
+  const char* src = reinterpret_cast<const char*>(mcopy_src_);
+  char* dst = reinterpret_cast<char*>(mcopy_dst_);
+  for (size_t part : mcopy_parts_) {
+    DCAACC_CUDA_CHECK(cudaMemcpyAsync(dst, src, part, cudaMemcpyHostToDevice, copy_stream_));
+    src += part;
+    dst += part;
+  }
 }
 
 void TpAccumulator::process() {

@@ -283,6 +283,7 @@ private:
   const double* mcopy_src_ = nullptr;
   double* mcopy_dst_ = nullptr;
   size_t mcopy_bytes_ = 0;
+  std::vector<size_t> mcopy_parts_;  // the sectors' bytes in it
   void flushMCopy();
   int n_max_batch_ = 0;   // largest order staged
   double sign_sum_ = 0;   // signs of the measurements accumulated since reset (sumTo moves them)

@@ -440,6 +440,42 @@ def test_device_resident_m_matches_host_m():
         assert rel_err(got, want) <= 1e-14
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+def test_host_m_side_by_side_in_separate_pinned_memory(precision):
+    """The matrices of a measurement next to one another in host memory that was pinned in two pieces: the upload
+    that joins neighbouring matrices may not span both."""
+    import mmap
+
+    import torch
+    from dca_b200.accumulators import TpAccumulator
+    w = _small("c1", n_range=(64, 64))  # 32 KB a matrix: whole pages
+    case = case_from_workload(w, 3)
+    want = run_gpu(case, precision=precision, max_batch=2)
+    size = 8 * 64 * 64
+    memory = mmap.mmap(-1, 2 * size)
+    both = np.frombuffer(memory, np.float64)
+    Ms = [both[64 * 64 * i:64 * 64 * (i + 1)].reshape(64, 64, order="F") for i in range(2)]
+    rt = torch.cuda.cudart()
+    torch.cuda.init()
+    for M in Ms:
+        assert int(rt.cudaHostRegister(M.ctypes.data, size, 0)) == 0
+    acc = TpAccumulator(case.G0, case.tp_params(precision=precision, max_batch=2))
+    acc.resetAccumulation(0)
+    try:
+        for m in case.measurements:
+            for M, s in zip(Ms, m.sectors):
+                M[...] = s.M
+            acc.accumulate(Ms, list(m.sectors), m.sign)
+            acc.synchronizeCopy()
+        acc.finalize()
+    finally:
+        torch.cuda.synchronize()
+        for M in Ms:
+            rt.cudaHostUnregister(M.ctypes.data)
+    for got, ref in zip(acc.get_G4(), want.get_G4()):
+        assert np.array_equal(got, ref)
+
+
 def test_lifecycle_and_errors():
     from dca_b200.accumulators import LogicError, TpAccumulator
     case, _ = golden("c1_mag")
