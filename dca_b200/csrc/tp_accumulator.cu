@@ -297,7 +297,9 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     // One band: FP32 on a 4x4 or 6x6 cluster, where the factoring saves 16 or 36 times the flops and the cluster
     // transform is an FFT (a batch of 64, Nw = 64: 0.47 against 0.66 ms; 6x6, Nw = 32, batch of 128: 2.3 against
     // 8.4 ms), and up to 8 sites (8 sites, Nw = 24 + 2, 0.094 against 0.091 ms, and 0.23 against 0.29 for a batch
-    // of 64 with n up to 400), whose G4 is then off by 1.6e-7 of the 64-bit sums instead of 4.3e-7.
+    // of 64 with n up to 400), whose G4 is then off by 1.6e-7 of the 64-bit sums instead of 4.3e-7.  Up to four sites, with as
+    // few orbitals' sums for a CTA's warps, only up to 512 vertices: 2x2, Nw = 24, a batch of 64, whole calls 0.354 against
+    // 0.349 ms (n 20..60), 0.756 against 0.717 (200..450), 1.75 against 1.53 (600..1000).
     // With the matrix of phases FP32 is the more precise one, and the slower one as long as the orders are low.  It is
     // taken where the tensor cores' G4 would be further off than on the kernels that had these calls before, for the
     // disconnected terms of a transfer subset: 16 sites (8x2, Nw = 32, a batch of 32, magnetic and pairing, three transfers,
@@ -319,7 +321,7 @@ void TpAccumulator::init(const dcaacc_tp_config& c, const double* G0) {
     const bool fact_on = fact_env && std::strcmp(fact_env, "1") == 0;
     const bool fact_tc = fact_env && std::strcmp(fact_env, "2") == 0;
     const bool ph = phChannels(dims_).n_channels == c.n_channels;
-    const bool factored = nb == 1 && (fft.on || nc <= 8 || (nc == 16 && !(ph && allTransfers())) ||
+    const bool factored = nb == 1 && (fft.on || (nc <= 8 && (nc > 4 || max_order_ <= 512)) || (nc == 16 && !(ph && allTransfers())) ||
                                       (nc == 36 && ph && !allTransfers()));
     front32_ = simt_only_ || (!fact_off && !fact_on && !fact_tc && factored && front32Applies(dims_, max_order_));
     tc_front_ = !front32_;

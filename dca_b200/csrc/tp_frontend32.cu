@@ -155,6 +155,11 @@ template <int WT, int L>
 struct Tile32 {
   static constexpr int kWarps = L == 6 && WT == 16 ? 16 : 8;  // 36 orbitals' sums leave room for one CTA per SM
   static constexpr int kThreads = 32 * kWarps;
+  // CTAs an SM: the matrix forms' steps are chains of short loops.  2x2, Nw = 24, a batch of 64, n 20..60, 100..200 and
+  // 200..450: row step 17, 47 and 129 us with two, 13, 36 and 98 with four; column step 29, 43 and 65 with two, 23, 35 and
+  // 53 with three (60 with four: spills).
+  static constexpr int kRowResident = L == 6 && WT == 16 ? 1 : L == 0 && WT == 8 ? 4 : 2;
+  static constexpr int kColResident = L == 6 && WT == 16 ? 1 : L == 0 && WT == 8 ? 3 : 2;
   static constexpr int kSub = WT / 4;           // frequencies of a lane
   static constexpr int kSums = kLong * WT + 1;  // stride of an orbital's sums
   static constexpr int kSlotBytes = 512 + 32 * WT;
@@ -443,7 +448,7 @@ __device__ inline double2 originPhase(const double2* __restrict__ Fb, int k, int
 // Row step.  grid (ceil(n_max / 32), ceil(frequencies / WT), n_sectors); X'(row - row0, j) at
 // x_off + j rows + row - row0.  L: cluster FFT (4, 6) or 0; NB: bands (1, 2, 3), 0 for any number.
 template <int WT, int L, int NB>
-__global__ void __launch_bounds__(Tile32<WT, L>::kThreads, L == 6 && WT == 16 ? 1 : 2)
+__global__ void __launch_bounds__(Tile32<WT, L>::kThreads, Tile32<WT, L>::kRowResident)
 rowTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, const int* __restrict__ row_start,
                      const float2* __restrict__ T2, const float* __restrict__ Ms, int Kr,
                      const double2* __restrict__ Fb, const double2* __restrict__ G0,
@@ -557,18 +562,25 @@ rowTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, 
           out[j * rows + static_cast<long>(w - w_lo) * R + b1 + nb * k] = v;
       };
       if constexpr (NB == 1) {
-        float2 s[4][2];
-        tile.template clusterSum<false, 2>(s, dims, 1, 0, wl, l0, k0);
+        auto momenta = [&](auto kc) {
+          constexpr int KC = decltype(kc)::value;
+          float2 s[4][KC];
+          tile.template clusterSum<false, KC>(s, dims, 1, 0, wl, l0, k0);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int k = k0 + lane % 8 + 8 * c;
-          if (k >= nc)
-            continue;
-          const float2 g = g0n(k);
+          for (int c = 0; c < KC; ++c) {
+            const int k = k0 + lane % 8 + 8 * c;
+            if (k >= nc)
+              continue;
+            const float2 g = g0n(k);
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            put(i, 0, k, cmul(g, s[i][c]));
-        }
+            for (int i = 0; i < 4; ++i)
+              put(i, 0, k, cmul(g, s[i][c]));
+          }
+        };
+        if (nc <= 8)  // half of sixteen momenta would be padding
+          momenta(std::integral_constant<int, 1>{});
+        else
+          momenta(std::integral_constant<int, 2>{});
       }
       else if constexpr (NB > 1) {
         float2 s[NB][4][1];
@@ -625,7 +637,7 @@ __device__ inline float2 addDelta(float2 v, double beta, double2 g) {
 // Column step.  grid (ceil(rows / 32), ceil(NwExt / WT), n_sectors), rows = D - row0.  gmax (or null):
 // [2 slot + spin] raised to the sector's largest |Re|, |Im| of G (float bits).
 template <int WT, int L, int NB>
-__global__ void __launch_bounds__(Tile32<WT, L>::kThreads, L == 6 && WT == 16 ? 1 : 2)
+__global__ void __launch_bounds__(Tile32<WT, L>::kThreads, Tile32<WT, L>::kColResident)
 colTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, const int* __restrict__ col_start,
                      const float4* __restrict__ T4, const double2* __restrict__ Fb, const double2* __restrict__ G0,
                      const __grid_constant__ ColFft fft, int row0, const float2* __restrict__ Xp, float2* __restrict__ G,
@@ -760,18 +772,25 @@ colTransform32Kernel(const TpDims dims, const SectorDesc* __restrict__ sectors, 
         out[((static_cast<long>(w1) * nw_ext + w2) * R + r) * R + b2 + nb * k2] = v;
       };
       if constexpr (NB == 1) {
-        float2 s[4][2];
-        tile.template clusterSum<true, 2>(s, dims, 1, 0, wl, l0, k0);
+        auto momenta = [&](auto kc) {
+          constexpr int KC = decltype(kc)::value;
+          float2 s[4][KC];
+          tile.template clusterSum<true, KC>(s, dims, 1, 0, wl, l0, k0);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int k = k0 + lane % 8 + 8 * c;
-          if (k >= nc)
-            continue;
-          const float2 g = to_f2(g0[k]);
+          for (int c = 0; c < KC; ++c) {
+            const int k = k0 + lane % 8 + 8 * c;
+            if (k >= nc)
+              continue;
+            const float2 g = to_f2(g0[k]);
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            put(i, 0, k, cmul(s[i][c], g));
-        }
+            for (int i = 0; i < 4; ++i)
+              put(i, 0, k, cmul(s[i][c], g));
+          }
+        };
+        if (nc <= 8)  // half of sixteen momenta would be padding
+          momenta(std::integral_constant<int, 1>{});
+        else
+          momenta(std::integral_constant<int, 2>{});
       }
       else if constexpr (NB > 1) {
         float2 s[NB][4][1];

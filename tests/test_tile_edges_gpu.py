@@ -191,6 +191,18 @@ def test_fp64_whole_g_when_not_symmetric():
     assert TpAccumulator(g0, params).mirror_mode() == 0
 
 
+@pytest.mark.parametrize("cluster,max_order,fp32", [("2x2", 512, True), ("2x2", 513, False), ("2x1", 600, False),
+                                                    ("3x2", 600, True)])
+def test_front_end_of_small_clusters(oracle_lib, cluster, max_order, fp32):
+    """Up to four sites: the FP32 front-end up to 512 vertices, orders up to the handle's limit."""
+    rng = np.random.default_rng(17)
+    cl = CLUSTERS[cluster]
+    orders = [(max_order, 3), (0, max_order - 1), (127, 257)]
+    params = _params(1, cl, 5, 9, [2, 4], [0], [0, 1], orders, precision=1, max_batch=3)
+    acc = _compare(oracle_lib, _g0(rng, 1, cl, 9), _measurements(rng, 1, cl.nc, orders), params, MIXED_TOL)
+    assert ("row32" in acc.tuning_report()) == fp32 and ("tc_row_order" in acc.tuning_report()) != fp32
+
+
 @pytest.mark.parametrize("cluster,channels,k_ex,fp32,mode", [
     ("8x2", [2], [15], True, 3), ("8x2", [4], [15], True, 0), ("8x2", [2, 3], list(range(16)), False, 3),
     ("9x4", [2], [35], True, 1), ("9x4", [4], [35], False, 0), ("9x4", [2, 4], [35, 1, 2], False, 0),
